@@ -30,7 +30,7 @@
 extern "C" {
 #endif
 
-#define IMN_ABI_VERSION 4
+#define IMN_ABI_VERSION 5
 
 typedef enum ImnStatus {
   IMN_OK = 0,
@@ -74,14 +74,18 @@ typedef struct ImnModel {
   const int32_t* M_mulm_rowadr;
   const int32_t* M_mulm_col;
   const int32_t* M_mulm_madr;
-  /* the same table, one word per entry: col | madr << 16 (2 nM - nv entries);
-   * built once per model by the host layer                                    */
-  const uint32_t* M_mulm_pack;
+  /* the same rows dealt to 32 lanes for the fused kernel, built once per model by the
+   * host layer: [n_mulm_batches][32][4] words col | madr << 16, four entries of one
+   * row per (batch, lane).  A row starts with a batch of its own; in the batch that
+   * ends it bits 8-10 of word 0 hold the entries used (1 to 4) and bits 8-14 of word 1
+   * the dof; bits 8-10 of word 0 are 0 in every other batch.                   */
+  const uint32_t* M_mulm_lanes;
   /* constants that live in the upstream solver module                         */
   float alpha_noise_eps;          /* solver._ALPHA_NOISE_EPS                    */
   int32_t overflow_iterations;    /* types.OverflowType.ITERATIONS bit          */
   int32_t overflow_ls_iterations; /* types.OverflowType.LS_ITERATIONS bit       */
   int32_t warn_overflow;          /* opt.warn_overflow mask (device printf)     */
+  int32_t n_mulm_batches;         /* batches of M_mulm_lanes                    */
 } ImnModel;
 
 /* Data-side buffers of one batch of worlds: the fields of mujoco_warp `Data`

@@ -15,7 +15,7 @@ I32 = C.c_int32
 I64 = C.c_int64
 F32 = C.c_float
 
-IMN_ABI_VERSION = 4
+IMN_ABI_VERSION = 5
 
 IMN_OK = 0
 IMN_ERR_NULL = -1
@@ -45,11 +45,12 @@ class ImnModel(C.Structure):
         ("M_mulm_rowadr", P),
         ("M_mulm_col", P),
         ("M_mulm_madr", P),
-        ("M_mulm_pack", P),
+        ("M_mulm_lanes", P),
         ("alpha_noise_eps", F32),
         ("overflow_iterations", I32),
         ("overflow_ls_iterations", I32),
         ("warn_overflow", I32),
+        ("n_mulm_batches", I32),
     ]
 
 

@@ -78,32 +78,32 @@ def _upstream_constants() -> tuple[float, int, int]:
     return c["alpha_noise_eps"], c["overflow_iterations"], c["overflow_ls_iterations"]
 
 
-def _mulm_pack(m: Any):
-    """The packed M_mulm table of a model; built once (and cached on the model) for
+def _mulm_lanes(m: Any):
+    """The lane program of a model's M_mulm rows; built once (and cached on the model) for
     Model objects that come from mujoco-warp and do not carry it."""
-    pack = getattr(m, "M_mulm_pack", None)
-    if pack is None:
-        pack = getattr(m, "_imn_mulm_pack", None)
-    if pack is None:
+    lanes = getattr(m, "M_mulm_lanes", None)
+    if lanes is None:
+        lanes = getattr(m, "_imn_mulm_lanes", None)
+    if lanes is None:
         import numpy as np
 
         from .arrays import device_of, to_host
-        from .mjw_model import pack_mulm
+        from .mjw_model import mulm_lane_program
 
         col, madr = m.M_mulm_col, m.M_mulm_madr
-        host = pack_mulm(to_host(col), to_host(madr))
+        host = mulm_lane_program(to_host(m.M_mulm_rowadr), to_host(col), to_host(madr), int(m.nv))
         if isinstance(col, np.ndarray):
-            pack = host
+            lanes = host
         else:
             import torch
 
             # on the device that holds the model's tables, not torch's current one
-            pack = torch.from_numpy(host).to(device_of(col))
+            lanes = torch.from_numpy(host).to(device_of(col))
         try:
-            m._imn_mulm_pack = pack
+            m._imn_mulm_lanes = lanes
         except AttributeError:
             pass
-    return pack
+    return lanes
 
 
 def model_struct(m: Any) -> abi.ImnModel:
@@ -127,7 +127,8 @@ def model_struct(m: Any) -> abi.ImnModel:
     s.M_mulm_rowadr = addr(m.M_mulm_rowadr)
     s.M_mulm_col = addr(m.M_mulm_col)
     s.M_mulm_madr = addr(m.M_mulm_madr)
-    s.M_mulm_pack = addr(_mulm_pack(m))
+    lanes = _mulm_lanes(m)
+    s.M_mulm_lanes, s.n_mulm_batches = addr(lanes), int(shape(lanes)[0])
     s.alpha_noise_eps = eps
     s.overflow_iterations = ovf_it
     s.overflow_ls_iterations = ovf_ls

@@ -139,8 +139,8 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
   s.ids = s.state + r4;
   s.frows = s.ids + r4;  // rows with a nonzero force, ascending
   s.uni = reinterpret_cast<int*>(smem + g.oUni);
-  s.mulm_rowadr = m.M_mulm_rowadr;
-  s.mulm_pack = m.M_mulm_pack;
+  s.mulm_lanes = m.M_mulm_lanes, s.mulm_batches = m.n_mulm_batches;
+  s.M_rowadr = m.M_rowadr, s.M_rownnz = m.M_rownnz, s.M_colind = m.M_colind;
   s.jbar = bar;
   s.jphase = reinterpret_cast<int*>(smem + g.oBar) + 2;  // the barrier itself takes two words
   s.jfail = s.jphase + 1;
@@ -569,8 +569,8 @@ static int validate(const ImnModel* m, const ImnData* d, const ImnCtx* cx) {
   if (m->iterations <= 0) return set_error("imn_solve: iterations must be positive"), IMN_ERR_UNSUPPORTED;
   if (m->n_tolerance <= 0 || m->n_ls_tolerance <= 0 || m->n_meaninertia <= 0)
     return set_error("imn_solve: empty option array"), IMN_ERR_SHAPE;
-  const void* need[] = {m->opt_tolerance, m->opt_ls_tolerance, m->stat_meaninertia, m->M_mulm_rowadr,
-                        m->M_mulm_pack, d->nefc, d->ne, d->nf, d->qacc_smooth, d->qacc_warmstart,
+  const void* need[] = {m->opt_tolerance, m->opt_ls_tolerance, m->stat_meaninertia, m->M_rowadr,
+                        m->M_rownnz, m->M_colind, m->M_mulm_lanes, d->nefc, d->ne, d->nf, d->qacc_smooth, d->qacc_warmstart,
                         d->qfrc_smooth, d->efc_J, d->efc_D, d->efc_aref, d->efc_frictionloss, d->M, d->qacc,
                         d->qfrc_constraint, d->efc_Ma, d->efc_force, d->efc_state, d->solver_niter,
                         d->overflow};
@@ -583,6 +583,7 @@ static int validate(const ImnModel* m, const ImnData* d, const ImnCtx* cx) {
   if (d->J_ld_row > 4 * (int64_t)m->nv + 64)
     return set_error("imn_solve: efc.J row stride %lld is far larger than nv %d", (long long)d->J_ld_row, m->nv),
            IMN_ERR_SHAPE;
+  if (m->n_mulm_batches <= 0) return set_error("imn_solve: empty M_mulm_lanes program"), IMN_ERR_SHAPE;
   if (m->nM >= (1 << 16)) return set_error("imn_solve: nM exceeds 16-bit indices"), IMN_ERR_LIMIT;
   if (cx->grad && cx->grad_ld < m->nv) return set_error("imn_solve: ctx.grad stride < nv"), IMN_ERR_SHAPE;
   if (cx->sparse_plan) {

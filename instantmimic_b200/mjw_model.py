@@ -68,7 +68,7 @@ class Model:
     M_mulm_rowadr: Any
     M_mulm_col: Any
     M_mulm_madr: Any
-    M_mulm_pack: Any  # col | madr << 16 per entry of the M_mulm tables
+    M_mulm_lanes: Any  # the M_mulm rows dealt to 32 lanes (mulm_lane_program)
     block_dim: SimpleNamespace = field(
         default_factory=lambda: SimpleNamespace(linesearch_iterative=32)
     )
@@ -208,13 +208,34 @@ def mulm_tables(rowadr, rownnz, colind, nv: int):
     return as32(adr), as32(col), as32(madr)
 
 
-def pack_mulm(col, madr) -> np.ndarray:
-    """One word per entry of the M_mulm tables: col | madr << 16."""
-    col = np.asarray(col).astype(np.int64)
-    madr = np.asarray(madr).astype(np.int64)
-    if col.size and (col.max() >= 1 << 16 or madr.max() >= 1 << 16):
-        raise ValueError("M_mulm indices exceed 16 bits")
-    return (col | (madr << 16)).astype(np.uint32).view(np.int32)
+def mulm_lane_program(rowadr, col, madr, nv: int) -> np.ndarray:
+    """The M_mulm rows dealt to the 32 lanes of a warp: (batches, 32, 4) words
+    ``col | madr << 16`` (layout in include/imnewton.h, ``M_mulm_lanes``).  Rows go longest
+    first to the lane with the fewest batches so far, so the program is hardly longer than
+    its longest row although nv may exceed 32."""
+    rowadr = np.asarray(rowadr, dtype=np.int64)
+    col = np.asarray(col, dtype=np.int64)
+    madr = np.asarray(madr, dtype=np.int64)
+    if nv > 128 or (madr.size and madr.max() >= 1 << 16):
+        return np.zeros((1, 32, 4), np.int32)  # outside the fused path
+    lanes: list[list[list[int]]] = [[] for _ in range(32)]
+    for i in sorted(range(nv), key=lambda i: (rowadr[i] - rowadr[i + 1], i)):
+        lane = min(range(32), key=lambda q: len(lanes[q]))
+        k0, k1 = int(rowadr[i]), int(rowadr[i + 1])
+        words = [int(col[k]) | int(madr[k]) << 16 for k in range(k0, k1)]
+        for at in range(0, max(len(words), 1), 4):
+            batch = words[at:at + 4]
+            used = len(batch)
+            batch += [0] * (4 - used)
+            if at + 4 >= len(words):
+                batch[0] |= used << 8
+                batch[1] |= i << 8
+            lanes[lane].append(batch)
+    out = np.zeros((max(len(q) for q in lanes), 32, 4), np.int64)
+    for lane, program in enumerate(lanes):
+        for b, batch in enumerate(program):
+            out[b, lane] = batch
+    return out.astype(np.uint32).view(np.int32)
 
 
 def put_model(
@@ -309,7 +330,7 @@ def put_model(
         M_mulm_rowadr=madr_row,
         M_mulm_col=mcol,
         M_mulm_madr=madr,
-        M_mulm_pack=pack_mulm(mcol, madr),
+        M_mulm_lanes=mulm_lane_program(madr_row, mcol, madr, nv),
         body_parentid=body_parentid,
         body_dofadr=body_dofadr,
         body_dofnum=body_dofnum,

@@ -151,15 +151,15 @@ def load(path: str | Path) -> tuple[Model, Data, SimpleNamespace | None, SimpleN
         **{n: g(f"model/opt/{n}") for n in _OPT_ARRAYS},
     )
     nv = int(e["model/nv"])
-    pack = None
+    lanes = None
     if g("model/M_mulm_col") is not None and g("model/M_mulm_madr") is not None:
-        pack = mjw_model.pack_mulm(e["model/M_mulm_col"], e["model/M_mulm_madr"])
+        lanes = mjw_model.mulm_lane_program(e["model/M_mulm_rowadr"], e["model/M_mulm_col"], e["model/M_mulm_madr"], nv)
     m = Model(
         nv=nv, nv_pad=int(e["model/nv_pad"]), opt=opt, stat=Statistic(meaninertia=g("model/stat/meaninertia")),
         is_sparse=bool(int(e["model/is_sparse"])), dof_parentid=g("model/dof_parentid"),
         M_rowadr=g("model/M_rowadr"), M_rownnz=g("model/M_rownnz"), M_colind=g("model/M_colind"),
         M_hinit_i=g("model/M_hinit_i"), M_mulm_rowadr=g("model/M_mulm_rowadr"), M_mulm_col=g("model/M_mulm_col"),
-        M_mulm_madr=g("model/M_mulm_madr"), M_mulm_pack=pack,
+        M_mulm_madr=g("model/M_mulm_madr"), M_mulm_lanes=lanes,
         body_parentid=g("model/body_parentid"), body_dofadr=g("model/body_dofadr"),
         body_dofnum=g("model/body_dofnum"), neq=int(e["model/neq"]), nflex=int(e["model/nflex"]),
         ntendon=int(e["model/ntendon"]), geom_bodyid=g("model/geom_bodyid"),
