@@ -89,26 +89,32 @@ __device__ __forceinline__ Vec3 row_at(const Row& r, float alpha, bool absolute)
     o.c0 = r.f * (alpha * r.j);
   return o;
 }
-// The same for a plain inequality row (limit or pyramidal contact edge): cost
-// 0.5 D x^2 while x < 0, else nothing.  Branch-free; identical values to row_at.
-__device__ __forceinline__ Row make_row_ineq(bool valid, float D, float ja, float j) {
-  Row r;
-  r.f = 0.0f, r.D = D, r.ja = ja, r.j = j, r.rf = -1.0f;
-  r.z0 = valid ? (ja >= 0.0f ? IMN_STATE_SATISFIED : IMN_STATE_QUADRATIC) : -1;
+// A plain inequality row (limit or pyramidal contact edge: cost 0.5 D x^2 while x < 0, else
+// nothing) prepared for evaluation at several step sizes.  The values equal row_at's.  A lane
+// without a row takes D = 0, ja = 1, j = 0, which contributes exact zeros everywhere.
+struct IneqRow {
+  float ja, j, jvD, h, q1r, hD, neg_cost0;
+  bool on0;
+};
+__device__ __forceinline__ IneqRow ineq_row(float D, float ja, float j) {
+  IneqRow r;
+  r.ja = ja, r.j = j;
   r.jvD = j * D;
   r.h = j * r.jvD;
   r.q1r = r.jvD * ja;
-  r.cost0 = r.z0 == IMN_STATE_QUADRATIC ? ((0.5f * D) * ja) * ja : 0.0f;
+  r.hD = 0.5f * D;
+  r.on0 = ja < 0.0f;
+  r.neg_cost0 = r.on0 ? -((r.hD * ja) * ja) : 0.0f;
   return r;
 }
-__device__ __forceinline__ Vec3 row_at_ineq(const Row& r, float alpha, bool absolute) {
+// acc += (cost(alpha) - cost(0), slope, curvature)
+__device__ __forceinline__ void ineq_add(const IneqRow& r, float alpha, float half_alpha, Vec3& acc) {
   const float x = fmaf(alpha, r.j, r.ja);
-  const bool valid = r.z0 >= 0, on = valid && x < 0.0f, on0 = r.z0 == IMN_STATE_QUADRATIC;
-  const float cx = on ? ((0.5f * r.D) * x) * x : 0.0f;
-  float c0 = on == on0 ? (on ? alpha * fmaf(0.5f * alpha, r.h, r.q1r) : 0.0f) : cx - r.cost0;
-  if (absolute) c0 = r.cost0;
-  if (!valid) c0 = 0.0f;
-  return v3(c0, on ? r.jvD * x : 0.0f, on ? r.h : 0.0f);
+  const bool on = x < 0.0f;
+  const float same = alpha * fmaf(half_alpha, r.h, r.q1r), enter = (r.hD * x) * x;
+  acc.c0 = acc.c0 + (on ? (r.on0 ? same : enter) : r.neg_cost0);
+  const float slope = r.jvD * x;
+  if (on) acc.c1 = acc.c1 + slope, acc.c2 = acc.c2 + r.h;
 }
 __device__ __forceinline__ Vec3 eval_quad(float q1, float q2, float alpha) {
   return v3(fmaf(alpha, q1, (alpha * alpha) * q2) + 0.0f, fmaf(2.0f * alpha, q2, q1), 2.0f * q2);
@@ -150,19 +156,39 @@ __device__ __forceinline__ float logical_block_sum(int n, int bd, int lane, F te
   return s;
 }
 
-// Shuffle-down trees of N values at once (independent chains interleave), lane 0
-// broadcast, then "+0" per later logical warp of the line search
-// (newton_stages.py:39-49).
+// Lane sums of N values at once in the order of N shuffle-down trees, broadcast, then "+0" per
+// later logical warp of the line search (newton_stages.py:39-49).  A tree's steps only ever need
+// half, a quarter, ... of the lanes, so two values share each step: one half of the lanes goes on
+// with the first value, the other half with the second (an addition's operands may come in
+// either order), and after five steps value k sits in lanes of its own.  Nine values take 16
+// shuffles and additions plus the broadcasts instead of 45.
 template <int N>
-__device__ __forceinline__ void ls_sum(float (&v)[N], int bd) {
+__device__ __forceinline__ void ls_sum(float (&v)[N], int bd, int lane) {
+  constexpr int N1 = (N + 1) / 2, N2 = (N1 + 1) / 2, N3 = (N2 + 1) / 2, N4 = (N3 + 1) / 2;
+  static_assert(N4 == 1, "at most 16 values");
+  float a[N1], b[N2], c[N3], d[N4];
+  auto fold = [&](auto& out, auto& in, int n, int off) {
+    const bool up = (lane & off) != 0;
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) v[k] = v[k] + __shfl_down_sync(IMN_FULL_MASK, v[k], off);
-  }
+    for (int k = 0; k < n; k += 2) {
+      if (k + 1 < n) {
+        const float keep = up ? in[k + 1] : in[k], send = up ? in[k] : in[k + 1];
+        out[k / 2] = keep + __shfl_xor_sync(IMN_FULL_MASK, send, off);
+      } else {
+        out[k / 2] = in[k] + __shfl_xor_sync(IMN_FULL_MASK, in[k], off);
+      }
+    }
+  };
+  fold(a, v, N, 16);
+  fold(b, a, N1, 8);
+  fold(c, b, N2, 4);
+  fold(d, c, N3, 2);
+  const float e = d[0] + __shfl_xor_sync(IMN_FULL_MASK, d[0], 1);
 #pragma unroll
   for (int k = 0; k < N; ++k) {
-    v[k] = __shfl_sync(IMN_FULL_MASK, v[k], 0);
+    // value k went up at step s when its index at that step was odd
+    const int src = ((k & 1) ? 16 : 0) | ((k & 2) ? 8 : 0) | ((k & 4) ? 4 : 0) | ((k & 8) ? 2 : 0);
+    v[k] = __shfl_sync(IMN_FULL_MASK, e, src);
     if (bd == 64) v[k] = v[k] + 0.0f;
   }
 }
