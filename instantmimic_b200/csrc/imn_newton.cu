@@ -54,7 +54,7 @@ struct Geom {
   int nv, njmax, ldj, ldu, nM, bd;
   int jrows;  // rows of J held in shared memory (njmax when resident, else 32)
   // offsets in 4-byte words; every region starts on a 16-byte boundary
-  int oBar, oJ, oA, oVec, nv4, oRowF, oRowI, r4, oUni, total;
+  int oBar, oJ, oA, oVec, nv4, oRowF, oRowI, oMask, mwords, r4, oUni, total;
   // polls a copy wait may take before the world gives up, and the failure-path test
   // switch: when set no bulk copy is issued (plain loads bring the data) while the
   // barrier is told to expect bytes, so the wait runs out with nothing in flight
@@ -82,13 +82,16 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   int o = 0;
   g.oBar = o, o += 4;
   // a streamed tile may start up to three floats into its buffer and end on a 16-byte boundary
-  g.oJ = o, o += up4(g.jrows * g.ldj) + (resident ? 0 : 8);
+  // a dense block reads up to three floats past a row; the gathered rows are up4(nv) floats apart
+  g.oJ = o, o += (resident ? up4(g.jrows * g.ldj + 3) : max(up4(32 * g.ldj) + 8, 32 * g.nv4));
   // dense: H and its factor share one (nv+1) x ldu array; sparse plan: packed H | N | 1/D
   g.oA = o, o += sp ? up4(sp->nfac) + up4(sp->nslots) + up4(m.nv) : (m.nv + 1) * g.ldu;
   // dof vectors; the dense factor needs two more (forward-solve scratch, 1 / pivot)
   g.oVec = o, o += (sp ? 6 : 8) * g.nv4;
-  g.oRowF = o, o += 5 * g.r4;
+  g.oRowF = o, o += 4 * g.r4;
   g.oRowI = o, o += up4(3 * g.r4 / 2);  // three 16-bit row lists
+  g.mwords = (m.nv + 31) / 32;
+  g.oMask = o, o += g.mwords * g.r4;
   g.oUni = o, o += up4(m.nv + 1);
   g.total = o;
   g.wait_polls = g_wait_polls;
@@ -133,8 +136,9 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
   s.Jaref = smem + g.oRowF;
   s.jv = s.Jaref + r4;
   s.Dsm = s.jv + r4;
-  s.floss = s.Dsm + r4;
-  s.force = s.floss + r4;
+  s.force = s.Dsm + r4;
+  s.masks = reinterpret_cast<uint32_t*>(smem + g.oMask);
+  s.mwords = g.mwords, s.r4 = r4;
   s.state = reinterpret_cast<uint16_t*>(smem + g.oRowI);
   s.ids = s.state + r4;
   s.frows = s.ids + r4;  // rows with a nonzero force, ascending
@@ -166,6 +170,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
   bool search_unchanged = false, ls_exhausted = false;
   int st_passes = 0, st_flips = 0, st_factor = 0, st_grad = 0;  // work counters (ctx.stats)
   bool have = false, first = true;
+  bool outside = false;  // a row of the world leaves the sparse plan's pattern
   bool taken = false;  // this CTA's world was taken
 
 #pragma unroll 1
@@ -186,6 +191,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         dofo = (size_t)w * d.dof_ld, efco = (size_t)w * d.efc_ld;
         s.Jg = d.efc_J + (d.J_world_offset ? (size_t)d.J_world_offset[w] : (size_t)w * d.J_ld_world);
         s.M = d.M + (size_t)w * d.M_ld;
+        s.floss = d.efc_frictionloss + efco;
 
         // ---- load: TMA bulk copies for the 16-byte-aligned bulk of every array, plain
         // loads for the ragged ends ---------------------------------------------------
@@ -195,10 +201,9 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
           const float* src;
           int n;
         };
-        const Src srcs[6] = {
+        const Src srcs[5] = {
             {s.Jsm, s.Jg, JRES ? nefc * s.ldj : 0},
             {s.Dsm, d.efc_D + efco, nefc},
-            {s.floss, d.efc_frictionloss + efco, nefc},
             {s.jv, d.efc_aref + efco, nefc},  // aref is parked in jv until Jaref is formed
             {s.qacc, q0 + dofo, nv},
             {s.qfs, d.qfrc_smooth + dofo, nv},
@@ -211,19 +216,19 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         const bool bulk = !(g.withhold_copies & 1);
         uint32_t tx = 0;
 #pragma unroll
-        for (int k = 0; k < 6; ++k)
+        for (int k = 0; k < 5; ++k)
           if (bulk && (reinterpret_cast<uintptr_t>(srcs[k].src) & 15) == 0) tx += (uint32_t)(srcs[k].n & ~3) * 4u;
         if (lane == 0) {
           mbar_expect_tx(bar, bulk ? tx : 16u);
 #pragma unroll
-          for (int k = 0; k < 6; ++k) {
+          for (int k = 0; k < 5; ++k) {
             const uint32_t bytes =
                 bulk && (reinterpret_cast<uintptr_t>(srcs[k].src) & 15) == 0 ? (uint32_t)(srcs[k].n & ~3) * 4u : 0u;
             if (bytes) bulk_g2s(srcs[k].dst, srcs[k].src, bytes, bar);
           }
         }
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
+        for (int k = 0; k < 5; ++k) {
           const int done_n = bulk && (reinterpret_cast<uintptr_t>(srcs[k].src) & 15) == 0 ? (srcs[k].n & ~3) : 0;
 #pragma unroll 1
           for (int i = done_n + lane; i < srcs[k].n; i += 32) srcs[k].dst[i] = srcs[k].src[i];
@@ -298,7 +303,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
 #pragma unroll 1
       for (int base = 0; base < nefc; base += 32) {
         const int r = base + lane;
-        bool flip = false, changed = false;
+        bool flip = false, changed = false, leaves = false;
         float f = 0.0f;
         if (r < nefc) {
           const float nj = first ? s.Jaref[r] : rounded_step(s.Jaref[r], alpha, s.jv[r]);
@@ -316,10 +321,11 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
           flip = first ? ns == IMN_STATE_QUADRATIC
                        : (old == IMN_STATE_QUADRATIC) != (ns == IMN_STATE_QUADRATIC);
           changed = old != ns;
+          leaves = ns != IMN_STATE_QUADRATIC;
         }
         const unsigned below = (1u << lane) - 1u;
         const unsigned fm = __ballot_sync(IMN_FULL_MASK, flip);
-        if (flip) s.ids[quad_count + __popc(fm & below)] = r;
+        if (flip) s.ids[quad_count + __popc(fm & below)] = r | (leaves ? 0x8000 : 0);
         quad_count += __popc(fm);
         state_count += __popc(__ballot_sync(IMN_FULL_MASK, changed));
         const unsigned nz = __ballot_sync(IMN_FULL_MASK, f != 0.0f);
@@ -356,23 +362,23 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         PROF(8);
         decrement = 0.0f;
         grad_scale = 1.0f;
-        if (first) {
+        if (first || quad_count > 0) {
+          if (SPARSE && first) {
+            bool bad = false;
+#pragma unroll 1
+            for (int r = lane; r < nefc; r += 32) bad = bad || row_outside(s.masks, r4, g.mwords, r, sp.pmask);
+            outside = __any_sync(IMN_FULL_MASK, bad);
+          }
           if (SPARSE)
-            assemble_hessian_sparse<JRES>(s, quad_count, sp);
+            hessian_sparse<JRES>(s, quad_count, first, outside, sp);
           else
-            assemble_hessian<JRES>(s, quad_count);
-        } else if (quad_count > 0) {
-          update_hessian<JRES, SPARSE>(s, quad_count, sp);
+            hessian_dense<JRES>(s, quad_count, first);
         }
         PROF(9);
         if (SPARSE) {
           // refactor the packed H, or solve with the resident factor
           // (sparse_hessian.py:490-547)
           if (first || quad_count > 0) {
-            if (!first) {
-#pragma unroll 1
-              for (int q = lane; q < sp.nfac; q += 32) s.N[q] = s.Hp[q];
-            }
             sp_load_rhs(sp, s.N, s.grad, lane);
             IMN_MARK(s, 1);
             sp_factor_sweeps(sp, s.N, s.iD, lane);
@@ -439,7 +445,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
       d.efc_state[efco + r] = s.state[r];
       if (cx.Jaref) cx.Jaref[efco + r] = s.Jaref[r];
       if (cx.jv) cx.jv[efco + r] = s.jv[r];
-      if (cx.quad_changed_ids && r < quad_count) cx.quad_changed_ids[efco + r] = s.ids[r];
+      if (cx.quad_changed_ids && r < quad_count) cx.quad_changed_ids[efco + r] = s.ids[r] & 0x7FFF;
     }
     if (cx.dof_union && !rowless)
 #pragma unroll 1
@@ -561,7 +567,7 @@ static const int kResidentBudget = kMaxSmem / 4;
 static int validate(const ImnModel* m, const ImnData* d, const ImnCtx* cx) {
   if (!m || !d || !cx) return set_error("imn_solve: NULL struct"), IMN_ERR_NULL;
   if (d->nworld < 0 || d->njmax < 0) return set_error("imn_solve: negative extent"), IMN_ERR_SHAPE;
-  if (d->njmax >= (1 << 16)) return set_error("imn_solve: njmax %d exceeds 16-bit row indices", d->njmax), IMN_ERR_LIMIT;
+  if (d->njmax >= (1 << 15)) return set_error("imn_solve: njmax %d exceeds 15-bit row indices", d->njmax), IMN_ERR_LIMIT;
   if (m->nv <= 0 || m->nv > 79 || m->nv_pad % 16 != 0 || m->nv_pad > 80 || m->nv_pad <= m->nv)
     return set_error("imn_solve: nv %d / nv_pad %d outside the fused path (0 < nv <= 79, nv_pad %% 16 == 0, nv < nv_pad <= 80)",
                      m->nv, m->nv_pad),

@@ -20,11 +20,14 @@ struct World {
   // the shared memory they would take holds more worlds per SM instead (measured: humanoid
   // 0.792 -> 0.785 ms per 8192 worlds, SNU-like 1.820 -> 1.736 ms per 4096)
   const float* M;
-  float *Jaref, *jv, *Dsm, *floss, *force;
-  // row states and the two row lists are 16-bit (njmax < 65536): shared memory per
+  float *Jaref, *jv, *Dsm, *force;
+  const float* floss;  // global memory: only friction-loss rows read it
+  // row states and the two row lists are 16-bit (njmax < 32768: bit 15 is a flag in ids): shared memory per
   // world decides how many worlds an SM holds
   uint16_t *state, *ids, *frows;
   int* uni;
+  uint32_t* masks;  // the dofs each row touches (store_mask)
+  int mwords, r4;
   const float* Jg;    // this world's J in global memory
   const float *Jbeg, *Jend;  // first element and one past the last row of the whole J array
   // streamed J: the copy barrier of the row tile, the parity of its next phase and the
@@ -91,9 +94,84 @@ __device__ __forceinline__ const float* j_tile(const World& s, int base) {
   __syncwarp();
   return s.Jsm;
 }
+// Rows of the list s.ids (bit 15: the row leaves the QUADRATIC set, its D counts negative) as the
+// Hessian stages read them.  A resident J is read in place.  Streamed rows are gathered into the
+// tile, up to 32 listed rows at a time and up4(nv) floats apart: the stages read a row many times
+// over, and taking its elements from global memory each time was a half of the whole solve at
+// 64 dofs x 512 rows.
+struct ListRow {
+  const float* J;
+  float D;
+};
 template <bool JRES>
-__device__ __forceinline__ float j_at(const World& s, int r, int i) {
-  return JRES ? s.Jsm[r * s.ldj + i] : s.Jg[(size_t)r * s.ldj + i];
+__device__ __forceinline__ ListRow list_row(const World& s, int t, int t0) {
+  const int id = s.ids[t], r = id & 0x7FFF;
+  ListRow o;
+  o.J = JRES ? s.Jsm + r * s.ldj : s.Jsm + (t - t0) * ((s.nv + 3) & ~3);
+  o.D = __int_as_float(__float_as_int(s.Dsm[r]) ^ ((id & 0x8000) << 16));
+  return o;
+}
+template <bool JRES>
+__device__ __forceinline__ void gather_rows(const World& s, int t0, int t1) {
+  if (JRES) return;
+  __syncwarp();  // every lane is done with the tile's previous contents
+  const int ld = (s.nv + 3) & ~3, lane = s.lane;
+  const int ids = t0 + lane < t1 ? s.ids[t0 + lane] & 0x7FFF : 0;
+  uint32_t dst = smem_u32(s.Jsm + lane);
+#pragma unroll 4
+  for (int t = t0; t < t1; ++t, dst += 4u * ld) {
+    const float* src = s.Jg + (size_t)__shfl_sync(IMN_FULL_MASK, ids, t - t0) * s.ldj + lane;
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      if (32 * q + lane < s.nv)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 128u * q), "l"(src + 32 * q) : "memory");
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  // a later tile may arrive through the async proxy into the same buffer
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+}
+
+// The dofs each row touches, as s.mwords 32-bit words per row in shared memory (word q of row r at
+// s.masks[q * r4 + r]), formed once per world while the first pass has the row in hand (lane = row).
+// The Hessian stages need them at every change of the active set: for the dofs the flipped rows
+// touch, and to know that no row leaves the sparse plan's pattern.
+__device__ __forceinline__ void store_mask(const World& s, const float* Jr, int r) {
+#pragma unroll 1
+  for (int q = 0; q < s.mwords; ++q) {
+    unsigned m = 0u;
+    const int n = min(32, s.nv - 32 * q);
+#pragma unroll 4
+    for (int i = 0; i < n; ++i) m |= (unsigned)(Jr[32 * q + i] != 0.0f) << i;
+    s.masks[q * s.r4 + r] = m;
+  }
+}
+// Whether row r's dofs are not all coupled in the plan's pattern.
+__device__ __forceinline__ bool row_outside(const uint32_t* masks, int r4, int mwords, int r, const uint32_t* pmask) {
+  bool bad = false;
+#pragma unroll 1
+  for (int q = 0; q < mwords; ++q)
+#pragma unroll 1
+    for (unsigned left = masks[q * r4 + r]; left; left &= left - 1u) {
+      const int d = 32 * q + __ffs(left) - 1;
+#pragma unroll 1
+      for (int p = 0; p < mwords; ++p) bad = bad || (masks[p * r4 + r] & ~__ldg(pmask + d * mwords + p)) != 0u;
+    }
+  return bad;
+}
+// The dofs of the flipped rows, ascending, and their count (ctx.newton_dof_union).
+__device__ __forceinline__ void write_union(const World& s, int count) {
+  int n = 0;
+#pragma unroll 1
+  for (int q = 0; q < s.mwords; ++q) {
+    unsigned m = 0u;
+#pragma unroll 1
+    for (int t = s.lane; t < count; t += 32) m |= s.masks[q * s.r4 + (s.ids[t] & 0x7FFF)];
+    m = __reduce_or_sync(IMN_FULL_MASK, m);
+    if ((m >> s.lane) & 1u) s.uni[n + __popc(m & ((1u << s.lane) - 1u))] = 32 * q + s.lane;
+    n += __popc(m);
+  }
+  if (s.lane == 0) s.uni[s.nv] = n;
 }
 
 // outM = M v over the symmetric rows (newton_fusion.py:171-176) and
@@ -151,6 +229,7 @@ __device__ __forceinline__ void products(const World& s, const float* v, float* 
           total = total + p;
       }
       outJ[r] = total;
+      if (minus) store_mask(s, Jr, r);  // the first pass
     }
     if (!JRES) __syncwarp();
   }
@@ -190,214 +269,175 @@ __device__ __forceinline__ float full_gradient(const World& s, int nfr) {
   return logical_block_sum(nv, s.bd, lane, [&](int i, float acc) { return fmaf(s.grad[i], s.grad[i], acc); });
 }
 
-// H = M + J^T diag(D, QUADRATIC rows) J on the upper triangle, every entry summing
-// its rows in ascending order.  H[r][c] (r <= c) lives at A[(c+1)*ldu + r].
-// The QUADRATIC rows arrive as the ascending list s.ids[0, nq) (built by the row
-// update of the initial pass).
+// The Hessian from the listed rows, dense form.  First call: H = M + sum D J^T J over the
+// QUADRATIC rows, every entry starting from M and summing its rows in ascending order.  Later:
+// every entry's change is summed over the flipped rows in list order (newton_stages.py:651-701)
+// and added to H.  H[r][c] (r <= c) lives at A[(c+1)*ldu + r]; the sums of a list that does not fit
+// one tile wait in the factor's half of the array (U[r][c] at A[r*ldu + c]), which is dead until
+// the factorisation that follows.
+// A lane owns 4 x 4 blocks of the upper triangle: eight values of a row feed 16 fused
+// multiply-adds, so the stage is bound by arithmetic instead of by shared-memory reads (an entry
+// per lane reads two values and looks its row up for every multiply-add).
 template <bool JRES>
-__device__ __forceinline__ void assemble_hessian(const World& s, int nq) {
+__device__ __forceinline__ void hessian_dense(const World& s, int count, bool first) {
   const int lane = s.lane, nv = s.nv, ldu = s.ldu;
   float* A = s.A;
+  if (first) {
 #pragma unroll 4
-  for (int e = lane; e < (nv + 1) * ldu; e += 32) A[e] = 0.0f;
-  __syncwarp();
-#pragma unroll 1
-  for (int i = lane; i < nv; i += 32) {
-    const int e0 = __ldg(s.M_rowadr + i), n = __ldg(s.M_rownnz + i);
-#pragma unroll 4
-    for (int k = 0; k < n; ++k) A[(i + 1) * ldu + __ldg(s.M_colind + e0 + k)] = __ldg(s.M + e0 + k);
-  }
-  __syncwarp();
-  const int npair = nv * (nv + 1) / 2;
-  // six entries per lane at a time: a row's D is read once per six entries and the six
-  // running sums overlap; every entry still receives its rows in ascending order
-  constexpr int Q = 6;
-  int k_lo = 0;
-#pragma unroll 1
-  for (int base = 0; base < s.nefc && k_lo < nq; base += 32) {
-    const float* Jt = j_tile<JRES>(s, base);
-    const int row_hi = JRES ? s.nefc : base + 32;
-    int k_hi = k_lo;
-    while (k_hi < nq && s.ids[k_hi] < row_hi) ++k_hi;
-#pragma unroll 1
-    for (int e0 = 0; e0 < npair && k_hi > k_lo; e0 += 32 * Q) {
-      float acc[Q];
-      int ij[Q];
-#pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        const int e = e0 + 32 * q + lane;
-        int pi = 0, pj = 0;
-        if (e < npair) pair_lookup(e, pi, pj);
-        ij[q] = e < npair ? (pi | (pj << 16)) : -1;
-        acc[q] = e < npair ? A[(pj + 1) * ldu + pi] : 0.0f;
-      }
-#pragma unroll 1
-      for (int k = k_lo; k < k_hi; ++k) {
-        const int r = s.ids[k];
-        const float Dr = s.Dsm[r];
-        const float* Jr = Jt + (r - base) * s.ldj;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-          const int pi = ij[q] < 0 ? 0 : (ij[q] & 0xFFFF), pj = ij[q] < 0 ? 0 : (ij[q] >> 16);
-          acc[q] = fmaf(Jr[pi] * Dr, Jr[pj], acc[q]);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < Q; ++q)
-        if (ij[q] >= 0) A[((ij[q] >> 16) + 1) * ldu + (ij[q] & 0xFFFF)] = acc[q];
-    }
-    k_lo = k_hi;
-    if (JRES) break;
+    for (int e = lane; e < (nv + 1) * ldu; e += 32) A[e] = 0.0f;
     __syncwarp();
+#pragma unroll 1
+    for (int i = lane; i < nv; i += 32) {
+      const int e0 = __ldg(s.M_rowadr + i), n = __ldg(s.M_rownnz + i);
+#pragma unroll 4
+      for (int k = 0; k < n; ++k) A[(i + 1) * ldu + __ldg(s.M_colind + e0 + k)] = __ldg(s.M + e0 + k);
+    }
   }
+  const int nb = (nv + 3) >> 2, nblock = nb * (nb + 1) / 2;
+  const int step = JRES ? max(count, 1) : 32;
+#pragma unroll 1
+  for (int t0 = 0; t0 < count; t0 += step) {
+    const int t1 = min(t0 + step, count);
+    gather_rows<JRES>(s, t0, t1);
+    __syncwarp();
+    IMN_MARK(s, 22);
+    const bool keep = t0 > 0 || first, last = t1 == count;
+#pragma unroll 1
+    for (int b0 = 0; b0 < nblock; b0 += 32) {
+      const bool live = b0 + lane < nblock;
+      int bi, bj;
+      pair_lookup(min(b0 + lane, nblock - 1), bi, bj);
+      const int i0 = 4 * bi, j0 = 4 * bj;
+      float acc[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const bool in = i0 + i <= j0 + j && j0 + j < nv;
+          acc[i][j] = !(keep && in) ? 0.0f : t0 > 0 ? A[(i0 + i) * ldu + j0 + j] : A[(j0 + j + 1) * ldu + i0 + i];
+        }
+#pragma unroll 2
+      for (int t = t0; t < t1; ++t) {
+        const ListRow row = list_row<JRES>(s, t, t0);
+        float a[4], b[4];
+        if (JRES) {  // rows lie at their own stride, on any boundary
+#pragma unroll
+          for (int k = 0; k < 4; ++k) a[k] = row.J[i0 + k], b[k] = row.J[j0 + k];
+        } else {
+          const float4 fa = *reinterpret_cast<const float4*>(row.J + i0), fb = *reinterpret_cast<const float4*>(row.J + j0);
+          a[0] = fa.x, a[1] = fa.y, a[2] = fa.z, a[3] = fa.w, b[0] = fb.x, b[1] = fb.y, b[2] = fb.z, b[3] = fb.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float ad = a[i] * row.D;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ad, b[j], acc[i][j]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (live && i0 + i <= j0 + j && j0 + j < nv) {
+            float* h = A + (j0 + j + 1) * ldu + i0 + i;
+            if (!last)
+              A[(i0 + i) * ldu + j0 + j] = acc[i][j];
+            else
+              *h = first ? acc[i][j] : *h + acc[i][j];
+          }
+    }
+  }
+  if (!first) write_union(s, count);
   __syncwarp();
+  IMN_MARK(s, 18);
 }
 
-// Rows whose QUADRATIC membership flipped -> dofs they touch (ascending), then
-// the pair update of H in the listed row order (newton_stages.py:651-701).
-// With a sparse plan (SP != nullptr) the entry lands in the packed H through the
-// plan's pair table; an entry outside the pattern is dropped and counted
-// (sparse_hessian.py:501-527).
-template <bool JRES, bool SPARSE>
-__device__ __forceinline__ void update_hessian(const World& s, int count, const ImnSparsePlan& SP) {
-  const int lane = s.lane, nv = s.nv, ldu = s.ldu;
-  int n = 0;
-#pragma unroll 1
-  for (int base = 0; base < nv; base += 32) {
-    const int dof = base + lane;
-    bool hit = false;
-    if (dof < nv)
-#pragma unroll 1
-      for (int t = 0; t < count && !hit; ++t) hit = j_at<JRES>(s, s.ids[t], dof) != 0.0f;
-    const unsigned hm = __ballot_sync(IMN_FULL_MASK, hit);
-    if (hit) s.uni[n + __popc(hm & ((1u << lane) - 1u))] = dof;
-    n += __popc(hm);
+// Pattern violations, for a world that has a row outside the pattern: at the first call one per
+// QUADRATIC row with D != 0, later one per pair of touched dofs without a slot whose H entry the
+// flipped rows change (sparse_hessian.py:501-527, 619-620).
+__device__ __noinline__ void count_violations(bool first, const float* Jw, int ld, int nv, const float* Dsm, const uint32_t* masks,
+                                              int r4, int mwords, const uint16_t* ids, int count, const uint32_t* pmask,
+                                              const int* pair, float* viol, int world, int lane) {
+  if (first) {
+    for (int t = lane; t < count; t += 32)
+      if (Dsm[ids[t]] != 0.0f && row_outside(masks, r4, mwords, ids[t], pmask)) sp_violation(viol, world, "has a constraint row");
+    return;
   }
-  if (lane == 0) s.uni[nv] = n;
-  __syncwarp();
-  IMN_MARK(s, 12);
-  const int npu = n * (n + 1) / 2;
-  // several pairs per lane at a time: the listed rows are walked once per group and the
-  // sums overlap their latencies; each sum still takes its rows in list order.  Four,
-  // except two in the resident-J kernel with the sparse plan, where the smaller code is
-  // worth more (measured: 2 % faster there; 1-3 % slower with the dense factor, 2-8 %
-  // slower with streamed J).
-  constexpr int Q = (JRES && SPARSE) ? 2 : 4;
-#pragma unroll 1
-  for (int base = 0; base < npu; base += 32 * Q) {
-    int row[Q], col[Q], sl[Q];
-    float delta[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const bool in = base + 32 * q + lane < npu;
-      int pi = 0, pj = 0;
-      if (in) pair_lookup(base + 32 * q + lane, pi, pj);
-      row[q] = in ? s.uni[pi] : 0, col[q] = in ? s.uni[pj] : 0;
-      // looked up ahead of the sum so that the table's latency is hidden behind it
-      sl[q] = in ? (SPARSE ? __ldg(SP.pair + row[q] * nv + col[q]) : 0) : -2;
-      delta[q] = 0.0f;
-    }
-#pragma unroll 1
+  for (int e = lane; e < nv * (nv + 1) / 2; e += 32) {
+    int i, j;
+    pair_lookup(e, i, j);
+    if (__ldg(pair + i * nv + j) >= 0) continue;
+    float delta = 0.0f;
     for (int t = 0; t < count; ++t) {
-      const int r = s.ids[t];
-      const float Dr = s.state[r] == IMN_STATE_QUADRATIC ? s.Dsm[r] : -s.Dsm[r];
+      const int id = ids[t], r = id & 0x7FFF;
+      const float* J = Jw + (size_t)r * ld;
+      const float D = (id & 0x8000) ? -Dsm[r] : Dsm[r];
+      if (J[i] != 0.0f && J[j] != 0.0f) delta = fmaf(D * J[i], J[j], delta);
+    }
+    if (delta != 0.0f) sp_violation(viol, world, "updates an H entry");
+  }
+}
+
+// The same on the pattern slots of a sparse plan (sparse_hessian.py:501-527, 571-637): first call
+// M + sum D J^T J, later H plus the flipped rows' change; the result goes to the packed H and to N,
+// where the factorisation starts.  Every slot is summed, whether the rows touch it or not: slot
+// tables are read coalesced once per call, a slot costs four instructions per row, and no pair list
+// of touched dofs has to be formed and looked up.  `outside`: the world has a row whose dofs do not
+// all lie in the pattern.  Sums of a list that does not fit one tile wait in N.
+template <bool JRES>
+__device__ __forceinline__ void hessian_sparse(const World& s, int count, bool first, bool outside, const ImnSparsePlan& SP) {
+  const int lane = s.lane, nv = s.nv, nfac = SP.nfac;
+  constexpr int Q = JRES ? 10 : 12;
+  const int step = JRES ? max(count, 1) : 32;
+  // a list without rows still has to place M (first call)
+  int t0 = 0;
+  do {
+    const int t1 = min(t0 + step, count);
+    gather_rows<JRES>(s, t0, t1);
+    IMN_MARK(s, 22);
+    const bool last = t1 == count;
+#pragma unroll 1
+    for (int base = 0; base < nfac; base += 32 * Q) {
+      float acc[Q];
+      int a[Q], b[Q];
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
-        const float a = j_at<JRES>(s, r, row[q]), b = j_at<JRES>(s, r, col[q]);
-        if (a != 0.0f && b != 0.0f) delta[q] = fmaf(Dr * a, b, delta[q]);
+        const int sl = min(base + 32 * q + lane, nfac - 1);
+        a[q] = __ldg(SP.s_a + sl), b[q] = __ldg(SP.s_b + sl);
+        acc[q] = 0.0f;
+        if (t0 > 0) {
+          acc[q] = s.N[sl];
+        } else if (first) {
+          const int e = __ldg(SP.s_m + sl);
+          if (e >= 0) acc[q] = __ldg(s.M + e);
+        }
       }
-    }
+#pragma unroll 1
+      for (int t = t0; t < t1; ++t) {
+        const ListRow row = list_row<JRES>(s, t, t0);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      if (sl[q] != -2 && delta[q] != 0.0f) {
-        if (SPARSE) {
-          if (sl[q] >= 0)
-            s.Hp[sl[q]] = s.Hp[sl[q]] + delta[q];
-          else
-            sp_violation(s.viol, s.world, "updates an H entry");
-        } else {
-          s.A[(col[q] + 1) * ldu + row[q]] = s.A[(col[q] + 1) * ldu + row[q]] + delta[q];
+        for (int q = 0; q < Q; ++q) acc[q] = fmaf(row.J[a[q]] * row.D, row.J[b[q]], acc[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int sl = base + 32 * q + lane;
+        if (sl < nfac) {
+          if (last) {
+            if (!first) acc[q] = s.Hp[sl] + acc[q];
+            s.Hp[sl] = acc[q];
+          }
+          s.N[sl] = acc[q];
         }
       }
     }
-  }
+    t0 = t1;
+  } while (t0 < count);
+  if (!first) write_union(s, count);
+  if (outside)
+    count_violations(first, JRES ? s.Jsm : s.Jg, s.ldj, nv, s.Dsm, s.masks, s.r4, s.mwords, s.ids, count, SP.pmask, SP.pair, s.viol,
+                     s.world, lane);
   __syncwarp();
-  IMN_MARK(s, 13);
-}
-
-// Sparse plan: H = M + J^T diag(D, QUADRATIC rows) J on the pattern slots, each slot
-// summing its rows in ascending order; every active row's dof support must lie in
-// the pattern (sparse_hessian.py:571-637).  Leaves the packed H in both N and Hp.
-// A lane keeps the running sums of ten slots in registers and walks the QUADRATIC
-// rows once per ten slots: the row's D is read once, and ten independent sums overlap
-// their latencies.  The QUADRATIC rows arrive as the ascending list s.ids[0, nq).
-template <bool JRES>
-__device__ __forceinline__ void assemble_hessian_sparse(const World& s, int nq, const ImnSparsePlan& SP) {
-  const int lane = s.lane, nv = s.nv, nfac = SP.nfac, words = (nv + 31) >> 5;
-#pragma unroll 1
-  for (int a = 0; a < nq; ++a) {
-    const int r = s.ids[a];
-    if (s.Dsm[r] == 0.0f) continue;
-    unsigned rm[3] = {0u, 0u, 0u};
-#pragma unroll
-    for (int q = 0; q < 3; ++q)
-      if (q < words) {
-        const int d = q * 32 + lane;
-        rm[q] = __ballot_sync(IMN_FULL_MASK, d < nv && j_at<JRES>(s, r, d) != 0.0f);
-      }
-    bool bad = false;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const int d = q * 32 + lane;
-      if (q < words && d < nv && ((rm[q] >> lane) & 1u)) {
-#pragma unroll
-        for (int p = 0; p < 3; ++p)
-          if (p < words) bad = bad || (rm[p] & ~__ldg(SP.pmask + d * words + p)) != 0u;
-      }
-    }
-    if (__any_sync(IMN_FULL_MASK, bad) && lane == 0) sp_violation(s.viol, s.world, "has a constraint row");
-  }
-  __syncwarp();
-  constexpr int Q = 10;
-#pragma unroll 1
-  for (int base = 0; base < nfac; base += 32 * Q) {
-    float acc[Q];
-    int ab[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const int sl = base + 32 * q + lane;
-      acc[q] = 0.0f, ab[q] = 0;
-      if (sl < nfac) {
-        const int e = __ldg(SP.s_m + sl);
-        ab[q] = (int)__ldg(SP.s_a + sl) | ((int)__ldg(SP.s_b + sl) << 16);
-        acc[q] = e >= 0 ? __ldg(s.M + e) : 0.0f;
-      }
-    }
-    // rows in ascending order; a streamed J passes through its 32-row tile
-    int k = 0;
-#pragma unroll 1
-    for (int row0 = 0; row0 < s.nefc && k < nq; row0 += 32) {
-      const float* Jt = j_tile<JRES>(s, row0);
-      const int row1 = JRES ? s.nefc : row0 + 32;
-#pragma unroll 1
-      for (; k < nq; ++k) {
-        const int r = s.ids[k];
-        if (r >= row1) break;
-        const float Dr = s.Dsm[r];
-        const float* Jr = Jt + (r - row0) * s.ldj;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) acc[q] = fmaf(Jr[ab[q] & 0xFFFF] * Dr, Jr[ab[q] >> 16], acc[q]);
-      }
-      if (JRES) break;
-      __syncwarp();
-    }
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const int sl = base + 32 * q + lane;
-      if (sl < nfac) s.N[sl] = acc[q], s.Hp[sl] = acc[q];
-    }
-  }
-  __syncwarp();
+  IMN_MARK(s, 18);
 }
 
 }  // namespace imn
