@@ -75,10 +75,10 @@ typedef struct ImnModel {
   const int32_t* M_mulm_col;
   const int32_t* M_mulm_madr;
   /* the same rows dealt to 32 lanes for the fused kernel, built once per model by the
-   * host layer: [n_mulm_batches][32][4] words col | madr << 16, four entries of one
-   * row per (batch, lane).  A row starts with a batch of its own; in the batch that
-   * ends it bits 8-10 of word 0 hold the entries used (1 to 4) and bits 8-14 of word 1
-   * the dof; bits 8-10 of word 0 are 0 in every other batch.                   */
+   * host layer: [n_mulm_batches + 1][32][4] words 4 col | 4 madr << 16 (byte offsets), four
+   * entries of one row per (batch, lane).  A row starts with a batch of its own; its last
+   * batch is filled up with col = nv (a zero behind the vector) and bit 9 of word 0 is
+   * set.  Bits 9-15 of word 1 hold the row's dof.  The last batch is only prefetched.  */
   const uint32_t* M_mulm_lanes;
   /* constants that live in the upstream solver module                         */
   float alpha_noise_eps;          /* solver._ALPHA_NOISE_EPS                    */
@@ -177,6 +177,22 @@ typedef struct ImnSparsePlan {
   const uint32_t* fsweep;
   const uint32_t* bsweep;
   int32_t nfsweep, nbsweep;
+  /* What the fused kernel reads: the sweeps once more with every operand as a byte offset
+   * from N[0] (1/D starts up4(nslots) floats behind N), one record per (step, lane).  A
+   * sweep is as many steps as its entry with the most runs has runs; sweeps that neither
+   * have a term nor a diagonal entry are left out.
+   *   fstep [nfstep + 1][32][4]: {a | b << 16, d | slot << 16, terms | diagonal's 1/D << 16
+   *     (0: not a diagonal), flags}; a, b, d start at the lane's own first term of the run and
+   *     advance by the team width; flags bit 0 = the lane stores the entry, bit 1 = last step
+   *     of its level, bits 2-4 = log2(team), bit 5 = last step of its sweep, bit 6 = a
+   *     lane of the sweep holds a diagonal entry, bits 8-15 = most terms of a lane.
+   *   bstep [nbsweep + 1][32][2]: {slot | source's right-hand side << 16, source's 1/D |
+   *     destination's right-hand side << 16}; bit 0 of word 0 = the lane has work, of
+   *     word 1 = last of its level.
+   * The spare record at the end of both is only prefetched.  */
+  const uint32_t* fstep;
+  const uint32_t* bstep;
+  int32_t nfstep;
 } ImnSparsePlan;
 
 /* Solver context: the arrays mujoco_warp's `_create_solver_context` allocates

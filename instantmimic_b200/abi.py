@@ -116,6 +116,10 @@ SPARSE_TABLES = (
 )
 
 
+# the same sweeps with every operand as a byte offset (uint32; sparse_hessian.pack_steps)
+SPARSE_STEPS = ("fstep", "bstep")
+
+
 class ImnSparsePlan(C.Structure):
     _fields_ = [
         ("nv", I32),
@@ -127,7 +131,7 @@ class ImnSparsePlan(C.Structure):
         ("nentries", I32),
         ("nruns", I32),
         ("nback", I32),
-    ] + [(name, P) for name, _ in SPARSE_TABLES] + [("nfsweep", I32), ("nbsweep", I32)]
+    ] + [(name, P) for name, _ in SPARSE_TABLES] + [("nfsweep", I32), ("nbsweep", I32)] + [(name, P) for name in SPARSE_STEPS] + [("nfstep", I32)]
 
 
 class ImnCtx(C.Structure):

@@ -128,7 +128,7 @@ def model_struct(m: Any) -> abi.ImnModel:
     s.M_mulm_col = addr(m.M_mulm_col)
     s.M_mulm_madr = addr(m.M_mulm_madr)
     lanes = _mulm_lanes(m)
-    s.M_mulm_lanes, s.n_mulm_batches = addr(lanes), int(shape(lanes)[0])
+    s.M_mulm_lanes, s.n_mulm_batches = addr(lanes), int(shape(lanes)[0]) - 1
     s.alpha_noise_eps = eps
     s.overflow_iterations = ovf_it
     s.overflow_ls_iterations = ovf_ls

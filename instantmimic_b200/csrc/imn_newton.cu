@@ -77,13 +77,13 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   g.nM = m.nM;
   g.bd = m.nv_pad >= 64 ? 64 : 32;
   g.jrows = resident ? d.njmax : 32;
-  g.nv4 = up4(m.nv);
+  g.nv4 = up4(m.nv + 1);  // M_mulm_lanes reads a zero behind a vector
   g.r4 = up4(d.njmax);
   int o = 0;
   g.oBar = o, o += 4;
   // a streamed tile may start up to three floats into its buffer and end on a 16-byte boundary
   // a dense block reads up to three floats past a row; the gathered rows are up4(nv) floats apart
-  g.oJ = o, o += (resident ? up4(g.jrows * g.ldj + 3) : max(up4(32 * g.ldj) + 8, 32 * g.nv4));
+  g.oJ = o, o += (resident ? up4(g.jrows * g.ldj + 3) : max(up4(32 * g.ldj) + 8, 32 * up4(m.nv)));
   // dense: H and its factor share one (nv+1) x ldu array; sparse plan: packed H | N | 1/D
   g.oA = o, o += sp ? up4(sp->nfac) + up4(sp->nslots) + up4(m.nv) : (m.nv + 1) * g.ldu;
   // dof vectors; the dense factor needs two more (forward-solve scratch, 1 / pivot)
@@ -235,6 +235,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         }
 #pragma unroll 1
         for (int i = lane; i < nv; i += 32) s.search[i] = 0.0f, s.mv[i] = 0.0f, s.grad[i] = 0.0f;
+        if (lane == 0) s.search[nv] = 0.0f, s.qacc[nv] = 0.0f;
 #pragma unroll 1
         for (int i = lane; i <= nv; i += 32) s.uni[i] = 0;
         // bounded wait for the copies; when it runs out the copies get one more bounded wait
@@ -381,13 +382,13 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
           if (first || quad_count > 0) {
             sp_load_rhs(sp, s.N, s.grad, lane);
             IMN_MARK(s, 1);
-            sp_factor_sweeps(sp, s.N, s.iD, lane);
+            sp_factor_steps(sp, s.N, lane);
             IMN_MARK(s, 2);
           } else {
             sp_forward(sp, s.N, s.iD, s.grad, lane);
             IMN_MARK(s, 3);
           }
-          sp_backward_sweeps(sp, s.N, s.iD, s.grad, s.search, s.bd, lane, search_dot, decrement);
+          sp_backward_steps(sp, s.N, s.iD, s.grad, s.search, s.bd, lane, search_dot, decrement);
           IMN_MARK(s, 4);
         } else {
           factor_solve(s, first || quad_count > 0, search_dot, decrement);
@@ -601,7 +602,7 @@ static int validate(const ImnModel* m, const ImnData* d, const ImnCtx* cx) {
     if (!sp->lvl_ptr || !sp->lvl_team || !sp->ent_slot || !sp->ent_col || !sp->run_ptr || !sp->run_ab ||
         !sp->run_kl || !sp->orig || !sp->b_lvl || !sp->b_slot || !sp->b_src || !sp->b_dst || !sp->pair ||
         !sp->f_lvl || !sp->f_row || !sp->row_start || !sp->rk_ptr || !sp->rk || !sp->pmask || !sp->s_a ||
-        !sp->s_b || !sp->s_m || !sp->fsweep || !sp->bsweep || sp->nfsweep <= 0 || sp->nbsweep < 0)
+        !sp->s_b || !sp->s_m || !sp->fstep || !sp->bstep || sp->nfstep <= 0 || sp->nbsweep < 0)
       return set_error("imn_solve: a sparse plan table is NULL"), IMN_ERR_NULL;
   }
   return IMN_OK;

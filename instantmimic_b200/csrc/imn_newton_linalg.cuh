@@ -191,19 +191,16 @@ __device__ __forceinline__ void products(const World& s, const float* v, float* 
     const uint4* prog = reinterpret_cast<const uint4*>(s.mulm_lanes) + lane;
     uint4 p = __ldg(prog);
     float acc = 0.0f;
+    const auto M = [&](uint32_t w) { return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(s.M) + (w >> 16))); };
+    const auto V = [&](uint32_t w) { return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(v) + (w & 0x1FCu)); };
 #pragma unroll 1
-    for (int b = 1; b <= s.mulm_batches; ++b) {
-      const uint4 nxt = __ldg(prog + 32 * min(b, s.mulm_batches - 1));
-      const float m0 = __ldg(s.M + (p.x >> 16)), m1 = __ldg(s.M + (p.y >> 16)), m2 = __ldg(s.M + (p.z >> 16)),
-                  m3 = __ldg(s.M + (p.w >> 16));
-      const float a0 = fmaf(m0, v[p.x & 0x7F], acc), a1 = fmaf(m1, v[p.y & 0x7F], a0),
-                  a2 = fmaf(m2, v[p.z & 0x7F], a1), a3 = fmaf(m3, v[p.w & 0x7F], a2);
-      const int used = (p.x >> 8) & 7;  // 0: the row goes on
-      acc = a3;
-      if (used) {
-        outM[(p.y >> 8) & 0x7F] = used == 1 ? a0 : used == 2 ? a1 : used == 3 ? a2 : a3;
-        acc = 0.0f;
-      }
+    for (int b = s.mulm_batches; b > 0; --b) {
+      prog += 32;
+      const uint4 nxt = __ldg(prog);
+      const float m0 = M(p.x), m1 = M(p.y), m2 = M(p.z), m3 = M(p.w);
+      acc = fmaf(m3, V(p.w), fmaf(m2, V(p.z), fmaf(m1, V(p.y), fmaf(m0, V(p.x), acc))));
+      outM[(p.y >> 9) & 0x7F] = acc;  // stored with every batch of the row: no branch, and the last one stays
+      if (p.x & 0x200u) acc = 0.0f;
       p = nxt;
     }
   }

@@ -111,7 +111,7 @@ extern "C" int imn_sparse_plan_create(const ImnSparsePlan* host, ImnSparsePlan**
   if (!host || !out) return imn::set_error("imn_sparse_plan_create: NULL argument"), IMN_ERR_NULL;
   *out = nullptr;
   if (host->nv <= 0 || host->nfac <= 0 || host->nlevels <= 0 || host->nentries <= 0 || host->nruns < 0 ||
-      host->nback < 0 || host->nfsweep < 0 || host->nbsweep < 0 || !host->rk_ptr)
+      host->nback < 0 || host->nfsweep < 0 || host->nbsweep < 0 || host->nfstep < 0 || !host->rk_ptr)
     return imn::set_error("imn_sparse_plan_create: malformed plan"), IMN_ERR_SHAPE;
   const int nv = host->nv, words = (nv + 31) / 32;
   const size_t nrk = host->rk_ptr[nv] > 0 ? host->rk_ptr[nv] : 1;
@@ -133,6 +133,8 @@ extern "C" int imn_sparse_plan_create(const ImnSparsePlan* host, ImnSparsePlan**
       TAB(f_row, nv), TAB(row_start, nv), TAB(rk_ptr, nv + 1), TAB(rk, nrk), TAB(pmask, nv * words),
       TAB(s_a, host->nfac), TAB(s_b, host->nfac), TAB(s_m, host->nfac), TAB(gat, host->nfac),
       TAB(fsweep, (size_t)host->nfsweep * 128), TAB(bsweep, (size_t)host->nbsweep * 32),
+      TAB(fstep, host->nfstep > 0 ? ((size_t)host->nfstep + 1) * 128 : 0),
+      TAB(bstep, host->nfstep > 0 ? ((size_t)host->nbsweep + 1) * 64 : 0),
   };
 #undef TAB
   size_t total = 0;

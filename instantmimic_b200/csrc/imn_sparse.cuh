@@ -62,48 +62,63 @@ __device__ __forceinline__ void sp_factor_levels(const ImnSparsePlan& P, float* 
   }
 }
 
-// The same factorisation driven by the per-(sweep, lane) records (ImnSparsePlan::
-// fsweep): one 128-bit load gives a lane its entry, the entry's first run and the
-// sweep's team width, and the next sweep's record is fetched while the current one is
-// worked on, so no table load sits on the dependent path.  The term loop is kept
-// rolled: taking terms in groups of four or two (loads first) was measured 2-4 % slower
-// on the whole kernel, which is bound by instruction fetch.
-__device__ __forceinline__ float sp_run_terms(const float* N, const float* iD, uint32_t ab, uint32_t kl, int tl,
-                                              int T, float v) {
-  const float* pa = N + (ab & 0xFFFFu);
-  const float* pb = N + (ab >> 16);
-  const float* pd = iD + (kl & 0xFFFFu);
-  const int len = (int)(kl >> 16);
-  int t = tl;
-#pragma unroll 1
-  for (; t < len; t += T) v = fmaf(pa[t] * pb[t], pd[t], v);
-  return v;
+// The same factorisation driven by the step records (ImnSparsePlan::fstep): one 128-bit load,
+// issued a step ahead, gives a lane its run of terms and its entry as byte offsets from N[0], so
+// that a term costs its three reads, two multiplications and a predicate.  Teams of one lane, where
+// most terms are, take four terms per trip with constant offsets between them; reads past a lane's
+// last term stay inside the world's shared memory and are not added.  (A lane that took the terms
+// of its run one by one from scaled indices spent 180 cycles per term step: 34-dof humanoid, 8192
+// worlds, 15 k cycles per factorisation.)
+__device__ __forceinline__ float sp_at(const float* N, uint32_t offset) {
+  return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(N) + offset);
 }
-
-__device__ __forceinline__ void sp_factor_sweeps(const ImnSparsePlan& P, float* N, float* iD, int lane) {
-  const uint4* tab = reinterpret_cast<const uint4*>(P.fsweep) + lane;
-  const int ns = P.nfsweep;
+__device__ __forceinline__ void sp_factor_steps(const ImnSparsePlan& P, float* N, int lane) {
+  const uint4* tab = reinterpret_cast<const uint4*>(P.fstep) + lane;
   uint4 cur = __ldg(tab);
+  float v = 0.0f;
 #pragma unroll 1
-  for (int s = 0; s < ns; ++s) {
-    const uint4 nxt = __ldg(tab + 32 * min(s + 1, ns - 1));
-    const uint32_t fl = cur.w;
-    const int T = 1 << ((fl >> 2) & 7), tl = lane & (T - 1);
-    const bool has = (fl & 1u) != 0u;
-    float v = 0.0f;
-    if (has) {
-      v = sp_run_terms(N, iD, cur.y, cur.z, tl, T, v);
-      const int extra = (fl >> 8) & 0xFF, r0 = fl >> 16;
+  for (int s = P.nfstep; s > 0; --s) {
+    tab += 32;
+    const uint4 nxt = __ldg(tab);
+    const uint32_t fl = cur.w, slot = cur.y >> 16;
+    uint32_t a = cur.x & 0xFFFFu, b = cur.x >> 16, d = cur.y & 0xFFFFu;
+    int cnt = (int)(cur.z & 0xFFFFu);
+    const float start = sp_at(N, slot);
+    int left = (int)((fl >> 8) & 0xFFu);
+    if ((fl & 0x1Cu) == 0u) {
 #pragma unroll 1
-      for (int r = r0; r < r0 + extra; ++r) v = sp_run_terms(N, iD, __ldg(P.run_ab + r), __ldg(P.run_kl + r), tl, T, v);
+      for (; left > 0; left -= 4, cnt -= 4, a += 16, b += 16, d += 16) {
+        float p[4], q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) p[k] = sp_at(N, a + 4 * k) * sp_at(N, b + 4 * k), q[k] = sp_at(N, d + 4 * k);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (cnt > k) v = fmaf(p[k], q[k], v);
+      }
+    } else {
+      const uint32_t stride = 4u << ((fl >> 2) & 7u);
+#pragma unroll 1
+      for (; left > 0; left -= 2, cnt -= 2) {
+        const float p0 = sp_at(N, a) * sp_at(N, b), q0 = sp_at(N, d);
+        a += stride, b += stride, d += stride;
+        const float p1 = sp_at(N, a) * sp_at(N, b), q1 = sp_at(N, d);
+        a += stride, b += stride, d += stride;
+        if (cnt > 0) v = fmaf(p0, q0, v);
+        if (cnt > 1) v = fmaf(p1, q1, v);
+      }
     }
+    if (fl & 32u) {
+      const int T = 1 << ((fl >> 2) & 7u);
 #pragma unroll 1
-    for (int off = T >> 1; off > 0; off >>= 1) v = v + __shfl_down_sync(IMN_FULL_MASK, v, off, T);
-    if (has && tl == 0) {
-      const int sl = cur.x & 0xFFFF, col = (int)(cur.x >> 16) - 1;
-      const float w = N[sl] - v;
-      N[sl] = w;
-      if (col >= 0) iD[col] = 1.0f / w;
+      for (int off = T >> 1; off > 0; off >>= 1) v = v + __shfl_down_sync(IMN_FULL_MASK, v, off, T);
+      const float w = start - v;
+      if (fl & 1u) *reinterpret_cast<float*>(reinterpret_cast<char*>(N) + slot) = w;
+      if (fl & 64u) {
+        const uint32_t diag = cur.z >> 16;
+        const float inv = 1.0f / (diag ? w : 1.0f);
+        if (diag) *reinterpret_cast<float*>(reinterpret_cast<char*>(N) + diag) = inv;
+      }
+      v = 0.0f;
     }
     if (fl & 2u) __syncwarp();
     cur = nxt;
@@ -170,21 +185,22 @@ __device__ __forceinline__ void sp_backward(const ImnSparsePlan& P, float* N, co
   __syncwarp();
 }
 
-// sp_backward driven by the per-(sweep, lane) records (ImnSparsePlan::bsweep).
-__device__ __forceinline__ void sp_backward_sweeps(const ImnSparsePlan& P, float* N, const float* iD,
-                                                   const float* grad, float* search, int bd, int lane,
-                                                   float& sum0, float& sum1) {
-  const int rhs = P.nfac, n = P.nv, ns = P.nbsweep;
-  const uint32_t* tab = P.bsweep + lane;
-  uint32_t cur = ns ? __ldg(tab) : 0u;
+// sp_backward driven by the step records (ImnSparsePlan::bstep).
+__device__ __forceinline__ void sp_backward_steps(const ImnSparsePlan& P, float* N, const float* iD,
+                                                  const float* grad, float* search, int bd, int lane,
+                                                  float& sum0, float& sum1) {
+  const int rhs = P.nfac, n = P.nv;
+  const uint2* tab = reinterpret_cast<const uint2*>(P.bstep) + lane;
+  uint2 cur = __ldg(tab);
 #pragma unroll 1
-  for (int s = 0; s < ns; ++s) {
-    const uint32_t nxt = __ldg(tab + 32 * min(s + 1, ns - 1));
-    if (cur & (1u << 30)) {
-      const int i = (cur >> 16) & 0x7F, j = (cur >> 23) & 0x7F;
-      N[rhs + j] = fmaf(-N[cur & 0xFFFFu], N[rhs + i] * iD[i], N[rhs + j]);
-    }
-    if (cur >> 31) __syncwarp();
+  for (int s = P.nbsweep; s > 0; --s) {
+    tab += 32;
+    const uint2 nxt = __ldg(tab);
+    const uint32_t to = cur.y >> 16;
+    const float x = sp_at(N, cur.x >> 16) * sp_at(N, cur.y & 0xFFFCu);
+    const float r = fmaf(-sp_at(N, cur.x & 0xFFFCu), x, sp_at(N, to));
+    if (cur.x & 1u) *reinterpret_cast<float*>(reinterpret_cast<char*>(N) + to) = r;
+    if (cur.y & 1u) __syncwarp();
     cur = nxt;
   }
   float ra = 0.0f, rb = 0.0f;

@@ -47,6 +47,7 @@ class SparseHessianPlan:
     nfac: int
     tables: dict = field(repr=False)
     adjacency: list = field(repr=False)
+    steps: dict = field(default_factory=dict, repr=False)  # the fused kernel's step records (pack_steps)
     struct: Any = field(default=None, repr=False)
     device_tables: Any = field(default=None, repr=False)
 
@@ -364,6 +365,7 @@ def build_plan(m: Any, body_groups: Sequence[Sequence[int]], block: int, path: s
     return SparseHessianPlan(
         nv=nv, nv_pad=nv_pad, block=block, nslots=nslots, nterms=nterms, levels=len(levels),
         density=nfac / (nv * (nv + 1) / 2), path=path, nfac=nfac, tables=tables, adjacency=adj,
+        steps=pack_steps(tables, nv, nfac) if path == "fused" else {},
     )
 
 
@@ -413,6 +415,55 @@ def _pack_sweeps(raw: dict) -> tuple[list[int], list[int]]:
     return fs, bs
 
 
+def pack_steps(t: dict, nv: int, nfac: int) -> dict:
+    """The sweep records with every operand as a byte offset from N[0] and one record per run
+    of terms (layout in include/imnewton.h): the kernel neither scales indices nor looks further
+    runs up, and sweeps without a term or a diagonal entry, which change nothing, are dropped."""
+    rec = t["fsweep"].astype(np.int64).reshape(-1, 32, 4)
+    run_ab, run_kl = t["run_ab"].astype(np.int64), t["run_kl"].astype(np.int64)
+    inv0 = (nfac + nv + 3) // 4 * 4  # 1/D behind N
+    if 4 * (inv0 + nv) >= 1 << 16:
+        raise ValueError("sparse plan exceeds the step records' 16-bit byte offsets")
+    flags = rec[..., 3]
+    team = 1 << ((flags >> 2) & 7)
+    tl = np.arange(32) % team
+    has, col, slot = (flags & 1) == 1, (rec[..., 0] >> 16) - 1, rec[..., 0] & 0xFFFF
+    diag = has & (col >= 0) & (tl == 0)
+    extra, r0 = np.where(has, (flags >> 8) & 0xFF, 0), flags >> 16
+    ends_level = (flags[:, 0] & 2).astype(np.int64)
+    # step d of a sweep: the d-th run of every lane's entry
+    depth = 1 + int(extra.max(initial=0))
+    out = np.zeros((rec.shape[0], depth, 32, 4), np.int64)
+    for d in range(depth):
+        if d == 0:
+            ab, kl = rec[..., 1], np.where(has, rec[..., 2], 0)
+        else:
+            at = np.minimum(r0 + d - 1, max(run_ab.size - 1, 0))
+            ab, kl = run_ab[at], np.where(extra >= d, run_kl[at], 0)
+        terms = np.maximum(0, -(-((kl >> 16) - tl) // team))
+        some = terms > 0
+        out[:, d, :, 0] = np.where(some, 4 * ((ab & 0xFFFF) + tl) | 4 * ((ab >> 16) + tl) << 16, 0)
+        out[:, d, :, 1] = np.where(some, 4 * (inv0 + (kl & 0xFFFF) + tl), 0) | 4 * slot << 16
+        out[:, d, :, 2] = terms | np.where(diag, 4 * (inv0 + col), 0) << 16
+        out[:, d, :, 3] = (has & (tl == 0)) | (flags & 0x1C) | terms.max(axis=1)[:, None] << 8
+    steps = []
+    for s in range(rec.shape[0]):
+        n = 1 + int(extra[s].max(initial=0))
+        if n == 1 and not diag[s].any() and not (out[s, 0, 0, 3] >> 8):
+            if steps and ends_level[s]:
+                steps[-1][:, 3] |= 2
+            continue
+        out[s, n - 1, :, 3] |= 32 | ends_level[s] | (64 if diag[s].any() else 0)
+        steps += list(out[s, :n])
+    b = t["bsweep"].astype(np.int64).reshape(-1, 32)
+    src, dst, work = (b >> 16) & 0x7F, (b >> 23) & 0x7F, ((b >> 30) & 1) == 1
+    back = np.zeros((b.shape[0] + 1, 32, 2), np.int64)
+    back[:-1, :, 0] = np.where(work, 4 * (b & 0xFFFF) | 4 * (nfac + src) << 16 | 1, 0)
+    back[:-1, :, 1] = np.where(work, 4 * (inv0 + src) | 4 * (nfac + dst) << 16, 0) | (b >> 31)
+    pack = lambda a: (a & 0xFFFFFFFF).astype(np.uint32).reshape(-1)  # noqa: E731
+    return {"fstep": pack(np.stack(steps + [np.zeros((32, 4), np.int64)])), "bstep": pack(back), "nfstep": len(steps)}
+
+
 def plan_struct(plan: SparseHessianPlan, arrays: dict) -> abi.ImnSparsePlan:
     """C-ABI struct over ``arrays`` (host numpy for the oracle, device tensors for CUDA)."""
     st = abi.ImnSparsePlan()
@@ -427,11 +478,14 @@ def plan_struct(plan: SparseHessianPlan, arrays: dict) -> abi.ImnSparsePlan:
     st.nbsweep = int(plan.tables["bsweep"].shape[0]) // 32
     if not st.nfsweep:
         st.fsweep = st.bsweep = None
+    for name in abi.SPARSE_STEPS:
+        setattr(st, name, addr(arrays.get(name)))
+    st.nfstep = int(plan.steps.get("nfstep", 0))
     return st
 
 
 def host_struct(plan: SparseHessianPlan) -> abi.ImnSparsePlan:
-    return plan_struct(plan, plan.tables)
+    return plan_struct(plan, {**plan.tables, **plan.steps})
 
 
 def upload(plan: SparseHessianPlan, device: Any = "cuda") -> SparseHessianPlan:
@@ -439,8 +493,7 @@ def upload(plan: SparseHessianPlan, device: Any = "cuda") -> SparseHessianPlan:
     import torch
 
     dev = {}
-    for name, _ in abi.SPARSE_TABLES:
-        t = plan.tables[name]
+    for name, t in [(n, plan.tables[n]) for n, _ in abi.SPARSE_TABLES] + [(n, plan.steps[n]) for n in abi.SPARSE_STEPS if plan.steps]:
         # torch has no uint16/uint32 arithmetic types; ship the raw bytes
         dev[name] = torch.from_numpy(t.view(np.uint8).copy()).to(device)
     plan.device_tables = dev
@@ -459,7 +512,7 @@ class NativePlan:
         from .. import _lib
 
         host = host_struct(plan)
-        self._keep = plan.tables  # the host tables must outlive the call only
+        self._keep = (plan.tables, plan.steps)  # the host tables must outlive the call only
         out = C.POINTER(abi.ImnSparsePlan)()
         _lib.check(_lib.lib().imn_sparse_plan_create(C.byref(host), C.byref(out)), "imn_sparse_plan_create")
         self._ptr = out

@@ -209,29 +209,31 @@ def mulm_tables(rowadr, rownnz, colind, nv: int):
 
 
 def mulm_lane_program(rowadr, col, madr, nv: int) -> np.ndarray:
-    """The M_mulm rows dealt to the 32 lanes of a warp: (batches, 32, 4) words
-    ``col | madr << 16`` (layout in include/imnewton.h, ``M_mulm_lanes``).  Rows go longest
-    first to the lane with the fewest batches so far, so the program is hardly longer than
-    its longest row although nv may exceed 32."""
+    """The M_mulm rows dealt to the 32 lanes of a warp: (batches + 1, 32, 4) words (layout in
+    include/imnewton.h, ``M_mulm_lanes``).  Rows go longest first to the lane with the fewest
+    batches so far, so the program is hardly longer than its longest row although nv may
+    exceed 32."""
     rowadr = np.asarray(rowadr, dtype=np.int64)
     col = np.asarray(col, dtype=np.int64)
     madr = np.asarray(madr, dtype=np.int64)
-    if nv > 128 or (madr.size and madr.max() >= 1 << 16):
-        return np.zeros((1, 32, 4), np.int32)  # outside the fused path
+    if nv > 127 or (madr.size and madr.max() >= 1 << 14):
+        return np.zeros((2, 32, 4), np.int32)  # outside the fused path
     lanes: list[list[list[int]]] = [[] for _ in range(32)]
     for i in sorted(range(nv), key=lambda i: (rowadr[i] - rowadr[i + 1], i)):
         lane = min(range(32), key=lambda q: len(lanes[q]))
         k0, k1 = int(rowadr[i]), int(rowadr[i + 1])
-        words = [int(col[k]) | int(madr[k]) << 16 for k in range(k0, k1)]
+        words = [4 * int(col[k]) | 4 * int(madr[k]) << 16 for k in range(k0, k1)]
+        idle = 4 * nv | (4 * int(madr[k1 - 1]) << 16 if k1 > k0 else 0)
         for at in range(0, max(len(words), 1), 4):
             batch = words[at:at + 4]
-            used = len(batch)
-            batch += [0] * (4 - used)
-            if at + 4 >= len(words):
-                batch[0] |= used << 8
-                batch[1] |= i << 8
+            batch += [idle] * (4 - len(batch))
+            batch[0] |= (at + 4 >= len(words)) << 9
+            batch[1] |= i << 9
             lanes[lane].append(batch)
-    out = np.zeros((max(len(q) for q in lanes), 32, 4), np.int64)
+    # a lane that is done goes on with a row of zeros that ends up behind the vector
+    out = np.zeros((max(len(q) for q in lanes) + 1, 32, 4), np.int64)
+    out[:, :] = [4 * nv] * 4
+    out[:, :, 1] |= nv << 9
     for lane, program in enumerate(lanes):
         for b, batch in enumerate(program):
             out[b, lane] = batch
