@@ -843,7 +843,7 @@ def main():
             "solver": {
                 "niter_mean": float(niter.mean()),
                 "niter_max": int(niter.max()),
-                "smem_bytes_per_world": int(info.smem_bytes),
+                "smem_bytes_per_world": int(info.smem_bytes) // int(info.worlds_per_cta),
                 "line_search_passes_mean": float(stats[:, 0].mean()),
                 "factorisations_mean": float(stats[:, 2].mean()),
             },

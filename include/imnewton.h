@@ -240,6 +240,11 @@ typedef struct ImnCtx {
                          * (summed over iterations), [2] factorisations (the initial
                          * one included), [3] full gradient evaluations (the initial
                          * one included)                                          */
+  int32_t* work_counter; /* optional scratch (1), no counterpart in the reference: hands the
+                         * worlds that do not fit the GPU at once to the first warp that
+                         * is free; without it every warp takes a fixed share.  Solves that
+                         * may overlap need counters of their own, as they need contexts
+                         * of their own                                           */
 } ImnCtx;
 
 /* Tree-structured L'DL plan (tree_ldl.py:47-57, 105-170) as an instruction

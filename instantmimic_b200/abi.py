@@ -161,6 +161,7 @@ class ImnCtx(C.Structure):
         ("sparse_plan", C.POINTER(ImnSparsePlan)),
         ("world_order", P),
         ("stats", P),
+        ("work_counter", P),
     ]
 
 

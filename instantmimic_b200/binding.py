@@ -257,6 +257,7 @@ def ctx_struct(d_struct: abi.ImnData, ctx: Any, nsolving: Any, sparse_plan_struc
     if stats is not None and (tuple(shape(stats)) != (d_struct.nworld, 4) or elem_strides(stats) != (4, 1)):
         raise ValueError("ctx.stats must be a contiguous (nworld, 4) int32 array")
     s.stats = addr(stats)
+    s.work_counter = addr(get("work_counter"))
     return s
 
 

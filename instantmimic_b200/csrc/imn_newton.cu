@@ -55,6 +55,10 @@ struct Geom {
   int jrows;  // rows of J held in shared memory (njmax when resident, else 32)
   // offsets in 4-byte words; every region starts on a 16-byte boundary
   int oBar, oJ, oA, oVec, nv4, oRowF, oRowI, oMask, mwords, r4, oUni, total;
+  // tables in shared memory (Tables), in words from its start; the worlds' slices (`total` words
+  // each, offsets above) follow at `tab` words.  warps: worlds in hand per CTA
+  bool tsm;
+  int tM, tF, tB, tS, tO, tab, warps;
   // polls a copy wait may take before the world gives up, and the failure-path test
   // switch: when set no bulk copy is issued (plain loads bring the data) while the
   // barrier is told to expect bytes, so the wait runs out with nothing in flight
@@ -65,6 +69,12 @@ struct Geom {
 static int g_wait_polls = 1 << 22;
 static int g_withhold_copies = 0;
 
+
+// Largest dynamic shared memory one CTA may opt into on sm_100 (227 KB).
+static const int kMaxSmem = 227 * 1024;
+// Most warps (worlds in hand) of a CTA: bounds the registers at 128 with a resident J, 168 with a
+// streamed one, whose worlds take more shared memory and are fewer.
+static const int kResidentWarps = 16, kStreamedWarps = 12;
 
 static inline int up4(int n) { return (n + 3) & ~3; }
 
@@ -94,6 +104,15 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   g.oMask = o, o += g.mwords * g.r4;
   g.oUni = o, o += up4(m.nv + 1);
   g.total = o;
+  int t = 0;
+  g.tM = t, t += (m.n_mulm_batches + 1) * 128;
+  g.tF = t, t += sp ? (sp->nfstep + 1) * 128 : 0;
+  g.tB = t, t += sp ? (sp->nbsweep + 1) * 64 : 0;
+  g.tS = t, t += sp ? up4(sp->nfac) : 0;
+  g.tO = t, t += sp ? up4(m.nv) : 0;
+  // tables stay in global memory when they would take more than a third of an SM's shared memory
+  g.tsm = 4 * t <= kMaxSmem / 3;
+  g.tab = g.tsm ? t : 0;
   g.wait_polls = g_wait_polls;
   g.withhold_copies = g_withhold_copies;
   return g;
@@ -108,16 +127,22 @@ __device__ __noinline__ void warn_limit(int which, unsigned limit) {
     printf("solver iterations limit reached - please increase iterations to %u\n", limit);
 }
 
-// One warp solves one world: the CTA's.  The solve is written as one loop whose trip is
-// "take the world if none is in hand, else run one pass of it" rather than as a load
-// followed by a pass loop: the same statements, but the compiler lays the single loop
-// out better (measured: 0.836 -> 0.796 ms per 8192 humanoid worlds at the same
+// A CTA holds `warps` worlds in hand, a warp each, and as many CTAs as there are SMs share the batch:
+// every table of the model and the plan then exists once per SM in shared memory.  Read from global
+// memory by one-world CTAs the tables cost about 210 cycles per trip of the loops they drive,
+// whatever the distance of the prefetch.  The warps of a CTA never wait for one another after the
+// tables have arrived.  A warp's first world is number warp * grid + CTA of the launch order, further
+// ones come from a counter.
+// The solve is written as one loop whose trip is "take a world if none is in hand, else run one
+// pass of it" rather than as a load followed by a pass loop: the same statements, but the compiler
+// lays the single loop out better (measured: 0.836 -> 0.796 ms per 8192 humanoid worlds at the same
 // occupancy).
-template <bool JRES, bool SPARSE, bool STATS>
+template <bool JRES, bool SPARSE, bool STATS, bool TSM>
 __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& d, const ImnCtx& cx, const Geom& g,
                                               const ImnSparsePlan& sp) {
-  extern __shared__ __align__(16) float smem[];
-  const int lane = threadIdx.x;
+  extern __shared__ __align__(16) float smem_all[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* smem = smem_all + g.tab + warp * g.total;
   const int nv = g.nv, R = g.njmax, nv4 = g.nv4, r4 = g.r4;
 
   void* bar = smem + g.oBar;
@@ -143,7 +168,18 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
   s.ids = s.state + r4;
   s.frows = s.ids + r4;  // rows with a nonzero force, ascending
   s.uni = reinterpret_cast<int*>(smem + g.oUni);
-  s.mulm_lanes = m.M_mulm_lanes, s.mulm_batches = m.n_mulm_batches;
+  s.mulm_batches = m.n_mulm_batches;
+  if (TSM) {
+    s.tab.mulm = reinterpret_cast<const uint4*>(smem_all + g.tM);
+    s.tab.fstep = reinterpret_cast<const uint4*>(smem_all + g.tF);
+    s.tab.bstep = reinterpret_cast<const uint2*>(smem_all + g.tB);
+    s.tab.slots = reinterpret_cast<const uint32_t*>(smem_all + g.tS);
+    s.tab.orig = reinterpret_cast<const uint32_t*>(smem_all + g.tO);
+  } else {
+    s.tab.mulm = reinterpret_cast<const uint4*>(m.M_mulm_lanes);
+    s.tab.fstep = reinterpret_cast<const uint4*>(sp.fstep);
+    s.tab.bstep = reinterpret_cast<const uint2*>(sp.bstep);
+  }
   s.M_rowadr = m.M_rowadr, s.M_rownnz = m.M_rownnz, s.M_colind = m.M_colind;
   s.jbar = bar;
   s.jphase = reinterpret_cast<int*>(smem + g.oBar) + 2;  // the barrier itself takes two words
@@ -155,8 +191,29 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
   s.Jbeg = d.efc_J;
   s.Jend = d.efc_J + (d.J_world_offset ? (size_t)d.J_elems
                                        : (size_t)(d.nworld - 1) * d.J_ld_world + (size_t)d.njmax * d.J_ld_row);
-  if (lane == 0) mbar_init(bar, 1);
+  if (lane == 0) mbar_init(bar, 1), *s.jphase = 0;
   __syncwarp();
+  if (TSM) {
+    auto stage = [&](int at, const void* src, int words) {
+#pragma unroll 1
+      for (int i = threadIdx.x; i < words / 4; i += blockDim.x)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_all + at + 4 * i)),
+                     "l"(static_cast<const uint4*>(src) + i)
+                     : "memory");
+    };
+    stage(g.tM, m.M_mulm_lanes, (m.n_mulm_batches + 1) * 128);
+    if (SPARSE) {
+      stage(g.tF, sp.fstep, (sp.nfstep + 1) * 128);
+      stage(g.tB, sp.bstep, (sp.nbsweep + 1) * 64);
+#pragma unroll 4
+      for (int i = threadIdx.x; i < sp.nfac; i += blockDim.x)
+        reinterpret_cast<uint32_t*>(smem_all + g.tS)[i] =
+            4u * __ldg(sp.s_a + i) | (4u * __ldg(sp.s_b + i)) << 9 | (uint32_t)(__ldg(sp.s_m + i) + 1) << 18;
+      for (int i = threadIdx.x; i < nv; i += blockDim.x) reinterpret_cast<uint32_t*>(smem_all + g.tO)[i] = __ldg(sp.orig + i);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+  }
 
   PROF_DECL;
   // the world in hand
@@ -171,15 +228,22 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
   int st_passes = 0, st_flips = 0, st_factor = 0, st_grad = 0;  // work counters (ctx.stats)
   bool have = false, first = true;
   bool outside = false;  // a row of the world leaves the sparse plan's pattern
-  bool taken = false;  // this CTA's world was taken
+  int idx = warp * (int)gridDim.x + (int)blockIdx.x;  // the next world's place in the launch order
+  bool turn = false;  // the first world was taken
 
 #pragma unroll 1
   for (;;) {
-    if (!have && !taken) {
-      // ---- take the world ------------------------------------------------------------
-      taken = true;
+    if (!have) {
+      // ---- take a world --------------------------------------------------------------
+      if (turn && cx.work_counter) {
+        if (lane == 0) idx = (int)gridDim.x * g.warps + atomicAdd(cx.work_counter, 1);
+        idx = __shfl_sync(IMN_FULL_MASK, idx, 0);
+      } else if (turn) {
+        idx += (int)gridDim.x * g.warps;
+      }
+      turn = true;
+      if (idx >= d.nworld) break;
       {
-        const int idx = (int)blockIdx.x;
         w = cx.world_order ? cx.world_order[idx] : idx;
         s.world = w;
         s.viol = (SPARSE && cx.hfactor) ? cx.hfactor + ((size_t)w + 1) * m.nv_pad * m.nv_pad - 1 : nullptr;
@@ -208,8 +272,13 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
             {s.qacc, q0 + dofo, nv},
             {s.qfs, d.qfrc_smooth + dofo, nv},
         };
+        __syncwarp();  // every lane has left the previous world
+        const uint32_t load_phase = (uint32_t)*s.jphase;
+        // the previous world's values were written through the generic proxy
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
         if (lane == 0) {
-          *s.jphase = 1;  // phase 0 is the load below
+          *s.jphase = (int)(load_phase ^ 1u);
           *s.jfail = 0;
         }
         __syncwarp();
@@ -239,15 +308,19 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
 #pragma unroll 1
         for (int i = lane; i <= nv; i += 32) s.uni[i] = 0;
         // bounded wait for the copies; when it runs out the copies get one more bounded wait
-        // (they write this CTA's shared memory, which the SM hands to the next CTA once
-        // this one is gone), then the world is left unsolved with the time-out bit set
+        // (they write shared memory that the warp's next world takes over), then the world is left
+        // unsolved with the time-out bit set and the barrier starts anew
         bool arrived = false;
 #pragma unroll 1
-        for (int tries = 0; tries < g.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(bar, 0);
+        for (int tries = 0; tries < g.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(bar, load_phase);
         if (!arrived) {
 #pragma unroll 1
-          for (int tries = 0; tries < g.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(bar, 0);
-          if (lane == 0) d.overflow[w] |= IMN_OVERFLOW_COPY_TIMEOUT;
+          for (int tries = 0; tries < g.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(bar, load_phase);
+          if (lane == 0) {
+            d.overflow[w] |= IMN_OVERFLOW_COPY_TIMEOUT;
+            mbar_restart(bar, 1);
+            *s.jphase = 0;
+          }
         } else {
           have = true, first = true;
           search_dot = 0.0f, grad_dot = 0.0f, grad_scale = 1.0f, decrement = 0.0f;
@@ -263,7 +336,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         PROF(0);
       }
     }
-    if (!have) break;
+    if (!have) continue;
 
     // Pass 0 is the initialisation (newton_fusion.py:431-472): Jaref = J qacc - aref,
     // Ma = M qacc, row states, gradient, full Hessian, factor, first search direction.
@@ -273,7 +346,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
       // one call site: Ma = M qacc, Jaref = J qacc - aref on pass 0; mv = M search,
       // jv = J search afterwards
       if (first || !search_unchanged)
-        products<JRES>(s, first ? s.qacc : s.search, first ? s.Ma : s.mv, first ? s.Jaref : s.jv,
+        products<JRES, TSM>(s, first ? s.qacc : s.search, first ? s.Ma : s.mv, first ? s.Jaref : s.jv,
                        first ? s.jv : nullptr);
       __syncwarp();
       PROF(5);
@@ -371,7 +444,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
             outside = __any_sync(IMN_FULL_MASK, bad);
           }
           if (SPARSE)
-            hessian_sparse<JRES>(s, quad_count, first, outside, sp);
+            hessian_sparse<JRES, TSM>(s, quad_count, first, outside, sp);
           else
             hessian_dense<JRES>(s, quad_count, first);
         }
@@ -380,15 +453,15 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
           // refactor the packed H, or solve with the resident factor
           // (sparse_hessian.py:490-547)
           if (first || quad_count > 0) {
-            sp_load_rhs(sp, s.N, s.grad, lane);
+            sp_load_rhs<TSM>(sp, s.tab, s.N, s.grad, lane);
             IMN_MARK(s, 1);
-            sp_factor_steps(sp, s.N, lane);
+            sp_factor_steps<TSM>(sp, s.tab, s.N, lane);
             IMN_MARK(s, 2);
           } else {
             sp_forward(sp, s.N, s.iD, s.grad, lane);
             IMN_MARK(s, 3);
           }
-          sp_backward_steps(sp, s.N, s.iD, s.grad, s.search, s.bd, lane, search_dot, decrement);
+          sp_backward_steps<TSM>(sp, s.tab, s.N, s.iD, s.grad, s.search, s.bd, lane, search_dot, decrement);
           IMN_MARK(s, 4);
         } else {
           factor_solve(s, first || quad_count > 0, search_dot, decrement);
@@ -403,7 +476,11 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         bool arrived = false;
 #pragma unroll 1
         for (int tries = 0; tries < g.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(bar, parity);
-        if (lane == 0) d.overflow[w] |= IMN_OVERFLOW_COPY_TIMEOUT;
+        if (lane == 0) {
+          d.overflow[w] |= IMN_OVERFLOW_COPY_TIMEOUT;
+          mbar_restart(bar, 1);
+          *s.jphase = 0;
+        }
         finished = true, failed = true;
         break;
       }
@@ -502,34 +579,32 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
   PROF_FLUSH;
 }
 
-// Two entry points over the same body.  With J resident shared memory limits the worlds
-// per SM to about 14 at the humanoid's shapes; the register bound is set to match
-// (14 one-warp CTAs per SM: 144 registers, no spills).  Measured per 8192 humanoid worlds
-// with this bound at 1 (148 registers, one warp fewer per SM) 0.902 ms, 12: 0.899,
-// 13: 0.795, 14: 0.797, 15: 0.800, 16: 0.803.  The streamed variants hold more worlds per
-// SM in shared memory than an uncapped register count would allow, so theirs is capped at
-// 128 (16 warps per SM).
-// STATS compiles the work counters of ImnCtx.stats in: four more live values in a
-// kernel that is short of registers cost 9 % of its speed (measured), so the counting
-// variants run only for callers that pass the stats array.
-#ifndef IMN_RESIDENT_MIN_BLOCKS
-#define IMN_RESIDENT_MIN_BLOCKS 14
-#endif
-template <bool SPARSE, bool STATS>
-__global__ void __launch_bounds__(32, IMN_RESIDENT_MIN_BLOCKS) newton_kernel_resident(const ImnModel m, const ImnData d, const ImnCtx cx,
-                                                                   const Geom g, const ImnSparsePlan sp) {
-  newton_worlds<true, SPARSE, STATS>(m, d, cx, g, sp);
+// Two entry points over the same body, with the register bounds that follow from the most worlds
+// in hand (kResidentWarps, kStreamedWarps).
+// STATS compiles the work counters of ImnCtx.stats in: four more live values in a kernel that is
+// short of registers cost 9 % of its speed (measured), so the counting variants run only for
+// callers that pass the stats array.
+template <bool SPARSE, bool STATS, bool TSM>
+__global__ void __launch_bounds__(32 * kResidentWarps, 1)
+    newton_kernel_resident(const ImnModel m, const ImnData d, const ImnCtx cx, const Geom g, const ImnSparsePlan sp) {
+  newton_worlds<true, SPARSE, STATS, TSM>(m, d, cx, g, sp);
 }
-#ifndef IMN_STREAMED_MIN_BLOCKS
-#define IMN_STREAMED_MIN_BLOCKS 12
-#endif
+template <bool SPARSE, bool STATS, bool TSM>
+__global__ void __launch_bounds__(32 * kStreamedWarps, 1)
+    newton_kernel_streamed(const ImnModel m, const ImnData d, const ImnCtx cx, const Geom g, const ImnSparsePlan sp) {
+  newton_worlds<false, SPARSE, STATS, TSM>(m, d, cx, g, sp);
+}
+using Kernel = void (*)(ImnModel, ImnData, ImnCtx, Geom, ImnSparsePlan);
 template <bool SPARSE, bool STATS>
-__global__ void __launch_bounds__(32, IMN_STREAMED_MIN_BLOCKS) newton_kernel_streamed(const ImnModel m, const ImnData d, const ImnCtx cx,
-                                                                 const Geom g, const ImnSparsePlan sp) {
-  newton_worlds<false, SPARSE, STATS>(m, d, cx, g, sp);
+static Kernel newton_kernel(bool resident, bool tsm) {
+  return resident ? (tsm ? (Kernel)newton_kernel_resident<SPARSE, STATS, true> : (Kernel)newton_kernel_resident<SPARSE, STATS, false>)
+                  : (tsm ? (Kernel)newton_kernel_streamed<SPARSE, STATS, true> : (Kernel)newton_kernel_streamed<SPARSE, STATS, false>);
 }
 
-__global__ void fill_nsolving(int* nsolving, int value) { *nsolving = value; }
+__global__ void start_counters(int* nsolving, int* work_counter, int nworld) {
+  if (nsolving) *nsolving = nworld;
+  if (work_counter) *work_counter = 0;
+}
 
 // The hardware hands CTAs to SMs in index order and a world's solve time grows with
 // its row count, so worlds are launched by descending row count: the long solves
@@ -539,11 +614,12 @@ __global__ void fill_nsolving(int* nsolving, int value) { *nsolving = value; }
 // world is solved independently of which CTA takes it.
 #define IMN_ORDER_CLASSES 64
 __global__ void __launch_bounds__(1024) order_worlds_kernel(const int* __restrict__ nefc, int njmax, int nworld,
-                                                            int* __restrict__ order, int* nsolving) {
+                                                            int* __restrict__ order, int* nsolving, int* work_counter) {
   __shared__ int count[IMN_ORDER_CLASSES], start[IMN_ORDER_CLASSES];
   const int tid = threadIdx.x;
   if (tid < IMN_ORDER_CLASSES) count[tid] = 0;
   if (tid == 0 && nsolving) *nsolving = nworld;
+  if (tid == 0 && work_counter) *work_counter = 0;
   __syncthreads();
   // class 0 holds the largest row counts
   auto cls = [&](int n) {
@@ -560,8 +636,6 @@ __global__ void __launch_bounds__(1024) order_worlds_kernel(const int* __restric
   for (int w = tid; w < nworld; w += blockDim.x) order[atomicAdd(&start[cls(nefc[w])], 1)] = w;
 }
 
-// Largest dynamic shared memory one CTA may opt into on sm_100 (227 KB).
-static const int kMaxSmem = 227 * 1024;
 // Resident-J budget per world: keep at least 4 worlds per SM.
 static const int kResidentBudget = kMaxSmem / 4;
 
@@ -608,11 +682,16 @@ static int validate(const ImnModel* m, const ImnData* d, const ImnCtx* cx) {
   return IMN_OK;
 }
 
-// Worlds one SM holds at `bytes` of dynamic shared memory per one-warp CTA (1 KB is
-// reserved per CTA; `cap` is the register limit of the kernel variant).
-static int worlds_per_sm(int bytes, int cap = 16) {
-  const int n = (228 * 1024) / (bytes + 1024);
-  return n < cap ? n : cap;
+// Worlds one SM can have in hand.
+static int worlds_per_sm(const Geom& g, int most) {
+  const int n = (kMaxSmem - 4 * g.tab) / (4 * g.total);
+  return n < most ? n : most;
+}
+
+static int sm_count() {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+  return sms;
 }
 
 // J resident in shared memory or streamed through the 32-row tile.  Resident J is
@@ -621,19 +700,22 @@ static int worlds_per_sm(int bytes, int cap = 16) {
 // resident vs 16 streamed worlds per SM: resident 7 % faster; SNU-like (njmax 128) 4 vs
 // 7: streamed 1.22x faster; G1-like (njmax 250) 4 vs 11: streamed 1.6x faster.  Hence:
 // stream when it holds at least 1.6x the worlds.
-static int plan_launch(const ImnModel* m, const ImnData* d, const ImnSparsePlan* sp, Geom* g, bool* resident) {
+static int plan_launch(const ImnModel* m, const ImnData* d, const ImnSparsePlan* sp, Geom* g, bool* resident, int* grid) {
   const Geom gr = make_geom(*m, *d, true, sp);
   const Geom gs = make_geom(*m, *d, false, sp);
-  const bool fits = gr.total * 4 <= kResidentBudget;
-  if (fits && 10 * worlds_per_sm(gs.total * 4) < 16 * worlds_per_sm(gr.total * 4)) {
-    *g = gr, *resident = true;
-    return IMN_OK;
-  }
-  if (gs.total * 4 > kMaxSmem)
-    return set_error("imn_solve: njmax %d needs %d bytes of shared memory per world (max %d)", d->njmax,
-                     gs.total * 4, kMaxSmem),
+  const int nr = worlds_per_sm(gr, kResidentWarps), ns = worlds_per_sm(gs, kStreamedWarps);
+  const bool fits = gr.total * 4 <= kResidentBudget && nr >= 1;
+  *resident = fits && 10 * ns < 16 * nr;
+  *g = *resident ? gr : gs;
+  if (!*resident && ns < 1)
+    return set_error("imn_solve: njmax %d needs %d bytes of shared memory per world (max %d)", d->njmax, 4 * (gs.total + gs.tab),
+                     kMaxSmem),
            IMN_ERR_LIMIT;
-  *g = gs, *resident = false;
+  // one CTA per SM; a batch that does not fill the GPU is spread over all SMs
+  const int sms = sm_count(), most = *resident ? nr : ns, share = (d->nworld + sms - 1) / sms;
+  g->warps = share < 1 ? 1 : share < most ? share : most;
+  const int need = (d->nworld + g->warps - 1) / g->warps;
+  *grid = need < sms ? need : sms;
   return IMN_OK;
 }
 
@@ -663,13 +745,14 @@ extern "C" int imn_launch_info(const ImnModel* m, const ImnData* d, const ImnCtx
   if (rc) return rc;
   imn::Geom g;
   bool res;
-  rc = imn::plan_launch(m, d, cx->sparse_plan, &g, &res);
+  int grid = 0;
+  rc = imn::plan_launch(m, d, cx->sparse_plan, &g, &res, &grid);
   if (rc) return rc;
   out->world_threads = g.bd;
-  out->worlds_per_cta = 1;
-  out->smem_bytes = g.total * 4;
+  out->worlds_per_cta = g.warps;
+  out->smem_bytes = 4 * (g.tab + g.warps * g.total);
   out->j_resident = res ? 1 : 0;
-  out->grid = d->nworld;
+  out->grid = grid;
   return IMN_OK;
 }
 
@@ -680,35 +763,25 @@ extern "C" int imn_solve(const ImnModel* m, const ImnData* d, const ImnCtx* cx, 
   if (d->nworld == 0) return IMN_OK;
   imn::Geom g;
   bool res;
-  rc = imn::plan_launch(m, d, cx->sparse_plan, &g, &res);
+  int grid = 0;
+  rc = imn::plan_launch(m, d, cx->sparse_plan, &g, &res, &grid);
   if (rc) return rc;
-  const int bytes = g.total * 4;
-  using Kernel = void (*)(ImnModel, ImnData, ImnCtx, imn::Geom, ImnSparsePlan);
-  const bool sparse = cx->sparse_plan != nullptr;
+  const int bytes = 4 * (g.tab + g.warps * g.total);
+  const bool sparse = cx->sparse_plan != nullptr, stats = cx->stats != nullptr;
   const ImnSparsePlan sp = sparse ? *cx->sparse_plan : ImnSparsePlan{};
-  auto prepare = [](Kernel k, int smem) {
-    // many one-warp CTAs share an SM: ask for the largest shared-memory carve-out,
-    // otherwise the driver sizes it for a single CTA
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess && smem > 48 * 1024) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return e;
-  };
-  if (cx->world_order)
-    imn::order_worlds_kernel<<<1, 1024, 0, stream>>>(d->nefc, d->njmax, d->nworld, cx->world_order, cx->nsolving);
-  else if (cx->nsolving)
-    imn::fill_nsolving<<<1, 1, 0, stream>>>(cx->nsolving, d->nworld);
-
-  Kernel kern = sparse ? (res ? (Kernel)imn::newton_kernel_resident<true, false> : (Kernel)imn::newton_kernel_streamed<true, false>)
-                       : (res ? (Kernel)imn::newton_kernel_resident<false, false> : (Kernel)imn::newton_kernel_streamed<false, false>);
-  if (cx->stats)
-    kern = sparse ? (res ? (Kernel)imn::newton_kernel_resident<true, true> : (Kernel)imn::newton_kernel_streamed<true, true>)
-                  : (res ? (Kernel)imn::newton_kernel_resident<false, true> : (Kernel)imn::newton_kernel_streamed<false, true>);
+  const imn::Kernel kern = sparse ? (stats ? imn::newton_kernel<true, true>(res, g.tsm) : imn::newton_kernel<true, false>(res, g.tsm))
+                                  : (stats ? imn::newton_kernel<false, true>(res, g.tsm) : imn::newton_kernel<false, false>(res, g.tsm));
   {
-    const cudaError_t e = prepare(kern, bytes);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess && bytes > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess)
       return imn::set_error("imn_solve: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
-  kern<<<d->nworld, 32, bytes, stream>>>(*m, *d, *cx, g, sp);
+  if (cx->world_order)
+    imn::order_worlds_kernel<<<1, 1024, 0, stream>>>(d->nefc, d->njmax, d->nworld, cx->world_order, cx->nsolving, cx->work_counter);
+  else if (cx->nsolving || cx->work_counter)
+    imn::start_counters<<<1, 1, 0, stream>>>(cx->nsolving, cx->work_counter, d->nworld);
+  kern<<<grid, 32 * g.warps, bytes, stream>>>(*m, *d, *cx, g, sp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return imn::set_error("imn_solve: launch failed: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;

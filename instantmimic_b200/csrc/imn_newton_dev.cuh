@@ -15,6 +15,11 @@ __device__ __forceinline__ void mbar_init(void* bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
+// a barrier whose phase is unknown (its copies did not arrive) starts anew
+__device__ __forceinline__ void mbar_restart(void* bar, int count) {
+  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+  mbar_init(bar, count);
+}
 __device__ __forceinline__ void mbar_expect_tx(void* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");

@@ -37,7 +37,7 @@ struct World {
   int* jphase;
   int* jfail;
   int wait_polls, withhold_copies;
-  const uint32_t* mulm_lanes;  // ImnModel::M_mulm_lanes
+  Tables tab;
   int mulm_batches;
   const int *M_rowadr, *M_rownnz, *M_colind;
   // sparse plan only: packed H, N = L D with the carried row, 1/D, the world's
@@ -177,7 +177,7 @@ __device__ __forceinline__ void write_union(const World& s, int count) {
 // outM = M v over the symmetric rows (newton_fusion.py:171-176) and
 // outJ[r] = J[r,:] v (- minus[r]): one running sum per row; above 50 dofs in
 // 20-dof partials joined by plain adds (newton_stages.py:157-174).
-template <bool JRES>
+template <bool JRES, bool TSM>
 __device__ __forceinline__ void products(const World& s, const float* v, float* outM, float* outJ,
                                          const float* minus) {
   const int lane = s.lane, nv = s.nv;
@@ -188,15 +188,15 @@ __device__ __forceinline__ void products(const World& s, const float* v, float* 
   // reads of M, and dofs past 32 took a second round (34-dof model, 8192 worlds: 7000 -> 5900 cycles
   // of the world's warp per product; 56-dof model, 4096 worlds: 1745 -> 1669 us per solve).
   {
-    const uint4* prog = reinterpret_cast<const uint4*>(s.mulm_lanes) + lane;
-    uint4 p = __ldg(prog);
+    const uint4* prog = s.tab.mulm + lane;
+    uint4 p = tab_at<TSM>(prog);
     float acc = 0.0f;
     const auto M = [&](uint32_t w) { return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(s.M) + (w >> 16))); };
     const auto V = [&](uint32_t w) { return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(v) + (w & 0x1FCu)); };
 #pragma unroll 1
     for (int b = s.mulm_batches; b > 0; --b) {
       prog += 32;
-      const uint4 nxt = __ldg(prog);
+      const uint4 nxt = tab_at<TSM>(prog);
       const float m0 = M(p.x), m1 = M(p.y), m2 = M(p.z), m3 = M(p.w);
       acc = fmaf(m3, V(p.w), fmaf(m2, V(p.z), fmaf(m1, V(p.y), fmaf(m0, V(p.x), acc))));
       outM[(p.y >> 9) & 0x7F] = acc;  // stored with every batch of the row: no branch, and the last one stays
@@ -381,7 +381,7 @@ __device__ __noinline__ void count_violations(bool first, const float* Jw, int l
 // tables are read coalesced once per call, a slot costs four instructions per row, and no pair list
 // of touched dofs has to be formed and looked up.  `outside`: the world has a row whose dofs do not
 // all lie in the pattern.  Sums of a list that does not fit one tile wait in N.
-template <bool JRES>
+template <bool JRES, bool TSM>
 __device__ __forceinline__ void hessian_sparse(const World& s, int count, bool first, bool outside, const ImnSparsePlan& SP) {
   const int lane = s.lane, nv = s.nv, nfac = SP.nfac;
   constexpr int Q = JRES ? 10 : 12;
@@ -400,20 +400,20 @@ __device__ __forceinline__ void hessian_sparse(const World& s, int count, bool f
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const int sl = min(base + 32 * q + lane, nfac - 1);
-        a[q] = __ldg(SP.s_a + sl), b[q] = __ldg(SP.s_b + sl);
-        acc[q] = 0.0f;
-        if (t0 > 0) {
-          acc[q] = s.N[sl];
-        } else if (first) {
-          const int e = __ldg(SP.s_m + sl);
-          if (e >= 0) acc[q] = __ldg(s.M + e);
+        int e;
+        if (TSM) {
+          const uint32_t w = s.tab.slots[sl];
+          a[q] = w & 0x1FC, b[q] = (w >> 9) & 0x1FC, e = (int)(w >> 18) - 1;
+        } else {
+          a[q] = 4 * __ldg(SP.s_a + sl), b[q] = 4 * __ldg(SP.s_b + sl), e = first ? __ldg(SP.s_m + sl) : -1;
         }
+        acc[q] = t0 > 0 ? s.N[sl] : first && e >= 0 ? __ldg(s.M + e) : 0.0f;
       }
 #pragma unroll 1
       for (int t = t0; t < t1; ++t) {
         const ListRow row = list_row<JRES>(s, t, t0);
 #pragma unroll
-        for (int q = 0; q < Q; ++q) acc[q] = fmaf(row.J[a[q]] * row.D, row.J[b[q]], acc[q]);
+        for (int q = 0; q < Q; ++q) acc[q] = fmaf(sp_at(row.J, a[q]) * row.D, sp_at(row.J, b[q]), acc[q]);
       }
 #pragma unroll
       for (int q = 0; q < Q; ++q) {

@@ -15,6 +15,30 @@
 
 namespace imn {
 
+// The model's and the plan's tables as the fused kernel reads them.  TSM: copies in shared memory,
+// one per CTA (slots: 4 a | 4 b << 9 | (entry of M + 1) << 18; orig widened); else the arrays of
+// ImnModel / ImnSparsePlan in global memory, slots and orig through the plan.
+struct Tables {
+  const uint4 *mulm, *fstep;
+  const uint2* bstep;
+  const uint32_t *slots, *orig;
+};
+template <bool TSM, class T>
+__device__ __forceinline__ T tab_at(const T* p) {
+  return TSM ? *p : __ldg(p);
+}
+template <bool TSM>
+__device__ __forceinline__ int tab_orig(const Tables& tab, const ImnSparsePlan& P, int j) {
+  return TSM ? (int)tab.orig[j] : (int)__ldg(P.orig + j);
+}
+
+// N[rhs + j] = grad[dof of elimination index j]
+template <bool TSM>
+__device__ __forceinline__ void sp_load_rhs(const ImnSparsePlan& P, const Tables& tab, float* N, const float* grad, int lane) {
+#pragma unroll 1
+  for (int j = lane; j < P.nv; j += 32) N[P.nfac + j] = grad[tab_orig<TSM>(tab, P, j)];
+  __syncwarp();
+}
 // N[rhs + j] = grad[dof of elimination index j]
 __device__ __forceinline__ void sp_load_rhs(const ImnSparsePlan& P, float* N, const float* grad, int lane) {
 #pragma unroll 1
@@ -72,14 +96,15 @@ __device__ __forceinline__ void sp_factor_levels(const ImnSparsePlan& P, float* 
 __device__ __forceinline__ float sp_at(const float* N, uint32_t offset) {
   return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(N) + offset);
 }
-__device__ __forceinline__ void sp_factor_steps(const ImnSparsePlan& P, float* N, int lane) {
-  const uint4* tab = reinterpret_cast<const uint4*>(P.fstep) + lane;
-  uint4 cur = __ldg(tab);
+template <bool TSM>
+__device__ __forceinline__ void sp_factor_steps(const ImnSparsePlan& P, const Tables& tables, float* N, int lane) {
+  const uint4* tab = tables.fstep + lane;
+  uint4 cur = tab_at<TSM>(tab);
   float v = 0.0f;
 #pragma unroll 1
   for (int s = P.nfstep; s > 0; --s) {
     tab += 32;
-    const uint4 nxt = __ldg(tab);
+    const uint4 nxt = tab_at<TSM>(tab);
     const uint32_t fl = cur.w, slot = cur.y >> 16;
     uint32_t a = cur.x & 0xFFFFu, b = cur.x >> 16, d = cur.y & 0xFFFFu;
     int cnt = (int)(cur.z & 0xFFFFu);
@@ -186,16 +211,17 @@ __device__ __forceinline__ void sp_backward(const ImnSparsePlan& P, float* N, co
 }
 
 // sp_backward driven by the step records (ImnSparsePlan::bstep).
-__device__ __forceinline__ void sp_backward_steps(const ImnSparsePlan& P, float* N, const float* iD,
+template <bool TSM>
+__device__ __forceinline__ void sp_backward_steps(const ImnSparsePlan& P, const Tables& tables, float* N, const float* iD,
                                                   const float* grad, float* search, int bd, int lane,
                                                   float& sum0, float& sum1) {
   const int rhs = P.nfac, n = P.nv;
-  const uint2* tab = reinterpret_cast<const uint2*>(P.bstep) + lane;
-  uint2 cur = __ldg(tab);
+  const uint2* tab = tables.bstep + lane;
+  uint2 cur = tab_at<TSM>(tab);
 #pragma unroll 1
   for (int s = P.nbsweep; s > 0; --s) {
     tab += 32;
-    const uint2 nxt = __ldg(tab);
+    const uint2 nxt = tab_at<TSM>(tab);
     const uint32_t to = cur.y >> 16;
     const float x = sp_at(N, cur.x >> 16) * sp_at(N, cur.y & 0xFFFCu);
     const float r = fmaf(-sp_at(N, cur.x & 0xFFFCu), x, sp_at(N, to));
@@ -209,7 +235,7 @@ __device__ __forceinline__ void sp_backward_steps(const ImnSparsePlan& P, float*
     float s0 = 0.0f, s1 = 0.0f;
 #pragma unroll 1
     for (int j = lane + 32 * w; j < n; j += bd) {
-      const int d = __ldg(P.orig + j);
+      const int d = tab_orig<TSM>(tables, P, j);
       const float v = N[rhs + j] * iD[j];
       search[d] = -v;
       s0 = fmaf(v, v, s0);

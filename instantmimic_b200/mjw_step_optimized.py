@@ -49,6 +49,8 @@ class SolverContext:
         self.sparse_hessian_plan = None
         # scratch of the fused kernel: worlds ordered by row count (no counterpart upstream)
         self.world_order = i(W)
+        # and the counter from which its warps take further worlds
+        self.work_counter = i(1)
         # work counters of each world's solve (passes, flips, factorisations, gradients);
         # counting costs the kernel ~9 %, so the array exists only on request
         self.stats = i(W, 4) if with_stats else None
@@ -156,7 +158,7 @@ def log_kernel_selection(m: Any, d: Any, scratch: "OptimizedFwdPositionScratch")
                                         cache_on=scratch).launch_info()
         parts.append(
             f"solve: fused Newton kernel, J {'resident in shared memory' if info.j_resident else 'streamed in 32-row tiles'}, "
-            f"{info.smem_bytes} B shared memory per world, {caps['hessian_factor']}")
+            f"{info.smem_bytes // info.worlds_per_cta} B shared memory per world, {caps['hessian_factor']}")
     else:
         parts.append("solve: outside the fused path")
     parts.append(f"M factor/solve: {caps['m_factor_solve']}")
