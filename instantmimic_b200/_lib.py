@@ -44,15 +44,47 @@ def check(rc: int, what: str) -> None:
 def current_stream_handle(stream=None) -> int:
     """cudaStream_t of ``stream`` (torch stream, int, or None = torch's current)."""
     if stream is None:
-        import torch
-
-        return int(torch.cuda.current_stream().cuda_stream)
+        return _current_stream()
     if isinstance(stream, int):
         return stream
     return int(stream.cuda_stream)
 
 
+def _slow_current_stream() -> int:
+    import torch
+
+    return int(torch.cuda.current_stream().cuda_stream)
+
+
+def _current_stream() -> int:
+    """torch's current stream as a plain number; replaces itself at the first call, by the
+    accessor that builds no stream object where torch has it."""
+    global _current_stream
+    import torch
+
+    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    first = _slow_current_stream()  # initialises CUDA, and is what the fast accessor has to agree with
+    if raw is not None and device is not None and int(raw(device())) == first:
+        _current_stream = lambda: raw(device())  # noqa: E731
+    else:
+        _current_stream = _slow_current_stream
+    return first
+
+
 _NVTX = None
+
+
+def nvtx_enabled() -> bool:
+    """Whether C-ABI calls are wrapped in NVTX ranges (``IMN_NVTX=1``)."""
+    if _NVTX is None:
+        nvtx("")
+    return _NVTX is not _no_range
+
+
+def _no_range(name: str):
+    import contextlib
+
+    return contextlib.nullcontext()
 
 
 def nvtx(name: str):
@@ -62,7 +94,6 @@ def nvtx(name: str):
     (src/instantmimic/utils/mjw_step_optimized.py:2683, utils/warp_kernels.py:11-14)."""
     global _NVTX
     if _NVTX is None:
-        import contextlib
         import os
 
         if os.environ.get("IMN_NVTX", "0") not in ("", "0"):
@@ -70,5 +101,5 @@ def nvtx(name: str):
 
             _NVTX = torch.cuda.nvtx.range
         else:
-            _NVTX = lambda name: contextlib.nullcontext()  # noqa: E731
+            _NVTX = _no_range
     return _NVTX(name)

@@ -17,7 +17,7 @@ from typing import Any
 
 import numpy as np
 
-from .. import _lib, abi
+from .. import abi, calls
 from ..arrays import addr, elem_strides, is_contiguous, to_host
 
 # Small blocked tiles avoid the long dependency chain of a full-matrix tile
@@ -106,22 +106,17 @@ def create_blocked_dense_factor_solve_scratch(
 
 
 def _launch(scratch, M, y, U, x, active, nworld, rhs_count, mode, stream):
-    for name, a in (("y", y), ("x", x), ("U", U)):
-        if not is_contiguous(a):
-            raise ValueError(f"blocked dense factor/solve needs a contiguous {name}")
-    with _lib.nvtx("imn_blocked_dense_factor_solve"):
-        rc = _launch_call(scratch, M, y, U, x, active, nworld, rhs_count, mode, stream)
-    _lib.check(rc, "imn_blocked_dense_factor_solve")
+    def build():
+        for name, a in (("y", y), ("x", x), ("U", U)):
+            if not is_contiguous(a):
+                raise ValueError(f"blocked dense factor/solve needs a contiguous {name}")
+        return (C.byref(scratch.struct), addr(M) if M is not None else None, elem_strides(M)[0] if M is not None else 0,
+                addr(y), addr(U), addr(x), addr(active), int(nworld), int(rhs_count), int(mode)), None
 
-
-def _launch_call(scratch, M, y, U, x, active, nworld, rhs_count, mode, stream):
-    return _lib.lib().imn_blocked_dense_factor_solve(
-        C.byref(scratch.struct),
-        addr(M) if M is not None else None,
-        elem_strides(M)[0] if M is not None else 0,
-        addr(y), addr(U), addr(x), addr(active), int(nworld), int(rhs_count), int(mode),
-        _lib.current_stream_handle(stream),
-    )
+    buffers = tuple(a for a in (M, y, U, x, active) if a is not None)
+    # factor and solve-only calls are prepared side by side
+    calls.call(scratch, "imn_blocked_dense_factor_solve", buffers, (M is None, active is None, nworld, rhs_count, mode), build,
+               stream, slot=mode)
 
 
 def blocked_dense_factor_solve(

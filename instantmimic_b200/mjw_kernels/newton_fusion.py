@@ -10,7 +10,7 @@ from __future__ import annotations
 import ctypes as C
 from typing import Any
 
-from .. import _lib, abi, binding, types
+from .. import _lib, abi, binding, calls, types
 from ..arrays import is_device
 
 # CTAs per SM requested from the compiler for the reference's Warp kernel
@@ -113,6 +113,7 @@ class SolveCall:
         self.plan_struct = getattr(plan, "struct", None) if plan is not None and plan.path == "fused" else None
         self.c = binding.ctx_struct(self.d, ctx, nsolving, self.plan_struct)
         self.key = _key(m, d, ctx, nsolving)
+        self.args = (C.byref(self.m), C.byref(self.d), C.byref(self.c))
 
     def launch_info(self) -> abi.ImnLaunchInfo:
         info = abi.ImnLaunchInfo()
@@ -123,42 +124,56 @@ class SolveCall:
         return info
 
     def __call__(self, stream=None) -> None:
-        with _lib.nvtx("imn_solve"):
-            rc = _lib.lib().imn_solve(
-                C.byref(self.m), C.byref(self.d), C.byref(self.c), _lib.current_stream_handle(stream)
-            )
-        _lib.check(rc, "imn_solve")
+        if _lib.nvtx_enabled():
+            with _lib.nvtx("imn_solve"):
+                rc = _lib.lib().imn_solve(*self.args, _lib.current_stream_handle(stream))
+        else:
+            rc = _lib.lib().imn_solve(*self.args, _lib.current_stream_handle(stream))
+        if rc:
+            _lib.check(rc, "imn_solve")
 
 
 _KEY_DATA = ("nefc", "ne", "nf", "qacc_smooth", "qacc_warmstart", "qfrc_smooth", "M", "qacc",
-             "qfrc_constraint", "solver_niter", "overflow")
-_KEY_EFC = ("J", "D", "aref", "frictionloss", "force", "state", "Ma", "J_world_offset")
+             "qfrc_constraint", "solver_niter", "overflow", "efc.J", "efc.D", "efc.aref", "efc.frictionloss", "efc.force",
+             "efc.state", "efc.Ma")
 _KEY_CTX = ("Jaref", "jv", "search", "mv", "grad", "h", "hfactor", "quad_changed_ids", "newton_dof_union",
             "world_order", "stats", "work_counter") + binding._CTX_WORLD_ARRAYS
+_KEY_SCALARS = ("nv", "nv_pad", "is_sparse", "opt.iterations", "opt.ls_iterations", "opt.disableflags", "opt.solver",
+                "opt.integrator", "opt.cone", "block_dim.linesearch_iterative")
+_data, _ctx, _scalars = calls.getter(*_KEY_DATA), calls.getter(*_KEY_CTX), calls.getter(*_KEY_SCALARS)
+_options = calls.getter("opt.tolerance", "opt.ls_tolerance", "stat.meaninertia")
+
+
+def _ctx_arrays(ctx) -> tuple:
+    try:
+        return _ctx(ctx)
+    except AttributeError:
+        return tuple(getattr(ctx, n, None) for n in _KEY_CTX)
 
 
 def _key(m, d, ctx, nsolving):
     """Everything the cached structs were built from: the address of every buffer the
-    kernel is handed and the scalar options.  A caller that rebinds any of them gets
-    fresh structs instead of stale pointers."""
-    from ..arrays import addr
-
-    plan = getattr(ctx, "sparse_hessian_plan", None)
+    kernel is handed, the scalar options, and what ``eligible`` looks at.  A caller that rebinds
+    any of them gets fresh structs instead of stale pointers."""
     return (
-        id(m), id(d), id(ctx), id(plan), addr(nsolving),
-        tuple(addr(getattr(d, n)) for n in _KEY_DATA),
-        tuple(addr(getattr(d.efc, n, None)) for n in _KEY_EFC),
-        tuple(addr(getattr(ctx, n, None)) for n in _KEY_CTX),
-        addr(m.opt.tolerance), addr(m.opt.ls_tolerance), addr(m.stat.meaninertia),
-        int(m.opt.iterations), int(m.opt.ls_iterations), int(m.opt.disableflags),
-        int(getattr(m.opt, "warn_overflow", 0) or 0), int(d.nworld), int(d.njmax),
+        id(m), id(d), id(ctx), id(getattr(ctx, "sparse_hessian_plan", None)),
+        calls.pointers(_data(d)),
+        calls.optional_pointers(_ctx_arrays(ctx) + (nsolving, getattr(d.efc, "J_world_offset", None))),
+        calls.pointers(_options(m)), _scalars(m), getattr(m.opt, "warn_overflow", 0), d.nworld, d.njmax,
     )
+
+
+def cached_call(m: Any, d: Any, ctx: Any, nsolving: Any, holder: Any) -> SolveCall | None:
+    """The holder's prepared call when it was built from exactly these buffers and options (which
+    then also passed ``eligible``)."""
+    call = getattr(holder, "_imn_solve_call", None)
+    return call if call is not None and call.key == _key(m, d, ctx, nsolving) else None
 
 
 def solve_call(m: Any, d: Any, ctx: Any, nsolving: Any, cache_on: Any = None) -> SolveCall:
     holder = cache_on if cache_on is not None else ctx
-    call = getattr(holder, "_imn_solve_call", None)
-    if call is None or call.key != _key(m, d, ctx, nsolving):
+    call = cached_call(m, d, ctx, nsolving, holder)
+    if call is None:
         call = SolveCall(m, d, ctx, nsolving)
         try:
             holder._imn_solve_call = call

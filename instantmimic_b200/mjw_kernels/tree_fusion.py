@@ -25,7 +25,7 @@ from typing import Any
 
 import numpy as np
 
-from .. import _lib, abi, binding
+from .. import abi, binding, calls
 from ..arrays import addr, device_of, elem_strides, is_contiguous, is_device, length, shape, to_host
 
 
@@ -148,17 +148,29 @@ def _row_ld(a: Any) -> int:
     return elem_strides(a)[0]
 
 
+# what each stage's structs are built from: the model's tables, the scratch's, the batch's buffers
+_TREE = calls.getter("bodies", "offsets", "child_ptr", "child_ids")
+_TREE_DOFS = calls.getter("body_parentid", "body_dofadr", "body_dofnum", "dof_bodyid", "dof_parentid")
+_CRB_MODEL = calls.getter("body_parentid", "body_dofadr", "body_dofnum", "dof_bodyid", "dof_parentid", "dof_armature",
+                          "M_hinit_i", "M_colind")
+_CRB_DATA = calls.getter("cinert", "cdof", "crb", "M")
+_RNE_MODEL = calls.getter("body_parentid", "body_dofadr", "body_dofnum", "dof_bodyid", "dof_parentid", "opt.gravity")
+_RNE_DATA = calls.getter("cinert", "cvel", "cdof", "cdof_dot", "qvel", "cacc", "cfrc_int", "qfrc_bias")
+
+
 def accumulate(m: Any, d: Any, values: Any, components: int, skip_root_parent: bool, scratch: TreeReductionScratch,
                stream=None) -> None:
     """values[:, parent] += values[:, body], deepest level first (tree_fusion.py:138-170)."""
     _need(scratch, "accumulate")
-    nbody = length(m.body_parentid)
-    ptr = _per_body(values, d.nworld, nbody, components, "values")
-    with _lib.nvtx("imn_body_tree_accumulate"):
-        rc = _lib.lib().imn_body_tree_accumulate(
-            C.byref(tree_struct(m, scratch)), ptr, nbody * components, int(components), int(bool(skip_root_parent)),
-            int(d.nworld), _lib.current_stream_handle(stream))
-    _lib.check(rc, "imn_body_tree_accumulate")
+
+    def build():
+        nbody = length(m.body_parentid)
+        ptr = _per_body(values, d.nworld, nbody, components, "values")
+        t = tree_struct(m, scratch)
+        return (C.byref(t), ptr, nbody * components, int(components), int(bool(skip_root_parent)), int(d.nworld)), t
+
+    calls.call(d, "imn_body_tree_accumulate", (m.body_parentid, values, *_TREE(scratch)),
+               (components, skip_root_parent, d.nworld, scratch.levels), build, stream)
 
 
 def subtree_com_accumulate(m: Any, d: Any, scratch: TreeReductionScratch | None = None, stream=None) -> None:
@@ -169,26 +181,29 @@ def subtree_com_accumulate(m: Any, d: Any, scratch: TreeReductionScratch | None 
 def crb(m: Any, d: Any, scratch: TreeReductionScratch | None = None, stream=None) -> None:
     """d.crb and d.M from d.cinert and d.cdof (tree_fusion.py:186-206)."""
     _need(scratch, "crb")
-    nbody = length(m.body_parentid)
-    t = tree_struct(m, scratch, dofs=True, inertia=True)
-    with _lib.nvtx("imn_crb"):
-        rc = _lib.lib().imn_crb(
-            C.byref(t), _per_body(d.cinert, d.nworld, nbody, 10, "d.cinert"),
-            _per_body(d.cdof, d.nworld, m.nv, 6, "d.cdof"), _per_body(d.crb, d.nworld, nbody, 10, "d.crb"),
-            addr(d.M), _row_ld(d.M), int(d.nworld), _lib.current_stream_handle(stream))
-    _lib.check(rc, "imn_crb")
+
+    def build():
+        nbody = length(m.body_parentid)
+        t = tree_struct(m, scratch, dofs=True, inertia=True)
+        return (C.byref(t), _per_body(d.cinert, d.nworld, nbody, 10, "d.cinert"),
+                _per_body(d.cdof, d.nworld, m.nv, 6, "d.cdof"), _per_body(d.crb, d.nworld, nbody, 10, "d.crb"),
+                addr(d.M), _row_ld(d.M), int(d.nworld)), t
+
+    calls.call(d, "imn_crb", _CRB_MODEL(m) + _TREE(scratch) + _CRB_DATA(d), (m.nv, d.nworld, scratch.levels), build, stream)
 
 
 def rne(m: Any, d: Any, scratch: TreeReductionScratch | None = None, stream=None) -> None:
     """d.cacc, d.cfrc_int and d.qfrc_bias (tree_fusion.py:209-222)."""
     _need(scratch, "rne")
-    nbody = length(m.body_parentid)
-    t = tree_struct(m, scratch, dofs=True, gravity=True)
-    with _lib.nvtx("imn_rne"):
-        rc = _lib.lib().imn_rne(
-            C.byref(t), _per_body(d.cinert, d.nworld, nbody, 10, "d.cinert"),
-            _per_body(d.cvel, d.nworld, nbody, 6, "d.cvel"), _per_body(d.cdof, d.nworld, m.nv, 6, "d.cdof"),
-            _per_body(d.cdof_dot, d.nworld, m.nv, 6, "d.cdof_dot"), addr(d.qvel), _row_ld(d.qvel),
-            _per_body(d.cacc, d.nworld, nbody, 6, "d.cacc"), _per_body(d.cfrc_int, d.nworld, nbody, 6, "d.cfrc_int"),
-            addr(d.qfrc_bias), _row_ld(d.qfrc_bias), int(d.nworld), _lib.current_stream_handle(stream))
-    _lib.check(rc, "imn_rne")
+
+    def build():
+        nbody = length(m.body_parentid)
+        t = tree_struct(m, scratch, dofs=True, gravity=True)
+        return (C.byref(t), _per_body(d.cinert, d.nworld, nbody, 10, "d.cinert"),
+                _per_body(d.cvel, d.nworld, nbody, 6, "d.cvel"), _per_body(d.cdof, d.nworld, m.nv, 6, "d.cdof"),
+                _per_body(d.cdof_dot, d.nworld, m.nv, 6, "d.cdof_dot"), addr(d.qvel), _row_ld(d.qvel),
+                _per_body(d.cacc, d.nworld, nbody, 6, "d.cacc"), _per_body(d.cfrc_int, d.nworld, nbody, 6, "d.cfrc_int"),
+                addr(d.qfrc_bias), _row_ld(d.qfrc_bias), int(d.nworld)), t
+
+    calls.call(d, "imn_rne", _RNE_MODEL(m) + _TREE(scratch) + _RNE_DATA(d),
+               (m.nv, d.nworld, scratch.levels, m.opt.disableflags), build, stream)

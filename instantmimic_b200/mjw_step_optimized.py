@@ -17,7 +17,7 @@ from typing import Any, Sequence
 
 import numpy as np
 
-from . import _lib, binding
+from . import _lib, binding, calls
 from .arrays import to_host
 from .mjw_kernels import newton_fusion
 
@@ -321,6 +321,10 @@ def solve_with_scratch(
         raise RuntimeError("optimized solver scratch layout no longer matches model")
     if expected_compact:
         raise RuntimeError("compact (sleeping-island) solves are outside this solver's path")
+    call = newton_fusion.cached_call(m, d, ctx, nsolving, scratch)
+    if call is not None:
+        call(stream)
+        return
     if not newton_fusion.eligible(m, ctx, compact=False):
         raise RuntimeError(
             "model is outside the fused Newton path: " + "; ".join(newton_fusion.ineligible_reasons(m, ctx))
@@ -342,6 +346,7 @@ def _factor_solve_i_dense(
     factor_workspace: Any = None,
     tree_factor_solve: Any = None,
     stream=None,
+    slot: Any = None,
 ) -> None:
     """x = M^-1 y for M (or M - h qDeriv) in the model's CSR layout, choosing the
     kernel as the reference does (mjw_step_optimized.py:1030-1070): the tree L'DL when
@@ -350,13 +355,13 @@ def _factor_solve_i_dense(
     Cholesky that stands in for the reference's per-tile kernels (:793-838).  The tile
     plan is made by ``make_optimized_fwd_position_scratch`` and remembered on the
     model; without it the first call builds it, which allocates (call once outside
-    graph capture)."""
+    graph capture).  ``slot`` names the caller among those that solve with this batch in turn."""
     from .mjw_kernels import indexed_factor, tree_ldl
 
     if factor_workspace is not None and dense_factor_solve is None:
         raise RuntimeError("a retained factor workspace requires the blocked dense path")
     if tree_factor_solve is not None and not retain_factor and factor_workspace is None:
-        tree_ldl.tree_factor_solve(tree_factor_solve, M, x, y, stream=stream)
+        tree_ldl.tree_factor_solve(tree_factor_solve, M, x, y, stream=stream, owner=d, slot=slot)
         return
     if dense_factor_solve is not None:
         indexed_factor.blocked_dense_factor_solve(
@@ -439,7 +444,7 @@ def fwd_acceleration_solve(m: Any, d: Any, scratch: OptimizedFwdPositionScratch,
     ``fwd_acceleration_optimized`` (mjw_step_optimized.py:1274-1329)."""
     _factor_solve_i_dense(
         m, d, d.M, d.qacc_smooth, d.qfrc_smooth, scratch.dense_factor_solve,
-        tree_factor_solve=scratch.tree_factor_solve, stream=stream,
+        tree_factor_solve=scratch.tree_factor_solve, stream=stream, slot="acceleration",
     )
 
 
@@ -458,6 +463,10 @@ def append_ball_limit_rows(m: Any, d: Any, scratch: OptimizedFwdPositionScratch,
 
 
 # ---- the implicit-fast integrator's tail (mjw_step_optimized.py:5209-5297) --------------
+
+_IMPLICIT_MODEL = calls.getter("opt.timestep", "dof_damping", "M_elemid", "M_colind")
+_IMPLICIT_DATA = calls.getter("moment_rownnz", "moment_rowadr", "moment_colind", "actuator_moment")
+_ADVANCE_MODEL = calls.getter("opt.timestep", "jnt_type", "jnt_dofadr", "jnt_qposadr")
 
 
 def attach_implicit_scratch(m: Any, d: Any, scratch: OptimizedFwdPositionScratch, device: Any = "cuda") -> None:
@@ -520,10 +529,17 @@ def deriv_smooth_vel_dense_actuator_centric(m: Any, d: Any, out: Any, scratch: O
         raise RuntimeError("tendon damping and fluid terms are outside this assembly")
     from .arrays import addr, elem_strides
 
-    ps = binding.implicit_struct(m, d, getattr(scratch, "implicit_actuator_vel", None))
-    rc = _lib.lib().imn_implicit_matrix(C.byref(ps), addr(d.M), elem_strides(d.M)[0], addr(out),
-                                        elem_strides(out)[0], int(d.nworld), _lib.current_stream_handle(stream))
-    _lib.check(rc, "imn_implicit_matrix")
+    gain = getattr(scratch, "implicit_actuator_vel", None)
+
+    def build():
+        ps = binding.implicit_struct(m, d, gain)
+        return (C.byref(ps), addr(d.M), elem_strides(d.M)[0], addr(out), elem_strides(out)[0], int(d.nworld)), ps
+
+    nu = int(getattr(m, "nu", 0) or 0)
+    buffers = _IMPLICIT_MODEL(m) + (d.M, out)
+    if nu and gain is not None:
+        buffers += _IMPLICIT_DATA(d) + (gain,)
+    calls.call(d, "imn_implicit_matrix", buffers, (m.nv, nu, m.opt.disableflags, d.nworld), build, stream)
 
 
 def _advance_with_scratch(m: Any, d: Any, qacc: Any, scratch: OptimizedFwdPositionScratch | None = None,
@@ -544,10 +560,13 @@ def _advance_with_scratch(m: Any, d: Any, qacc: Any, scratch: OptimizedFwdPositi
         raise RuntimeError("actuator activations are outside this advance")
     from .arrays import addr, elem_strides
 
-    ps = binding.advance_struct(m, d)
-    rc = _lib.lib().imn_advance(C.byref(ps), addr(qacc), elem_strides(qacc)[0], int(d.nworld),
-                                _lib.current_stream_handle(stream))
-    _lib.check(rc, "imn_advance")
+    def build():
+        ps = binding.advance_struct(m, d)
+        return (C.byref(ps), addr(qacc), elem_strides(qacc)[0], int(d.nworld)), ps
+
+    time = getattr(d, "time", None)
+    buffers = _ADVANCE_MODEL(m) + (d.qvel, d.qpos, qacc) + (() if time is None else (time,))
+    calls.call(d, "imn_advance", buffers, (m.nv, m.nq, m.njnt, time is None, d.nworld), build, stream)
 
 
 def implicitfast_integrate(m: Any, d: Any, scratch: OptimizedFwdPositionScratch, stream=None) -> None:
@@ -566,6 +585,6 @@ def implicitfast_integrate(m: Any, d: Any, scratch: OptimizedFwdPositionScratch,
     deriv_smooth_vel_dense_actuator_centric(m, d, scratch.implicit_qderiv, scratch, stream=stream)
     _factor_solve_i_dense(
         m, d, scratch.implicit_qderiv, scratch.implicit_qacc, d.efc.Ma, scratch.dense_factor_solve,
-        tree_factor_solve=scratch.tree_factor_solve, stream=stream,
+        tree_factor_solve=scratch.tree_factor_solve, stream=stream, slot="implicit",
     )
     _advance_with_scratch(m, d, scratch.implicit_qacc, scratch, stream=stream)
