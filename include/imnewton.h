@@ -294,6 +294,16 @@ typedef struct ImnImplicit {
   const float* actuator_moment; /* (W, moment_ld)                                */
   int64_t moment_ld;
   const float* actuator_velocity_gain; /* (W, nu)                                */
+  /* Optional: with `ctrl` the gains are formed in the same launch, gain_a = g2_a ctrl_a +
+   * b2_a (stateless fixed / affine actuators), and stored to `velocity_gain_out`, which then
+   * stands in for actuator_velocity_gain.  Coefficients: (n_coefficients, nu), world w
+   * reads row w % n.                                                            */
+  const float* ctrl;           /* (W, nu) stride ctrl_ld */
+  int64_t ctrl_ld;
+  const float* gain_g2;
+  const float* gain_b2;
+  int32_t n_coefficients;
+  float* velocity_gain_out;    /* (W, nu) */
 } ImnImplicit;
 
 /* State advanced by the integrator (upstream _advance, called through

@@ -193,7 +193,8 @@ class ImnImplicit(C.Structure):
     _fields_ = [
         ("nv", I32), ("nM", I32), ("nu", I32), ("actuation", I32), ("damper", I32), ("timestep", P), ("n_timestep", I32),
         ("dof_damping", P), ("M_elemid", P), ("moment_rownnz", P), ("moment_rowadr", P), ("moment_colind", P),
-        ("actuator_moment", P), ("moment_ld", I64), ("actuator_velocity_gain", P),
+        ("actuator_moment", P), ("moment_ld", I64), ("actuator_velocity_gain", P), ("ctrl", P), ("ctrl_ld", I64), ("gain_g2", P), ("gain_b2", P),
+        ("n_coefficients", I32), ("velocity_gain_out", P),
     ]
 
 

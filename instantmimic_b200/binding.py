@@ -273,8 +273,9 @@ def _timestep(m: Any) -> tuple[int, int]:
     return addr(h), n
 
 
-def implicit_struct(m: Any, d: Any, velocity_gain: Any) -> abi.ImnImplicit:
-    """``velocity_gain``: (nworld, nu) d(actuator force)/d(actuator velocity), or None."""
+def implicit_struct(m: Any, d: Any, velocity_gain: Any, coefficients: Any = None) -> abi.ImnImplicit:
+    """``velocity_gain``: (nworld, nu) d(actuator force)/d(actuator velocity), or None.  With
+    ``coefficients`` (g2, b2 per actuator) the kernel forms it from ``d.ctrl`` and stores it there."""
     c = upstream_constants()
     s = abi.ImnImplicit()
     flags = int(m.opt.disableflags)
@@ -300,6 +301,11 @@ def implicit_struct(m: Any, d: Any, velocity_gain: Any) -> abi.ImnImplicit:
         s.moment_colind, s.actuator_moment = addr(d.moment_colind), addr(d.actuator_moment)
         s.moment_ld = elem_strides(d.actuator_moment)[0]
         s.actuator_velocity_gain = addr(velocity_gain)
+        if coefficients is not None:
+            g2, b2 = coefficients
+            s.ctrl, s.ctrl_ld = addr(d.ctrl), _row_ld(d.ctrl)
+            s.gain_g2, s.gain_b2, s.n_coefficients = addr(g2), addr(b2), (length(g2) if len(shape(g2)) == 2 else 1)
+            s.velocity_gain_out = addr(velocity_gain)
     return s
 
 

@@ -525,6 +525,12 @@ def deriv_smooth_vel_dense_actuator_centric(m: Any, d: Any, out: Any, scratch: O
     """out = M - h qDeriv in M's layout (mjw_step_optimized.py:4172-4412): actuator term
     from ``scratch.implicit_actuator_vel`` and the per-world moment rows, joint damping.
     Models with tendons or fluid forces keep the upstream assembly."""
+    _implicit_matrix(m, d, out, scratch, None, stream)
+
+
+def _implicit_matrix(m: Any, d: Any, out: Any, scratch: OptimizedFwdPositionScratch, coefficients: Any, stream) -> None:
+    """The assembly with the velocity gains of the scratch, or with gains formed from
+    ``coefficients`` and the controls in the same launch (and left in the scratch)."""
     if int(getattr(m, "ntendon", 0) or 0) or bool(getattr(m, "has_fluid", False)):
         raise RuntimeError("tendon damping and fluid terms are outside this assembly")
     from .arrays import addr, elem_strides
@@ -532,14 +538,32 @@ def deriv_smooth_vel_dense_actuator_centric(m: Any, d: Any, out: Any, scratch: O
     gain = getattr(scratch, "implicit_actuator_vel", None)
 
     def build():
-        ps = binding.implicit_struct(m, d, gain)
+        ps = binding.implicit_struct(m, d, gain, coefficients)
         return (C.byref(ps), addr(d.M), elem_strides(d.M)[0], addr(out), elem_strides(out)[0], int(d.nworld)), ps
 
     nu = int(getattr(m, "nu", 0) or 0)
     buffers = _IMPLICIT_MODEL(m) + (d.M, out)
     if nu and gain is not None:
         buffers += _IMPLICIT_DATA(d) + (gain,)
+    if coefficients is not None:
+        buffers += (d.ctrl, *coefficients)
     calls.call(d, "imn_implicit_matrix", buffers, (m.nv, nu, m.opt.disableflags, d.nworld), build, stream)
+
+
+def _fused_gain_coefficients(m: Any, d: Any, scratch: Any):
+    """The prepared (g2, b2) when the assembly can form the gains itself: float32 rows per
+    actuator, for all worlds or for each."""
+    import torch
+
+    pair = getattr(scratch, "implicit_gain_coefficients", None)
+    if pair is None:
+        return None
+    shapes = {tuple(t.shape) for t in pair}
+    nu = int(m.nu)
+    if shapes <= {(nu,)} or shapes <= {(1, nu)} or shapes <= {(int(d.nworld), nu)}:
+        if all(t.dtype == torch.float32 and t.is_contiguous() for t in pair):
+            return pair
+    return None
 
 
 def _advance_with_scratch(m: Any, d: Any, qacc: Any, scratch: OptimizedFwdPositionScratch | None = None,
@@ -581,8 +605,12 @@ def implicitfast_integrate(m: Any, d: Any, scratch: OptimizedFwdPositionScratch,
     if scratch.implicit_qderiv is None or scratch.implicit_qacc is None:
         raise RuntimeError("implicit-fast scratch is not attached (attach_implicit_scratch)")
     if int(getattr(m, "nu", 0) or 0) and not (int(m.opt.disableflags) & B.upstream_constants()["disable_actuation"]):
-        actuator_velocity_gain(m, d, scratch.implicit_actuator_vel, scratch)
-    deriv_smooth_vel_dense_actuator_centric(m, d, scratch.implicit_qderiv, scratch, stream=stream)
+        coefficients = _fused_gain_coefficients(m, d, scratch)
+        if coefficients is None:
+            actuator_velocity_gain(m, d, scratch.implicit_actuator_vel, scratch)
+    else:
+        coefficients = None
+    _implicit_matrix(m, d, scratch.implicit_qderiv, scratch, coefficients, stream)
     _factor_solve_i_dense(
         m, d, scratch.implicit_qderiv, scratch.implicit_qacc, d.efc.Ma, scratch.dense_factor_solve,
         tree_factor_solve=scratch.tree_factor_solve, stream=stream, slot="implicit",

@@ -208,3 +208,43 @@ def test_implicitfast_integrate_entry(oracle, cuda_device):
     h = float(m.opt.timestep[0])
     got = mjw_model.to_host(dd)
     assert np.abs(got.qvel - (d.qvel + h * exact)).max() <= 1e-4 * (np.abs(exact).max() + 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nu,shape", [(28, "ball"), (33, "ball"), (70, "ball"), (1, "hinge"), (32, "hinge"), (5, "clash")])
+def test_gains_formed_in_the_assembly_and_batches_of_moment_rows(oracle, cuda_device, nu, shape):
+    """The assembly that forms the velocity gains itself equals gain call + assembly bit for bit, and
+    the oracle: three-dof rows with one nonzero moment (ball-joint motors), rows of one dof, and
+    three-dof rows whose actuators meet on the same entries."""
+    import torch
+
+    from instantmimic_b200 import mjw_step_optimized as runtime
+
+    m, d = _problem(worlds=37, nu=nu, seed=nu, single=True)[:2]
+    rng = np.random.default_rng(nu)
+    W, n = d.nworld, (1 if shape == "hinge" else 3)
+    first = rng.integers(6, m.nv - 3, (W, nu)) if shape != "clash" else np.full((W, nu), 6)
+    d.moment_rownnz = np.full((W, nu), n, np.int32)
+    d.moment_rowadr = np.tile(np.arange(nu, dtype=np.int32) * n, (W, 1))
+    d.moment_colind = (first[..., None] + np.arange(n)).reshape(W, -1).astype(np.int32)
+    moment = rng.normal(size=(W, nu, n)).astype(np.float32)
+    if shape == "ball":
+        moment *= np.eye(3, dtype=np.float32)[rng.integers(0, 3, (W, nu))]
+    d.actuator_moment = moment.reshape(W, -1).copy()
+    d.ctrl = rng.uniform(-1, 1, (W, nu)).astype(np.float32)
+    m.actuator_gaintype = np.full(nu, int(types.GainType.AFFINE), np.int32)
+    m.actuator_biastype = np.full(nu, int(types.BiasType.AFFINE), np.int32)
+    m.actuator_dyntype = np.zeros(nu, np.int32)
+    m.actuator_gainprm = rng.normal(size=(nu, 10)).astype(np.float32)
+    m.actuator_biasprm = -rng.uniform(1, 20, (nu, 10)).astype(np.float32)
+    md, dd = mjw_model.to_device(m, cuda_device), mjw_model.to_device(d, cuda_device)
+    scratch = runtime.make_optimized_fwd_position_scratch(md, dd, cuda_device)
+    runtime.attach_implicit_scratch(md, dd, scratch, cuda_device)
+    runtime.actuator_velocity_gain(md, dd, scratch.implicit_actuator_vel, scratch)
+    runtime.deriv_smooth_vel_dense_actuator_centric(md, dd, scratch.implicit_qderiv, scratch)
+    A, gains = scratch.implicit_qderiv.clone(), scratch.implicit_actuator_vel.clone()
+    scratch.implicit_qderiv.zero_(), scratch.implicit_actuator_vel.zero_()
+    runtime._implicit_matrix(md, dd, scratch.implicit_qderiv, scratch, runtime._fused_gain_coefficients(md, dd, scratch), None)
+    torch.cuda.synchronize()
+    assert torch.equal(gains, scratch.implicit_actuator_vel) and torch.equal(A, scratch.implicit_qderiv)
+    np.testing.assert_array_equal(A.cpu().numpy(), oracle.implicit_matrix(m, d, gains.cpu().numpy()))
