@@ -11,19 +11,127 @@
 // (or grad) and subtracts U[t][r] * U[t][c] for t = 0, 1, ... with fused
 // multiply-adds; the pivot is sqrtf; the row is scaled by the reciprocal pivot.
 //
-// Mapping: 16 rows at a time.  A lane owns up to three columns c = b0 + lane +
-// 32k and keeps the block's 16 running sums of each in registers.  Phase 1 adds
-// the terms of all earlier rows (one shared-memory read of U[t][c] and four
-// 128-bit broadcast reads of U[t][b0..b0+15] feed 16 fused multiply-adds).
-// Phase 2 eliminates the block's rows one by one with warp shuffles: the pivot
-// row's entry of column b0+j is in lane j, so no shared-memory round trip and no
-// barrier separates the 16 steps.  The register file is shifted by one row per
-// step so that the loop body is the same code for every row.
+// Mapping: 16 rows at a time.  A lane owns K columns c = b0 + lane + 32k (K = 1 or 2 by the
+// columns that are left; columns past the 64th follow when the block's rows are done) and keeps the block's 16 running sums of each in registers.  Phase 1 adds
+// the terms of all earlier rows (one shared-memory read of U[t][c] per column and four 128-bit
+// broadcast reads of U[t][b0..b0+15] feed 16 K fused multiply-adds).  Phase 2 eliminates the block's
+// rows.  Its chain per row is scale -> own square -> shuffle -> root -> reciprocal: the pivot of row
+// r + 1 is its lane's own sum after row r, which that lane has at once, so it travels while the
+// other sums wait for row r to come back from shared memory as four broadcast reads (the block's
+// entries of a row sit in 16 lanes; fetched by 15 shuffles each row cost 700 cycles).  Four rows per
+// trip, so that every sum has a fixed register and the reads start on 16-byte boundaries.
 #pragma once
 
 #include "imn_newton_linalg.cuh"
 
 namespace imn {
+
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+template <int K>
+__device__ __forceinline__ void factor_block(const World& s, int b0) {
+  const int lane = s.lane, nv = s.nv, ldu = s.ldu, nr = min(16, nv - b0);
+  float* A = s.A;
+  float acc[K][16];
+  int cc[K];
+  bool valid[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int c = b0 + lane + 32 * k;
+    valid[k] = c <= nv;
+    cc[k] = valid[k] ? c : nv;
+    // H column cc (rows b0..), or grad for the carried column; rows below the diagonal and past the
+    // last hold values that are never stored or read by another lane
+    const float* src = (cc[k] < nv ? A + (cc[k] + 1) * ldu : s.grad) + b0;
+#pragma unroll
+    for (int g = 0; g < 16; g += 4) {
+      const float4 h = g < nr ? ld4(src + g) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      acc[k][g] = h.x, acc[k][g + 1] = h.y, acc[k][g + 2] = h.z, acc[k][g + 3] = h.w;
+    }
+  }
+  // phase 1: terms of rows t < b0
+#pragma unroll 2
+  for (int t = 0; t < b0; ++t) {
+    const float* Ut = A + t * ldu;
+    float uc[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) uc[k] = Ut[cc[k]];
+#pragma unroll
+    for (int g = 0; g < 16; g += 4) {
+      const float4 u = ld4(Ut + b0 + g);  // past the last row: values of the next rows, never stored
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        acc[k][g] = fmaf(-u.x, uc[k], acc[k][g]), acc[k][g + 1] = fmaf(-u.y, uc[k], acc[k][g + 1]);
+        acc[k][g + 2] = fmaf(-u.z, uc[k], acc[k][g + 2]), acc[k][g + 3] = fmaf(-u.w, uc[k], acc[k][g + 3]);
+      }
+    }
+  }
+  IMN_MARK(s, 12);
+  // phase 2: acc[k][q] belongs to row g + q
+  float pv = __shfl_sync(IMN_FULL_MASK, acc[0][0], 0);
+#pragma unroll 1
+  for (int g = 0; g < nr; g += 4) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = g + q;
+      if (r >= nr) break;  // warp-uniform
+      const float dg = sqrtf(pv), rinv = 1.0f / dg;
+      float* Ur = A + (b0 + r) * ldu;
+      float u[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) u[k] = acc[k][q] * rinv;
+      pv = __shfl_sync(IMN_FULL_MASK, fmaf(-u[0], u[0], acc[0][q + 1]), r + 1);
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (valid[k] && cc[k] >= b0 + r) Ur[cc[k]] = k == 0 && lane == r ? dg : u[k];
+      if (lane == 0) s.dinv[b0 + r] = rinv;
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < 16; h += 4) {
+        const float4 m = ld4(Ur + b0 + g + h);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          if (h > q) acc[k][h] = fmaf(-m.x, u[k], acc[k][h]);
+          if (h + 1 > q) acc[k][h + 1] = fmaf(-m.y, u[k], acc[k][h + 1]);
+          if (h + 2 > q) acc[k][h + 2] = fmaf(-m.z, u[k], acc[k][h + 2]);
+          if (h + 3 > q) acc[k][h + 3] = fmaf(-m.w, u[k], acc[k][h + 3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int h = 0; h < 16; ++h) acc[k][h] = h < 12 ? acc[k][h + 4] : 0.0f;
+  }
+  __syncwarp();
+  IMN_MARK(s, 13);
+}
+
+// The block's rows at one column c0 + lane behind the 64 of factor_block: the same sums, scaled with the
+// stored reciprocals.
+__device__ __forceinline__ void factor_follow(const World& s, int b0, int c0) {
+  const int nv = s.nv, ldu = s.ldu, nr = min(16, nv - b0), c = c0 + s.lane, cc = min(c, nv);
+  float* A = s.A;
+  float acc[16];
+  const float* src = (cc < nv ? A + (cc + 1) * ldu : s.grad) + b0;
+#pragma unroll
+  for (int g = 0; g < 16; ++g) acc[g] = g < nr ? src[g] : 0.0f;
+#pragma unroll 1
+  for (int t = 0; t < b0; ++t) {
+    const float uc = A[t * ldu + cc];
+#pragma unroll
+    for (int g = 0; g < 16; ++g) acc[g] = fmaf(-A[t * ldu + b0 + g], uc, acc[g]);
+  }
+#pragma unroll 1
+  for (int r = 0; r < nr; ++r) {
+    float* Ur = A + (b0 + r) * ldu;
+    const float u = acc[0] * s.dinv[b0 + r];
+    if (c <= nv) Ur[c] = u;
+#pragma unroll
+    for (int h = 1; h < 16; ++h) acc[h - 1] = fmaf(-Ur[min(b0 + r + h, nv)], u, acc[h]);
+  }
+  __syncwarp();
+}
 
 __device__ __forceinline__ void factor_solve(const World& s, bool factor, float& sum0, float& sum1) {
   const int lane = s.lane, nv = s.nv, ldu = s.ldu;
@@ -31,85 +139,12 @@ __device__ __forceinline__ void factor_solve(const World& s, bool factor, float&
   if (factor) {
 #pragma unroll 1
     for (int b0 = 0; b0 < nv; b0 += 16) {
-      const int nr = min(16, nv - b0);
-      const int ng = (nr + 3) >> 2;
-      float acc[3][16];
-      int cc[3];
-      bool act[3], valid[3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const int c = b0 + lane + 32 * k;
-        act[k] = b0 + 32 * k <= nv;  // warp-uniform: the slot holds at least one column
-        valid[k] = c <= nv;
-        cc[k] = valid[k] ? c : nv;
-        if (act[k]) {
-          // H column cc (rows b0..), or grad for the carried column; rows below the
-          // diagonal hold values that are never stored or read by another lane
-          const float* src = (cc[k] < nv ? A + (cc[k] + 1) * ldu : s.grad) + b0;
-#pragma unroll
-          for (int gi = 0; gi < 4; ++gi) {
-            float4 h = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (gi < ng) h = *reinterpret_cast<const float4*>(src + 4 * gi);
-            acc[k][4 * gi] = h.x, acc[k][4 * gi + 1] = h.y, acc[k][4 * gi + 2] = h.z, acc[k][4 * gi + 3] = h.w;
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) acc[k][i] = 0.0f;
-        }
-      }
-      // phase 1: terms of rows t < b0
-#pragma unroll 1
-      for (int t = 0; t < b0; ++t) {
-        const float* Ut = A + t * ldu;
-        float ur[16];
-#pragma unroll
-        for (int gi = 0; gi < 4; ++gi) {
-          float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (gi < ng) u = *reinterpret_cast<const float4*>(Ut + b0 + 4 * gi);
-          ur[4 * gi] = u.x, ur[4 * gi + 1] = u.y, ur[4 * gi + 2] = u.z, ur[4 * gi + 3] = u.w;
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-          if (act[k]) {
-            const float uc = Ut[cc[k]];
-#pragma unroll
-            for (int gi = 0; gi < 4; ++gi)
-              if (gi < ng) {  // warp-uniform: a short last block skips its absent rows
-#pragma unroll
-                for (int i = 4 * gi; i < 4 * gi + 4; ++i) acc[k][i] = fmaf(-ur[i], uc, acc[k][i]);
-              }
-          }
-      }
-      IMN_MARK(s, 12);
-      // phase 2: eliminate the block's rows; acc[k][0] is always the current row
-#pragma unroll 1
-      for (int r = 0; r < nr; ++r) {
-        const float pv = __shfl_sync(IMN_FULL_MASK, acc[0][0], r);
-        const float dg = sqrtf(pv);
-        const float rinv = 1.0f / dg;
-        float u[3];
-        float* Ur = A + (b0 + r) * ldu;
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-          if (act[k]) {
-            u[k] = acc[k][0] * rinv;
-            if (k == 0 && lane == r) u[k] = dg;
-            if (valid[k] && cc[k] >= b0 + r) Ur[cc[k]] = u[k];
-          }
-        if (lane == 0) s.dinv[b0 + r] = rinv;
-        float um[16];  // um[j] = U[b0+r][b0+r+j], held by lane r+j
-#pragma unroll
-        for (int j = 1; j < 16; ++j) um[j] = __shfl_sync(IMN_FULL_MASK, u[0], (r + j) & 31);
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-          if (act[k]) {
-#pragma unroll
-            for (int j = 1; j < 16; ++j) acc[k][j - 1] = fmaf(-um[j], u[k], acc[k][j]);
-            acc[k][15] = 0.0f;
-          }
-      }
-      __syncwarp();
-      IMN_MARK(s, 13);
+      const int columns = nv + 1 - b0;
+      if (columns <= 32)
+        factor_block<1>(s, b0);
+      else
+        factor_block<2>(s, b0);
+      if (columns > 64) factor_follow(s, b0, b0 + 64);
     }
   } else {
     // forward substitution with the stored factor: unknown r receives its terms
