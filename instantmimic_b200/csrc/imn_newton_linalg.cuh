@@ -234,30 +234,29 @@ __device__ __forceinline__ void products(const World& s, const float* v, float* 
 
 // grad = Ma - qfrc_smooth - J^T force over the rows with a nonzero force (a zero
 // force leaves the running sums unchanged), then grad_dot
-// (newton_stages.py:785-795).
+// (newton_stages.py:785-795).  Lane = dof.  Every element of J is used once, so a streamed J is read
+// straight from global memory (coalesced), without the detour through the tile; the listed rows go
+// several at a time so that their reads overlap.
 template <bool JRES>
 __device__ __forceinline__ float full_gradient(const World& s, int nfr) {
   const int lane = s.lane, nv = s.nv;
   float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
   const int i0 = lane, i1 = lane + 32, i2 = lane + 64;
   const bool h0 = i0 < nv, h1 = i1 < nv, h2 = i2 < nv;
-  int a = 0;
+  constexpr int B = JRES ? 4 : 8;
+  const float* J = (JRES ? s.Jsm : s.Jg) + lane;
 #pragma unroll 1
-  for (int base = 0; base < s.nefc; base += 32) {
-    const float* Jt = j_tile<JRES>(s, base);
-    const int hi = JRES ? s.nefc : base + 32;
-#pragma unroll 2
-    for (; a < nfr; ++a) {
-      const int r = s.frows[a];
-      if (r >= hi) break;
-      const float f = s.force[r];
-      const float* Jr = Jt + (r - base) * s.ldj;
-      if (h0) s0 = fmaf(Jr[i0], f, s0);
-      if (h1) s1 = fmaf(Jr[i1], f, s1);
-      if (h2) s2 = fmaf(Jr[i2], f, s2);
+  for (int a = 0; a < nfr; a += B) {
+    float f[B], j0[B], j1[B], j2[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      const int r = s.frows[min(a + k, nfr - 1)];
+      f[k] = a + k < nfr ? s.force[r] : 0.0f;  // past the end the last row again, without a force
+      const float* Jr = J + (size_t)r * s.ldj;
+      j0[k] = h0 ? Jr[0] : 0.0f, j1[k] = h1 ? Jr[32] : 0.0f, j2[k] = h2 ? Jr[64] : 0.0f;
     }
-    if (JRES) break;
-    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < B; ++k) s0 = fmaf(j0[k], f[k], s0), s1 = fmaf(j1[k], f[k], s1), s2 = fmaf(j2[k], f[k], s2);
   }
   if (h0) s.grad[i0] = (s.Ma[i0] - s.qfs[i0]) - s0;
   if (h1) s.grad[i1] = (s.Ma[i1] - s.qfs[i1]) - s1;
