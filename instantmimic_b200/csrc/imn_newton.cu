@@ -51,7 +51,8 @@ __device__ unsigned long long g_prof[16];
 #define IMN_OVERFLOW_COPY_TIMEOUT (1 << 30)
 
 struct Geom {
-  int nv, njmax, ldj, ldu, nM, bd;
+  int nv, njmax, ldj, ldp, ldu, nM, bd;
+  bool j16;  // a streamed J is copied row by row and read 16 bytes at a time (j_tile)
   int jrows;  // rows of J held in shared memory (njmax when resident, else 32)
   // offsets in 4-byte words; every region starts on a 16-byte boundary
   int oBar, oJ, oA, oVec, nv4, oRowF, oRowI, oMask, mwords, r4, oUni, total;
@@ -93,7 +94,13 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   g.oBar = o, o += 4;
   // a streamed tile may start up to three floats into its buffer and end on a 16-byte boundary
   // a dense block reads up to three floats past a row; the gathered rows are up4(nv) floats apart
-  g.oJ = o, o += (resident ? up4(g.jrows * g.ldj + 3) : max(up4(32 * g.ldj) + 8, 32 * up4(m.nv)));
+  g.ldp = 4 * ((m.nv / 4) | 1);
+  g.j16 = !resident && m.nv % 4 == 0 && d.J_ld_row % 4 == 0 && !d.J_world_offset && d.J_ld_world % 4 == 0 &&
+          (reinterpret_cast<uintptr_t>(d.efc_J) & 15) == 0;
+  if (g.j16)
+    g.oJ = o, o += 32 * g.ldp;
+  else
+    g.oJ = o, o += (resident ? up4(g.jrows * g.ldj + 3) : max(up4(32 * g.ldj) + 8, 32 * up4(m.nv)));
   // dense: H and its factor share one (nv+1) x ldu array; sparse plan: packed H | N | 1/D
   g.oA = o, o += sp ? up4(sp->nfac) + up4(sp->nslots) + up4(m.nv) : (m.nv + 1) * g.ldu;
   // dof vectors; the dense factor needs two more (forward-solve scratch, 1 / pivot)
@@ -137,7 +144,7 @@ __device__ __noinline__ void warn_limit(int which, unsigned limit) {
 // pass of it" rather than as a load followed by a pass loop: the same statements, but the compiler
 // lays the single loop out better (measured: 0.836 -> 0.796 ms per 8192 humanoid worlds at the same
 // occupancy).
-template <bool JRES, bool SPARSE, bool STATS, bool TSM>
+template <bool JRES, bool J16, bool SPARSE, bool STATS, bool TSM>
 __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& d, const ImnCtx& cx, const Geom& g,
                                               const ImnSparsePlan& sp) {
   extern __shared__ __align__(16) float smem_all[];
@@ -147,7 +154,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
 
   void* bar = smem + g.oBar;
   World s;
-  s.nv = nv, s.ldj = g.ldj, s.ldu = g.ldu, s.bd = g.bd, s.lane = lane, s.nM = g.nM;
+  s.nv = nv, s.ldj = g.ldj, s.ldp = g.ldp, s.ldu = g.ldu, s.bd = g.bd, s.lane = lane, s.nM = g.nM;
   s.Jsm = smem + g.oJ;
   s.A = smem + g.oA;
   s.qacc = smem + g.oVec;
@@ -346,7 +353,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
       // one call site: Ma = M qacc, Jaref = J qacc - aref on pass 0; mv = M search,
       // jv = J search afterwards
       if (first || !search_unchanged)
-        products<JRES, TSM>(s, first ? s.qacc : s.search, first ? s.Ma : s.mv, first ? s.Jaref : s.jv,
+        products<JRES, J16, TSM>(s, first ? s.qacc : s.search, first ? s.Ma : s.mv, first ? s.Jaref : s.jv,
                        first ? s.jv : nullptr);
       __syncwarp();
       PROF(5);
@@ -444,9 +451,9 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
             outside = __any_sync(IMN_FULL_MASK, bad);
           }
           if (SPARSE)
-            hessian_sparse<JRES, TSM>(s, quad_count, first, outside, sp);
+            hessian_sparse<JRES, J16, TSM>(s, quad_count, first, outside, sp);
           else
-            hessian_dense<JRES>(s, quad_count, first);
+            hessian_dense<JRES, J16>(s, quad_count, first);
         }
         PROF(9);
         if (SPARSE) {
@@ -587,18 +594,23 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
 template <bool SPARSE, bool STATS, bool TSM>
 __global__ void __launch_bounds__(32 * kResidentWarps, 1)
     newton_kernel_resident(const ImnModel m, const ImnData d, const ImnCtx cx, const Geom g, const ImnSparsePlan sp) {
-  newton_worlds<true, SPARSE, STATS, TSM>(m, d, cx, g, sp);
+  newton_worlds<true, false, SPARSE, STATS, TSM>(m, d, cx, g, sp);
 }
-template <bool SPARSE, bool STATS, bool TSM>
+template <bool J16, bool SPARSE, bool STATS, bool TSM>
 __global__ void __launch_bounds__(32 * kStreamedWarps, 1)
     newton_kernel_streamed(const ImnModel m, const ImnData d, const ImnCtx cx, const Geom g, const ImnSparsePlan sp) {
-  newton_worlds<false, SPARSE, STATS, TSM>(m, d, cx, g, sp);
+  newton_worlds<false, J16, SPARSE, STATS, TSM>(m, d, cx, g, sp);
 }
 using Kernel = void (*)(ImnModel, ImnData, ImnCtx, Geom, ImnSparsePlan);
+template <bool SPARSE, bool STATS, bool TSM>
+static Kernel newton_kernel(bool resident, bool j16) {
+  return resident ? (Kernel)newton_kernel_resident<SPARSE, STATS, TSM>
+         : j16    ? (Kernel)newton_kernel_streamed<true, SPARSE, STATS, TSM>
+                  : (Kernel)newton_kernel_streamed<false, SPARSE, STATS, TSM>;
+}
 template <bool SPARSE, bool STATS>
-static Kernel newton_kernel(bool resident, bool tsm) {
-  return resident ? (tsm ? (Kernel)newton_kernel_resident<SPARSE, STATS, true> : (Kernel)newton_kernel_resident<SPARSE, STATS, false>)
-                  : (tsm ? (Kernel)newton_kernel_streamed<SPARSE, STATS, true> : (Kernel)newton_kernel_streamed<SPARSE, STATS, false>);
+static Kernel newton_kernel(bool resident, const Geom& g) {
+  return g.tsm ? newton_kernel<SPARSE, STATS, true>(resident, g.j16) : newton_kernel<SPARSE, STATS, false>(resident, g.j16);
 }
 
 __global__ void start_counters(int* nsolving, int* work_counter, int nworld) {
@@ -769,8 +781,8 @@ extern "C" int imn_solve(const ImnModel* m, const ImnData* d, const ImnCtx* cx, 
   const int bytes = 4 * (g.tab + g.warps * g.total);
   const bool sparse = cx->sparse_plan != nullptr, stats = cx->stats != nullptr;
   const ImnSparsePlan sp = sparse ? *cx->sparse_plan : ImnSparsePlan{};
-  const imn::Kernel kern = sparse ? (stats ? imn::newton_kernel<true, true>(res, g.tsm) : imn::newton_kernel<true, false>(res, g.tsm))
-                                  : (stats ? imn::newton_kernel<false, true>(res, g.tsm) : imn::newton_kernel<false, false>(res, g.tsm));
+  const imn::Kernel kern = sparse ? (stats ? imn::newton_kernel<true, true>(res, g) : imn::newton_kernel<true, false>(res, g))
+                                  : (stats ? imn::newton_kernel<false, true>(res, g) : imn::newton_kernel<false, false>(res, g));
   {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e == cudaSuccess && bytes > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);

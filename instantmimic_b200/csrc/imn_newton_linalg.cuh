@@ -13,7 +13,7 @@ namespace imn {
 
 // Shared-memory view of one world plus the per-world constants.
 struct World {
-  int nv, ldj, ldu, bd, nefc, ne, nef, lane, nM;
+  int nv, ldj, ldp, ldu, bd, nefc, ne, nef, lane, nM;
   float *Jsm, *A, *qacc, *Ma, *search, *mv, *grad, *qfs, *xsm, *dinv;
   // the world's M stays in global memory: its nM values are read once per iteration by
   // `products` (independent loads, issued together) and once by the Hessian assembly, and
@@ -56,37 +56,50 @@ struct World {
 #define IMN_MARK(s, k)
 #endif
 
-// Rows [base, base+32) of J: resident rows are addressed in place, otherwise they
-// are staged through the 32-row tile.
-template <bool JRES>
+// Rows [base, base+32) of J: resident rows are addressed in place, otherwise they are staged
+// through the 32-row tile by TMA bulk copies on the world's mbarrier; the wait is bounded.
+// J16 (streamed only; nv, the row stride and every row multiples of four floats): one copy per row,
+// a row per lane, to a stride of ldp floats, a multiple of four with ldp / 4 odd.  With lane = row the
+// 128-bit reads of eight consecutive lanes then hit eight different groups of four banks; at their
+// own stride the rows of such models (56, 64 floats) put 4 or all 32 lanes on one bank.
+// (64 dofs x 512 rows, 4096 worlds: 7326 -> 4816 us per solve; 56 x 128: 1206 -> 1189.)
+// Otherwise rows keep their own stride and the tile is one contiguous copy.
+template <bool JRES, bool J16>
 __device__ __forceinline__ const float* j_tile(const World& s, int base) {
   if (JRES) return s.Jsm + base * s.ldj;
+  IMN_MARK(s, 23);
   __syncwarp();  // every lane is done with the previous tile
-  const int n = min(32, s.nefc - base) * s.ldj;
+  const int rows = min(32, s.nefc - base), n = rows * s.ldj;
   const float* src = s.Jg + (size_t)base * s.ldj;
-  // One TMA bulk copy on the world's mbarrier; the wait is bounded.  A bulk copy wants
-  // 16-byte aligned ends, so the smallest aligned range around the rows is copied (up
-  // to three floats of the neighbouring rows on either side, still inside the J
+  // A bulk copy wants 16-byte aligned ends, so the smallest aligned range around a run of rows is
+  // copied (up to three floats of the neighbouring rows on either side, still inside the J
   // array) and the tile starts `head` floats into the buffer.
-  const int head = (int)((reinterpret_cast<uintptr_t>(src) & 15) >> 2);
-  const uint32_t bytes = (uint32_t)((head + n + 3) & ~3) * 4u;
+  const int head = J16 ? 0 : (int)((reinterpret_cast<uintptr_t>(src) & 15) >> 2);
+  const uint32_t bytes = J16 ? (uint32_t)(rows * s.nv) * 4u : (uint32_t)((head + n + 3) & ~3) * 4u;
   // after a copy that timed out the barrier's phase is unknown: the world is lost (the
   // caller checks jfail at the end of the pass) and the rest of the pass uses plain loads
-  if (src - head >= s.Jbeg && src - head + (bytes >> 2) <= s.Jend && !*s.jfail) {
+  if ((J16 || (src - head >= s.Jbeg && src - head + (bytes >> 2) <= s.Jend)) && !*s.jfail) {
     const uint32_t parity = (uint32_t)*s.jphase;
     __syncwarp();
     if (s.lane == 0) {
       mbar_expect_tx(s.jbar, bytes);
-      if (!(s.withhold_copies & 2)) bulk_g2s(s.Jsm, src - head, bytes, s.jbar);
+      if (!J16 && !(s.withhold_copies & 2)) bulk_g2s(s.Jsm, src - head, bytes, s.jbar);
       *s.jphase = (int)(parity ^ 1u);
+    }
+    if (J16) {
+      __syncwarp();  // the barrier expects the bytes before the first of them arrives
+      if (s.lane < rows && !(s.withhold_copies & 2))
+        bulk_g2s(s.Jsm + s.lane * s.ldp, src + (size_t)s.lane * s.ldj, (uint32_t)s.nv * 4u, s.jbar);
     }
     bool arrived = false;
 #pragma unroll 1
     for (int tries = 0; tries < s.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(s.jbar, parity);
     if (!arrived && s.lane == 0) *s.jfail = 1;
     __syncwarp();
+    IMN_MARK(s, 17);
     return s.Jsm + head;
   }
+  if (J16) return s.Jsm;  // a lost world: its results are never written
 #pragma unroll 4
   for (int i = s.lane; i < n; i += 32) s.Jsm[i] = src[i];
   // the next tile may arrive through the async proxy into the same buffer
@@ -94,6 +107,7 @@ __device__ __forceinline__ const float* j_tile(const World& s, int base) {
   __syncwarp();
   return s.Jsm;
 }
+
 // Rows of the list s.ids (bit 15: the row leaves the QUADRATIC set, its D counts negative) as the
 // Hessian stages read them.  A resident J is read in place.  Streamed rows are gathered into the
 // tile, up to 32 listed rows at a time and up4(nv) floats apart: the stages read a row many times
@@ -111,13 +125,21 @@ __device__ __forceinline__ ListRow list_row(const World& s, int t, int t0) {
   o.D = __int_as_float(__float_as_int(s.Dsm[r]) ^ ((id & 0x8000) << 16));
   return o;
 }
-template <bool JRES>
+template <bool JRES, bool J16>
 __device__ __forceinline__ void gather_rows(const World& s, int t0, int t1) {
   if (JRES) return;
   __syncwarp();  // every lane is done with the tile's previous contents
   const int ld = (s.nv + 3) & ~3, lane = s.lane;
   const int ids = t0 + lane < t1 ? s.ids[t0 + lane] & 0x7FFF : 0;
   uint32_t dst = smem_u32(s.Jsm + lane);
+  if (J16) {
+    dst = smem_u32(s.Jsm + 4 * lane);
+#pragma unroll 4
+    for (int t = t0; t < t1; ++t, dst += 4u * ld) {
+      const float* src = s.Jg + (size_t)__shfl_sync(IMN_FULL_MASK, ids, t - t0) * s.ldj + 4 * lane;
+      if (4 * lane < s.nv) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    }
+  } else
 #pragma unroll 4
   for (int t = t0; t < t1; ++t, dst += 4u * ld) {
     const float* src = s.Jg + (size_t)__shfl_sync(IMN_FULL_MASK, ids, t - t0) * s.ldj + lane;
@@ -177,7 +199,7 @@ __device__ __forceinline__ void write_union(const World& s, int count) {
 // outM = M v over the symmetric rows (newton_fusion.py:171-176) and
 // outJ[r] = J[r,:] v (- minus[r]): one running sum per row; above 50 dofs in
 // 20-dof partials joined by plain adds (newton_stages.py:157-174).
-template <bool JRES, bool TSM>
+template <bool JRES, bool J16, bool TSM>
 __device__ __forceinline__ void products(const World& s, const float* v, float* outM, float* outJ,
                                          const float* minus) {
   const int lane = s.lane, nv = s.nv;
@@ -208,18 +230,26 @@ __device__ __forceinline__ void products(const World& s, const float* v, float* 
   const int chunk = nv > 50 ? 20 : nv;
 #pragma unroll 1
   for (int base = 0; base < s.nefc; base += 32) {
-    const float* Jt = j_tile<JRES>(s, base);
+    const float* Jt = j_tile<JRES, J16>(s, base);
     const int r = base + lane;
     if (r < s.nefc) {
-      const float* Jr = Jt + lane * s.ldj;
+      const float* Jr = Jt + lane * (J16 ? s.ldp : s.ldj);
       const float sub = minus ? minus[r] : 0.0f;
       float total = 0.0f;
 #pragma unroll 1
       for (int s0 = 0; s0 < nv; s0 += chunk) {
         float p = 0.0f;
         const int e = min(s0 + chunk, nv);
+        if (J16) {
+#pragma unroll 5
+          for (int i = s0; i < e; i += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(Jr + i), x = *reinterpret_cast<const float4*>(v + i);
+            p = fmaf(a.w, x.w, fmaf(a.z, x.z, fmaf(a.y, x.y, fmaf(a.x, x.x, p))));
+          }
+        } else {
 #pragma unroll 4
-        for (int i = s0; i < e; ++i) p = fmaf(Jr[i], v[i], p);
+          for (int i = s0; i < e; ++i) p = fmaf(Jr[i], v[i], p);
+        }
         if (s0 == 0)
           total = minus ? p - sub : (nv > 50 ? 0.0f + p : p);
         else
@@ -274,7 +304,7 @@ __device__ __forceinline__ float full_gradient(const World& s, int nfr) {
 // A lane owns 4 x 4 blocks of the upper triangle: eight values of a row feed 16 fused
 // multiply-adds, so the stage is bound by arithmetic instead of by shared-memory reads (an entry
 // per lane reads two values and looks its row up for every multiply-add).
-template <bool JRES>
+template <bool JRES, bool J16>
 __device__ __forceinline__ void hessian_dense(const World& s, int count, bool first) {
   const int lane = s.lane, nv = s.nv, ldu = s.ldu;
   float* A = s.A;
@@ -294,7 +324,7 @@ __device__ __forceinline__ void hessian_dense(const World& s, int count, bool fi
 #pragma unroll 1
   for (int t0 = 0; t0 < count; t0 += step) {
     const int t1 = min(t0 + step, count);
-    gather_rows<JRES>(s, t0, t1);
+    gather_rows<JRES, J16>(s, t0, t1);
     __syncwarp();
     IMN_MARK(s, 22);
     const bool keep = t0 > 0 || first, last = t1 == count;
@@ -380,7 +410,7 @@ __device__ __noinline__ void count_violations(bool first, const float* Jw, int l
 // tables are read coalesced once per call, a slot costs four instructions per row, and no pair list
 // of touched dofs has to be formed and looked up.  `outside`: the world has a row whose dofs do not
 // all lie in the pattern.  Sums of a list that does not fit one tile wait in N.
-template <bool JRES, bool TSM>
+template <bool JRES, bool J16, bool TSM>
 __device__ __forceinline__ void hessian_sparse(const World& s, int count, bool first, bool outside, const ImnSparsePlan& SP) {
   const int lane = s.lane, nv = s.nv, nfac = SP.nfac;
   constexpr int Q = JRES ? 10 : 12;
@@ -389,7 +419,7 @@ __device__ __forceinline__ void hessian_sparse(const World& s, int count, bool f
   int t0 = 0;
   do {
     const int t1 = min(t0 + step, count);
-    gather_rows<JRES>(s, t0, t1);
+    gather_rows<JRES, J16>(s, t0, t1);
     IMN_MARK(s, 22);
     const bool last = t1 == count;
 #pragma unroll 1
