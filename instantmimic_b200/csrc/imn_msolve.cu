@@ -87,124 +87,227 @@ __global__ void tree_ldl_kernel(const int4* __restrict__ prog, const int* __rest
 // order as the plain row-by-row statement of the algorithm (ascending t).
 static const int kDenseWarps = 4;
 
-// LW lanes work on one world: 32 (a warp per world), or 16 for models whose n + carry
-// columns fit three columns per lane of a half-warp (<= 48), where a whole warp would leave
-// half its lanes without a column for most of the factorisation; a warp then factors two
-// worlds at once.  `l` is the lane within the team, `base` the team's first lane (shuffle
-// sources are base | lane-in-team).
-template <int LW>
-__device__ __forceinline__ void dense_factor_carry(float* A, float* dinv, const int n, const int nc, const int ldu,
-                                                   const int l, const int base) {
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// A warp per world, `l` its lane.  What bounds the kernel is the chain of a world's rows and the warps
+// an SM holds to cover it: registers for 28 warps per SM (models up to 64 columns), so that 4096 worlds are
+// in flight at once.  4096 humanoid worlds, three right-hand sides, then one with the stored factor:
+// 104 us with two worlds per warp, three column groups throughout and 15 shuffles per row; 95 at 24
+// warps per SM; 69 as it is (65536 worlds: 1432 -> 958).  Two worlds per warp halve the warps and take
+// three column groups for one or two: slower at every batch size.
+//
+// Rows b0 .. b0 + 15 at the K column groups that are left.  As in the Newton factor
+// (imn_newton_factor.cuh): the pivot of row r + 1 is its own lane's sum after row r and travels at
+// once, the row's block entries come back from shared memory as broadcast reads, four rows per trip.
+template <int K>
+__device__ __forceinline__ void dense_block(float* A, float* dinv, const int b0, const int n, const int nc, const int ldu,
+                                            const int l) {
+  const int nr = min(16, n - b0);
+  float acc[K][16];
+  int cc[K];
+  bool valid[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int c = b0 + l + 32 * k;
+    valid[k] = c < nc;
+    cc[k] = valid[k] ? c : nc - 1;
+    const float* src = A + (cc[k] + 1) * ldu + b0;
+#pragma unroll
+    for (int g = 0; g < 16; g += 4) {
+      const float4 h = g < nr ? ld4(src + g) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      acc[k][g] = h.x, acc[k][g + 1] = h.y, acc[k][g + 2] = h.z, acc[k][g + 3] = h.w;
+    }
+  }
+  // terms of the rows above the block
+#pragma unroll 2
+  for (int t = 0; t < b0; ++t) {
+    const float* Ut = A + t * ldu;
+    float uc[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) uc[k] = Ut[cc[k]];
+#pragma unroll
+    for (int g = 0; g < 16; g += 4) {
+      const float4 u = ld4(Ut + b0 + g);  // past the last row: values that end in sums nobody stores
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        acc[k][g] = fmaf(-u.x, uc[k], acc[k][g]), acc[k][g + 1] = fmaf(-u.y, uc[k], acc[k][g + 1]);
+        acc[k][g + 2] = fmaf(-u.z, uc[k], acc[k][g + 2]), acc[k][g + 3] = fmaf(-u.w, uc[k], acc[k][g + 3]);
+      }
+    }
+  }
+  __syncwarp();  // row b0 of U goes where column b0 - 1 stood
+  float pv = __shfl_sync(IMN_FULL_MASK, acc[0][0], 0);
+#pragma unroll 1
+  for (int g = 0; g < nr; g += 4) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = g + q;
+      if (r >= nr) break;  // uniform: one model
+      const float dg = sqrtf(pv), rinv = 1.0f / dg;
+      float* Ur = A + (b0 + r) * ldu;
+      float u[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) u[k] = acc[k][q] * rinv;
+      pv = __shfl_sync(IMN_FULL_MASK, fmaf(-u[0], u[0], acc[0][q + 1]), r + 1);
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (valid[k] && cc[k] >= b0 + r) Ur[cc[k]] = k == 0 && l == r ? dg : u[k];
+      if (l == 0) dinv[b0 + r] = rinv;
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < 16; h += 4) {
+        const float4 m = ld4(Ur + b0 + g + h);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          if (h > q) acc[k][h] = fmaf(-m.x, u[k], acc[k][h]);
+          if (h + 1 > q) acc[k][h + 1] = fmaf(-m.y, u[k], acc[k][h + 1]);
+          if (h + 2 > q) acc[k][h + 2] = fmaf(-m.z, u[k], acc[k][h + 2]);
+          if (h + 3 > q) acc[k][h + 3] = fmaf(-m.w, u[k], acc[k][h + 3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int h = 0; h < 16; ++h) acc[k][h] = h < 12 ? acc[k][h + 4] : 0.0f;
+  }
+  __syncwarp();
+}
+
+template <int KM>
+__device__ __forceinline__ void dense_factor_carry(float* A, float* dinv, const int n, const int nc, const int ldu, const int l) {
 #pragma unroll 1
   for (int b0 = 0; b0 < n; b0 += 16) {
-    const int nr = min(16, n - b0);
-    const int ng = (nr + 3) >> 2;
-    float acc[3][16];
-    int cc[3];
-    bool act[3], valid[3];
+    if (nc - b0 <= 32)
+      dense_block<1>(A, dinv, b0, n, nc, ldu, l);
+    else if (KM == 2 || nc - b0 <= 64)
+      dense_block<2>(A, dinv, b0, n, nc, ldu, l);
+    else
+      dense_block<KM>(A, dinv, b0, n, nc, ldu, l);
+  }
+}
+
+// Forward substitution with the stored factor for right-hand sides [q0, q0 + RQ): a lane keeps rows
+// l, l + 32, l + 64 of each in registers, so that a column of U is read once for all of them
+// and the only traffic between lanes is the finished unknown.  Unknown r receives its terms in
+// ascending order.
+template <int KM, int RQ>
+__device__ __forceinline__ void dense_forward(const float* A, const float* dinv, float* X, const int n, const int ldu,
+                                              const int rhs, const int q0, const int l) {
+  float x[RQ][KM];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const int c = b0 + l + LW * k;
-      act[k] = b0 + LW * k < nc;  // uniform over the team (and over the warp: one model)
-      valid[k] = c < nc;
-      cc[k] = valid[k] ? c : nc - 1;
-      if (act[k]) {
-        const float* src = A + (cc[k] + 1) * ldu + b0;
+  for (int k = 0; k < KM; ++k)
 #pragma unroll
-        for (int gi = 0; gi < 4; ++gi) {
-          float4 h = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (gi < ng) h = *reinterpret_cast<const float4*>(src + 4 * gi);
-          acc[k][4 * gi] = h.x, acc[k][4 * gi + 1] = h.y, acc[k][4 * gi + 2] = h.z, acc[k][4 * gi + 3] = h.w;
-        }
-      } else {
+    for (int j = 0; j < RQ; ++j) x[j][k] = l + 32 * k < n && q0 + j < rhs ? X[(l + 32 * k) * rhs + q0 + j] : 0.0f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc[k][i] = 0.0f;
-      }
-    }
-    // terms of the rows above the block
+  for (int kb = 0; kb < KM; ++kb) {
+    const int tn = min(32, n - 32 * kb);
 #pragma unroll 2
-    for (int t = 0; t < b0; ++t) {
-      const float* Ut = A + t * ldu;
-      float ur[16];
+    for (int tl = 0; tl < tn; ++tl) {
+      const int t = 32 * kb + tl;
+      const float di = dinv[t];
+      float a[KM];
 #pragma unroll
-      for (int gi = 0; gi < 4; ++gi) {
-        float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (gi < ng) u = *reinterpret_cast<const float4*>(Ut + b0 + 4 * gi);
-        ur[4 * gi] = u.x, ur[4 * gi + 1] = u.y, ur[4 * gi + 2] = u.z, ur[4 * gi + 3] = u.w;
+      for (int k = kb; k < KM; ++k) {
+        const int r = l + 32 * k;
+        a[k] = r > t && r < n ? A[t * ldu + r] : 0.0f;
       }
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
-        if (act[k]) {
-          const float uc = Ut[cc[k]];
+      for (int j = 0; j < RQ; ++j) {
+        const float yt = __shfl_sync(IMN_FULL_MASK, x[j][kb], tl) * di;
 #pragma unroll
-          for (int gi = 0; gi < 4; ++gi)
-            if (gi < ng) {  // warp-uniform: a short last block skips its absent rows
-#pragma unroll
-              for (int i = 4 * gi; i < 4 * gi + 4; ++i) acc[k][i] = fmaf(-ur[i], uc, acc[k][i]);
-            }
-        }
+        for (int k = kb; k < KM; ++k) x[j][k] = fmaf(-a[k], yt, x[j][k]);
+        if (l == tl) x[j][kb] = yt;
+      }
     }
-    // the block's own rows, one by one; acc[k][0] is always the current row.  Row b0 + r's
-    // column is held by lane r of the team (k = 0); the rows below it inside the block by
-    // lanes r + 1 .. 15 (later sources wrap and feed slots that are never read).
+  }
+#pragma unroll
+  for (int k = 0; k < KM; ++k)
+#pragma unroll
+    for (int j = 0; j < RQ; ++j)
+      if (l + 32 * k < n && q0 + j < rhs) X[(l + 32 * k) * rhs + q0 + j] = x[j][k];
+  __syncwarp();
+}
+
+// Back substitution of the same right-hand sides in 16-row blocks from the last: later blocks'
+// columns first (ascending), then the block's own columns from its last inwards.  The upper half of
+// the warp takes the next RQ right-hand sides.
+template <int RQ>
+__device__ __forceinline__ void dense_back(const float* A, const float* dinv, float* X, const int n, const int ldu, const int rhs,
+                                           int q0, const int l) {
+  q0 += (l >> 4) * RQ;
+  const int l16 = l & 15;
 #pragma unroll 1
-    for (int r = 0; r < nr; ++r) {
-      const float pv = __shfl_sync(IMN_FULL_MASK, acc[0][0], base | r);
-      const float dg = sqrtf(pv);
-      const float rinv = 1.0f / dg;
-      float u[3];
-      float* Ur = A + (b0 + r) * ldu;
+  for (int b0 = ((n - 1) / 16) * 16; b0 >= 0; b0 -= 16) {
+    const int b1 = min(b0 + 16, n), r = min(b0 + l16, n - 1);
+    const bool mine = b0 + l16 < b1;
+    const float* Ur = A + r * ldu;
+    const float di = dinv[r];
+    float acc[RQ];
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
-        if (act[k]) {
-          u[k] = acc[k][0] * rinv;
-          if (k == 0 && l == r) u[k] = dg;
-          if (valid[k] && cc[k] >= b0 + r) Ur[cc[k]] = u[k];
-        }
-      if (l == 0) dinv[b0 + r] = rinv;
-      float um[16];
+    for (int j = 0; j < RQ; ++j) acc[j] = mine && q0 + j < rhs ? X[r * rhs + q0 + j] : 0.0f;
+    int c = b1;
+#pragma unroll 2
+    for (; c + 4 <= n; c += 4) {
+      const float4 u = ld4(Ur + c);
+      const float uu[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-      for (int j = 1; j < 16; ++j) um[j] = __shfl_sync(IMN_FULL_MASK, u[0], base | ((r + j) & (LW - 1)));
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
-        if (act[k]) {
-#pragma unroll
-          for (int j = 1; j < 16; ++j) acc[k][j - 1] = fmaf(-um[j], u[k], acc[k][j]);
-          acc[k][15] = 0.0f;
-        }
+        for (int j = 0; j < RQ; ++j) acc[j] = fmaf(-uu[i], X[(c + i) * rhs + min(q0 + j, rhs - 1)], acc[j]);
     }
+#pragma unroll 1
+    for (; c < n; ++c)
+#pragma unroll
+      for (int j = 0; j < RQ; ++j) acc[j] = fmaf(-Ur[c], X[c * rhs + min(q0 + j, rhs - 1)], acc[j]);
+#pragma unroll 2
+    for (int c = b1 - 1; c >= b0; --c) {
+      const float u = Ur[c];
+#pragma unroll
+      for (int j = 0; j < RQ; ++j) {
+        const float xc = __shfl_sync(IMN_FULL_MASK, acc[j] * di, (l & ~15) | (c - b0));
+        if (b0 + l16 < c) acc[j] = fmaf(-u, xc, acc[j]);
+      }
+    }
+    // row b0 + l16 is final: its unknown is its sum scaled
+#pragma unroll
+    for (int j = 0; j < RQ; ++j)
+      if (mine && q0 + j < rhs) X[r * rhs + q0 + j] = acc[j] * di;
     __syncwarp();
   }
 }
 
-template <int LW>
-__global__ void __launch_bounds__(32 * kDenseWarps)
+template <int KM, int RQ>
+__device__ __forceinline__ void dense_substitute(const float* A, const float* dinv, float* X, const int n, const int ldu,
+                                                 const int rhs, const int carried, const int l) {
+#pragma unroll 1
+  for (int q = carried; q < rhs; q += RQ) dense_forward<KM, RQ>(A, dinv, X, n, ldu, rhs, q, l);
+#pragma unroll 1
+  for (int q = 0; q < rhs; q += 2 * RQ) dense_back<RQ>(A, dinv, X, n, ldu, rhs, q, l);
+}
+
+template <int KM>
+__global__ void __launch_bounds__(32 * kDenseWarps, KM == 2 ? 7 : 4)
     blocked_dense_kernel(const int nv, const int pad, const int nM, const int* __restrict__ indices,
                          const float* __restrict__ identity, const float* __restrict__ M, const int64_t M_ld,
                          const float* __restrict__ y, float* __restrict__ Ug, float* __restrict__ x,
                          const int* __restrict__ active, const int rhs, const int mode, const int carry,
-                         const int ldu, const int per_world, const int nworld) {
+                         const int ldu, const int per_world, const int vec, const int nworld) {
   extern __shared__ __align__(16) float sm[];
-  constexpr int kPer = 32 / LW;  // worlds per warp
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int l = lane & (LW - 1), base = lane & ~(LW - 1), sub = lane / LW;
-  const int first = (blockIdx.x * kDenseWarps + warp) * kPer;
-  if (first >= nworld) return;
-  const int wreal = first + sub;
-  // a team without a world, or with an inactive one, runs along on the warp's first
-  // world (the shuffles are full-warp) and stores nothing
-  bool live = wreal < nworld;
-  if (live && active && active[wreal] == 0) live = false;
-  if (!__any_sync(IMN_FULL_MASK, live)) return;
-  const int w = wreal < nworld ? wreal : first;
+  const int l = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int w = blockIdx.x * kDenseWarps + warp;
+  if (w >= nworld || (active && active[w] == 0)) return;
   const int n = nv, nc = n + carry;
-  float* A = sm + (warp * kPer + sub) * per_world;
+  float* A = sm + warp * per_world;
   float* dinv = A + (nc + 1) * ldu;
   float* X = dinv + ((n + 3) & ~3);
   float* Uw = Ug + (size_t)w * pad * pad;
   const int nblk = pad >> 4;
+  // four columns per lane of a row of U, several rows at a time (pad <= 80)
+  const int quads = pad >> 2, vrows = 32 / quads;
+  const int vr = l / quads < vrows ? l / quads : n, c = 4 * (l % quads);
   const float* yw = y + (size_t)w * n * rhs;
-  for (int q = l; q < n * rhs; q += LW) X[q] = yw[q];
+  for (int q = l; q < n * rhs; q += 32) X[q] = yw[q];
   if (mode == 0) {
     // gather the blocks on and above the diagonal: table entry
     // ((kb*nblk + ib)*16 + r)*16 + c addresses M's value of (16 kb + r, 16 ib + c);
@@ -214,89 +317,69 @@ __global__ void __launch_bounds__(32 * kDenseWarps)
       for (int ib = kb; ib < nblk; ++ib) {
         const int* tab = indices + ((kb * nblk + ib) << 8);
 #pragma unroll 4
-        for (int q = l; q < 256; q += LW) {
+        for (int q = l; q < 256; q += 32) {
           const int row = 16 * kb + (q >> 4), colm = 16 * ib + (q & 15);
           const int idx = __ldg(tab + q);
           if (row <= colm && colm < n) A[(colm + 1) * ldu + row] = idx < nM ? __ldg(Mw + idx) : 0.0f;
         }
       }
     __syncwarp();
-    for (int e = l; e < n * carry; e += LW) {
+    for (int e = l; e < n * carry; e += 32) {
       const int r = e / carry, q = e - r * carry;
       A[(n + q + 1) * ldu + r] = X[r * rhs + q];
     }
     __syncwarp();
-    dense_factor_carry<LW>(A, dinv, n, nc, ldu, l, base);
-    // the factor, padded: zeros below the diagonal, the padded diagonal's own root
-    if (live) {
+    dense_factor_carry<KM>(A, dinv, n, nc, ldu, l);
+    // the factor, padded: zeros below the diagonal, the padded diagonal's own root; four columns
+    // per store where the workspace allows it
+    if (vec) {
+#pragma unroll 4
+      for (int r = vr; r < n; r += vrows) {
+        const float4 a = c < ldu ? ld4(A + r * ldu + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float4 o;
+        o.x = c >= r && c < n ? a.x : 0.0f, o.y = c + 1 >= r && c + 1 < n ? a.y : 0.0f;
+        o.z = c + 2 >= r && c + 2 < n ? a.z : 0.0f, o.w = c + 3 >= r && c + 3 < n ? a.w : 0.0f;
+        *reinterpret_cast<float4*>(Uw + r * pad + c) = o;
+      }
+    } else {
       for (int r = 0; r < n; ++r) {
         const float* Ar = A + r * ldu;
         float* Ur = Uw + r * pad;
 #pragma unroll 3
-        for (int c = l; c < pad; c += LW) Ur[c] = (c >= r && c < n) ? Ar[c] : 0.0f;
-      }
-      for (int r = n; r < pad; ++r) {
-        const float dg = sqrtf(identity[((r & 15) << 4) | (r & 15)]);
-        for (int c = l; c < pad; c += LW) Uw[r * pad + c] = c == r ? dg : 0.0f;
+        for (int c = l; c < pad; c += 32) Ur[c] = (c >= r && c < n) ? Ar[c] : 0.0f;
       }
     }
-    for (int e = l; e < n * carry; e += LW) {
+    for (int r = n; r < pad; ++r) {
+      const float dg = sqrtf(identity[((r & 15) << 4) | (r & 15)]);
+      for (int c = l; c < pad; c += 32) Uw[r * pad + c] = c == r ? dg : 0.0f;
+    }
+    for (int e = l; e < n * carry; e += 32) {
       const int r = e / carry, q = e - r * carry;
       X[r * rhs + q] = A[r * ldu + n + q];
     }
   } else {
-    for (int r = 0; r < n; ++r)
-      for (int c = r + l; c < n; c += LW) A[r * ldu + c] = Uw[r * pad + c];
+    if (vec) {
+#pragma unroll 8
+      for (int r = vr; r < n; r += vrows)
+        if (c + 3 >= r && c < n) *reinterpret_cast<float4*>(A + r * ldu + c) = *reinterpret_cast<const float4*>(Uw + r * pad + c);
+    } else {
+      for (int r = 0; r < n; ++r)
+        for (int c = r + l; c < n; c += 32) A[r * ldu + c] = Uw[r * pad + c];
+    }
     __syncwarp();
-    for (int r = l; r < n; r += LW) dinv[r] = 1.0f / A[r * ldu + r];
+    for (int r = l; r < n; r += 32) dinv[r] = 1.0f / A[r * ldu + r];
   }
   __syncwarp();
-  // forward substitution with the stored factor for the right-hand sides that did
-  // not ride along: unknown r receives its terms in ascending order
-  const int q0 = mode == 0 ? carry : 0;
-  if (q0 < rhs) {
-    const int nq = rhs - q0;
-    for (int t = 0; t < n; ++t) {
-      const float di = dinv[t];
-      for (int q = l; q < nq; q += LW) X[t * rhs + q0 + q] = X[t * rhs + q0 + q] * di;
-      __syncwarp();
-      for (int e = l; e < (n - t - 1) * nq; e += LW) {
-        const int r = t + 1 + e / nq, q = q0 + e % nq;
-        X[r * rhs + q] = fmaf(-A[t * ldu + r], X[t * rhs + q], X[r * rhs + q]);
-      }
-      __syncwarp();
-    }
-  }
-  // back substitution in 16-row blocks from the last: later blocks' columns first
-  // (ascending), then the block's own columns from its last inwards; a team of 32 lanes
-  // takes two right-hand sides at a time on its two halves, a team of 16 one
-  constexpr int kRhsAtOnce = LW / 16;
-  for (int qb = 0; qb < rhs; qb += kRhsAtOnce) {
-    const int q = qb + (l >> 4), l16 = l & 15;
-    const bool hasq = q < rhs;
-    for (int b0 = ((n - 1) / 16) * 16; b0 >= 0; b0 -= 16) {
-      const int b1 = min(b0 + 16, n);
-      const int r = b0 + l16;
-      const float* Ur = A + r * ldu;
-      float acc = 0.0f, di = 0.0f;
-      if (r < b1 && hasq) {
-        acc = X[r * rhs + q];
-        di = dinv[r];
-#pragma unroll 2
-        for (int c = b1; c < n; ++c) acc = fmaf(-Ur[c], X[c * rhs + q], acc);
-      }
-      for (int c = b1 - 1; c >= b0; --c) {
-        const float xc = __shfl_sync(IMN_FULL_MASK, acc * di, (lane & ~15) | (c - b0));
-        if (r < c && hasq) acc = fmaf(-Ur[c], xc, acc);
-        if (l16 == 0 && hasq) X[c * rhs + q] = xc;
-      }
-      __syncwarp();
-    }
-  }
-  if (live) {
-    float* xw = x + (size_t)w * n * rhs;
-    for (int q = l; q < n * rhs; q += LW) xw[q] = X[q];
-  }
+  // right-hand sides one, two or four at a time
+  const int carried = mode == 0 ? carry : 0;
+  if (rhs == 1)
+    dense_substitute<KM, 1>(A, dinv, X, n, ldu, rhs, carried, l);
+  else if (rhs == 2)
+    dense_substitute<KM, 2>(A, dinv, X, n, ldu, rhs, carried, l);
+  else
+    dense_substitute<KM, 4>(A, dinv, X, n, ldu, rhs, carried, l);
+  float* xw = x + (size_t)w * n * rhs;
+  for (int q = l; q < n * rhs; q += 32) xw[q] = X[q];
 }
 
 }  // namespace imn
@@ -347,14 +430,15 @@ extern "C" int imn_blocked_dense_factor_solve(const ImnBlockedPlan* plan, const 
   if (n > 80) return imn::set_error("imn_blocked_dense_factor_solve: nv %d above 80", n), IMN_ERR_UNSUPPORTED;
   // right-hand sides that ride through the factorisation as extra columns
   const int carry = mode == 0 ? (rhs_count < 96 - n ? rhs_count : 96 - n) : 0;
-  const int ldu = (n + carry + 3) & ~3;
-  const int per_world = (n + carry + 1) * ldu + ((n + 3) & ~3) + ((n * rhs_count + 3) & ~3);
-  // two worlds per warp when every column of the factorisation has a place on 16 lanes
-  // and the batch is large enough to keep the GPU full that way
-  const bool half = n + carry <= 48 && nworld >= 2048;
-  const int per_cta = imn::kDenseWarps * (half ? 2 : 1);
+  // rows of an odd number of quads: 128-bit reads of one quad from consecutive rows meet no bank twice
+  // (the largest models with many right-hand sides only fit without)
+  auto floats = [&](int ld) { return (n + carry + 1) * ld + ((n + 3) & ~3) + ((n * rhs_count + 3) & ~3); };
+  int ldu = 4 * (((n + carry + 3) >> 2) | 1);
+  if (sizeof(float) * (size_t)floats(ldu) * imn::kDenseWarps > 227 * 1024) ldu = (n + carry + 3) & ~3;
+  const int per_world = floats(ldu);
+  const int per_cta = imn::kDenseWarps;
   const size_t bytes = sizeof(float) * (size_t)per_world * per_cta;
-  auto kernel = half ? imn::blocked_dense_kernel<16> : imn::blocked_dense_kernel<32>;
+  auto kernel = n + carry <= 64 ? imn::blocked_dense_kernel<2> : imn::blocked_dense_kernel<3>;
   if (bytes > 227 * 1024)
     return imn::set_error("imn_blocked_dense_factor_solve: %zu bytes of shared memory needed (max %d)", bytes,
                           227 * 1024),
@@ -368,9 +452,10 @@ extern "C" int imn_blocked_dense_factor_solve(const ImnBlockedPlan* plan, const 
       return imn::set_error("imn_blocked_dense_factor_solve: cudaFuncSetAttribute: %s", cudaGetErrorString(e)),
              IMN_ERR_LAUNCH;
   }
+  const int vec = (reinterpret_cast<uintptr_t>(U) & 15) == 0;  // pad is a multiple of 16 floats
   kernel<<<(nworld + per_cta - 1) / per_cta, 32 * imn::kDenseWarps, bytes, (cudaStream_t)stream>>>(
       plan->nv, plan->pad, plan->nM, plan->indices, plan->identity, M, M_ld, y, U, x, active, rhs_count, mode, carry, ldu,
-      per_world, nworld);
+      per_world, vec, nworld);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return imn::set_error("imn_blocked_dense_factor_solve: launch failed: %s", cudaGetErrorString(e)),

@@ -1,0 +1,34 @@
+"""Blocked dense factor + solve around the edges of its launch rules: the column counts where the
+two-group kernel ends (64), right-hand sides around the groups they are solved in, and a workspace that
+does not lie on a 16-byte boundary."""
+
+import numpy as np
+import pytest
+
+from instantmimic_b200 import mjw_model
+from instantmimic_b200.mjw_kernels import indexed_factor
+
+from test_msolve import _blocked_case
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nv,rhs,offset", [(63, 1, 0), (64, 1, 0), (60, 4, 1), (33, 5, 1), (34, 9, 0), (48, 18, 3)])
+def test_dense_factor_edges(oracle, cuda_device, nv, rhs, offset):
+    import torch
+
+    worlds = 10
+    m, Mv, _, pad, layout, ident, y = _blocked_case(nv, worlds, rhs)
+    md = mjw_model.to_device(m, cuda_device)
+    dd = mjw_model.to_device(mjw_model.make_data(m, worlds, 4), cuda_device)
+    scratch = indexed_factor.create_blocked_dense_factor_solve_scratch(md, dd, cuda_device)
+    Mt, yt = torch.from_numpy(Mv).to(cuda_device), torch.from_numpy(y).to(cuda_device)
+    active = torch.ones(worlds, dtype=torch.int32, device=cuda_device)
+    x, x2 = torch.zeros_like(yt), torch.zeros_like(yt)
+    U = torch.zeros(worlds * pad * pad + 4, device=cuda_device)[offset:offset + worlds * pad * pad].view(worlds, pad, pad)
+    indexed_factor.factor_multi_solve(scratch, Mt, yt, active, U, x, rhs)
+    indexed_factor.multi_solve(scratch, U, yt, active, x2, rhs)
+    want_x, want_U = oracle.blocked_dense_factor_solve(nv, pad, layout, ident, Mv, y)
+    np.testing.assert_array_equal(x.cpu().numpy(), want_x)
+    np.testing.assert_array_equal(x2.cpu().numpy(), want_x)
+    np.testing.assert_array_equal(U.cpu().numpy(), want_U)
