@@ -91,7 +91,7 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   g.nv4 = up4(m.nv + 1);  // M_mulm_lanes reads a zero behind a vector
   g.r4 = up4(d.njmax);
   int o = 0;
-  g.oBar = o, o += 4;
+  g.oBar = o, o += 8;  // load barrier, its phase, jfail; tile barrier (J16), its phase
   // a streamed tile may start up to three floats into its buffer and end on a 16-byte boundary
   // a dense block reads up to three floats past a row; the gathered rows are up4(nv) floats apart
   g.ldp = 4 * ((m.nv / 4) | 1);
@@ -188,9 +188,10 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
     s.tab.bstep = reinterpret_cast<const uint2*>(sp.bstep);
   }
   s.M_rowadr = m.M_rowadr, s.M_rownnz = m.M_rownnz, s.M_colind = m.M_colind;
-  s.jbar = bar;
-  s.jphase = reinterpret_cast<int*>(smem + g.oBar) + 2;  // the barrier itself takes two words
-  s.jfail = s.jphase + 1;
+  int* const load_phase_at = reinterpret_cast<int*>(smem + g.oBar) + 2;  // the barrier itself takes two words
+  s.jbar = J16 ? smem + g.oBar + 4 : bar;  // J16: every lane arrives at the tiles' own barrier
+  s.jphase = load_phase_at + (J16 ? 4 : 0);
+  s.jfail = load_phase_at + 1;
   s.wait_polls = g.wait_polls, s.withhold_copies = g.withhold_copies;
   s.Hp = s.A;
   s.N = s.A + (SPARSE ? ((sp.nfac + 3) & ~3) : 0);
@@ -198,7 +199,10 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
   s.Jbeg = d.efc_J;
   s.Jend = d.efc_J + (d.J_world_offset ? (size_t)d.J_elems
                                        : (size_t)(d.nworld - 1) * d.J_ld_world + (size_t)d.njmax * d.J_ld_row);
-  if (lane == 0) mbar_init(bar, 1), *s.jphase = 0;
+  if (lane == 0) {
+    mbar_init(bar, 1), *load_phase_at = 0;
+    if (J16) mbar_init(s.jbar, 32), *s.jphase = 0;
+  }
   __syncwarp();
   if (TSM) {
     auto stage = [&](int at, const void* src, int words) {
@@ -280,12 +284,12 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
             {s.qfs, d.qfrc_smooth + dofo, nv},
         };
         __syncwarp();  // every lane has left the previous world
-        const uint32_t load_phase = (uint32_t)*s.jphase;
+        const uint32_t load_phase = (uint32_t)*load_phase_at;
         // the previous world's values were written through the generic proxy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) {
-          *s.jphase = (int)(load_phase ^ 1u);
+          *load_phase_at = (int)(load_phase ^ 1u);
           *s.jfail = 0;
         }
         __syncwarp();
@@ -326,7 +330,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
           if (lane == 0) {
             d.overflow[w] |= IMN_OVERFLOW_COPY_TIMEOUT;
             mbar_restart(bar, 1);
-            *s.jphase = 0;
+            *load_phase_at = 0;
           }
         } else {
           have = true, first = true;
@@ -482,10 +486,10 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         const uint32_t parity = (uint32_t)*s.jphase ^ 1u;
         bool arrived = false;
 #pragma unroll 1
-        for (int tries = 0; tries < g.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(bar, parity);
+        for (int tries = 0; tries < g.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(s.jbar, parity);
         if (lane == 0) {
           d.overflow[w] |= IMN_OVERFLOW_COPY_TIMEOUT;
-          mbar_restart(bar, 1);
+          mbar_restart(s.jbar, J16 ? 32 : 1);
           *s.jphase = 0;
         }
         finished = true, failed = true;

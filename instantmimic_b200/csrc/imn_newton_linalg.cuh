@@ -56,14 +56,28 @@ struct World {
 #define IMN_MARK(s, k)
 #endif
 
+// J16: the elements of up to 32 rows in pieces of 16 bytes, consecutive lanes on consecutive pieces,
+// nv / 4 pieces per row; f(row, piece) copies one.
+template <typename F>
+__device__ __forceinline__ void each_piece(const World& s, int rows, F f) {
+  const int n = s.nv >> 2, dr = 32 / n, dc = 32 - dr * n;
+  int row = s.lane / n, c = s.lane - row * n;
+#pragma unroll 4
+  while (row < rows) {
+    f(row, c);
+    row += dr, c += dc;
+    if (c >= n) c -= n, ++row;
+  }
+}
+
 // Rows [base, base+32) of J: resident rows are addressed in place, otherwise they are staged
-// through the 32-row tile by TMA bulk copies on the world's mbarrier; the wait is bounded.
-// J16 (streamed only; nv, the row stride and every row multiples of four floats): one copy per row,
-// a row per lane, to a stride of ldp floats, a multiple of four with ldp / 4 odd.  With lane = row the
-// 128-bit reads of eight consecutive lanes then hit eight different groups of four banks; at their
-// own stride the rows of such models (56, 64 floats) put 4 or all 32 lanes on one bank.
-// (64 dofs x 512 rows, 4096 worlds: 7326 -> 4816 us per solve; 56 x 128: 1206 -> 1189.)
-// Otherwise rows keep their own stride and the tile is one contiguous copy.
+// through the 32-row tile; the wait for the copies is bounded.
+// J16 (streamed only; nv, the row stride and every row multiples of four floats): 16-byte copies to a
+// row stride of ldp floats, a multiple of four with ldp / 4 odd.  With lane = row the 128-bit reads of
+// eight consecutive lanes then hit eight different groups of four banks; at their own stride the rows
+// of such models (56, 64 floats) put 4 or all 32 lanes on one bank.  (64 dofs x 512 rows, 4096
+// worlds: 7326 -> 4816 us per solve with a bulk copy per row; 4621 with the pieces.)
+// Otherwise rows keep their own stride and the tile is one contiguous TMA bulk copy.
 template <bool JRES, bool J16>
 __device__ __forceinline__ const float* j_tile(const World& s, int base) {
   if (JRES) return s.Jsm + base * s.ldj;
@@ -75,21 +89,22 @@ __device__ __forceinline__ const float* j_tile(const World& s, int base) {
   // copied (up to three floats of the neighbouring rows on either side, still inside the J
   // array) and the tile starts `head` floats into the buffer.
   const int head = J16 ? 0 : (int)((reinterpret_cast<uintptr_t>(src) & 15) >> 2);
-  const uint32_t bytes = J16 ? (uint32_t)(rows * s.nv) * 4u : (uint32_t)((head + n + 3) & ~3) * 4u;
+  const uint32_t bytes = (uint32_t)((head + n + 3) & ~3) * 4u;
   // after a copy that timed out the barrier's phase is unknown: the world is lost (the
   // caller checks jfail at the end of the pass) and the rest of the pass uses plain loads
   if ((J16 || (src - head >= s.Jbeg && src - head + (bytes >> 2) <= s.Jend)) && !*s.jfail) {
     const uint32_t parity = (uint32_t)*s.jphase;
     __syncwarp();
-    if (s.lane == 0) {
-      mbar_expect_tx(s.jbar, bytes);
-      if (!J16 && !(s.withhold_copies & 2)) bulk_g2s(s.Jsm, src - head, bytes, s.jbar);
-      *s.jphase = (int)(parity ^ 1u);
-    }
     if (J16) {
-      __syncwarp();  // the barrier expects the bytes before the first of them arrives
-      if (s.lane < rows && !(s.withhold_copies & 2))
-        bulk_g2s(s.Jsm + s.lane * s.ldp, src + (size_t)s.lane * s.ldj, (uint32_t)s.nv * 4u, s.jbar);
+      if (s.lane == 0) *s.jphase = (int)(parity ^ 1u);
+      if (!(s.withhold_copies & 2)) {
+        each_piece(s, rows, [&](int row, int c) { copy16(s.Jsm + row * s.ldp + 4 * c, src + (size_t)row * s.ldj + 4 * c); });
+        mbar_arrive_copies(s.jbar);
+      }
+    } else if (s.lane == 0) {
+      mbar_expect_tx(s.jbar, bytes);
+      if (!(s.withhold_copies & 2)) bulk_g2s(s.Jsm, src - head, bytes, s.jbar);
+      *s.jphase = (int)(parity ^ 1u);
     }
     bool arrived = false;
 #pragma unroll 1
@@ -130,16 +145,16 @@ __device__ __forceinline__ void gather_rows(const World& s, int t0, int t1) {
   if (JRES) return;
   __syncwarp();  // every lane is done with the tile's previous contents
   const int ld = (s.nv + 3) & ~3, lane = s.lane;
+  if (J16) {
+    each_piece(s, t1 - t0, [&](int row, int c) {
+      copy16(s.Jsm + row * ld + 4 * c, s.Jg + (size_t)(s.ids[t0 + row] & 0x7FFF) * s.ldj + 4 * c);
+    });
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    return;
+  }
   const int ids = t0 + lane < t1 ? s.ids[t0 + lane] & 0x7FFF : 0;
   uint32_t dst = smem_u32(s.Jsm + lane);
-  if (J16) {
-    dst = smem_u32(s.Jsm + 4 * lane);
-#pragma unroll 4
-    for (int t = t0; t < t1; ++t, dst += 4u * ld) {
-      const float* src = s.Jg + (size_t)__shfl_sync(IMN_FULL_MASK, ids, t - t0) * s.ldj + 4 * lane;
-      if (4 * lane < s.nv) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-    }
-  } else
 #pragma unroll 4
   for (int t = t0; t < t1; ++t, dst += 4u * ld) {
     const float* src = s.Jg + (size_t)__shfl_sync(IMN_FULL_MASK, ids, t - t0) * s.ldj + lane;
