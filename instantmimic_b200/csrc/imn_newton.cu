@@ -1,4 +1,4 @@
-// imn_newton.cu -- the fused Newton constraint solve, one warp per world.
+// imn_newton.cu -- the fused Newton constraint solve, a warp or a small team of warps per world.
 //
 // One launch replaces the reference's whole solve pipeline
 // (mjw_step_optimized.py:2588-2680): _solve_init_dof, the init of
@@ -7,16 +7,17 @@
 // newton_fusion.py:170-296 and the final qfrc_constraint_from_grad.
 //
 // B200 mapping.  The solve is latency-bound small dense algebra (nv <= 79), not a
-// tensor-core contraction, so the design goal is to touch HBM exactly once: a CTA
-// is one warp that owns one world.  Its J and row data arrive in shared memory
+// tensor-core contraction, so the design goal is to touch HBM exactly once: a warp owns a world, one
+// CTA per SM holds as many worlds as fit.  A world's J and row data arrive in shared memory
 // through TMA bulk copies (cp.async.bulk, one mbarrier; M, read once per iteration,
 // stays in global memory and comes through L1), the Hessian, its
 // Cholesky factor and every vector stay on chip for all iterations, and the
-// results are written once.  A warp needs no block barrier (only __syncwarp),
-// lane reductions are shuffle trees, and the hardware CTA scheduler balances
-// worlds whose iteration counts differ; worlds are launched by descending row count
-// so that the long solves start first.  Models whose J would leave room for few
-// worlds per SM stream it through a 32-row tile (TMA bulk copies from L2) instead.
+// results are written once.  A warp needs no block barrier (only __syncwarp) and
+// lane reductions are shuffle trees; a warp that has finished a world takes the next from a
+// counter, worlds with many rows first, so that iteration counts that differ leave no SM waiting.
+// Models whose J would leave room for few worlds per SM stream it through a 32-row tile (TMA bulk
+// copies or 16-byte pieces from L2) instead.  Where the worlds in hand leave warps of an SM unused (small
+// batches, very large worlds) a team of two to four warps shares each world (plan_launch).
 // The initialisation runs through the same code as an iteration (as "iteration 0"
 // without a line search): the kernel is bound by instruction fetch and latency, so
 // every stage exists once.
@@ -39,7 +40,7 @@ namespace imn {
 __device__ unsigned long long g_prof[16];
 #define PROF_DECL long long prof_t = clock64(); long long prof_acc[16] = {0}; s.prof_acc = prof_acc; s.prof_t = &prof_t
 #define PROF(k) do { const long long t_ = clock64(); prof_acc[k] += t_ - prof_t; prof_t = t_; } while (0)
-#define PROF_FLUSH do { if (lane == 0) for (int k_ = 0; k_ < 16; ++k_) atomicAdd(&g_prof[k_], (unsigned long long)prof_acc[k_]); } while (0)
+#define PROF_FLUSH do { if (tid == 0) for (int k_ = 0; k_ < 16; ++k_) atomicAdd(&g_prof[k_], (unsigned long long)prof_acc[k_]); } while (0)
 #else
 #define PROF_DECL
 #define PROF(k)
@@ -60,6 +61,8 @@ struct Geom {
   // each, offsets above) follow at `tab` words.  warps: worlds in hand per CTA
   bool tsm;
   int tM, tF, tB, tS, tO, tab, warps;
+  // warps per world (make_geom); the tiles of a streamed J are `tile` words apart
+  int parts, tile, oBox;
   // polls a copy wait may take before the world gives up, and the failure-path test
   // switch: when set no bulk copy is issued (plain loads bring the data) while the
   // barrier is told to expect bytes, so the wait runs out with nothing in flight
@@ -79,7 +82,7 @@ static const int kResidentWarps = 16, kStreamedWarps = 12;
 
 static inline int up4(int n) { return (n + 3) & ~3; }
 
-static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const ImnSparsePlan* sp = nullptr) {
+static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const ImnSparsePlan* sp, int parts) {
   Geom g;
   g.nv = m.nv;
   g.njmax = d.njmax;
@@ -91,16 +94,16 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   g.nv4 = up4(m.nv + 1);  // M_mulm_lanes reads a zero behind a vector
   g.r4 = up4(d.njmax);
   int o = 0;
-  g.oBar = o, o += 8;  // load barrier, its phase, jfail; tile barrier (J16), its phase
+  g.parts = parts;
+  g.oBar = o, o += 8 * parts;  // per warp: load barrier, its phase, jfail; tile barrier (J16), its phase
+  g.oBox = o, o += parts > 1 ? 12 : 0;  // single values for the team
   // a streamed tile may start up to three floats into its buffer and end on a 16-byte boundary
   // a dense block reads up to three floats past a row; the gathered rows are up4(nv) floats apart
   g.ldp = 4 * ((m.nv / 4) | 1);
   g.j16 = !resident && m.nv % 4 == 0 && d.J_ld_row % 4 == 0 && !d.J_world_offset && d.J_ld_world % 4 == 0 &&
           (reinterpret_cast<uintptr_t>(d.efc_J) & 15) == 0;
-  if (g.j16)
-    g.oJ = o, o += 32 * g.ldp;
-  else
-    g.oJ = o, o += (resident ? up4(g.jrows * g.ldj + 3) : max(up4(32 * g.ldj) + 8, 32 * up4(m.nv)));
+  g.tile = resident ? up4(g.jrows * g.ldj + 3) : g.j16 ? 32 * g.ldp : max(up4(32 * g.ldj) + 8, 32 * up4(m.nv));
+  g.oJ = o, o += resident ? g.tile : parts * g.tile;
   // dense: H and its factor share one (nv+1) x ldu array; sparse plan: packed H | N | 1/D
   g.oA = o, o += sp ? up4(sp->nfac) + up4(sp->nslots) + up4(m.nv) : (m.nv + 1) * g.ldu;
   // dof vectors; the dense factor needs two more (forward-solve scratch, 1 / pivot)
@@ -134,28 +137,37 @@ __device__ __noinline__ void warn_limit(int which, unsigned limit) {
     printf("solver iterations limit reached - please increase iterations to %u\n", limit);
 }
 
-// A CTA holds `warps` worlds in hand, a warp each, and as many CTAs as there are SMs share the batch:
-// every table of the model and the plan then exists once per SM in shared memory.  Read from global
-// memory by one-world CTAs the tables cost about 210 cycles per trip of the loops they drive,
-// whatever the distance of the prefetch.  The warps of a CTA never wait for one another after the
-// tables have arrived.  A warp's first world is number warp * grid + CTA of the launch order, further
-// ones come from a counter.
+// A CTA holds `warps` worlds in hand, a warp (or a team of `parts` warps) each, and as many CTAs as there
+// are SMs share the batch: every table of the model and the plan then exists once per SM in shared
+// memory.  Read from global memory by one-world CTAs the tables cost about 210 cycles per trip of the
+// loops they drive, whatever the distance of the prefetch.  The worlds of a CTA never wait for one another
+// after the tables have arrived.  A slot's first world is number slot * grid + CTA of the launch order,
+// further ones come from a counter.
+// A team (TEAM) runs the same statements: every warp takes the same decisions from values in shared
+// memory, part 0 does the stages that are one chain and passes its results on in `box`, every stage that
+// others read from ends in team_sync.
 // The solve is written as one loop whose trip is "take a world if none is in hand, else run one
 // pass of it" rather than as a load followed by a pass loop: the same statements, but the compiler
 // lays the single loop out better (measured: 0.836 -> 0.796 ms per 8192 humanoid worlds at the same
 // occupancy).
-template <bool JRES, bool J16, bool SPARSE, bool STATS, bool TSM>
+template <bool JRES, bool J16, bool SPARSE, bool STATS, bool TSM, bool TEAM>
 __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& d, const ImnCtx& cx, const Geom& g,
                                               const ImnSparsePlan& sp) {
   extern __shared__ __align__(16) float smem_all[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float* smem = smem_all + g.tab + warp * g.total;
+  // the first warps of the teams come first, so that they are spread over the SM's four schedulers
+  const int part = TEAM ? warp / g.warps : 0, slot = TEAM ? warp - part * g.warps : warp;
+  const int tid = lane + 32 * part, threads = TEAM ? 32 * g.parts : 32;  // of the world's team
+  float* smem = smem_all + g.tab + slot * g.total;
   const int nv = g.nv, R = g.njmax, nv4 = g.nv4, r4 = g.r4;
 
-  void* bar = smem + g.oBar;
+  void* bar = smem + g.oBar + 8 * part;  // copy barriers per warp
   World s;
   s.nv = nv, s.ldj = g.ldj, s.ldp = g.ldp, s.ldu = g.ldu, s.bd = g.bd, s.lane = lane, s.nM = g.nM;
+  s.part = part, s.parts = g.parts, s.team_bar = 1 + slot, s.tile_words = g.tile;
+  s.box = reinterpret_cast<int*>(smem + g.oBox);
   s.Jsm = smem + g.oJ;
+  s.tile = s.Jsm + (JRES ? 0 : part * g.tile);
   s.A = smem + g.oA;
   s.qacc = smem + g.oVec;
   s.Ma = s.qacc + nv4;
@@ -188,8 +200,8 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
     s.tab.bstep = reinterpret_cast<const uint2*>(sp.bstep);
   }
   s.M_rowadr = m.M_rowadr, s.M_rownnz = m.M_rownnz, s.M_colind = m.M_colind;
-  int* const load_phase_at = reinterpret_cast<int*>(smem + g.oBar) + 2;  // the barrier itself takes two words
-  s.jbar = J16 ? smem + g.oBar + 4 : bar;  // J16: every lane arrives at the tiles' own barrier
+  int* const load_phase_at = static_cast<int*>(bar) + 2;  // the barrier itself takes two words
+  s.jbar = J16 ? static_cast<float*>(bar) + 4 : bar;  // J16: every lane arrives at the tiles' own barrier
   s.jphase = load_phase_at + (J16 ? 4 : 0);
   s.jfail = load_phase_at + 1;
   s.wait_polls = g.wait_polls, s.withhold_copies = g.withhold_copies;
@@ -239,7 +251,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
   int st_passes = 0, st_flips = 0, st_factor = 0, st_grad = 0;  // work counters (ctx.stats)
   bool have = false, first = true;
   bool outside = false;  // a row of the world leaves the sparse plan's pattern
-  int idx = warp * (int)gridDim.x + (int)blockIdx.x;  // the next world's place in the launch order
+  int idx = slot * (int)gridDim.x + (int)blockIdx.x;  // the next world's place in the launch order
   bool turn = false;  // the first world was taken
 
 #pragma unroll 1
@@ -247,12 +259,17 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
     if (!have) {
       // ---- take a world --------------------------------------------------------------
       if (turn && cx.work_counter) {
-        if (lane == 0) idx = (int)gridDim.x * g.warps + atomicAdd(cx.work_counter, 1);
+        if (tid == 0) idx = (int)gridDim.x * g.warps + atomicAdd(cx.work_counter, 1);
         idx = __shfl_sync(IMN_FULL_MASK, idx, 0);
       } else if (turn) {
         idx += (int)gridDim.x * g.warps;
       }
       turn = true;
+      if (TEAM) {  // part 0 takes the world; past the barrier every warp has left the previous one
+        if (tid == 0) s.box[0] = idx;
+        team_sync<TEAM>(s);
+        idx = s.box[0];
+      }
       if (idx >= d.nworld) break;
       {
         w = cx.world_order ? cx.world_order[idx] : idx;
@@ -284,55 +301,65 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
             {s.qfs, d.qfrc_smooth + dofo, nv},
         };
         __syncwarp();  // every lane has left the previous world
-        const uint32_t load_phase = (uint32_t)*load_phase_at;
-        // the previous world's values were written through the generic proxy
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) {
-          *load_phase_at = (int)(load_phase ^ 1u);
-          *s.jfail = 0;
-        }
-        __syncwarp();
-        const bool bulk = !(g.withhold_copies & 1);
-        uint32_t tx = 0;
+        bool arrived = false;
+        if (TEAM && lane == 0) *s.jfail = 0;
+        if (!TEAM || part == 0) {
+          const uint32_t load_phase = (uint32_t)*load_phase_at;
+          // the previous world's values were written through the generic proxy
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            *load_phase_at = (int)(load_phase ^ 1u);
+            *s.jfail = 0;
+          }
+          __syncwarp();
+          const bool bulk = !(g.withhold_copies & 1);
+          uint32_t tx = 0;
 #pragma unroll
-        for (int k = 0; k < 5; ++k)
-          if (bulk && (reinterpret_cast<uintptr_t>(srcs[k].src) & 15) == 0) tx += (uint32_t)(srcs[k].n & ~3) * 4u;
-        if (lane == 0) {
-          mbar_expect_tx(bar, bulk ? tx : 16u);
+          for (int k = 0; k < 5; ++k)
+            if (bulk && (reinterpret_cast<uintptr_t>(srcs[k].src) & 15) == 0) tx += (uint32_t)(srcs[k].n & ~3) * 4u;
+          if (lane == 0) {
+            mbar_expect_tx(bar, bulk ? tx : 16u);
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+              const uint32_t bytes =
+                  bulk && (reinterpret_cast<uintptr_t>(srcs[k].src) & 15) == 0 ? (uint32_t)(srcs[k].n & ~3) * 4u : 0u;
+              if (bytes) bulk_g2s(srcs[k].dst, srcs[k].src, bytes, bar);
+            }
+          }
 #pragma unroll
           for (int k = 0; k < 5; ++k) {
-            const uint32_t bytes =
-                bulk && (reinterpret_cast<uintptr_t>(srcs[k].src) & 15) == 0 ? (uint32_t)(srcs[k].n & ~3) * 4u : 0u;
-            if (bytes) bulk_g2s(srcs[k].dst, srcs[k].src, bytes, bar);
+            const int done_n = bulk && (reinterpret_cast<uintptr_t>(srcs[k].src) & 15) == 0 ? (srcs[k].n & ~3) : 0;
+#pragma unroll 1
+            for (int i = done_n + lane; i < srcs[k].n; i += 32) srcs[k].dst[i] = srcs[k].src[i];
           }
-        }
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-          const int done_n = bulk && (reinterpret_cast<uintptr_t>(srcs[k].src) & 15) == 0 ? (srcs[k].n & ~3) : 0;
 #pragma unroll 1
-          for (int i = done_n + lane; i < srcs[k].n; i += 32) srcs[k].dst[i] = srcs[k].src[i];
-        }
+          for (int i = lane; i < nv; i += 32) s.search[i] = 0.0f, s.mv[i] = 0.0f, s.grad[i] = 0.0f;
+          if (lane == 0) s.search[nv] = 0.0f, s.qacc[nv] = 0.0f;
 #pragma unroll 1
-        for (int i = lane; i < nv; i += 32) s.search[i] = 0.0f, s.mv[i] = 0.0f, s.grad[i] = 0.0f;
-        if (lane == 0) s.search[nv] = 0.0f, s.qacc[nv] = 0.0f;
-#pragma unroll 1
-        for (int i = lane; i <= nv; i += 32) s.uni[i] = 0;
-        // bounded wait for the copies; when it runs out the copies get one more bounded wait
-        // (they write shared memory that the warp's next world takes over), then the world is left
-        // unsolved with the time-out bit set and the barrier starts anew
-        bool arrived = false;
-#pragma unroll 1
-        for (int tries = 0; tries < g.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(bar, load_phase);
-        if (!arrived) {
+          for (int i = lane; i <= nv; i += 32) s.uni[i] = 0;
+          // bounded wait for the copies; when it runs out the copies get one more bounded wait
+          // (they write shared memory that the warp's next world takes over), then the world is left
+          // unsolved with the time-out bit set and the barrier starts anew
 #pragma unroll 1
           for (int tries = 0; tries < g.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(bar, load_phase);
-          if (lane == 0) {
-            d.overflow[w] |= IMN_OVERFLOW_COPY_TIMEOUT;
-            mbar_restart(bar, 1);
-            *load_phase_at = 0;
+          if (!arrived) {
+            bool late = false;
+#pragma unroll 1
+            for (int tries = 0; tries < g.wait_polls && !late; ++tries) late = mbar_try_wait(bar, load_phase);
+            if (lane == 0) {
+              d.overflow[w] |= IMN_OVERFLOW_COPY_TIMEOUT;
+              mbar_restart(bar, 1);
+              *load_phase_at = 0;
+            }
           }
-        } else {
+        }
+        if (TEAM) {
+          if (tid == 0) s.box[1] = arrived;
+          team_sync<TEAM>(s);
+          arrived = s.box[1] != 0;
+        }
+        if (arrived) {
           have = true, first = true;
           search_dot = 0.0f, grad_dot = 0.0f, grad_scale = 1.0f, decrement = 0.0f;
           improvement = 0.0f, alpha = 0.0f;
@@ -357,9 +384,9 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
       // one call site: Ma = M qacc, Jaref = J qacc - aref on pass 0; mv = M search,
       // jv = J search afterwards
       if (first || !search_unchanged)
-        products<JRES, J16, TSM>(s, first ? s.qacc : s.search, first ? s.Ma : s.mv, first ? s.Jaref : s.jv,
+        products<JRES, J16, TSM, TEAM>(s, first ? s.qacc : s.search, first ? s.Ma : s.mv, first ? s.Jaref : s.jv,
                        first ? s.jv : nullptr);
-      __syncwarp();
+      team_sync<TEAM>(s);
       PROF(5);
       if (rowless) {
         finished = true;
@@ -367,7 +394,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
       }
       float noise_floor = 0.0f;
       bool ls_converged = true;
-      if (!first) {
+      if (!first && part == 0) {  // the search and the row lists are part 0's
         const LineSearchResult ls =
             line_search(s, search_dot, tolerance, ls_tolerance, scale, m.alpha_noise_eps, m.ls_iterations);
         alpha = ls.alpha, improvement = ls.improvement, noise_floor = ls.noise_floor;
@@ -386,7 +413,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
       state_count = 0;
       int nfr = 0;
 #pragma unroll 1
-      for (int base = 0; base < nefc; base += 32) {
+      for (int base = part == 0 ? 0 : nefc; base < nefc; base += 32) {
         const int r = base + lane;
         bool flip = false, changed = false, leaves = false;
         float f = 0.0f;
@@ -417,11 +444,20 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         if (f != 0.0f) s.frows[nfr + __popc(nz & below)] = r;
         nfr += __popc(nz);
       }
+      if (TEAM) {
+        if (tid == 0) {
+          s.box[2] = quad_count, s.box[3] = state_count, s.box[4] = nfr, s.box[7] = ls_converged;
+          s.box[8] = __float_as_int(alpha), s.box[9] = __float_as_int(improvement), s.box[10] = __float_as_int(noise_floor);
+        }
+        team_sync<TEAM>(s);
+        quad_count = s.box[2], state_count = s.box[3], nfr = s.box[4], ls_converged = s.box[7] != 0;
+        alpha = __int_as_float(s.box[8]), improvement = __int_as_float(s.box[9]), noise_floor = __int_as_float(s.box[10]);
+      }
       if (!first) {
         ls_exhausted = fabsf(alpha) < noise_floor;
         if (ls_exhausted) state_count += 1;
         if (!ls_converged) {
-          if ((m.warn_overflow & m.overflow_ls_iterations) && lane == 0) warn_limit(0, (unsigned)m.ls_iterations);
+          if ((m.warn_overflow & m.overflow_ls_iterations) && tid == 0) warn_limit(0, (unsigned)m.ls_iterations);
           overflow |= m.overflow_ls_iterations;
         }
       }
@@ -438,7 +474,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         decrement *= rsq;
         grad_scale = ns;
       } else {
-        grad_dot = full_gradient<JRES>(s, nfr);
+        grad_dot = full_gradient<JRES, TEAM>(s, nfr);
         if (STATS) {
           ++st_grad;
           if (!first) st_flips += quad_count;
@@ -455,12 +491,14 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
             outside = __any_sync(IMN_FULL_MASK, bad);
           }
           if (SPARSE)
-            hessian_sparse<JRES, J16, TSM>(s, quad_count, first, outside, sp);
+            hessian_sparse<JRES, J16, TSM, TEAM>(s, quad_count, first, outside, sp);
           else
-            hessian_dense<JRES, J16>(s, quad_count, first);
+            hessian_dense<JRES, J16, TEAM>(s, quad_count, first);
         }
         PROF(9);
-        if (SPARSE) {
+        // the factorisation is a chain of levels or rows: part 0's
+        if (TEAM && part != 0) {
+        } else if (SPARSE) {
           // refactor the packed H, or solve with the resident factor
           // (sparse_hessian.py:490-547)
           if (first || quad_count > 0) {
@@ -477,18 +515,30 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         } else {
           factor_solve(s, first || quad_count > 0, search_dot, decrement);
         }
+        if (TEAM) {
+          if (tid == 0) s.box[5] = __float_as_int(search_dot), s.box[6] = __float_as_int(decrement);
+          team_sync<TEAM>(s);
+          search_dot = __int_as_float(s.box[5]), decrement = __int_as_float(s.box[6]);
+        }
         PROF(10);
       }
-      if (!JRES && *s.jfail) {
+      bool lost = !JRES && *s.jfail;
+      if (TEAM && !JRES) {  // the flags are raised by `products`, a barrier or more ago
+        const int* flags = reinterpret_cast<const int*>(smem + g.oBar) + 3;  // jfail of each warp
+#pragma unroll 1
+        for (int p = 0; p < g.parts; ++p) lost = lost || flags[8 * p] != 0;
+      }
+      if (lost) {
         // a tile copy of this pass did not complete within its wait limit, so the pass
         // worked on stale rows: give the copy one more bounded wait (it writes this
         // CTA's shared memory), then leave the world unsolved, results unwritten
         const uint32_t parity = (uint32_t)*s.jphase ^ 1u;
-        bool arrived = false;
+        bool arrived = TEAM && !*s.jfail;  // a team: each warp its own copy
+        const bool restart = !arrived;
 #pragma unroll 1
         for (int tries = 0; tries < g.wait_polls && !arrived; ++tries) arrived = mbar_try_wait(s.jbar, parity);
-        if (lane == 0) {
-          d.overflow[w] |= IMN_OVERFLOW_COPY_TIMEOUT;
+        if (tid == 0) d.overflow[w] |= IMN_OVERFLOW_COPY_TIMEOUT;
+        if (restart && lane == 0) {
           mbar_restart(s.jbar, J16 ? 32 : 1);
           *s.jphase = 0;
         }
@@ -506,10 +556,10 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
                              0.5f * decrement / scale < tolerance;
       if (converged || niter == m.iterations) {
         if (!converged) {
-          if ((m.warn_overflow & m.overflow_iterations) && lane == 0) warn_limit(1, (unsigned)m.iterations);
+          if ((m.warn_overflow & m.overflow_iterations) && tid == 0) warn_limit(1, (unsigned)m.iterations);
           overflow |= m.overflow_iterations;
         }
-        if (lane == 0 && cx.nsolving) atomicAdd(cx.nsolving, -1);
+        if (tid == 0 && cx.nsolving) atomicAdd(cx.nsolving, -1);
         finished = true;
       }
     } while (false);
@@ -520,7 +570,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
 
     // ---- results (once) ---------------------------------------------------------
 #pragma unroll 1
-    for (int i = lane; i < nv; i += 32) {
+    for (int i = tid; i < nv; i += threads) {
       d.qacc[dofo + i] = s.qacc[i];
       d.efc_Ma[dofo + i] = s.Ma[i];
       d.qfrc_constraint[dofo + i] = rowless ? 0.0f : fmaf(-grad_scale, s.grad[i], s.Ma[i] - s.qfs[i]);
@@ -529,7 +579,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
       if (cx.grad) cx.grad[(size_t)w * cx.grad_ld + i] = s.grad[i];
     }
 #pragma unroll 1
-    for (int r = lane; r < nefc; r += 32) {
+    for (int r = tid; r < nefc; r += threads) {
       d.efc_force[efco + r] = s.force[r];
       d.efc_state[efco + r] = s.state[r];
       if (cx.Jaref) cx.Jaref[efco + r] = s.Jaref[r];
@@ -538,7 +588,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
     }
     if (cx.dof_union && !rowless)
 #pragma unroll 1
-      for (int i = lane; i <= nv; i += 32) cx.dof_union[(size_t)w * (nv + 1) + i] = s.uni[i];
+      for (int i = tid; i <= nv; i += threads) cx.dof_union[(size_t)w * (nv + 1) + i] = s.uni[i];
     if (SPARSE && !rowless && cx.hfactor && cx.h) {
       // packed H | N | 1/D, the reference's hfactor layout (sparse_hessian.py:488-489).
       // The factor never leaves the chip here, so it is written only for callers that
@@ -546,9 +596,9 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
       // last element is always live.
       float* Uf = cx.hfactor + (size_t)w * m.nv_pad * m.nv_pad;
 #pragma unroll 1
-      for (int q = lane; q < sp.nfac; q += 32) Uf[q] = s.Hp[q], Uf[sp.nfac + q] = s.N[q];
+      for (int q = tid; q < sp.nfac; q += threads) Uf[q] = s.Hp[q], Uf[sp.nfac + q] = s.N[q];
 #pragma unroll 1
-      for (int q = lane; q < nv; q += 32) Uf[2 * sp.nfac + q] = s.iD[q];
+      for (int q = tid; q < nv; q += threads) Uf[2 * sp.nfac + q] = s.iD[q];
     }
     if (!SPARSE && !rowless) {
       const size_t ho = (size_t)w * m.nv_pad * m.nv_pad;
@@ -556,15 +606,15 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
 #pragma unroll 1
         for (int r = 0; r < nv; ++r)
 #pragma unroll 1
-          for (int c = r + lane; c < nv; c += 32) cx.h[ho + (size_t)r * m.nv_pad + c] = s.A[(c + 1) * s.ldu + r];
+          for (int c = r + tid; c < nv; c += threads) cx.h[ho + (size_t)r * m.nv_pad + c] = s.A[(c + 1) * s.ldu + r];
       if (cx.hfactor)
 #pragma unroll 1
         for (int r = 0; r < nv; ++r)
 #pragma unroll 1
-          for (int c = r + lane; c < nv; c += 32) cx.hfactor[ho + (size_t)r * m.nv_pad + c] = s.A[r * s.ldu + c];
+          for (int c = r + tid; c < nv; c += threads) cx.hfactor[ho + (size_t)r * m.nv_pad + c] = s.A[r * s.ldu + c];
     }
     PROF(11);
-    if (lane == 0) {
+    if (tid == 0) {
       d.solver_niter[w] = niter;
       if (overflow) d.overflow[w] |= overflow;
       if (cx.search_dot) cx.search_dot[w] = search_dot;
@@ -595,26 +645,32 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
 // STATS compiles the work counters of ImnCtx.stats in: four more live values in a kernel that is
 // short of registers cost 9 % of its speed (measured), so the counting variants run only for
 // callers that pass the stats array.
-template <bool SPARSE, bool STATS, bool TSM>
+template <bool SPARSE, bool STATS, bool TSM, bool TEAM>
 __global__ void __launch_bounds__(32 * kResidentWarps, 1)
     newton_kernel_resident(const ImnModel m, const ImnData d, const ImnCtx cx, const Geom g, const ImnSparsePlan sp) {
-  newton_worlds<true, false, SPARSE, STATS, TSM>(m, d, cx, g, sp);
+  newton_worlds<true, false, SPARSE, STATS, TSM, TEAM>(m, d, cx, g, sp);
 }
-template <bool J16, bool SPARSE, bool STATS, bool TSM>
+template <bool J16, bool SPARSE, bool STATS, bool TSM, bool TEAM>
 __global__ void __launch_bounds__(32 * kStreamedWarps, 1)
     newton_kernel_streamed(const ImnModel m, const ImnData d, const ImnCtx cx, const Geom g, const ImnSparsePlan sp) {
-  newton_worlds<false, J16, SPARSE, STATS, TSM>(m, d, cx, g, sp);
+  newton_worlds<false, J16, SPARSE, STATS, TSM, TEAM>(m, d, cx, g, sp);
 }
 using Kernel = void (*)(ImnModel, ImnData, ImnCtx, Geom, ImnSparsePlan);
-template <bool SPARSE, bool STATS, bool TSM>
+template <bool SPARSE, bool STATS, bool TSM, bool TEAM>
 static Kernel newton_kernel(bool resident, bool j16) {
-  return resident ? (Kernel)newton_kernel_resident<SPARSE, STATS, TSM>
-         : j16    ? (Kernel)newton_kernel_streamed<true, SPARSE, STATS, TSM>
-                  : (Kernel)newton_kernel_streamed<false, SPARSE, STATS, TSM>;
+  return resident ? (Kernel)newton_kernel_resident<SPARSE, STATS, TSM, TEAM>
+         : j16    ? (Kernel)newton_kernel_streamed<true, SPARSE, STATS, TSM, TEAM>
+                  : (Kernel)newton_kernel_streamed<false, SPARSE, STATS, TSM, TEAM>;
+}
+template <bool SPARSE, bool STATS, bool TSM>
+static Kernel newton_kernel(bool resident, const Geom& g) {
+  if constexpr (!STATS)
+    if (g.parts > 1) return newton_kernel<SPARSE, STATS, TSM, true>(resident, g.j16);
+  return newton_kernel<SPARSE, STATS, TSM, false>(resident, g.j16);
 }
 template <bool SPARSE, bool STATS>
 static Kernel newton_kernel(bool resident, const Geom& g) {
-  return g.tsm ? newton_kernel<SPARSE, STATS, true>(resident, g.j16) : newton_kernel<SPARSE, STATS, false>(resident, g.j16);
+  return g.tsm ? newton_kernel<SPARSE, STATS, true>(resident, g) : newton_kernel<SPARSE, STATS, false>(resident, g);
 }
 
 __global__ void start_counters(int* nsolving, int* work_counter, int nworld) {
@@ -622,12 +678,11 @@ __global__ void start_counters(int* nsolving, int* work_counter, int nworld) {
   if (work_counter) *work_counter = 0;
 }
 
-// The hardware hands CTAs to SMs in index order and a world's solve time grows with
-// its row count, so worlds are launched by descending row count: the long solves
-// start first and the launch ends with short ones instead of a few stragglers.  One
-// CTA sorts the worlds into 64 classes of row count (counting sort through shared
-// memory); the order inside a class depends on atomics and is irrelevant: every
-// world is solved independently of which CTA takes it.
+// A world's solve time grows with its row count, so worlds are taken by descending row
+// count: the long solves start first and the launch ends with short ones instead of a few
+// stragglers.  One CTA sorts the worlds into 64 classes of row count (counting sort through
+// shared memory); the order inside a class depends on atomics and is irrelevant: every
+// world is solved independently of which warp takes it.
 #define IMN_ORDER_CLASSES 64
 __global__ void __launch_bounds__(1024) order_worlds_kernel(const int* __restrict__ nefc, int njmax, int nworld,
                                                             int* __restrict__ order, int* nsolving, int* work_counter) {
@@ -716,9 +771,20 @@ static int sm_count() {
 // resident vs 16 streamed worlds per SM: resident 7 % faster; SNU-like (njmax 128) 4 vs
 // 7: streamed 1.22x faster; G1-like (njmax 250) 4 vs 11: streamed 1.6x faster.  Hence:
 // stream when it holds at least 1.6x the worlds.
-static int plan_launch(const ImnModel* m, const ImnData* d, const ImnSparsePlan* sp, Geom* g, bool* resident, int* grid) {
-  const Geom gr = make_geom(*m, *d, true, sp);
-  const Geom gs = make_geom(*m, *d, false, sp);
+//
+// Warps per world: a world's rows, dofs and Hessian entries can be dealt to several warps; the line
+// search, the row lists and the factor cannot, and each stage costs a barrier.  A team of p warps is taken
+// for sqrt(p) times one: the choice is the largest (worlds in hand) x sqrt(team).  That is one warp where
+// the worlds in hand fill the SM's registers, more for batches of few worlds per SM (1024 34-dof
+// worlds, two warps: 182 -> 174 us; 1000 35-dof worlds, dense: 436 -> 411; 16 worlds, four warps, solve and
+// the rest of a step: 174 -> 161) and for worlds so large that few fit (64 dofs x 512 rows: 5 worlds of a warp
+// 4621 us, 3 of four warps 4153).
+static const int kMaxParts = 4;
+
+static int plan_launch(const ImnModel* m, const ImnData* d, const ImnSparsePlan* sp, bool stats, Geom* g, bool* resident,
+                       int* grid) {
+  const Geom gr = make_geom(*m, *d, true, sp, 1);
+  const Geom gs = make_geom(*m, *d, false, sp, 1);
   const int nr = worlds_per_sm(gr, kResidentWarps), ns = worlds_per_sm(gs, kStreamedWarps);
   const bool fits = gr.total * 4 <= kResidentBudget && nr >= 1;
   *resident = fits && 10 * ns < 16 * nr;
@@ -728,8 +794,15 @@ static int plan_launch(const ImnModel* m, const ImnData* d, const ImnSparsePlan*
                      kMaxSmem),
            IMN_ERR_LIMIT;
   // one CTA per SM; a batch that does not fill the GPU is spread over all SMs
-  const int sms = sm_count(), most = *resident ? nr : ns, share = (d->nworld + sms - 1) / sms;
-  g->warps = share < 1 ? 1 : share < most ? share : most;
+  const int sms = sm_count(), share = max((d->nworld + sms - 1) / sms, 1);
+  g->warps = min(share, *resident ? nr : ns);
+  for (int parts = 2; parts <= kMaxParts && !stats; ++parts) {  // the counting kernels know no teams
+    Geom team = make_geom(*m, *d, *resident, sp, parts);
+    const int n = min(share, worlds_per_sm(team, (*resident ? kResidentWarps : kStreamedWarps) / parts));
+    if ((float)n * sqrtf((float)parts) <= (float)g->warps * sqrtf((float)g->parts)) continue;
+    team.warps = n;
+    *g = team;
+  }
   const int need = (d->nworld + g->warps - 1) / g->warps;
   *grid = need < sms ? need : sms;
   return IMN_OK;
@@ -762,7 +835,7 @@ extern "C" int imn_launch_info(const ImnModel* m, const ImnData* d, const ImnCtx
   imn::Geom g;
   bool res;
   int grid = 0;
-  rc = imn::plan_launch(m, d, cx->sparse_plan, &g, &res, &grid);
+  rc = imn::plan_launch(m, d, cx->sparse_plan, cx->stats != nullptr, &g, &res, &grid);
   if (rc) return rc;
   out->world_threads = g.bd;
   out->worlds_per_cta = g.warps;
@@ -780,7 +853,7 @@ extern "C" int imn_solve(const ImnModel* m, const ImnData* d, const ImnCtx* cx, 
   imn::Geom g;
   bool res;
   int grid = 0;
-  rc = imn::plan_launch(m, d, cx->sparse_plan, &g, &res, &grid);
+  rc = imn::plan_launch(m, d, cx->sparse_plan, cx->stats != nullptr, &g, &res, &grid);
   if (rc) return rc;
   const int bytes = 4 * (g.tab + g.warps * g.total);
   const bool sparse = cx->sparse_plan != nullptr, stats = cx->stats != nullptr;
@@ -797,7 +870,7 @@ extern "C" int imn_solve(const ImnModel* m, const ImnData* d, const ImnCtx* cx, 
     imn::order_worlds_kernel<<<1, 1024, 0, stream>>>(d->nefc, d->njmax, d->nworld, cx->world_order, cx->nsolving, cx->work_counter);
   else if (cx->nsolving || cx->work_counter)
     imn::start_counters<<<1, 1, 0, stream>>>(cx->nsolving, cx->work_counter, d->nworld);
-  kern<<<grid, 32 * g.warps, bytes, stream>>>(*m, *d, *cx, g, sp);
+  kern<<<grid, 32 * g.warps * g.parts, bytes, stream>>>(*m, *d, *cx, g, sp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return imn::set_error("imn_solve: launch failed: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;

@@ -14,6 +14,11 @@ namespace imn {
 // Shared-memory view of one world plus the per-world constants.
 struct World {
   int nv, ldj, ldp, ldu, bd, nefc, ne, nef, lane, nM;
+  // a team of `parts` warps may share the world (the TEAM kernels), each with a row tile, a copy barrier
+  // and its words of its own; `box` carries single values from part 0 to the others
+  int part, parts, team_bar, tile_words;
+  int* box;
+  float* tile;
   float *Jsm, *A, *qacc, *Ma, *search, *mv, *grad, *qfs, *xsm, *dinv;
   // the world's M stays in global memory: its nM values are read once per iteration by
   // `products` (independent loads, issued together) and once by the Hessian assembly, and
@@ -49,6 +54,20 @@ struct World {
   long long* prof_t;
 #endif
 };
+
+// The warps of a world's team wait for one another, on the team's own barrier; a team of one warp has
+// its lanes to order.
+template <bool TEAM>
+__device__ __forceinline__ void team_sync(const World& s) {
+  if (TEAM)
+    asm volatile("bar.sync %0, %1;" ::"r"(s.team_bar), "r"(32 * s.parts) : "memory");
+  else
+    __syncwarp();
+}
+template <bool TEAM>
+__device__ __forceinline__ int team_part(const World& s) { return TEAM ? s.part : 0; }
+template <bool TEAM>
+__device__ __forceinline__ int team_parts(const World& s) { return TEAM ? s.parts : 1; }
 
 #ifdef IMN_PROFILE
 #define IMN_MARK(s, k) do { const long long t_ = clock64(); (s).prof_acc[k] += t_ - *(s).prof_t; *(s).prof_t = t_; } while (0)
@@ -98,12 +117,12 @@ __device__ __forceinline__ const float* j_tile(const World& s, int base) {
     if (J16) {
       if (s.lane == 0) *s.jphase = (int)(parity ^ 1u);
       if (!(s.withhold_copies & 2)) {
-        each_piece(s, rows, [&](int row, int c) { copy16(s.Jsm + row * s.ldp + 4 * c, src + (size_t)row * s.ldj + 4 * c); });
+        each_piece(s, rows, [&](int row, int c) { copy16(s.tile + row * s.ldp + 4 * c, src + (size_t)row * s.ldj + 4 * c); });
         mbar_arrive_copies(s.jbar);
       }
     } else if (s.lane == 0) {
       mbar_expect_tx(s.jbar, bytes);
-      if (!(s.withhold_copies & 2)) bulk_g2s(s.Jsm, src - head, bytes, s.jbar);
+      if (!(s.withhold_copies & 2)) bulk_g2s(s.tile, src - head, bytes, s.jbar);
       *s.jphase = (int)(parity ^ 1u);
     }
     bool arrived = false;
@@ -112,15 +131,15 @@ __device__ __forceinline__ const float* j_tile(const World& s, int base) {
     if (!arrived && s.lane == 0) *s.jfail = 1;
     __syncwarp();
     IMN_MARK(s, 17);
-    return s.Jsm + head;
+    return s.tile + head;
   }
-  if (J16) return s.Jsm;  // a lost world: its results are never written
+  if (J16) return s.tile;  // a lost world: its results are never written
 #pragma unroll 4
-  for (int i = s.lane; i < n; i += 32) s.Jsm[i] = src[i];
+  for (int i = s.lane; i < n; i += 32) s.tile[i] = src[i];
   // the next tile may arrive through the async proxy into the same buffer
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncwarp();
-  return s.Jsm;
+  return s.tile;
 }
 
 // Rows of the list s.ids (bit 15: the row leaves the QUADRATIC set, its D counts negative) as the
@@ -128,35 +147,46 @@ __device__ __forceinline__ const float* j_tile(const World& s, int base) {
 // tile, up to 32 listed rows at a time and up4(nv) floats apart: the stages read a row many times
 // over, and taking its elements from global memory each time was a half of the whole solve at
 // 64 dofs x 512 rows.
+// place of the at-th gathered row (a team has a tile of 32 per warp)
+template <bool TEAM>
+__device__ __forceinline__ float* gathered(const World& s, int at, int ld) {
+  return TEAM ? s.Jsm + (at >> 5) * s.tile_words + (at & 31) * ld : s.Jsm + at * ld;
+}
 struct ListRow {
   const float* J;
   float D;
 };
-template <bool JRES>
+template <bool JRES, bool TEAM>
 __device__ __forceinline__ ListRow list_row(const World& s, int t, int t0) {
   const int id = s.ids[t], r = id & 0x7FFF;
   ListRow o;
-  o.J = JRES ? s.Jsm + r * s.ldj : s.Jsm + (t - t0) * ((s.nv + 3) & ~3);
+  const int at = t - t0, ld = (s.nv + 3) & ~3;
+  o.J = JRES ? s.Jsm + r * s.ldj : gathered<TEAM>(s, at, ld);
   o.D = __int_as_float(__float_as_int(s.Dsm[r]) ^ ((id & 0x8000) << 16));
   return o;
 }
-template <bool JRES, bool J16>
+template <bool JRES, bool J16, bool TEAM>
 __device__ __forceinline__ void gather_rows(const World& s, int t0, int t1) {
   if (JRES) return;
-  __syncwarp();  // every lane is done with the tile's previous contents
+  team_sync<TEAM>(s);  // every lane is done with the tile's previous contents
+  int at = 0;  // a team's warps gather a share of the rows each
+  if (TEAM) {
+    const int share = (t1 - t0 + s.parts - 1) / s.parts;
+    at = share * s.part, t1 = min(t1, t0 + at + share), t0 += at;
+  }
   const int ld = (s.nv + 3) & ~3, lane = s.lane;
   if (J16) {
     each_piece(s, t1 - t0, [&](int row, int c) {
-      copy16(s.Jsm + row * ld + 4 * c, s.Jg + (size_t)(s.ids[t0 + row] & 0x7FFF) * s.ldj + 4 * c);
+      copy16(gathered<TEAM>(s, at + row, ld) + 4 * c, s.Jg + (size_t)(s.ids[t0 + row] & 0x7FFF) * s.ldj + 4 * c);
     });
     asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();
+    team_sync<TEAM>(s);
     return;
   }
   const int ids = t0 + lane < t1 ? s.ids[t0 + lane] & 0x7FFF : 0;
-  uint32_t dst = smem_u32(s.Jsm + lane);
 #pragma unroll 4
-  for (int t = t0; t < t1; ++t, dst += 4u * ld) {
+  for (int t = t0; t < t1; ++t) {
+    const uint32_t dst = smem_u32(gathered<TEAM>(s, at + t - t0, ld) + lane);
     const float* src = s.Jg + (size_t)__shfl_sync(IMN_FULL_MASK, ids, t - t0) * s.ldj + lane;
 #pragma unroll
     for (int q = 0; q < 3; ++q)
@@ -166,7 +196,7 @@ __device__ __forceinline__ void gather_rows(const World& s, int t0, int t1) {
   asm volatile("cp.async.wait_all;" ::: "memory");
   // a later tile may arrive through the async proxy into the same buffer
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  __syncwarp();
+  team_sync<TEAM>(s);
 }
 
 // The dofs each row touches, as s.mwords 32-bit words per row in shared memory (word q of row r at
@@ -214,17 +244,19 @@ __device__ __forceinline__ void write_union(const World& s, int count) {
 // outM = M v over the symmetric rows (newton_fusion.py:171-176) and
 // outJ[r] = J[r,:] v (- minus[r]): one running sum per row; above 50 dofs in
 // 20-dof partials joined by plain adds (newton_stages.py:157-174).
-template <bool JRES, bool J16, bool TSM>
+template <bool JRES, bool J16, bool TSM, bool TEAM>
 __device__ __forceinline__ void products(const World& s, const float* v, float* outM, float* outJ,
                                          const float* minus) {
   const int lane = s.lane, nv = s.nv;
+  // a team deals the tiles of 32 rows to its warps, M v to the warp that is next
+  const int part = team_part<TEAM>(s), stride = 32 * team_parts<TEAM>(s);
   // M v by the lane program: a lane owns whole rows and forms each row's sum in table order,
   // four entries per batch.  The program is read coalesced and a batch ahead, so that the reads
   // of M (global, L1) and v of a batch are issued together.  With a lane per dof and the row table
   // itself, the table reads touched up to 18 cache lines per instruction, stood in front of the
   // reads of M, and dofs past 32 took a second round (34-dof model, 8192 worlds: 7000 -> 5900 cycles
   // of the world's warp per product; 56-dof model, 4096 worlds: 1745 -> 1669 us per solve).
-  {
+  if (!TEAM || ((s.nefc + 31) >> 5) % s.parts == part) {
     const uint4* prog = s.tab.mulm + lane;
     uint4 p = tab_at<TSM>(prog);
     float acc = 0.0f;
@@ -244,7 +276,7 @@ __device__ __forceinline__ void products(const World& s, const float* v, float* 
   IMN_MARK(s, 16);
   const int chunk = nv > 50 ? 20 : nv;
 #pragma unroll 1
-  for (int base = 0; base < s.nefc; base += 32) {
+  for (int base = 32 * part; base < s.nefc; base += stride) {
     const float* Jt = j_tile<JRES, J16>(s, base);
     const int r = base + lane;
     if (r < s.nefc) {
@@ -282,12 +314,15 @@ __device__ __forceinline__ void products(const World& s, const float* v, float* 
 // (newton_stages.py:785-795).  Lane = dof.  Every element of J is used once, so a streamed J is read
 // straight from global memory (coalesced), without the detour through the tile; the listed rows go
 // several at a time so that their reads overlap.
-template <bool JRES>
+template <bool JRES, bool TEAM>
 __device__ __forceinline__ float full_gradient(const World& s, int nfr) {
   const int lane = s.lane, nv = s.nv;
   float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
   const int i0 = lane, i1 = lane + 32, i2 = lane + 64;
-  const bool h0 = i0 < nv, h1 = i1 < nv, h2 = i2 < nv;
+  const int part = team_part<TEAM>(s), parts = team_parts<TEAM>(s);  // 32 dofs per warp of a team, in turn
+  const bool h0 = i0 < nv && (!TEAM || part == 0), h1 = i1 < nv && (!TEAM || 1 % parts == part),
+             h2 = i2 < nv && (!TEAM || 2 % parts == part);
+  if (TEAM && 32 * part >= nv) nfr = 0;
   constexpr int B = JRES ? 4 : 8;
   const float* J = (JRES ? s.Jsm : s.Jg) + lane;
 #pragma unroll 1
@@ -306,7 +341,7 @@ __device__ __forceinline__ float full_gradient(const World& s, int nfr) {
   if (h0) s.grad[i0] = (s.Ma[i0] - s.qfs[i0]) - s0;
   if (h1) s.grad[i1] = (s.Ma[i1] - s.qfs[i1]) - s1;
   if (h2) s.grad[i2] = (s.Ma[i2] - s.qfs[i2]) - s2;
-  __syncwarp();
+  team_sync<TEAM>(s);
   return logical_block_sum(nv, s.bd, lane, [&](int i, float acc) { return fmaf(s.grad[i], s.grad[i], acc); });
 }
 
@@ -319,32 +354,33 @@ __device__ __forceinline__ float full_gradient(const World& s, int nfr) {
 // A lane owns 4 x 4 blocks of the upper triangle: eight values of a row feed 16 fused
 // multiply-adds, so the stage is bound by arithmetic instead of by shared-memory reads (an entry
 // per lane reads two values and looks its row up for every multiply-add).
-template <bool JRES, bool J16>
+template <bool JRES, bool J16, bool TEAM>
 __device__ __forceinline__ void hessian_dense(const World& s, int count, bool first) {
+  const int at = 32 * team_part<TEAM>(s), stride = 32 * team_parts<TEAM>(s);  // a team's warps take turns
   const int lane = s.lane, nv = s.nv, ldu = s.ldu;
   float* A = s.A;
   if (first) {
 #pragma unroll 4
-    for (int e = lane; e < (nv + 1) * ldu; e += 32) A[e] = 0.0f;
-    __syncwarp();
+    for (int e = at + lane; e < (nv + 1) * ldu; e += stride) A[e] = 0.0f;
+    team_sync<TEAM>(s);
 #pragma unroll 1
-    for (int i = lane; i < nv; i += 32) {
+    for (int i = at + lane; i < nv; i += stride) {
       const int e0 = __ldg(s.M_rowadr + i), n = __ldg(s.M_rownnz + i);
 #pragma unroll 4
       for (int k = 0; k < n; ++k) A[(i + 1) * ldu + __ldg(s.M_colind + e0 + k)] = __ldg(s.M + e0 + k);
     }
   }
   const int nb = (nv + 3) >> 2, nblock = nb * (nb + 1) / 2;
-  const int step = JRES ? max(count, 1) : 32;
+  const int step = JRES ? max(count, 1) : stride;
 #pragma unroll 1
   for (int t0 = 0; t0 < count; t0 += step) {
     const int t1 = min(t0 + step, count);
-    gather_rows<JRES, J16>(s, t0, t1);
-    __syncwarp();
+    gather_rows<JRES, J16, TEAM>(s, t0, t1);
+    if (JRES || !TEAM) team_sync<TEAM>(s);
     IMN_MARK(s, 22);
     const bool keep = t0 > 0 || first, last = t1 == count;
 #pragma unroll 1
-    for (int b0 = 0; b0 < nblock; b0 += 32) {
+    for (int b0 = at; b0 < nblock; b0 += stride) {
       const bool live = b0 + lane < nblock;
       int bi, bj;
       pair_lookup(min(b0 + lane, nblock - 1), bi, bj);
@@ -359,7 +395,7 @@ __device__ __forceinline__ void hessian_dense(const World& s, int count, bool fi
         }
 #pragma unroll 2
       for (int t = t0; t < t1; ++t) {
-        const ListRow row = list_row<JRES>(s, t, t0);
+        const ListRow row = list_row<JRES, TEAM>(s, t, t0);
         float a[4], b[4];
         if (JRES) {  // rows lie at their own stride, on any boundary
 #pragma unroll
@@ -388,8 +424,8 @@ __device__ __forceinline__ void hessian_dense(const World& s, int count, bool fi
           }
     }
   }
-  if (!first) write_union(s, count);
-  __syncwarp();
+  if (!first && at == 0) write_union(s, count);
+  team_sync<TEAM>(s);
   IMN_MARK(s, 18);
 }
 
@@ -425,20 +461,22 @@ __device__ __noinline__ void count_violations(bool first, const float* Jw, int l
 // tables are read coalesced once per call, a slot costs four instructions per row, and no pair list
 // of touched dofs has to be formed and looked up.  `outside`: the world has a row whose dofs do not
 // all lie in the pattern.  Sums of a list that does not fit one tile wait in N.
-template <bool JRES, bool J16, bool TSM>
+template <bool JRES, bool J16, bool TSM, bool TEAM>
 __device__ __forceinline__ void hessian_sparse(const World& s, int count, bool first, bool outside, const ImnSparsePlan& SP) {
   const int lane = s.lane, nv = s.nv, nfac = SP.nfac;
-  constexpr int Q = JRES ? 10 : 12;
-  const int step = JRES ? max(count, 1) : 32;
+  // slots a lane sums at a time: few in a team, whose warps take turns at the slots
+  constexpr int Q = TEAM ? 5 : JRES ? 10 : 12;
+  const int part = team_part<TEAM>(s), parts = team_parts<TEAM>(s);
+  const int step = JRES ? max(count, 1) : 32 * parts;
   // a list without rows still has to place M (first call)
   int t0 = 0;
   do {
     const int t1 = min(t0 + step, count);
-    gather_rows<JRES, J16>(s, t0, t1);
+    gather_rows<JRES, J16, TEAM>(s, t0, t1);
     IMN_MARK(s, 22);
     const bool last = t1 == count;
 #pragma unroll 1
-    for (int base = 0; base < nfac; base += 32 * Q) {
+    for (int base = 32 * Q * part; base < nfac; base += 32 * Q * parts) {
       float acc[Q];
       int a[Q], b[Q];
 #pragma unroll
@@ -455,7 +493,7 @@ __device__ __forceinline__ void hessian_sparse(const World& s, int count, bool f
       }
 #pragma unroll 1
       for (int t = t0; t < t1; ++t) {
-        const ListRow row = list_row<JRES>(s, t, t0);
+        const ListRow row = list_row<JRES, TEAM>(s, t, t0);
 #pragma unroll
         for (int q = 0; q < Q; ++q) acc[q] = fmaf(sp_at(row.J, a[q]) * row.D, sp_at(row.J, b[q]), acc[q]);
       }
@@ -473,11 +511,11 @@ __device__ __forceinline__ void hessian_sparse(const World& s, int count, bool f
     }
     t0 = t1;
   } while (t0 < count);
-  if (!first) write_union(s, count);
-  if (outside)
+  if (!first && part == 0) write_union(s, count);
+  if (outside && part == 0)
     count_violations(first, JRES ? s.Jsm : s.Jg, s.ldj, nv, s.Dsm, s.masks, s.r4, s.mwords, s.ids, count, SP.pmask, SP.pair, s.viol,
                      s.world, lane);
-  __syncwarp();
+  team_sync<TEAM>(s);
   IMN_MARK(s, 18);
 }
 
