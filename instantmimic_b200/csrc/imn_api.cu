@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(256) mul_m_kernel(const int nv, const int* __r
                                                     float* __restrict__ out, const int64_t out_ld,
                                                     float* __restrict__ copy_to, int* __restrict__ niter,
                                                     float* __restrict__ zero, const int nworld) {
+  chain_begin();
   extern __shared__ uint32_t tab[];  // packed (col | madr << 16) entries, then nv + 1 row starts
   const int nnz = rowadr[nv];
   int* radr = reinterpret_cast<int*>(tab + nnz);
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
                       float* __restrict__ copy_to, int* __restrict__ niter, float* __restrict__ zero, const int nworld,
                       const int bulk) {
   extern __shared__ __align__(16) float tile[];
+  chain_begin();
   const int nnz = rowadr[nv];
   float* Mt = tile + 4;  // the first 16 bytes hold the mbarrier
   float* vt = Mt + ((32 * nM + 3) & ~3);
@@ -201,10 +203,9 @@ static int launch_mul_m(const ImnModel* m, const float* M, int64_t M_ld, const f
         e = cudaFuncSetAttribute(mul_m_tile_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return set_error("mul_m: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
-      mul_m_tile_kernel<<<(nworld + 31) / 32, 32 * kTileWarps, tile_bytes, stream>>>(
-          m->nv, m->nM, m->M_mulm_rowadr, m->M_mulm_col, m->M_mulm_madr, M, M_ld, v, v_ld, out, out_ld, copy_to, niter,
-          zero, nworld, bulk);
-      e = cudaGetLastError();
+      e = launch_chained(mul_m_tile_kernel, (nworld + 31) / 32, 32 * kTileWarps, tile_bytes, stream, m->nv, m->nM,
+                         m->M_mulm_rowadr, m->M_mulm_col, m->M_mulm_madr, M, M_ld, v, v_ld, out, out_ld, copy_to, niter, zero,
+                         nworld, bulk);
       if (e != cudaSuccess) return set_error("mul_m: launch failed: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
       return IMN_OK;
     }
@@ -216,9 +217,8 @@ static int launch_mul_m(const ImnModel* m, const float* M, int64_t M_ld, const f
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   }
   const int grid = min((nworld + warps - 1) / warps, sms * 8);
-  mul_m_kernel<<<grid, warps * 32, bytes, stream>>>(m->nv, m->M_mulm_rowadr, m->M_mulm_col, m->M_mulm_madr, M, M_ld,
-                                                    v, v_ld, out, out_ld, copy_to, niter, zero, nworld);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_chained(mul_m_kernel, grid, warps * 32, bytes, stream, m->nv, m->M_mulm_rowadr, m->M_mulm_col,
+                                       m->M_mulm_madr, M, M_ld, v, v_ld, out, out_ld, copy_to, niter, zero, nworld);
   if (e != cudaSuccess) return set_error("mul_m: launch failed: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;
 }

@@ -185,6 +185,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
     tree_accumulate_kernel(const ImnBodyTree T, float* __restrict__ values, const int64_t world_ld, const int C,
                            const int skip_root_parent, const int nworld) {
   extern __shared__ __align__(16) float tree_smem[];
+  chain_begin();
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int n = T.nbody * C;
@@ -205,6 +206,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
     crb_kernel(const ImnBodyTree T, const float* __restrict__ cinert, const float* __restrict__ cdof,
                float* __restrict__ crb, float* __restrict__ M, const int64_t M_ld, const int nworld) {
   extern __shared__ __align__(16) float tree_smem[];
+  chain_begin();
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int sl = t.sl, w = t.w;
@@ -244,6 +246,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
                const int64_t qvel_ld, float* __restrict__ cacc_out, float* __restrict__ cfrc_out,
                float* __restrict__ qfrc_bias, const int64_t bias_ld, const int nworld) {
   extern __shared__ __align__(16) float tree_smem[];
+  chain_begin();
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int sl = t.sl, w = t.w;
@@ -311,6 +314,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
                    const float* __restrict__ cdof, float* __restrict__ cvel_out, float* __restrict__ cdof_dot_out,
                    const int nworld) {
   extern __shared__ __align__(16) float tree_smem[];
+  chain_begin();
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int sl = t.sl, w = t.w;
@@ -421,8 +425,8 @@ static int launch_tree(const char* who, void (*kernel)(Args...), int gw, size_t 
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return set_error("%s: cudaFuncSetAttribute: %s", who, cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
-  kernel<<<(nworld + per_cta - 1) / per_cta, 32 * kTreeWarps, bytes, (cudaStream_t)stream>>>(args...);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e =
+      launch_chained(kernel, (nworld + per_cta - 1) / per_cta, 32 * kTreeWarps, bytes, (cudaStream_t)stream, args...);
   if (e != cudaSuccess) return set_error("%s: launch failed: %s", who, cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;
 }
@@ -441,8 +445,7 @@ static int launch_tile(const char* who, void (*kernel)(Args...), size_t bytes, i
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return set_error("%s: cudaFuncSetAttribute: %s", who, cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
-  kernel<<<(nworld + 31) / 32, 32 * kTileWarps, bytes, (cudaStream_t)stream>>>(args...);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_chained(kernel, (nworld + 31) / 32, 32 * kTileWarps, bytes, (cudaStream_t)stream, args...);
   if (e != cudaSuccess) return set_error("%s: launch failed: %s", who, cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;
 }

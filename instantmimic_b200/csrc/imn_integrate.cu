@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(32 * kMatrixWarps)
     implicit_matrix_kernel(const ImnImplicit P, const float* __restrict__ M, const int64_t M_ld,
                            float* __restrict__ out, const int64_t out_ld, const int nworld) {
   extern __shared__ float qd_all[];
+  chain_begin();
   const int lane = threadIdx.x & 31, w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= nworld) return;
   const int row = (P.nM + 3) & ~3;
@@ -229,6 +230,7 @@ __host__ __device__ inline int advance_stride(int n) { return (n & 3) == 0 ? (n 
 __global__ void __launch_bounds__(32 * kAdvanceWarps)
     advance_kernel(const ImnAdvance P, const float* __restrict__ qacc, const int64_t qacc_ld, const int nworld) {
   extern __shared__ __align__(16) float rows[];
+  chain_begin();
   // row strides: the lanes of a warp read the same element of 32 rows; a row length that
   // shares a factor of 4 or more with the 32 banks is padded to an odd stride
   const int tq = advance_stride(P.nq), tv = advance_stride(P.nv);
@@ -308,9 +310,8 @@ extern "C" int imn_implicit_matrix(const ImnImplicit* p, const float* M, int64_t
     if (e != cudaSuccess)
       return imn::set_error("imn_implicit_matrix: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
-  imn::implicit_matrix_kernel<<<(nworld + warps - 1) / warps, 32 * warps, bytes, (cudaStream_t)stream>>>(*p, M, M_ld, out, out_ld,
-                                                                                                         nworld);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = imn::launch_chained(imn::implicit_matrix_kernel, (nworld + warps - 1) / warps, 32 * warps, bytes,
+                                            (cudaStream_t)stream, *p, M, M_ld, out, out_ld, nworld);
   if (e != cudaSuccess) return imn::set_error("imn_implicit_matrix: launch failed: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;
 }
@@ -330,9 +331,8 @@ extern "C" int imn_advance(const ImnAdvance* p, const float* qacc, int64_t qacc_
     if (e != cudaSuccess)
       return imn::set_error("imn_advance: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
-  imn::advance_kernel<<<(unsigned)((nworld + 31) / 32), 32 * imn::kAdvanceWarps, bytes, (cudaStream_t)stream>>>(
-      *p, qacc, qacc_ld, nworld);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = imn::launch_chained(imn::advance_kernel, (unsigned)((nworld + 31) / 32), 32 * imn::kAdvanceWarps, bytes,
+                                            (cudaStream_t)stream, *p, qacc, qacc_ld, nworld);
   if (e != cudaSuccess) return imn::set_error("imn_advance: launch failed: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;
 }

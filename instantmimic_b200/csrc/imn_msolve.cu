@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, KM == 2 ? 7 : 4)
                          const int* __restrict__ active, const int rhs, const int mode, const int carry,
                          const int ldu, const int per_world, const int vec, const int nworld) {
   extern __shared__ __align__(16) float sm[];
+  chain_begin();
   const int l = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int w = blockIdx.x * kDenseWarps + warp;
   if (w >= nworld || (active && active[w] == 0)) return;
@@ -453,10 +454,9 @@ extern "C" int imn_blocked_dense_factor_solve(const ImnBlockedPlan* plan, const 
              IMN_ERR_LAUNCH;
   }
   const int vec = (reinterpret_cast<uintptr_t>(U) & 15) == 0;  // pad is a multiple of 16 floats
-  kernel<<<(nworld + per_cta - 1) / per_cta, 32 * imn::kDenseWarps, bytes, (cudaStream_t)stream>>>(
-      plan->nv, plan->pad, plan->nM, plan->indices, plan->identity, M, M_ld, y, U, x, active, rhs_count, mode, carry, ldu,
-      per_world, vec, nworld);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = imn::launch_chained(kernel, (nworld + per_cta - 1) / per_cta, 32 * imn::kDenseWarps, bytes,
+                                            (cudaStream_t)stream, plan->nv, plan->pad, plan->nM, plan->indices, plan->identity,
+                                            M, M_ld, y, U, x, active, rhs_count, mode, carry, ldu, per_world, vec, nworld);
   if (e != cudaSuccess)
     return imn::set_error("imn_blocked_dense_factor_solve: launch failed: %s", cudaGetErrorString(e)),
            IMN_ERR_LAUNCH;

@@ -63,6 +63,7 @@ struct Geom {
   int tM, tF, tB, tS, tO, tab, warps;
   // warps per world (make_geom); the tiles of a streamed J are `tile` words apart
   int parts, tile, oBox;
+  bool early;  // the launch before this one is its own counter kernel, which writes no table
   // polls a copy wait may take before the world gives up, and the failure-path test
   // switch: when set no bulk copy is issued (plain loads bring the data) while the
   // barrier is told to expect bytes, so the wait runs out with nothing in flight
@@ -216,6 +217,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
     if (J16) mbar_init(s.jbar, 32), *s.jphase = 0;
   }
   __syncwarp();
+  if (!g.early) chain_wait();
   if (TSM) {
     auto stage = [&](int at, const void* src, int words) {
 #pragma unroll 1
@@ -237,6 +239,8 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
   }
+  if (g.early) chain_wait();
+  chain_release();
 
   PROF_DECL;
   // the world in hand
@@ -674,6 +678,7 @@ static Kernel newton_kernel(bool resident, const Geom& g) {
 }
 
 __global__ void start_counters(int* nsolving, int* work_counter, int nworld) {
+  chain_begin();
   if (nsolving) *nsolving = nworld;
   if (work_counter) *work_counter = 0;
 }
@@ -689,6 +694,7 @@ __global__ void __launch_bounds__(1024) order_worlds_kernel(const int* __restric
   __shared__ int count[IMN_ORDER_CLASSES], start[IMN_ORDER_CLASSES];
   const int tid = threadIdx.x;
   if (tid < IMN_ORDER_CLASSES) count[tid] = 0;
+  chain_begin();
   if (tid == 0 && nsolving) *nsolving = nworld;
   if (tid == 0 && work_counter) *work_counter = 0;
   __syncthreads();
@@ -866,12 +872,14 @@ extern "C" int imn_solve(const ImnModel* m, const ImnData* d, const ImnCtx* cx, 
     if (e != cudaSuccess)
       return imn::set_error("imn_solve: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
+  cudaError_t e = cudaSuccess;
   if (cx->world_order)
-    imn::order_worlds_kernel<<<1, 1024, 0, stream>>>(d->nefc, d->njmax, d->nworld, cx->world_order, cx->nsolving, cx->work_counter);
+    e = imn::launch_chained(imn::order_worlds_kernel, 1, 1024, 0, stream, d->nefc, d->njmax, d->nworld, cx->world_order,
+                            cx->nsolving, cx->work_counter);
   else if (cx->nsolving || cx->work_counter)
-    imn::start_counters<<<1, 1, 0, stream>>>(cx->nsolving, cx->work_counter, d->nworld);
-  kern<<<grid, 32 * g.warps * g.parts, bytes, stream>>>(*m, *d, *cx, g, sp);
-  cudaError_t e = cudaGetLastError();
+    e = imn::launch_chained(imn::start_counters, 1, 1, 0, stream, cx->nsolving, cx->work_counter, d->nworld);
+  g.early = cx->world_order || cx->nsolving || cx->work_counter;
+  if (e == cudaSuccess) e = imn::launch_chained(kern, grid, 32 * g.warps * g.parts, bytes, stream, *m, *d, *cx, g, sp);
   if (e != cudaSuccess) return imn::set_error("imn_solve: launch failed: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;
 }

@@ -234,6 +234,8 @@ std::string generate(const std::string& name, const int32_t* prog, const int32_t
          ") " + name + "(const float* __restrict__ M, long long M_ld, const float* __restrict__ y,\n"
          "    long long y_ld, float* __restrict__ x, long long x_ld, int nworld, int bulk) {\n"
          "  extern __shared__ __align__(16) float slots[];\n"
+         "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");  // chain_begin of imn_common.cuh\n"
+         "  if (gridDim.x <= 64) asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n"
          "  const int lw = threadIdx.x & 31, part = threadIdx.x >> 5;\n"
          "  const int world = blockIdx.x * 32 + lw;\n"
          "  const bool live = world < nworld;\n"
@@ -492,8 +494,13 @@ extern "C" int imn_tree_ldl_compiled_solve(ImnTreeKernel* k, const float* M, int
   int bulk = k->staged && M_ld == k->nM && y_ld == k->nv && (reinterpret_cast<uintptr_t>(M) & 15) == 0 &&
              (reinterpret_cast<uintptr_t>(y) & 15) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   void* args[] = {&M, &mld, &y, &yld, &x, &xld, &nw, &bulk};
-  cudaError_t e = cudaLaunchKernel(reinterpret_cast<const void*>(k->kernel), dim3((nworld + 31) / 32),
-                                   dim3(32 * k->groups), args, bytes, (cudaStream_t)stream);
+  cudaLaunchAttribute follow;
+  follow.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  follow.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((nworld + 31) / 32), cfg.blockDim = dim3(32 * k->groups), cfg.dynamicSmemBytes = bytes;
+  cfg.stream = (cudaStream_t)stream, cfg.attrs = &follow, cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(k->kernel), args);
   if (e != cudaSuccess)
     return imn::set_error("imn_tree_ldl_compiled_solve: launch failed: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;
