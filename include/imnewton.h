@@ -178,14 +178,17 @@ typedef struct ImnSparsePlan {
   const uint32_t* bsweep;
   int32_t nfsweep, nbsweep;
   /* What the fused kernel reads: the sweeps once more with every operand as a byte offset
-   * from N[0] (1/D starts up4(nslots) floats behind N), one record per (step, lane).  A
-   * sweep is as many steps as its entry with the most runs has runs; sweeps that neither
-   * have a term nor a diagonal entry are left out.
+   * from N[0] (1/D starts up4(nslots) floats behind N), one record per (step, lane).  The
+   * entries of a level are dealt to its sweeps anew (most terms first); entries that neither
+   * have a term nor are a diagonal are left out.  A sweep is as many steps as its entry
+   * with the most runs has runs.
    *   fstep [nfstep + 1][32][4]: {a | b << 16, d | slot << 16, terms | diagonal's 1/D << 16
    *     (0: not a diagonal), flags}; a, b, d start at the lane's own first term of the run and
    *     advance by the team width; flags bit 0 = the lane stores the entry, bit 1 = last step
    *     of its level, bits 2-4 = log2(team), bit 5 = last step of its sweep, bit 6 = a
-   *     lane of the sweep holds a diagonal entry, bits 8-15 = most terms of a lane.
+   *     lane of the sweep holds a diagonal entry, bit 7 = this step and the next, two sweeps
+   *     of a level, are done together (bits 8-15 then count for both), bits 8-15 = most
+   *     terms of a lane.
    *   bstep [nbsweep + 1][32][2]: {slot | source's right-hand side << 16, source's 1/D |
    *     destination's right-hand side << 16}; bit 0 of word 0 = the lane has work, of
    *     word 1 = last of its level.
@@ -193,6 +196,7 @@ typedef struct ImnSparsePlan {
   const uint32_t* fstep;
   const uint32_t* bstep;
   int32_t nfstep;
+  int32_t pairs; /* whether fstep has steps marked with bit 7 */
 } ImnSparsePlan;
 
 /* Solver context: the arrays mujoco_warp's `_create_solver_context` allocates

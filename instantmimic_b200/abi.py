@@ -131,7 +131,7 @@ class ImnSparsePlan(C.Structure):
         ("nentries", I32),
         ("nruns", I32),
         ("nback", I32),
-    ] + [(name, P) for name, _ in SPARSE_TABLES] + [("nfsweep", I32), ("nbsweep", I32)] + [(name, P) for name in SPARSE_STEPS] + [("nfstep", I32)]
+    ] + [(name, P) for name, _ in SPARSE_TABLES] + [("nfsweep", I32), ("nbsweep", I32)] + [(name, P) for name in SPARSE_STEPS] + [("nfstep", I32), ("pairs", I32)]
 
 
 class ImnCtx(C.Structure):

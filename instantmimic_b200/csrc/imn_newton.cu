@@ -151,7 +151,7 @@ __device__ __noinline__ void warn_limit(int which, unsigned limit) {
 // pass of it" rather than as a load followed by a pass loop: the same statements, but the compiler
 // lays the single loop out better (measured: 0.836 -> 0.796 ms per 8192 humanoid worlds at the same
 // occupancy).
-template <bool JRES, bool J16, bool SPARSE, bool STATS, bool TSM, bool TEAM>
+template <bool JRES, bool J16, int SPARSE, bool STATS, bool TSM, bool TEAM>
 __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& d, const ImnCtx& cx, const Geom& g,
                                               const ImnSparsePlan& sp) {
   extern __shared__ __align__(16) float smem_all[];
@@ -508,7 +508,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
           if (first || quad_count > 0) {
             sp_load_rhs<TSM>(sp, s.tab, s.N, s.grad, lane);
             IMN_MARK(s, 1);
-            sp_factor_steps<TSM>(sp, s.tab, s.N, lane);
+            sp_factor_steps<TSM, SPARSE == 2>(sp, s.tab, s.N, lane);
             IMN_MARK(s, 2);
           } else {
             sp_forward(sp, s.N, s.iD, s.grad, lane);
@@ -646,33 +646,35 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
 
 // Two entry points over the same body, with the register bounds that follow from the most worlds
 // in hand (kResidentWarps, kStreamedWarps).
+// SPARSE: 0 the dense factor, 1 a sparse plan, 2 a sparse plan whose sweeps go in pairs (ImnSparsePlan::pairs):
+// beside the code for pairs the kernels of plans without them run 1 to 3 % slower.
 // STATS compiles the work counters of ImnCtx.stats in: four more live values in a kernel that is
 // short of registers cost 9 % of its speed (measured), so the counting variants run only for
 // callers that pass the stats array.
-template <bool SPARSE, bool STATS, bool TSM, bool TEAM>
+template <int SPARSE, bool STATS, bool TSM, bool TEAM>
 __global__ void __launch_bounds__(32 * kResidentWarps, 1)
     newton_kernel_resident(const ImnModel m, const ImnData d, const ImnCtx cx, const Geom g, const ImnSparsePlan sp) {
   newton_worlds<true, false, SPARSE, STATS, TSM, TEAM>(m, d, cx, g, sp);
 }
-template <bool J16, bool SPARSE, bool STATS, bool TSM, bool TEAM>
+template <bool J16, int SPARSE, bool STATS, bool TSM, bool TEAM>
 __global__ void __launch_bounds__(32 * kStreamedWarps, 1)
     newton_kernel_streamed(const ImnModel m, const ImnData d, const ImnCtx cx, const Geom g, const ImnSparsePlan sp) {
   newton_worlds<false, J16, SPARSE, STATS, TSM, TEAM>(m, d, cx, g, sp);
 }
 using Kernel = void (*)(ImnModel, ImnData, ImnCtx, Geom, ImnSparsePlan);
-template <bool SPARSE, bool STATS, bool TSM, bool TEAM>
+template <int SPARSE, bool STATS, bool TSM, bool TEAM>
 static Kernel newton_kernel(bool resident, bool j16) {
   return resident ? (Kernel)newton_kernel_resident<SPARSE, STATS, TSM, TEAM>
          : j16    ? (Kernel)newton_kernel_streamed<true, SPARSE, STATS, TSM, TEAM>
                   : (Kernel)newton_kernel_streamed<false, SPARSE, STATS, TSM, TEAM>;
 }
-template <bool SPARSE, bool STATS, bool TSM>
+template <int SPARSE, bool STATS, bool TSM>
 static Kernel newton_kernel(bool resident, const Geom& g) {
   if constexpr (!STATS)
     if (g.parts > 1) return newton_kernel<SPARSE, STATS, TSM, true>(resident, g.j16);
   return newton_kernel<SPARSE, STATS, TSM, false>(resident, g.j16);
 }
-template <bool SPARSE, bool STATS>
+template <int SPARSE, bool STATS>
 static Kernel newton_kernel(bool resident, const Geom& g) {
   return g.tsm ? newton_kernel<SPARSE, STATS, true>(resident, g) : newton_kernel<SPARSE, STATS, false>(resident, g);
 }
@@ -864,8 +866,9 @@ extern "C" int imn_solve(const ImnModel* m, const ImnData* d, const ImnCtx* cx, 
   const int bytes = 4 * (g.tab + g.warps * g.total);
   const bool sparse = cx->sparse_plan != nullptr, stats = cx->stats != nullptr;
   const ImnSparsePlan sp = sparse ? *cx->sparse_plan : ImnSparsePlan{};
-  const imn::Kernel kern = sparse ? (stats ? imn::newton_kernel<true, true>(res, g) : imn::newton_kernel<true, false>(res, g))
-                                  : (stats ? imn::newton_kernel<false, true>(res, g) : imn::newton_kernel<false, false>(res, g));
+  const imn::Kernel kern = !sparse    ? (stats ? imn::newton_kernel<0, true>(res, g) : imn::newton_kernel<0, false>(res, g))
+                           : sp.pairs ? (stats ? imn::newton_kernel<2, true>(res, g) : imn::newton_kernel<2, false>(res, g))
+                                      : (stats ? imn::newton_kernel<1, true>(res, g) : imn::newton_kernel<1, false>(res, g));
   {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e == cudaSuccess && bytes > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);

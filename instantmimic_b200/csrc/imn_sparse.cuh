@@ -96,7 +96,44 @@ __device__ __forceinline__ void sp_factor_levels(const ImnSparsePlan& P, float* 
 __device__ __forceinline__ float sp_at(const float* N, uint32_t offset) {
   return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(N) + offset);
 }
-template <bool TSM>
+// Two sweeps of a level, whose chains of reads and sums run side by side (56 dofs, levels of up to
+// three sweeps, 4096 worlds: 1187 -> 1090 us per solve; four terms per trip instead of two: 1125).
+__device__ __forceinline__ void sp_two_sweeps(float* N, const uint4 e, const uint4 g) {
+  uint32_t a = e.x & 0xFFFFu, b = e.x >> 16, d = e.y & 0xFFFFu, A = g.x & 0xFFFFu, B = g.x >> 16, D = g.y & 0xFFFFu;
+  int n = (int)(e.z & 0xFFFFu), m = (int)(g.z & 0xFFFFu);
+  const uint32_t slot = e.y >> 16, Slot = g.y >> 16, stride = 4u << ((e.w >> 2) & 7u);
+  const float start = sp_at(N, slot), Start = sp_at(N, Slot);
+  float v = 0.0f, V = 0.0f;
+#pragma unroll 1
+  for (int left = (int)((e.w >> 8) & 0xFFu); left > 0; left -= 2, n -= 2, m -= 2) {
+    const float p0 = sp_at(N, a) * sp_at(N, b), q0 = sp_at(N, d), P0 = sp_at(N, A) * sp_at(N, B), Q0 = sp_at(N, D);
+    a += stride, b += stride, d += stride, A += stride, B += stride, D += stride;
+    const float p1 = sp_at(N, a) * sp_at(N, b), q1 = sp_at(N, d), P1 = sp_at(N, A) * sp_at(N, B), Q1 = sp_at(N, D);
+    a += stride, b += stride, d += stride, A += stride, B += stride, D += stride;
+    if (n > 0) v = fmaf(p0, q0, v);
+    if (m > 0) V = fmaf(P0, Q0, V);
+    if (n > 1) v = fmaf(p1, q1, v);
+    if (m > 1) V = fmaf(P1, Q1, V);
+  }
+  const int T = 1 << ((e.w >> 2) & 7u);
+#pragma unroll 1
+  for (int off = T >> 1; off > 0; off >>= 1) {
+    const float x = __shfl_down_sync(IMN_FULL_MASK, v, off, T), X = __shfl_down_sync(IMN_FULL_MASK, V, off, T);
+    v = v + x, V = V + X;
+  }
+  const float w = start - v, W = Start - V;
+  char* at = reinterpret_cast<char*>(N);
+  if (e.w & 1u) *reinterpret_cast<float*>(at + slot) = w;
+  if (g.w & 1u) *reinterpret_cast<float*>(at + Slot) = W;
+  if ((e.w | g.w) & 64u) {
+    const uint32_t di = e.z >> 16, Di = g.z >> 16;
+    const float inv = 1.0f / (di ? w : 1.0f), Inv = 1.0f / (Di ? W : 1.0f);
+    if (di) *reinterpret_cast<float*>(at + di) = inv;
+    if (Di) *reinterpret_cast<float*>(at + Di) = Inv;
+  }
+}
+
+template <bool TSM, bool PAIR>
 __device__ __forceinline__ void sp_factor_steps(const ImnSparsePlan& P, const Tables& tables, float* N, int lane) {
   const uint4* tab = tables.fstep + lane;
   uint4 cur = tab_at<TSM>(tab);
@@ -106,6 +143,15 @@ __device__ __forceinline__ void sp_factor_steps(const ImnSparsePlan& P, const Ta
     tab += 32;
     const uint4 nxt = tab_at<TSM>(tab);
     const uint32_t fl = cur.w, slot = cur.y >> 16;
+    if (PAIR && (fl & 128u)) {  // two sweeps of the level at once
+      tab += 32;
+      const uint4 then = tab_at<TSM>(tab);
+      sp_two_sweeps(N, cur, nxt);
+      if (nxt.w & 2u) __syncwarp();
+      cur = then;
+      --s;
+      continue;
+    }
     uint32_t a = cur.x & 0xFFFFu, b = cur.x >> 16, d = cur.y & 0xFFFFu;
     int cnt = (int)(cur.z & 0xFFFFu);
     const float start = sp_at(N, slot);
