@@ -552,18 +552,31 @@ def _implicit_matrix(m: Any, d: Any, out: Any, scratch: OptimizedFwdPositionScra
 
 def _fused_gain_coefficients(m: Any, d: Any, scratch: Any):
     """The prepared (g2, b2) when the assembly can form the gains itself: float32 rows per
-    actuator, for all worlds or for each."""
+    actuator, for all worlds or for each, and a float32 row of controls per world next to them.  Other
+    controls (one row for all worlds, another type, another device) go through torch, which converts them."""
     import torch
+
+    from .arrays import as_torch, device_of, elem_strides, is_device
 
     pair = getattr(scratch, "implicit_gain_coefficients", None)
     if pair is None:
         return None
+    W, nu = int(d.nworld), int(m.nu)
     shapes = {tuple(t.shape) for t in pair}
-    nu = int(m.nu)
-    if shapes <= {(nu,)} or shapes <= {(1, nu)} or shapes <= {(int(d.nworld), nu)}:
-        if all(t.dtype == torch.float32 and t.is_contiguous() for t in pair):
-            return pair
-    return None
+    if not (shapes <= {(nu,)} or shapes <= {(1, nu)} or shapes <= {(W, nu)}):
+        return None
+    out, ctrl = as_torch(scratch.implicit_actuator_vel), d.ctrl
+    if any(t.dtype != torch.float32 or not t.is_contiguous() or t.device != out.device for t in pair):
+        return None
+    if tuple(ctrl.shape) != (W, nu):
+        return None
+    if isinstance(ctrl, torch.Tensor):
+        fits = ctrl.dtype == torch.float32 and ctrl.device == out.device
+    else:
+        fits = is_device(ctrl) and getattr(ctrl.dtype, "__name__", "") == "float32" and device_of(ctrl) == out.device
+    if not fits or elem_strides(ctrl)[1] != 1 or elem_strides(ctrl)[0] < nu:
+        return None
+    return pair
 
 
 def _advance_with_scratch(m: Any, d: Any, qacc: Any, scratch: OptimizedFwdPositionScratch | None = None,

@@ -248,3 +248,66 @@ def test_gains_formed_in_the_assembly_and_batches_of_moment_rows(oracle, cuda_de
     torch.cuda.synchronize()
     assert torch.equal(gains, scratch.implicit_actuator_vel) and torch.equal(A, scratch.implicit_qderiv)
     np.testing.assert_array_equal(A.cpu().numpy(), oracle.implicit_matrix(m, d, gains.cpu().numpy()))
+
+
+def _controls(ctrl, form):
+    """The controls (W, nu) of all-equal rows in another form with the same values."""
+    import torch
+
+    return {"one row": lambda: ctrl[:1].clone(), "expanded": lambda: ctrl[:1].expand(ctrl.shape),
+            "row of its own": lambda: ctrl[0].clone(), "every other": lambda: ctrl.repeat_interleave(2, 1)[:, ::2],
+            "transposed": lambda: ctrl.t().contiguous().t(), "float64": lambda: ctrl.double(),
+            "other device": lambda: ctrl.to("meta" if ctrl.device.type == "cpu" else "cpu"),
+            "padded rows": lambda: torch.cat((ctrl, ctrl), 1)[:, :ctrl.shape[1]]}[form]()
+
+
+CONTROL_FORMS = ("one row", "expanded", "row of its own", "every other", "transposed", "float64", "other device")
+
+
+@pytest.mark.parametrize("form", CONTROL_FORMS + ("padded rows",))
+def test_gains_are_formed_in_the_assembly_for_float_rows_of_controls_only(form):
+    """The assembly reads a float row of controls per world; any other form would be read out of
+    range or as other numbers and has to go through torch."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from instantmimic_b200 import mjw_step_optimized as runtime
+
+    W, nu = 3, 4
+    d = SimpleNamespace(nworld=W, ctrl=_controls(torch.ones(W, nu), form))
+    pair = (torch.ones(nu), torch.ones(nu))
+    scratch = SimpleNamespace(implicit_gain_coefficients=pair, implicit_actuator_vel=torch.zeros(W, nu))
+    got = runtime._fused_gain_coefficients(SimpleNamespace(nu=nu), d, scratch)
+    assert got is (pair if form == "padded rows" else None)
+    d.ctrl = torch.ones(W, nu)
+    scratch.implicit_gain_coefficients = tuple(t.to("meta") for t in pair)
+    assert runtime._fused_gain_coefficients(SimpleNamespace(nu=nu), d, scratch) is None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", CONTROL_FORMS + ("padded rows",))
+def test_implicitfast_integrate_takes_controls_of_every_form(cuda_device, form):
+    import torch
+
+    from instantmimic_b200 import mjw_step_optimized as runtime
+
+    m, d = _problem(worlds=37, nu=20)[:2]
+    rng = np.random.default_rng(5)
+    m.actuator_gaintype = np.full(m.nu, int(types.GainType.AFFINE), np.int32)
+    m.actuator_biastype = np.full(m.nu, int(types.BiasType.AFFINE), np.int32)
+    m.actuator_dyntype = np.zeros(m.nu, np.int32)
+    m.actuator_gainprm = rng.normal(size=(m.nu, 10)).astype(np.float32)
+    m.actuator_biasprm = -rng.uniform(1, 20, (m.nu, 10)).astype(np.float32)
+    d.ctrl = np.tile(rng.uniform(-1, 1, m.nu).astype(np.float32), (d.nworld, 1))
+    results = []
+    for f in (None, form):
+        md, dd = mjw_model.to_device(m, cuda_device), mjw_model.to_device(copy.deepcopy(d), cuda_device)
+        if f:
+            dd.ctrl = _controls(dd.ctrl, f)
+        scratch = runtime.make_optimized_fwd_position_scratch(md, dd, cuda_device)
+        runtime.attach_implicit_scratch(md, dd, scratch, cuda_device)
+        runtime.implicitfast_integrate(md, dd, scratch)
+        torch.cuda.synchronize()
+        results.append((scratch.implicit_actuator_vel, scratch.implicit_qderiv, dd.qvel, dd.qpos))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
