@@ -16,6 +16,12 @@ void set_error(const char* fmt, ...) {
   va_end(ap);
 }
 
+int sm_count() {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+  return sms;
+}
+
 // M v over the symmetric row tables, a bandwidth-bound pass: every CTA stages the
 // (model-wide) tables in shared memory once and its eight warps then walk worlds
 // with a grid stride.  A lane owns dofs lane, lane+32, ...; its loads of M and v
@@ -211,12 +217,7 @@ static int launch_mul_m(const ImnModel* m, const float* M, int64_t M_ld, const f
     }
   }
   const int warps = 8;
-  int sms = 148;
-  {
-    int dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  const int grid = min((nworld + warps - 1) / warps, sms * 8);
+  const int grid = min((nworld + warps - 1) / warps, sm_count() * 8);
   const cudaError_t e = launch_chained(mul_m_kernel, grid, warps * 32, bytes, stream, m->nv, m->M_mulm_rowadr, m->M_mulm_col,
                                        m->M_mulm_madr, M, M_ld, v, v_ld, out, out_ld, copy_to, niter, zero, nworld);
   if (e != cudaSuccess) return set_error("mul_m: launch failed: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;

@@ -19,6 +19,7 @@
 namespace imn {
 
 void set_error(const char* fmt, ...);
+int sm_count();  // of the current device; 148 where there is none
 
 // ---- launches that follow each other on a stream --------------------------------
 //

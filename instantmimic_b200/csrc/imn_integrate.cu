@@ -35,10 +35,20 @@ namespace imn {
 //                              once.  Motors on the axes of a ball joint store three dofs with one
 //                              nonzero moment, so their products land on three different diagonals;
 //   anything else              actuator by actuator.
-// Per 8192 humanoid worlds with 28 motors in three-dof rows the batch form takes 9 us where actuator
-// by actuator took 39 (the chain of dependent reads, 28 times).
+// Per 8192 humanoid worlds with 28 motors in three-dof rows the batch form takes 10 us where actuator
+// by actuator took 44 (the chain of dependent reads, 28 times).
+//
+// Two variants (imn_implicit_matrix chooses), same sums for any rows:
+//   ROWS   the batch form, and M fetched ahead.  64 registers a thread and a second shared-memory row for the
+//          marks: 32 warps per SM.
+//   !ROWS  neither: 32 registers, 64 warps per SM; rows of several dofs go actuator by actuator.
+// A pass over a large batch is bound by memory in flight, so the warps count where no row needs the
+// batch form; a batch of a wave or two is bound by one world's chain of reads, which the
+// fetched-ahead M shortens.  Servo rows (34 dofs, 28 actuators), us with / without ROWS: 512 worlds
+// 3.6 / 4.4, 4096 5.0 / 5.7, 8192 9.2 / 9.4, 16384 19.5 / 17.9, 65536 65.1 / 55.8 (199 MB: 3.6 TB/s).
 static const int kMatrixWarps = 8;
 static const int kRowDofs = 4;  // rows of the batch form
+static const int kRowsBlocksPerSm = 4;  // of the ROWS variant: 64 registers x 256 threads
 
 __device__ __forceinline__ void add_batch(float* qd, int e, float c, int lane) {
   const unsigned peers = __match_any_sync(IMN_FULL_MASK, e);
@@ -51,6 +61,7 @@ __device__ __forceinline__ void add_batch(float* qd, int e, float c, int lane) {
   }
 }
 
+template <bool ROWS>
 __global__ void __launch_bounds__(32 * kMatrixWarps)
     implicit_matrix_kernel(const ImnImplicit P, const float* __restrict__ M, const int64_t M_ld,
                            float* __restrict__ out, const int64_t out_ld, const int nworld) {
@@ -59,12 +70,12 @@ __global__ void __launch_bounds__(32 * kMatrixWarps)
   const int lane = threadIdx.x & 31, w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= nworld) return;
   const int row = (P.nM + 3) & ~3;
-  float* qd = qd_all + (threadIdx.x >> 5) * 2 * row;
+  float* qd = qd_all + (threadIdx.x >> 5) * (ROWS ? 2 : 1) * row;
   int* mark = reinterpret_cast<int*>(qd + row);  // the actuator of the batch that hit an entry last
   // M's entries are on their way while the actuators are worked on
-  constexpr int kAhead = 12;
+  constexpr int kAhead = ROWS ? 12 : 0;
   const float* Mw = M + (size_t)w * M_ld;
-  float m[kAhead];
+  float m[kAhead + 1];
 #pragma unroll
   for (int k = 0; k < kAhead; ++k) m[k] = lane + 32 * k < P.nM ? __ldg(Mw + lane + 32 * k) : 0.0f;
   const float h = P.timestep[w % P.n_timestep];
@@ -105,7 +116,7 @@ __global__ void __launch_bounds__(32 * kMatrixWarps)
         add_batch(qd, e, c, lane);
         continue;
       }
-      if (longest <= kRowDofs) {
+      if (ROWS && longest <= kRowDofs) {
         int dof[kRowDofs];
         float mo[kRowDofs];
 #pragma unroll
@@ -299,19 +310,26 @@ extern "C" int imn_implicit_matrix(const ImnImplicit* p, const float* M, int64_t
       (!p->gain_g2 || !p->gain_b2 || !p->velocity_gain_out || p->n_coefficients <= 0 || p->ctrl_ld < p->nu))
     return imn::set_error("imn_implicit_matrix: controls without gain coefficients or with a short stride"), IMN_ERR_NULL;
   if (nworld == 0) return IMN_OK;
-  const size_t per_warp = 2 * sizeof(float) * (size_t)((p->nM + 3) & ~3);  // qD and the marks
+  // A world whose moment row storage is no longer than nu holds one dof per actuator (or none for others
+  // beside a longer row): no work for the batch form.  Such batches, beyond two waves of its blocks (one of
+  // the other variant's), and an M whose marks would not fit take the variant without.
+  const size_t row_bytes = sizeof(float) * (size_t)((p->nM + 3) & ~3);
+  const bool several = p->nu > 0 && p->actuation && p->moment_ld > p->nu;
+  const bool few = (int64_t)nworld <= 2 * (int64_t)imn::sm_count() * imn::kRowsBlocksPerSm * imn::kMatrixWarps;
+  const bool rows = (several || few) && 2 * row_bytes <= 227 * 1024;
+  const auto kernel = rows ? imn::implicit_matrix_kernel<true> : imn::implicit_matrix_kernel<false>;
+  const size_t per_warp = (rows ? 2 : 1) * row_bytes;  // qD and the marks
   int warps = imn::kMatrixWarps;
   while (warps > 1 && per_warp * warps > 227 * 1024) warps /= 2;
   const size_t bytes = per_warp * warps;
   if (bytes > 227 * 1024) return imn::set_error("imn_implicit_matrix: nM %d too large", p->nM), IMN_ERR_LIMIT;
   if (bytes > 48 * 1024) {
-    cudaError_t e =
-        cudaFuncSetAttribute(imn::implicit_matrix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess)
       return imn::set_error("imn_implicit_matrix: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
-  const cudaError_t e = imn::launch_chained(imn::implicit_matrix_kernel, (nworld + warps - 1) / warps, 32 * warps, bytes,
-                                            (cudaStream_t)stream, *p, M, M_ld, out, out_ld, nworld);
+  const cudaError_t e = imn::launch_chained(kernel, (nworld + warps - 1) / warps, 32 * warps, bytes, (cudaStream_t)stream,
+                                            *p, M, M_ld, out, out_ld, nworld);
   if (e != cudaSuccess) return imn::set_error("imn_implicit_matrix: launch failed: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;
 }

@@ -767,12 +767,6 @@ static int worlds_per_sm(const Geom& g, int most) {
   return n < most ? n : most;
 }
 
-static int sm_count() {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-  return sms;
-}
-
 // J resident in shared memory or streamed through the 32-row tile.  Resident J is
 // read once from HBM; a streamed J is re-read from L2 in every stage but leaves room
 // for more worlds per SM.  Measured on B200 (dense factor): humanoid (njmax 64) 12

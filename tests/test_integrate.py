@@ -311,3 +311,59 @@ def test_implicitfast_integrate_takes_controls_of_every_form(cuda_device, form):
         torch.cuda.synchronize()
         results.append((scratch.implicit_actuator_vel, scratch.implicit_qderiv, dd.qvel, dd.qpos))
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+def test_one_dof_assembly_leaves_room_for_every_warp(tmp_path):
+    """The assembly variant of large batches of one-dof rows is bound by memory in flight: 64 warps per SM
+    (65536 registers), so 32 registers a thread; carrying the several-dof form's products and marks
+    costs half of the warps and a seventh of the speed."""
+    import re
+    import subprocess
+
+    from instantmimic_b200 import build
+
+    flags = [f for f in build.NVCC_FLAGS if f not in ("-shared", "-ldl")]
+    cmd = [build.nvcc(), *flags, "-Xptxas", "-v", "-c", str(build.CSRC / "imn_integrate.cu"), "-o", str(tmp_path / "x.o")]
+    log = subprocess.run(cmd, capture_output=True, text=True, check=True).stderr
+    used = [int(n) for n in re.findall(r"implicit_matrix_kernel.*?Used (\d+) registers", log, flags=re.S)]
+    assert used and min(used) <= 32, used
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("worlds", [9472, 9473])
+@pytest.mark.parametrize("shape", ["servo", "padded", "mixed", "none"])
+def test_both_assembly_variants(oracle, cuda_device, worlds, shape):
+    """Either side of the batch size at which one-dof rows change variant: rows of one dof, the same in
+    wider storage, storage of one dof per actuator that holds rows of three beside empty ones, and no
+    actuators."""
+    import torch
+
+    from instantmimic_b200 import mjw_step_optimized as runtime
+
+    nu = 0 if shape == "none" else 21
+    m, d = _problem(worlds=4, nu=nu, seed=11, single=True)[:2]
+    rng = np.random.default_rng(11)
+    if shape != "none":
+        n = np.tile([3, 0, 0], (4, nu // 3)) if shape == "mixed" else np.ones((4, nu), int)
+        width = nu + 5 if shape == "padded" else nu
+        d.moment_rownnz = n.astype(np.int32)
+        d.moment_rowadr = (np.cumsum(n, 1) - n).astype(np.int32)
+        d.moment_colind = np.zeros((4, width), np.int32)
+        d.moment_colind[:, :nu] = np.arange(nu) + 6
+        d.actuator_moment = rng.normal(size=(4, width)).astype(np.float32)
+    gain = -rng.uniform(1, 20, (4, nu)).astype(np.float32) if nu else None
+    md, dd = mjw_model.to_device(m, cuda_device), mjw_model.to_device(d, cuda_device)
+    dd.nworld = worlds
+    rep = lambda t: t.repeat(worlds // 4 + 1, 1)[:worlds].contiguous()  # noqa: E731
+    dd.M = rep(dd.M)
+    if nu:
+        for name in ("moment_rownnz", "moment_rowadr", "moment_colind", "actuator_moment"):
+            setattr(dd, name, rep(getattr(dd, name)))
+    from types import SimpleNamespace
+
+    scratch = SimpleNamespace(implicit_actuator_vel=rep(torch.from_numpy(gain).to(cuda_device)) if nu else None)
+    out = torch.empty_like(dd.M)
+    runtime.deriv_smooth_vel_dense_actuator_centric(md, dd, out, scratch)
+    torch.cuda.synchronize()
+    want = oracle.implicit_matrix(m, d, gain)
+    np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), np.resize(want, out.shape).view(np.uint32))
