@@ -35,6 +35,20 @@ def lib() -> C.CDLL:
     return _LIB
 
 
+_PACKED: dict = {}
+
+
+def packed(name: str):
+    """The library's function ``name``, taking its structs as the bytes of ``abi.packer``."""
+    fn = _PACKED.get(name)
+    if fn is None:
+        fn = lib()[name]  # a function object of its own, beside the one with struct arguments
+        fn.restype, kinds = abi.SYMBOLS[name]
+        fn.argtypes = [abi.P if issubclass(kind, C._Pointer) else kind for kind in kinds]
+        _PACKED[name] = fn
+    return fn
+
+
 def check(rc: int, what: str) -> None:
     if rc != 0:
         msg = lib().imn_last_error().decode(errors="replace")

@@ -9,6 +9,7 @@ check against).  Field order and types must match the header exactly;
 from __future__ import annotations
 
 import ctypes as C
+import struct
 
 P = C.c_void_p
 I32 = C.c_int32
@@ -235,6 +236,15 @@ class ImnLaunchInfo(C.Structure):
         ("j_resident", I32),
         ("grid", I32),
     ]
+
+
+def packer(cls):
+    """The function that packs a struct's fields, in their order, into bytes with the compiler's
+    layout; a NULL pointer is 0."""
+    codes = {I32: "i", I64: "q", F32: "f"}
+    layout = struct.Struct("".join(codes.get(kind, "P") for _, kind in cls._fields_) + "0q")
+    assert layout.size == C.sizeof(cls), cls
+    return layout.pack
 
 
 # name -> (restype, argtypes) of every symbol the header declares

@@ -13,6 +13,7 @@ Everything in the package that touches a caller's array goes through this module
 from __future__ import annotations
 
 import ctypes
+import operator
 from typing import Any
 
 import numpy as np
@@ -32,16 +33,60 @@ def _is_torch(a: Any) -> bool:
 def addr(a: Any) -> int | None:
     if a is None:
         return None
+    data_ptr = getattr(a, "data_ptr", None)
+    if data_ptr is not None:
+        return data_ptr()
     if isinstance(a, np.ndarray):
         return a.ctypes.data
-    if _is_torch(a):
-        return int(a.data_ptr())
     if hasattr(a, "ptr"):
         return int(a.ptr) if a.ptr else None
     iface = getattr(a, "__cuda_array_interface__", None)
     if iface is not None:
         return int(iface["data"][0])
     raise TypeError(f"cannot take the address of {type(a).__name__}")
+
+
+_DATA_PTR = _STRIDE = _CONTIGUOUS = None
+_SHAPE = operator.attrgetter("shape")
+
+
+def _torch_methods() -> None:
+    global _DATA_PTR, _STRIDE, _CONTIGUOUS
+    import torch
+
+    _DATA_PTR, _STRIDE, _CONTIGUOUS = torch.Tensor.data_ptr, torch.Tensor.stride, torch.Tensor.is_contiguous
+
+
+# Several arrays at once: torch tensors, the usual case, in one pass per property.
+
+def addrs(objs: tuple) -> tuple:
+    """The addresses, 0 for a missing array."""
+    if _DATA_PTR is None:
+        _torch_methods()
+    try:
+        return tuple(map(_DATA_PTR, objs))
+    except TypeError:
+        return tuple([0 if o is None else addr(o) or 0 for o in objs])
+
+
+def all_strides(objs: tuple) -> tuple:
+    """Strides in elements of each, None for a missing array."""
+    if _STRIDE is None:
+        _torch_methods()
+    try:
+        return tuple(map(_STRIDE, objs))
+    except TypeError:
+        return tuple([None if o is None else elem_strides(o) for o in objs])
+
+
+def dense(objs: tuple, shapes: list) -> bool:
+    """Whether every array is contiguous and of its shape."""
+    if _CONTIGUOUS is None:
+        _torch_methods()
+    try:
+        return list(map(_SHAPE, objs)) == shapes and all(map(_CONTIGUOUS, objs))
+    except TypeError:
+        return [tuple(o.shape) for o in objs] == shapes and all([is_contiguous(o) for o in objs])
 
 
 def shape(a: Any) -> tuple[int, ...]:
@@ -73,10 +118,11 @@ def itemsize(a: Any) -> int:
 
 def elem_strides(a: Any) -> tuple[int, ...]:
     """Strides in elements."""
+    stride = getattr(a, "stride", None)
+    if stride is not None:
+        return stride()
     if isinstance(a, np.ndarray):
         return tuple(int(s // a.itemsize) for s in a.strides)
-    if _is_torch(a):
-        return tuple(int(s) for s in a.stride())
     size = itemsize(a)
     out = []
     for s in a.strides:

@@ -8,8 +8,8 @@ from __future__ import annotations
 import ctypes as C
 from typing import Any
 
-from . import abi, types
-from .arrays import addr, elem_strides, is_contiguous, itemsize, length, shape
+from . import abi, calls, types
+from .arrays import addr, addrs, all_strides, dense, elem_strides, is_contiguous, itemsize, length, shape
 
 
 _UPSTREAM: dict | None = None
@@ -73,11 +73,6 @@ def upstream_constants(module_types: Any = None, module_solver: Any = None) -> d
     return out
 
 
-def _upstream_constants() -> tuple[float, int, int]:
-    c = upstream_constants()
-    return c["alpha_noise_eps"], c["overflow_iterations"], c["overflow_ls_iterations"]
-
-
 def _mulm_lanes(m: Any):
     """The lane program of a model's M_mulm rows; built once (and cached on the model) for
     Model objects that come from mujoco-warp and do not carry it."""
@@ -106,34 +101,25 @@ def _mulm_lanes(m: Any):
     return lanes
 
 
+_MODEL = calls.getter("opt.tolerance", "opt.ls_tolerance", "stat.meaninertia", "M_rowadr", "M_rownnz", "M_colind",
+                      "M_mulm_rowadr", "M_mulm_col", "M_mulm_madr")
+_pack_model = abi.packer(abi.ImnModel)
+
+
+def pack_model(m: Any) -> bytes:
+    c, opt = upstream_constants(), m.opt
+    arrays = (*_MODEL(m), _mulm_lanes(m))
+    tolerance, ls_tolerance, meaninertia, _, _, colind, _, _, _, lanes = arrays
+    return _pack_model(
+        m.nv, m.nv_pad, colind.shape[0], int(opt.iterations), int(opt.ls_iterations),
+        0 if int(opt.disableflags) & c["disable_warmstart"] else 1,
+        tolerance.shape[0], ls_tolerance.shape[0], meaninertia.shape[0], *addrs(arrays),
+        c["alpha_noise_eps"], c["overflow_iterations"], c["overflow_ls_iterations"],
+        int(getattr(opt, "warn_overflow", 0) or 0), lanes.shape[0] - 1)
+
+
 def model_struct(m: Any) -> abi.ImnModel:
-    eps, ovf_it, ovf_ls = _upstream_constants()
-    s = abi.ImnModel()
-    s.nv = int(m.nv)
-    s.nv_pad = int(m.nv_pad)
-    s.nM = int(shape(m.M_colind)[0])
-    s.iterations = int(m.opt.iterations)
-    s.ls_iterations = int(m.opt.ls_iterations)
-    s.warmstart = 0 if (int(m.opt.disableflags) & upstream_constants()["disable_warmstart"]) else 1
-    s.n_tolerance = length(m.opt.tolerance)
-    s.n_ls_tolerance = length(m.opt.ls_tolerance)
-    s.n_meaninertia = length(m.stat.meaninertia)
-    s.opt_tolerance = addr(m.opt.tolerance)
-    s.opt_ls_tolerance = addr(m.opt.ls_tolerance)
-    s.stat_meaninertia = addr(m.stat.meaninertia)
-    s.M_rowadr = addr(m.M_rowadr)
-    s.M_rownnz = addr(m.M_rownnz)
-    s.M_colind = addr(m.M_colind)
-    s.M_mulm_rowadr = addr(m.M_mulm_rowadr)
-    s.M_mulm_col = addr(m.M_mulm_col)
-    s.M_mulm_madr = addr(m.M_mulm_madr)
-    lanes = _mulm_lanes(m)
-    s.M_mulm_lanes, s.n_mulm_batches = addr(lanes), int(shape(lanes)[0]) - 1
-    s.alpha_noise_eps = eps
-    s.overflow_iterations = ovf_it
-    s.overflow_ls_iterations = ovf_ls
-    s.warn_overflow = int(getattr(m.opt, "warn_overflow", 0) or 0)
-    return s
+    return abi.ImnModel.from_buffer_copy(pack_model(m))
 
 
 def _row_ld(a: Any) -> int:
@@ -143,121 +129,110 @@ def _row_ld(a: Any) -> int:
     return st[0]
 
 
-def _same_ld(name: str, arrays: list[Any]) -> int:
-    lds = {_row_ld(a) for a in arrays if a is not None}
+def _same_ld(name: str, strides: tuple) -> int:
+    first = strides[0]
+    if first is not None and strides == (first,) * len(strides) and len(first) == 2 and first[1] == 1:
+        return first[0]
+    present = [st for st in strides if st is not None]
+    if any([st[-1] != 1 for st in present]):
+        raise ValueError("solver buffers need a unit innermost stride")
+    lds = {st[0] for st in present}
     if len(lds) != 1:
         raise ValueError(f"{name} arrays must share one world stride, got {sorted(lds)}")
     return lds.pop()
 
 
-def data_struct(m: Any, d: Any) -> abi.ImnData:
-    s = abi.ImnData()
-    s.nworld = int(d.nworld)
-    s.njmax = int(d.njmax)
-    s.nefc, s.ne, s.nf = addr(d.nefc), addr(d.ne), addr(d.nf)
-    s.qacc_smooth = addr(d.qacc_smooth)
-    s.qacc_warmstart = addr(d.qacc_warmstart)
-    s.qfrc_smooth = addr(d.qfrc_smooth)
-    s.dof_ld = _same_ld(
-        "dof",
-        [d.qacc_smooth, d.qacc_warmstart, d.qfrc_smooth, d.qacc, d.qfrc_constraint, d.efc.Ma],
-    )
-    s.efc_J = addr(d.efc.J)
-    if s.njmax > 0 and getattr(d.efc, "J_world_offset", None) is not None:
-        s.efc_ld = _same_ld(
-            "efc", [d.efc.D, d.efc.aref, d.efc.frictionloss, d.efc.force, d.efc.state]
-        )
-    elif s.njmax > 0:
-        js = elem_strides(d.efc.J)
-        if js[2] != 1:
-            raise ValueError("efc.J needs a unit innermost stride")
-        s.J_ld_world, s.J_ld_row = js[0], js[1]
-        s.efc_ld = _same_ld(
-            "efc", [d.efc.D, d.efc.aref, d.efc.frictionloss, d.efc.force, d.efc.state]
-        )
-    else:
-        # a model without constraint storage: the row arrays are empty, their strides
-        # carry no information, and only the rowless hand-off may be called
-        s.J_ld_world = s.J_ld_row = s.efc_ld = 0
-    s.efc_D = addr(d.efc.D)
-    s.efc_aref = addr(d.efc.aref)
-    s.efc_frictionloss = addr(d.efc.frictionloss)
-    s.M = addr(d.M)
-    s.M_ld = _row_ld(d.M)
-    s.qacc = addr(d.qacc)
-    s.qfrc_constraint = addr(d.qfrc_constraint)
-    s.efc_Ma = addr(d.efc.Ma)
-    s.efc_force = addr(d.efc.force)
-    s.efc_state = addr(d.efc.state)
-    s.solver_niter = addr(d.solver_niter)
-    s.overflow = addr(d.overflow)
+_DATA = calls.getter("nefc", "ne", "nf", "qacc_smooth", "qacc_warmstart", "qfrc_smooth", "efc.J", "efc.D", "efc.aref",
+                     "efc.frictionloss", "M", "qacc", "qfrc_constraint", "efc.Ma", "efc.force", "efc.state", "solver_niter",
+                     "overflow")
+_pack_data = abi.packer(abi.ImnData)
+
+
+def pack_data(m: Any, d: Any) -> tuple[bytes, int, int]:
+    """(ImnData, world stride of the dof arrays, of the row arrays)."""
+    nworld, njmax = int(d.nworld), int(d.njmax)
+    arrays = _DATA(d)
+    J, strides = arrays[6], all_strides(arrays[3:6] + arrays[10:14])
+    M_ld, inner = strides[3]
+    if inner != 1:
+        raise ValueError("solver buffers need a unit innermost stride")
+    dof_ld = _same_ld("dof", strides[:3] + strides[4:])
     offsets = getattr(d.efc, "J_world_offset", None)
+    ld_world = ld_row = efc_ld = offset_addr = elems = 0
     if offsets is not None:
         # compact J: (total rows, >= nv) with one int64 element offset per world
-        if itemsize(offsets) != 8 or length(offsets) < s.nworld:
+        if itemsize(offsets) != 8 or length(offsets) < nworld:
             raise ValueError("efc.J_world_offset must hold one int64 per world")
-        js = elem_strides(d.efc.J)
+        js = elem_strides(J)
         if len(js) != 2 or js[1] != 1:
             raise ValueError("a compact efc.J is a (rows, nv) array with a unit innermost stride")
-        s.J_world_offset = addr(offsets)
-        s.J_ld_world, s.J_ld_row = 0, js[0]
-        s.J_elems = int(shape(d.efc.J)[0]) * js[0]
-    return s
+        offset_addr = addr(offsets) or 0
+        ld_row = js[0]
+        elems = length(J) * js[0]
+    elif njmax > 0:
+        js = elem_strides(J)
+        if js[2] != 1:
+            raise ValueError("efc.J needs a unit innermost stride")
+        ld_world, ld_row = js[0], js[1]
+    if njmax > 0:
+        efc_ld = _same_ld("efc", all_strides(arrays[7:10] + arrays[14:16]))
+    # else: a model without constraint storage: the row arrays are empty, their strides carry no
+    # information, and only the rowless hand-off may be called
+    (a_nefc, a_ne, a_nf, a_smooth, a_warm, a_qfs, a_J, a_D, a_aref, a_loss, a_M, a_qacc, a_qfrc, a_Ma, a_force, a_state,
+     a_niter, a_overflow) = addrs(arrays)
+    packed = _pack_data(nworld, njmax, a_nefc, a_ne, a_nf, a_smooth, a_warm, a_qfs, dof_ld, a_J, ld_world, ld_row, a_D, a_aref,
+                        a_loss, efc_ld, a_M, M_ld, a_qacc, a_qfrc, a_Ma, a_force, a_state, a_niter, a_overflow,
+                        offset_addr, elems)
+    return packed, dof_ld, efc_ld
 
 
-_CTX_WORLD_ARRAYS = (
-    "search_dot",
-    "grad_dot",
-    "grad_scale",
-    "newton_decrement",
-    "improvement",
-    "alpha",
-    "done",
-    "search_unchanged",
-    "ls_exhausted",
-    "quad_changed_count",
-    "state_changed_count",
-)
+def data_struct(m: Any, d: Any) -> abi.ImnData:
+    return abi.ImnData.from_buffer_copy(pack_data(m, d)[0])
+
+
+_CTX_ARRAYS = ("Jaref", "jv", "search", "mv", "grad", "h", "hfactor", "search_dot", "grad_dot", "grad_scale",
+               "newton_decrement", "improvement", "alpha", "done", "search_unchanged", "ls_exhausted", "quad_changed_ids",
+               "quad_changed_count", "state_changed_count", "newton_dof_union", "world_order", "stats", "work_counter")
+_CTX_ROWS = ("Jaref", "jv", "search", "mv", "quad_changed_ids")
+_CTX = calls.getter(*_CTX_ARRAYS)
+_pack_ctx = abi.packer(abi.ImnCtx)
+
+
+def pack_ctx(nworld: int, dof_ld: int, efc_ld: int, ctx: Any, nsolving: Any, plan_address: int = 0) -> bytes:
+    """``ctx`` may omit any array (attribute missing or None): the kernel then skips
+    writing it back."""
+    try:
+        arrays = _CTX(ctx)
+    except AttributeError:
+        arrays = tuple([getattr(ctx, name, None) for name in _CTX_ARRAYS])
+    # grad, which has a stride of its own, and the arrays that share one with the row or dof arrays
+    grad_stride, *strides = all_strides((arrays[4], *arrays[:4], arrays[16]))
+    if grad_stride is not None and grad_stride[-1] != 1:
+        raise ValueError("solver buffers need a unit innermost stride")
+    rows, dofs = (efc_ld, 1), (dof_ld, 1)
+    if strides != [rows, rows, dofs, dofs, rows]:
+        for name, st, want in zip(_CTX_ROWS, strides, (rows, rows, dofs, dofs, rows)):
+            if st is not None and st[-1] != 1:
+                raise ValueError("solver buffers need a unit innermost stride")
+            if st is not None and st[0] != want[0]:
+                raise ValueError(f"ctx.{name} must share the world stride of the {'efc' if want is rows else 'dof'} arrays")
+    order, stats = arrays[20], arrays[21]
+    if order is not None and length(order) < nworld:
+        raise ValueError("ctx.world_order must hold one int32 per world")
+    if stats is not None and (tuple(stats.shape) != (nworld, 4) or elem_strides(stats) != (4, 1)):
+        raise ValueError("ctx.stats must be a contiguous (nworld, 4) int32 array")
+    try:
+        at = [0 if a is None else a.data_ptr() for a in arrays]
+    except AttributeError:
+        at = addrs(arrays)
+    return _pack_ctx(*at[:5], grad_stride[0] if grad_stride is not None else 0, *at[5:20], addr(nsolving) or 0, plan_address,
+                     *at[20:])
 
 
 def ctx_struct(d_struct: abi.ImnData, ctx: Any, nsolving: Any, sparse_plan_struct=None) -> abi.ImnCtx:
-    """``ctx`` may omit any array (attribute missing or None): the kernel then skips
-    writing it back."""
-    s = abi.ImnCtx()
-
-    def get(name):
-        return getattr(ctx, name, None) if ctx is not None else None
-
-    for name in ("Jaref", "jv", "quad_changed_ids"):
-        a = get(name)
-        if a is not None and _row_ld(a) != d_struct.efc_ld:
-            raise ValueError(f"ctx.{name} must share the world stride of the efc arrays")
-        setattr(s, name, addr(a))
-    for name in ("search", "mv"):
-        a = get(name)
-        if a is not None and _row_ld(a) != d_struct.dof_ld:
-            raise ValueError(f"ctx.{name} must share the world stride of the dof arrays")
-        setattr(s, name, addr(a))
-    g = get("grad")
-    s.grad = addr(g)
-    s.grad_ld = _row_ld(g) if g is not None else 0
-    s.h = addr(get("h"))
-    s.hfactor = addr(get("hfactor"))
-    for name in _CTX_WORLD_ARRAYS:
-        setattr(s, name, addr(get(name)))
-    s.dof_union = addr(get("newton_dof_union"))
-    s.nsolving = addr(nsolving)
+    s = abi.ImnCtx.from_buffer_copy(pack_ctx(d_struct.nworld, d_struct.dof_ld, d_struct.efc_ld, ctx, nsolving))
     if sparse_plan_struct is not None:
         s.sparse_plan = C.pointer(sparse_plan_struct)
-    order = get("world_order")
-    if order is not None and length(order) < d_struct.nworld:
-        raise ValueError("ctx.world_order must hold one int32 per world")
-    s.world_order = addr(order)
-    stats = get("stats")
-    if stats is not None and (tuple(shape(stats)) != (d_struct.nworld, 4) or elem_strides(stats) != (4, 1)):
-        raise ValueError("ctx.stats must be a contiguous (nworld, 4) int32 array")
-    s.stats = addr(stats)
-    s.work_counter = addr(get("work_counter"))
     return s
 
 
@@ -267,54 +242,64 @@ def _timestep(m: Any) -> tuple[int, int]:
     h = m.opt.timestep
     if isinstance(h, (int, float)) or h is None:
         raise ValueError("m.opt.timestep must be a float array of length 1 or nworld, next to the other arrays")
-    n = length(h)
+    n = h.shape[0]
     if n <= 0 or not is_contiguous(h):
         raise ValueError("m.opt.timestep must be a contiguous, non-empty float array")
     return addr(h), n
 
 
-def implicit_struct(m: Any, d: Any, velocity_gain: Any, coefficients: Any = None) -> abi.ImnImplicit:
+_pack_implicit, _pack_advance = abi.packer(abi.ImnImplicit), abi.packer(abi.ImnAdvance)
+
+
+def pack_implicit(m: Any, d: Any, velocity_gain: Any, coefficients: Any = None) -> bytes:
     """``velocity_gain``: (nworld, nu) d(actuator force)/d(actuator velocity), or None.  With
     ``coefficients`` (g2, b2 per actuator) the kernel forms it from ``d.ctrl`` and stores it there."""
-    c = upstream_constants()
-    s = abi.ImnImplicit()
-    flags = int(m.opt.disableflags)
-    s.nv, s.nM = int(m.nv), int(shape(m.M_colind)[0])
-    s.nu = int(getattr(m, "nu", 0) or 0)
-    s.actuation = 0 if flags & c["disable_actuation"] else 1
-    s.damper = 0 if flags & c["disable_damper"] else 1
-    s.timestep, s.n_timestep = _timestep(m)
-    s.dof_damping = addr(m.dof_damping)
-    s.M_elemid = addr(m.M_elemid)
-    if s.nu and s.actuation:
+    c, flags, nu, W = upstream_constants(), int(m.opt.disableflags), int(getattr(m, "nu", 0) or 0), int(d.nworld)
+    actuation = 0 if flags & c["disable_actuation"] else 1
+    timestep, n_timestep = _timestep(m)
+    tables = m.dof_damping, m.M_elemid
+    nnz = adr = col = moment = gain = moment_ld = ctrl = ctrl_ld = g2 = b2 = n_coefficients = 0
+    if nu and actuation:
         if velocity_gain is None:
             raise ValueError("an actuated model needs the actuators' velocity gains")
-        for name in ("moment_rownnz", "moment_rowadr"):
-            a = getattr(d, name)
-            if tuple(shape(a)) != (int(d.nworld), s.nu) or elem_strides(a) != (s.nu, 1):
-                raise ValueError(f"d.{name} must be a contiguous (nworld, nu) array")
-            setattr(s, name, addr(a))
-        if elem_strides(d.moment_colind) != elem_strides(d.actuator_moment) or elem_strides(d.actuator_moment)[1] != 1:
+        per_actuator = d.moment_rownnz, d.moment_rowadr, velocity_gain
+        if not dense(per_actuator, [(W, nu)] * 3):
+            for name, a in zip(("d.moment_rownnz", "d.moment_rowadr", "velocity gains"), per_actuator):
+                if tuple(a.shape) != (W, nu) or not is_contiguous(a):
+                    raise ValueError(f"{name} must be a contiguous (nworld, nu) array")
+        entries = d.moment_colind, d.actuator_moment
+        strides = all_strides(entries)
+        moment_ld, inner = strides[1]
+        if strides[0] != strides[1] or inner != 1:
             raise ValueError("d.moment_colind and d.actuator_moment must share one layout")
-        if tuple(shape(velocity_gain)) != (int(d.nworld), s.nu) or elem_strides(velocity_gain) != (s.nu, 1):
-            raise ValueError("velocity gains must be a contiguous (nworld, nu) array")
-        s.moment_colind, s.actuator_moment = addr(d.moment_colind), addr(d.actuator_moment)
-        s.moment_ld = elem_strides(d.actuator_moment)[0]
-        s.actuator_velocity_gain = addr(velocity_gain)
-        if coefficients is not None:
-            g2, b2 = coefficients
-            s.ctrl, s.ctrl_ld = addr(d.ctrl), _row_ld(d.ctrl)
-            s.gain_g2, s.gain_b2, s.n_coefficients = addr(g2), addr(b2), (length(g2) if len(shape(g2)) == 2 else 1)
-            s.velocity_gain_out = addr(velocity_gain)
-    return s
+        if coefficients is None:
+            damping, elemid, nnz, adr, gain, col, moment = addrs(tables + per_actuator + entries)
+        else:
+            dims = coefficients[0].shape
+            n_coefficients, ctrl_ld = dims[0] if len(dims) == 2 else 1, _row_ld(d.ctrl)
+            damping, elemid, nnz, adr, gain, col, moment, ctrl, g2, b2 = addrs(
+                tables + per_actuator + entries + (d.ctrl, *coefficients))
+    else:
+        damping, elemid = addrs(tables)
+    return _pack_implicit(m.nv, length(m.M_colind), nu, actuation, 0 if flags & c["disable_damper"] else 1, timestep, n_timestep,
+                          damping, elemid, nnz, adr, col, moment, moment_ld, gain, ctrl, ctrl_ld, g2, b2, n_coefficients,
+                          gain if ctrl else 0)
+
+
+def implicit_struct(m: Any, d: Any, velocity_gain: Any, coefficients: Any = None) -> abi.ImnImplicit:
+    return abi.ImnImplicit.from_buffer_copy(pack_implicit(m, d, velocity_gain, coefficients))
+
+
+def pack_advance(m: Any, d: Any) -> bytes:
+    timestep, n_timestep = _timestep(m)
+    state = d.qvel, d.qpos
+    (qvel_ld, qvel_in), (qpos_ld, qpos_in) = all_strides(state)
+    if qvel_in != 1 or qpos_in != 1:
+        raise ValueError("solver buffers need a unit innermost stride")
+    kind, dofadr, qposadr, qvel, qpos = addrs((m.jnt_type, m.jnt_dofadr, m.jnt_qposadr, *state))
+    return _pack_advance(m.nv, m.nq, m.njnt, timestep, n_timestep, kind, dofadr, qposadr, qvel, qvel_ld, qpos, qpos_ld,
+                         addr(getattr(d, "time", None)) or 0)
 
 
 def advance_struct(m: Any, d: Any) -> abi.ImnAdvance:
-    s = abi.ImnAdvance()
-    s.nv, s.nq, s.njnt = int(m.nv), int(m.nq), int(m.njnt)
-    s.timestep, s.n_timestep = _timestep(m)
-    s.jnt_type, s.jnt_dofadr, s.jnt_qposadr = addr(m.jnt_type), addr(m.jnt_dofadr), addr(m.jnt_qposadr)
-    s.qvel, s.qvel_ld = addr(d.qvel), _row_ld(d.qvel)
-    s.qpos, s.qpos_ld = addr(d.qpos), _row_ld(d.qpos)
-    s.time = addr(getattr(d, "time", None))
-    return s
+    return abi.ImnAdvance.from_buffer_copy(pack_advance(m, d))

@@ -106,17 +106,12 @@ def create_blocked_dense_factor_solve_scratch(
 
 
 def _launch(scratch, M, y, U, x, active, nworld, rhs_count, mode, stream):
-    def build():
-        for name, a in (("y", y), ("x", x), ("U", U)):
-            if not is_contiguous(a):
-                raise ValueError(f"blocked dense factor/solve needs a contiguous {name}")
-        return (C.byref(scratch.struct), addr(M) if M is not None else None, elem_strides(M)[0] if M is not None else 0,
-                addr(y), addr(U), addr(x), addr(active), int(nworld), int(rhs_count), int(mode)), None
-
-    buffers = tuple(a for a in (M, y, U, x, active) if a is not None)
-    # factor and solve-only calls are prepared side by side
-    calls.call(scratch, "imn_blocked_dense_factor_solve", buffers, (M is None, active is None, nworld, rhs_count, mode), build,
-               stream, slot=mode)
+    for name, a in (("y", y), ("x", x), ("U", U)):
+        if not is_contiguous(a):
+            raise ValueError(f"blocked dense factor/solve needs a contiguous {name}")
+    calls.call("imn_blocked_dense_factor_solve", (
+        C.byref(scratch.struct), addr(M), elem_strides(M)[0] if M is not None else 0, addr(y), addr(U), addr(x), addr(active),
+        int(nworld), int(rhs_count), int(mode)), stream)
 
 
 def blocked_dense_factor_solve(

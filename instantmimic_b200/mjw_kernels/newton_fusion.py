@@ -100,90 +100,34 @@ def attach_scratch(m: Any, d: Any, ctx: Any, device: Any) -> None:
 
 
 class SolveCall:
-    """The structs of one (Model, Data, context) triple, built once.
-
-    Struct construction walks ~60 attributes; a step pipeline calls the solve every
-    substep with the same buffers, so the result is cached on the scratch object
-    and only revalidated by address."""
+    """The packed structs of one (Model, Data, context) triple as its buffers are now.  Every solve
+    packs its own: a call is for one use (or for ``launch_info``) and is not kept."""
 
     def __init__(self, m: Any, d: Any, ctx: Any, nsolving: Any):
-        self.m = binding.model_struct(m)
-        self.d = binding.data_struct(m, d)
         plan = getattr(ctx, "sparse_hessian_plan", None)
+        # the plan's struct has to outlive the call
         self.plan_struct = getattr(plan, "struct", None) if plan is not None and plan.path == "fused" else None
-        self.c = binding.ctx_struct(self.d, ctx, nsolving, self.plan_struct)
-        self.key = _key(m, d, ctx, nsolving)
-        self.args = (C.byref(self.m), C.byref(self.d), C.byref(self.c))
+        data, dof_ld, efc_ld = binding.pack_data(m, d)
+        address = C.addressof(self.plan_struct) if self.plan_struct is not None else 0
+        self.args = (binding.pack_model(m), data, binding.pack_ctx(int(d.nworld), dof_ld, efc_ld, ctx, nsolving, address))
 
     def launch_info(self) -> abi.ImnLaunchInfo:
         info = abi.ImnLaunchInfo()
-        _lib.check(
-            _lib.lib().imn_launch_info(C.byref(self.m), C.byref(self.d), C.byref(self.c), C.byref(info)),
-            "imn_launch_info",
-        )
+        _lib.check(_lib.packed("imn_launch_info")(*self.args, C.byref(info)), "imn_launch_info")
         return info
 
     def __call__(self, stream=None) -> None:
-        if _lib.nvtx_enabled():
-            with _lib.nvtx("imn_solve"):
-                rc = _lib.lib().imn_solve(*self.args, _lib.current_stream_handle(stream))
-        else:
-            rc = _lib.lib().imn_solve(*self.args, _lib.current_stream_handle(stream))
-        if rc:
-            _lib.check(rc, "imn_solve")
-
-
-_KEY_DATA = ("nefc", "ne", "nf", "qacc_smooth", "qacc_warmstart", "qfrc_smooth", "M", "qacc",
-             "qfrc_constraint", "solver_niter", "overflow", "efc.J", "efc.D", "efc.aref", "efc.frictionloss", "efc.force",
-             "efc.state", "efc.Ma")
-_KEY_CTX = ("Jaref", "jv", "search", "mv", "grad", "h", "hfactor", "quad_changed_ids", "newton_dof_union",
-            "world_order", "stats", "work_counter") + binding._CTX_WORLD_ARRAYS
-_KEY_SCALARS = ("nv", "nv_pad", "is_sparse", "opt.iterations", "opt.ls_iterations", "opt.disableflags", "opt.solver",
-                "opt.integrator", "opt.cone", "block_dim.linesearch_iterative")
-_data, _ctx, _scalars = calls.getter(*_KEY_DATA), calls.getter(*_KEY_CTX), calls.getter(*_KEY_SCALARS)
-_options = calls.getter("opt.tolerance", "opt.ls_tolerance", "stat.meaninertia")
-
-
-def _ctx_arrays(ctx) -> tuple:
-    try:
-        return _ctx(ctx)
-    except AttributeError:
-        return tuple(getattr(ctx, n, None) for n in _KEY_CTX)
-
-
-def _key(m, d, ctx, nsolving):
-    """Everything the cached structs were built from: the address of every buffer the
-    kernel is handed, the scalar options, and what ``eligible`` looks at.  A caller that rebinds
-    any of them gets fresh structs instead of stale pointers."""
-    return (
-        id(m), id(d), id(ctx), id(getattr(ctx, "sparse_hessian_plan", None)),
-        calls.pointers(_data(d)),
-        calls.optional_pointers(_ctx_arrays(ctx) + (nsolving, getattr(d.efc, "J_world_offset", None))),
-        calls.pointers(_options(m)), _scalars(m), getattr(m.opt, "warn_overflow", 0), d.nworld, d.njmax,
-    )
-
-
-def cached_call(m: Any, d: Any, ctx: Any, nsolving: Any, holder: Any) -> SolveCall | None:
-    """The holder's prepared call when it was built from exactly these buffers and options (which
-    then also passed ``eligible``)."""
-    call = getattr(holder, "_imn_solve_call", None)
-    return call if call is not None and call.key == _key(m, d, ctx, nsolving) else None
+        calls.call("imn_solve", self.args, stream)
 
 
 def solve_call(m: Any, d: Any, ctx: Any, nsolving: Any, cache_on: Any = None) -> SolveCall:
-    holder = cache_on if cache_on is not None else ctx
-    call = cached_call(m, d, ctx, nsolving, holder)
-    if call is None:
-        call = SolveCall(m, d, ctx, nsolving)
-        try:
-            holder._imn_solve_call = call
-        except AttributeError:
-            pass
-    return call
+    """``cache_on`` is accepted for callers that name the scratch; nothing is kept on it."""
+    del cache_on
+    return SolveCall(m, d, ctx, nsolving)
 
 
 def run(m: Any, d: Any, ctx: Any, nsolving: Any, stream=None) -> None:
     """Init, every Newton iteration and the final force of all worlds: one launch
     (reference: init_context + run + qfrc_constraint_from_grad,
     newton_fusion.py:330-409, 431-472, 522-539)."""
-    solve_call(m, d, ctx, nsolving)(stream)
+    SolveCall(m, d, ctx, nsolving)(stream)

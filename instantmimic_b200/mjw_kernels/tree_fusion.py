@@ -19,14 +19,13 @@ path, so a missing scratch is an error.
 
 from __future__ import annotations
 
-import ctypes as C
 from dataclasses import dataclass, field
 from typing import Any
 
 import numpy as np
 
 from .. import abi, binding, calls
-from ..arrays import addr, device_of, elem_strides, is_contiguous, is_device, length, shape, to_host
+from ..arrays import addr, addrs, dense, device_of, elem_strides, is_contiguous, is_device, length, to_host
 
 
 @dataclass(frozen=True)
@@ -101,76 +100,92 @@ def _need(scratch: Any, who: str) -> None:
             f"{who}: this library has no per-level upstream path; pass the scratch of create_tree_reduction_scratch")
 
 
+_TREE = calls.getter("bodies", "offsets", "child_ptr", "child_ids")
+_DOFS = ("body_parentid", "body_dofadr", "body_dofnum", "dof_bodyid", "dof_parentid")
+_JOINT_TABLES = calls.getter(*_DOFS, "body_jntnum", "body_jntadr", "jnt_type")
+_INERTIA_TABLES = calls.getter(*_DOFS, "dof_armature", "M_hinit_i", "M_colind")
+_GRAVITY_TABLES = calls.getter(*_DOFS, "opt.gravity")
+_pack_tree = abi.packer(abi.ImnBodyTree)
+
+
+def _rows_of(a: Any, width: int, name: str, extent: str) -> int:
+    """Rows of a contiguous (n, width) or (width) option array."""
+    dims = a.shape
+    if dims[-1] != width or not is_contiguous(a):
+        raise ValueError(f"m.{name} must be a contiguous (n, {extent}) or ({extent}) array")
+    return dims[0] if len(dims) == 2 else 1
+
+
+# The C struct over the model's tables, one function per set of tables that a call reads.
+
+def pack_tree(m: Any, t: TreeReductionScratch) -> bytes:
+    """The tree alone."""
+    parent = m.body_parentid
+    at = addrs((parent, *_TREE(t)))
+    return _pack_tree(parent.shape[0], 0, 0, t.levels, *at, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, getattr(t, "team_lanes", 32))
+
+
+def pack_tree_joints(m: Any, t: TreeReductionScratch) -> bytes:
+    tables = _JOINT_TABLES(m)
+    parent, dofadr, dofnum, body, dof_parent, jntnum, jntadr, kind, *tree = addrs(tables + _TREE(t))
+    return _pack_tree(tables[0].shape[0], m.nv, 0, t.levels, parent, *tree, jntnum, jntadr, dofadr, dofnum, kind, body, dof_parent,
+                      0, 0, 0, 0, 0, 0, 0, getattr(t, "team_lanes", 32))
+
+
+def pack_tree_inertia(m: Any, t: TreeReductionScratch) -> bytes:
+    tables, nv = _INERTIA_TABLES(m), m.nv
+    parent, dofadr, dofnum, body, dof_parent, armature, rows, cols, *tree = addrs(tables + _TREE(t))
+    return _pack_tree(tables[0].shape[0], nv, tables[7].shape[0], t.levels, parent, *tree, 0, 0, dofadr, dofnum, 0, body, dof_parent,
+                      armature, _rows_of(tables[5], nv, "dof_armature", "nv"), rows, cols, 0, 0, 0, getattr(t, "team_lanes", 32))
+
+
+def pack_tree_gravity(m: Any, t: TreeReductionScratch) -> bytes:
+    tables = _GRAVITY_TABLES(m)
+    parent, dofadr, dofnum, body, dof_parent, gravity, *tree = addrs(tables + _TREE(t))
+    enabled = 0 if int(m.opt.disableflags) & binding.upstream_constants()["disable_gravity"] else 1
+    return _pack_tree(tables[0].shape[0], m.nv, 0, t.levels, parent, *tree, 0, 0, dofadr, dofnum, 0, body, dof_parent, 0, 0, 0, 0,
+                      gravity, _rows_of(tables[5], 3, "opt.gravity", "3"), enabled, getattr(t, "team_lanes", 32))
+
+
 def tree_struct(m: Any, scratch: TreeReductionScratch, *, dofs: bool = False, joints: bool = False,
                 inertia: bool = False, gravity: bool = False) -> abi.ImnBodyTree:
-    """The C struct over the model's tables; the flags name what the call reads."""
-    s = abi.ImnBodyTree()
-    s.nbody = length(m.body_parentid)
-    s.nlevels = int(scratch.levels)
-    s.body_parentid = addr(m.body_parentid)
-    s.level_bodies, s.level_offsets = addr(scratch.bodies), addr(scratch.offsets)
-    s.child_ptr, s.child_ids = addr(scratch.child_ptr), addr(scratch.child_ids)
-    s.team_lanes = int(getattr(scratch, "team_lanes", 32))
-    if dofs:
-        s.nv = int(m.nv)
-        s.body_dofadr, s.body_dofnum = addr(m.body_dofadr), addr(m.body_dofnum)
-        s.dof_bodyid, s.dof_parentid = addr(m.dof_bodyid), addr(m.dof_parentid)
-    if joints:
-        s.body_jntadr, s.body_jntnum, s.jnt_type = addr(m.body_jntadr), addr(m.body_jntnum), addr(m.jnt_type)
-    if inertia:
-        s.nM = length(m.M_colind)
-        arm = m.dof_armature
-        dims = shape(arm)
-        if dims[-1] != m.nv or not is_contiguous(arm):
-            raise ValueError("m.dof_armature must be a contiguous (n, nv) or (nv) array")
-        s.dof_armature, s.n_armature = addr(arm), (dims[0] if len(dims) == 2 else 1)
-        s.M_rowidx, s.M_colind = addr(m.M_hinit_i), addr(m.M_colind)
-    if gravity:
-        g = m.opt.gravity
-        dims = shape(g)
-        if dims[-1] != 3 or not is_contiguous(g):
-            raise ValueError("m.opt.gravity must be a contiguous (n, 3) or (3) array")
-        s.gravity, s.n_gravity = addr(g), (dims[0] if len(dims) == 2 else 1)
-        s.gravity_enabled = 0 if int(m.opt.disableflags) & binding.upstream_constants()["disable_gravity"] else 1
-    return s
+    """The struct for a call that reads the named tables (each set includes the dofs')."""
+    pack = pack_tree_inertia if inertia else pack_tree_gravity if gravity else pack_tree_joints if joints else pack_tree
+    return abi.ImnBodyTree.from_buffer_copy(pack(m, scratch))
 
 
 def _per_body(a: Any, nworld: int, nbody: int, width: int, name: str) -> int:
     """Address of a contiguous (nworld, nbody, width) float array (a Warp vector array has
     the same bytes with the last extent folded into its dtype)."""
-    dims = tuple(shape(a))
-    if dims not in ((nworld, nbody, width), (nworld, nbody)) or not is_contiguous(a):
+    if tuple(a.shape) not in ((nworld, nbody, width), (nworld, nbody)) or not is_contiguous(a):
         raise ValueError(f"{name} must be a contiguous ({nworld}, {nbody}, {width}) float array")
     return addr(a)
+
+
+def _all_per_body(arrays: tuple, nworld: int, extents: tuple, names: tuple) -> tuple:
+    """The same for several arrays; extents: (rows, width) of each."""
+    if dense(arrays, [(nworld, n, width) for n, width in extents]):
+        return addrs(arrays)
+    return tuple([_per_body(a, nworld, n, width, "d." + name) for a, (n, width), name in zip(arrays, extents, names)])
 
 
 def _row_ld(a: Any) -> int:
     return elem_strides(a)[0]
 
 
-# what each stage's structs are built from: the model's tables, the scratch's, the batch's buffers
-_TREE = calls.getter("bodies", "offsets", "child_ptr", "child_ids")
-_TREE_DOFS = calls.getter("body_parentid", "body_dofadr", "body_dofnum", "dof_bodyid", "dof_parentid")
-_CRB_MODEL = calls.getter("body_parentid", "body_dofadr", "body_dofnum", "dof_bodyid", "dof_parentid", "dof_armature",
-                          "M_hinit_i", "M_colind")
-_CRB_DATA = calls.getter("cinert", "cdof", "crb", "M")
-_RNE_MODEL = calls.getter("body_parentid", "body_dofadr", "body_dofnum", "dof_bodyid", "dof_parentid", "opt.gravity")
-_RNE_DATA = calls.getter("cinert", "cvel", "cdof", "cdof_dot", "qvel", "cacc", "cfrc_int", "qfrc_bias")
+_CRB = calls.getter("cinert", "cdof", "crb")
+_RNE_NAMES = ("cinert", "cvel", "cdof", "cdof_dot", "cacc", "cfrc_int")
+_RNE = calls.getter(*_RNE_NAMES)
 
 
 def accumulate(m: Any, d: Any, values: Any, components: int, skip_root_parent: bool, scratch: TreeReductionScratch,
                stream=None) -> None:
     """values[:, parent] += values[:, body], deepest level first (tree_fusion.py:138-170)."""
     _need(scratch, "accumulate")
-
-    def build():
-        nbody = length(m.body_parentid)
-        ptr = _per_body(values, d.nworld, nbody, components, "values")
-        t = tree_struct(m, scratch)
-        return (C.byref(t), ptr, nbody * components, int(components), int(bool(skip_root_parent)), int(d.nworld)), t
-
-    calls.call(d, "imn_body_tree_accumulate", (m.body_parentid, values, *_TREE(scratch)),
-               (components, skip_root_parent, d.nworld, scratch.levels), build, stream)
+    nbody = length(m.body_parentid)
+    calls.call("imn_body_tree_accumulate", (
+        pack_tree(m, scratch), _per_body(values, d.nworld, nbody, components, "values"), nbody * components, int(components),
+        int(bool(skip_root_parent)), int(d.nworld)), stream)
 
 
 def subtree_com_accumulate(m: Any, d: Any, scratch: TreeReductionScratch | None = None, stream=None) -> None:
@@ -182,28 +197,19 @@ def crb(m: Any, d: Any, scratch: TreeReductionScratch | None = None, stream=None
     """d.crb and d.M from d.cinert and d.cdof (tree_fusion.py:186-206)."""
     _need(scratch, "crb")
 
-    def build():
-        nbody = length(m.body_parentid)
-        t = tree_struct(m, scratch, dofs=True, inertia=True)
-        return (C.byref(t), _per_body(d.cinert, d.nworld, nbody, 10, "d.cinert"),
-                _per_body(d.cdof, d.nworld, m.nv, 6, "d.cdof"), _per_body(d.crb, d.nworld, nbody, 10, "d.crb"),
-                addr(d.M), _row_ld(d.M), int(d.nworld)), t
-
-    calls.call(d, "imn_crb", _CRB_MODEL(m) + _TREE(scratch) + _CRB_DATA(d), (m.nv, d.nworld, scratch.levels), build, stream)
+    nb, nv, W = length(m.body_parentid), m.nv, int(d.nworld)
+    cinert, cdof, crb = _all_per_body(_CRB(d), W, ((nb, 10), (nv, 6), (nb, 10)), ("cinert", "cdof", "crb"))
+    M = d.M
+    calls.call("imn_crb", (pack_tree_inertia(m, scratch), cinert, cdof, crb, addr(M), _row_ld(M), W), stream)
 
 
 def rne(m: Any, d: Any, scratch: TreeReductionScratch | None = None, stream=None) -> None:
     """d.cacc, d.cfrc_int and d.qfrc_bias (tree_fusion.py:209-222)."""
     _need(scratch, "rne")
 
-    def build():
-        nbody = length(m.body_parentid)
-        t = tree_struct(m, scratch, dofs=True, gravity=True)
-        return (C.byref(t), _per_body(d.cinert, d.nworld, nbody, 10, "d.cinert"),
-                _per_body(d.cvel, d.nworld, nbody, 6, "d.cvel"), _per_body(d.cdof, d.nworld, m.nv, 6, "d.cdof"),
-                _per_body(d.cdof_dot, d.nworld, m.nv, 6, "d.cdof_dot"), addr(d.qvel), _row_ld(d.qvel),
-                _per_body(d.cacc, d.nworld, nbody, 6, "d.cacc"), _per_body(d.cfrc_int, d.nworld, nbody, 6, "d.cfrc_int"),
-                addr(d.qfrc_bias), _row_ld(d.qfrc_bias), int(d.nworld)), t
-
-    calls.call(d, "imn_rne", _RNE_MODEL(m) + _TREE(scratch) + _RNE_DATA(d),
-               (m.nv, d.nworld, scratch.levels, m.opt.disableflags), build, stream)
+    nb, nv, W = length(m.body_parentid), m.nv, int(d.nworld)
+    cinert, cvel, cdof, cdof_dot, cacc, cfrc_int = _all_per_body(
+        _RNE(d), W, ((nb, 10), (nb, 6), (nv, 6), (nv, 6), (nb, 6), (nb, 6)), _RNE_NAMES)
+    qvel, qfrc_bias = d.qvel, d.qfrc_bias
+    calls.call("imn_rne", (pack_tree_gravity(m, scratch), cinert, cvel, cdof, cdof_dot, addr(qvel), _row_ld(qvel),
+                           cacc, cfrc_int, addr(qfrc_bias), _row_ld(qfrc_bias), W), stream)

@@ -8,7 +8,6 @@ runs upstream mujoco-warp's per-level launches; this package has no second path.
 
 from __future__ import annotations
 
-import ctypes as C
 from typing import Any
 
 from .. import calls
@@ -16,21 +15,13 @@ from ..arrays import addr, length
 from . import tree_fusion
 
 
-_MODEL = calls.getter("body_parentid", "body_dofadr", "body_dofnum", "dof_bodyid", "dof_parentid", "body_jntadr",
-                      "body_jntnum", "jnt_type")
-_DATA = calls.getter("qvel", "cdof", "cvel", "cdof_dot")
+_DATA = calls.getter("cdof", "cvel", "cdof_dot")
 
 
 def com_vel(m: Any, d: Any, tree: Any, stream=None) -> None:
     """d.cvel and d.cdof_dot from d.qvel and d.cdof."""
     tree_fusion._need(tree, "com_vel")
-
-    def build():
-        nbody = length(m.body_parentid)
-        t = tree_fusion.tree_struct(m, tree, dofs=True, joints=True)
-        return (C.byref(t), addr(d.qvel), tree_fusion._row_ld(d.qvel),
-                tree_fusion._per_body(d.cdof, d.nworld, m.nv, 6, "d.cdof"),
-                tree_fusion._per_body(d.cvel, d.nworld, nbody, 6, "d.cvel"),
-                tree_fusion._per_body(d.cdof_dot, d.nworld, m.nv, 6, "d.cdof_dot"), int(d.nworld)), t
-
-    calls.call(d, "imn_com_vel", _MODEL(m) + tree_fusion._TREE(tree) + _DATA(d), (m.nv, d.nworld, tree.levels), build, stream)
+    nb, nv, W, qvel = length(m.body_parentid), m.nv, int(d.nworld), d.qvel
+    cdof, cvel, cdof_dot = tree_fusion._all_per_body(_DATA(d), W, ((nv, 6), (nb, 6), (nv, 6)), ("cdof", "cvel", "cdof_dot"))
+    calls.call("imn_com_vel", (tree_fusion.pack_tree_joints(m, tree), addr(qvel), tree_fusion._row_ld(qvel), cdof, cvel,
+                               cdof_dot, W), stream)

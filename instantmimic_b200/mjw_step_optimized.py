@@ -9,7 +9,6 @@ a launch of hand-written CUDA through the C ABI; there is no other code path.
 
 from __future__ import annotations
 
-import ctypes as C
 import functools
 import logging
 from dataclasses import dataclass
@@ -18,8 +17,8 @@ from typing import Any, Sequence
 import numpy as np
 
 from . import _lib, binding, calls
-from .arrays import to_host
-from .mjw_kernels import newton_fusion
+from .arrays import addr, as_torch, device_of, elem_strides, is_device, table_to_host, to_host
+from .mjw_kernels import indexed_factor, newton_fusion, tree_ldl
 
 logger = logging.getLogger(__name__)
 
@@ -195,20 +194,15 @@ def mul_m(m: Any, d: Any, res: Any, vec: Any, stream=None, kernel: Any = None) -
     call, mjw_step_optimized.py:2252-2255).  With ``kernel`` (the model's generated
     straight-line kernel, ``mul_m_generated.compile_mul_m``) batches that fill the GPU run
     through it; the bits are the same."""
-    from .arrays import addr, elem_strides
-
     if kernel is not None and int(d.nworld) >= _GENERATED_MUL_M_MIN_WORLDS and addr(res) != addr(vec):
         from .mjw_kernels import mul_m_generated
 
         with _lib.nvtx("mul_m_generated"):
             mul_m_generated.mul_m(kernel, d.M, res, vec, stream)
         return
-    ms = binding.model_struct(m)
-    rc = _lib.lib().imn_mul_m(
-        C.byref(ms), addr(d.M), elem_strides(d.M)[0], addr(vec), elem_strides(vec)[0], addr(res),
-        elem_strides(res)[0], int(d.nworld), _lib.current_stream_handle(stream),
-    )
-    _lib.check(rc, "imn_mul_m")
+    calls.call("imn_mul_m", (
+        binding.pack_model(m), addr(d.M), elem_strides(d.M)[0], addr(vec), elem_strides(vec)[0], addr(res),
+        elem_strides(res)[0], int(d.nworld)), stream)
 
 
 def make_optimized_fwd_position_scratch(
@@ -224,8 +218,6 @@ def make_optimized_fwd_position_scratch(
     """Solver context, nsolving counter, the M-side factor/solve plans and the
     ``constraint_free`` decision (mjw_step_optimized.py:2237-2255, 2510-2585)."""
     import torch
-
-    from .mjw_kernels import indexed_factor, tree_ldl
 
     ctx = nsolving = None
     if d.njmax > 0 and m.nv > 0:
@@ -285,11 +277,7 @@ def _solver_compact_enabled(m: Any) -> bool:
 
 
 def _rowless_handoff(m: Any, d: Any, stream=None) -> None:
-    ms = binding.model_struct(m)
-    ds = binding.data_struct(m, d)
-    with _lib.nvtx("imn_rowless_handoff"):
-        rc = _lib.lib().imn_rowless_handoff(C.byref(ms), C.byref(ds), _lib.current_stream_handle(stream))
-    _lib.check(rc, "imn_rowless_handoff")
+    calls.call("imn_rowless_handoff", (binding.pack_model(m), binding.pack_data(m, d)[0]), stream)
 
 
 def solve_with_scratch(
@@ -321,17 +309,13 @@ def solve_with_scratch(
         raise RuntimeError("optimized solver scratch layout no longer matches model")
     if expected_compact:
         raise RuntimeError("compact (sleeping-island) solves are outside this solver's path")
-    call = newton_fusion.cached_call(m, d, ctx, nsolving, scratch)
-    if call is not None:
-        call(stream)
-        return
     if not newton_fusion.eligible(m, ctx, compact=False):
         raise RuntimeError(
             "model is outside the fused Newton path: " + "; ".join(newton_fusion.ineligible_reasons(m, ctx))
             + ".  This library has no other solver path: route such models to the upstream solve"
         )
     del use_optimized_kernel
-    newton_fusion.solve_call(m, d, ctx, nsolving, cache_on=scratch)(stream)
+    newton_fusion.run(m, d, ctx, nsolving, stream)
 
 
 def _factor_solve_i_dense(
@@ -346,7 +330,6 @@ def _factor_solve_i_dense(
     factor_workspace: Any = None,
     tree_factor_solve: Any = None,
     stream=None,
-    slot: Any = None,
 ) -> None:
     """x = M^-1 y for M (or M - h qDeriv) in the model's CSR layout, choosing the
     kernel as the reference does (mjw_step_optimized.py:1030-1070): the tree L'DL when
@@ -355,13 +338,11 @@ def _factor_solve_i_dense(
     Cholesky that stands in for the reference's per-tile kernels (:793-838).  The tile
     plan is made by ``make_optimized_fwd_position_scratch`` and remembered on the
     model; without it the first call builds it, which allocates (call once outside
-    graph capture).  ``slot`` names the caller among those that solve with this batch in turn."""
-    from .mjw_kernels import indexed_factor, tree_ldl
-
+    graph capture)."""
     if factor_workspace is not None and dense_factor_solve is None:
         raise RuntimeError("a retained factor workspace requires the blocked dense path")
     if tree_factor_solve is not None and not retain_factor and factor_workspace is None:
-        tree_ldl.tree_factor_solve(tree_factor_solve, M, x, y, stream=stream, owner=d, slot=slot)
+        tree_ldl.tree_factor_solve(tree_factor_solve, M, x, y, stream=stream)
         return
     if dense_factor_solve is not None:
         indexed_factor.blocked_dense_factor_solve(
@@ -370,14 +351,10 @@ def _factor_solve_i_dense(
         return
     if retain_factor:
         raise RuntimeError("a retained factor requires the blocked dense path (nv >= 32)")
-    from .arrays import is_device
-
     if not is_device(M):
         raise RuntimeError("no factor/solve path for host buffers: the M-side kernels need CUDA arrays")
     tile = getattr(m, "_imn_tile_factor_solve", None)
     if tile is None or tile.U.shape[0] < d.nworld:
-        from .arrays import device_of
-
         tile = indexed_factor.create_blocked_dense_factor_solve_scratch(m, d, device_of(M), minimum_nv=1)
         if tile is None:
             raise RuntimeError("no factor/solve plan for this model (nv == 0 or no inertia matrix)")
@@ -404,8 +381,6 @@ def refresh_sparse_hessian(m: Any, d: Any, scratch: OptimizedFwdPositionScratch,
         return "no solver context"
     plan, reason = sparse_hessian.plan_for_model(m, ctx, body_groups, newton_fusion.newton_block_dim(m))
     ctx.sparse_hessian_plan = None
-    if hasattr(scratch, "_imn_solve_call"):
-        del scratch._imn_solve_call
     if plan is None:
         return reason
     sparse_hessian.upload(plan, device)
@@ -444,7 +419,7 @@ def fwd_acceleration_solve(m: Any, d: Any, scratch: OptimizedFwdPositionScratch,
     ``fwd_acceleration_optimized`` (mjw_step_optimized.py:1274-1329)."""
     _factor_solve_i_dense(
         m, d, d.M, d.qacc_smooth, d.qfrc_smooth, scratch.dense_factor_solve,
-        tree_factor_solve=scratch.tree_factor_solve, stream=stream, slot="acceleration",
+        tree_factor_solve=scratch.tree_factor_solve, stream=stream,
     )
 
 
@@ -463,10 +438,6 @@ def append_ball_limit_rows(m: Any, d: Any, scratch: OptimizedFwdPositionScratch,
 
 
 # ---- the implicit-fast integrator's tail (mjw_step_optimized.py:5209-5297) --------------
-
-_IMPLICIT_MODEL = calls.getter("opt.timestep", "dof_damping", "M_elemid", "M_colind")
-_IMPLICIT_DATA = calls.getter("moment_rownnz", "moment_rowadr", "moment_colind", "actuator_moment")
-_ADVANCE_MODEL = calls.getter("opt.timestep", "jnt_type", "jnt_dofadr", "jnt_qposadr")
 
 
 def attach_implicit_scratch(m: Any, d: Any, scratch: OptimizedFwdPositionScratch, device: Any = "cuda") -> None:
@@ -490,7 +461,6 @@ def _velocity_gain_coefficients(m: Any):
     """(g2, b2) per actuator with d(force)/d(velocity) = g2 ctrl + b2, as tensors next to
     the model's tables; refuses actuator kinds whose derivative is upstream's."""
     from . import types as T
-    from .arrays import as_torch, table_to_host
 
     gain_t, bias_t, dyn_t = (table_to_host(getattr(m, n))
                              for n in ("actuator_gaintype", "actuator_biastype", "actuator_dyntype"))
@@ -511,8 +481,6 @@ def actuator_velocity_gain(m: Any, d: Any, out: Any, scratch: Any = None) -> Non
     bias = b0 + b1 length + b2 velocity, hence g2 ctrl + b2.  Muscle and user types, and
     actuators with activation dynamics, are refused.  With a scratch whose coefficients
     were prepared (``attach_implicit_scratch``) the call is device work only."""
-    from .arrays import as_torch
-
     coefficients = getattr(scratch, "implicit_gain_coefficients", None) if scratch is not None else None
     g2, b2 = coefficients if coefficients is not None else _velocity_gain_coefficients(m)
     torch_out = as_torch(out)
@@ -533,21 +501,11 @@ def _implicit_matrix(m: Any, d: Any, out: Any, scratch: OptimizedFwdPositionScra
     ``coefficients`` and the controls in the same launch (and left in the scratch)."""
     if int(getattr(m, "ntendon", 0) or 0) or bool(getattr(m, "has_fluid", False)):
         raise RuntimeError("tendon damping and fluid terms are outside this assembly")
-    from .arrays import addr, elem_strides
-
     gain = getattr(scratch, "implicit_actuator_vel", None)
-
-    def build():
-        ps = binding.implicit_struct(m, d, gain, coefficients)
-        return (C.byref(ps), addr(d.M), elem_strides(d.M)[0], addr(out), elem_strides(out)[0], int(d.nworld)), ps
-
-    nu = int(getattr(m, "nu", 0) or 0)
-    buffers = _IMPLICIT_MODEL(m) + (d.M, out)
-    if nu and gain is not None:
-        buffers += _IMPLICIT_DATA(d) + (gain,)
-    if coefficients is not None:
-        buffers += (d.ctrl, *coefficients)
-    calls.call(d, "imn_implicit_matrix", buffers, (m.nv, nu, m.opt.disableflags, d.nworld), build, stream)
+    M = d.M
+    calls.call("imn_implicit_matrix", (
+        binding.pack_implicit(m, d, gain, coefficients), addr(M), elem_strides(M)[0], addr(out), elem_strides(out)[0],
+        int(d.nworld)), stream)
 
 
 def _fused_gain_coefficients(m: Any, d: Any, scratch: Any):
@@ -556,25 +514,24 @@ def _fused_gain_coefficients(m: Any, d: Any, scratch: Any):
     controls (one row for all worlds, another type, another device) go through torch, which converts them."""
     import torch
 
-    from .arrays import as_torch, device_of, elem_strides, is_device
-
     pair = getattr(scratch, "implicit_gain_coefficients", None)
     if pair is None:
         return None
-    W, nu = int(d.nworld), int(m.nu)
-    shapes = {tuple(t.shape) for t in pair}
-    if not (shapes <= {(nu,)} or shapes <= {(1, nu)} or shapes <= {(W, nu)}):
+    W, nu, (g2, b2) = int(d.nworld), int(m.nu), pair
+    out, ctrl, dims = as_torch(scratch.implicit_actuator_vel).device, d.ctrl, tuple(g2.shape)
+    if dims not in ((nu,), (1, nu), (W, nu)) or b2.shape != g2.shape or tuple(ctrl.shape) != (W, nu):
         return None
-    out, ctrl = as_torch(scratch.implicit_actuator_vel), d.ctrl
-    if any(t.dtype != torch.float32 or not t.is_contiguous() or t.device != out.device for t in pair):
-        return None
-    if tuple(ctrl.shape) != (W, nu):
+    if not (g2.dtype == b2.dtype == torch.float32 and g2.is_contiguous() and b2.is_contiguous()
+            and g2.device == b2.device == out):
         return None
     if isinstance(ctrl, torch.Tensor):
-        fits = ctrl.dtype == torch.float32 and ctrl.device == out.device
+        fits = ctrl.dtype == torch.float32 and ctrl.device == out
     else:
-        fits = is_device(ctrl) and getattr(ctrl.dtype, "__name__", "") == "float32" and device_of(ctrl) == out.device
-    if not fits or elem_strides(ctrl)[1] != 1 or elem_strides(ctrl)[0] < nu:
+        fits = is_device(ctrl) and getattr(ctrl.dtype, "__name__", "") == "float32" and device_of(ctrl) == out
+    if not fits:
+        return None
+    ld, inner = elem_strides(ctrl)
+    if inner != 1 or ld < nu:
         return None
     return pair
 
@@ -595,15 +552,7 @@ def _advance_with_scratch(m: Any, d: Any, qacc: Any, scratch: OptimizedFwdPositi
         raise RuntimeError("an externally integrated qvel needs the caller's advance_call")
     if int(getattr(m, "na", 0) or 0):
         raise RuntimeError("actuator activations are outside this advance")
-    from .arrays import addr, elem_strides
-
-    def build():
-        ps = binding.advance_struct(m, d)
-        return (C.byref(ps), addr(qacc), elem_strides(qacc)[0], int(d.nworld)), ps
-
-    time = getattr(d, "time", None)
-    buffers = _ADVANCE_MODEL(m) + (d.qvel, d.qpos, qacc) + (() if time is None else (time,))
-    calls.call(d, "imn_advance", buffers, (m.nv, m.nq, m.njnt, time is None, d.nworld), build, stream)
+    calls.call("imn_advance", (binding.pack_advance(m, d), addr(qacc), elem_strides(qacc)[0], int(d.nworld)), stream)
 
 
 def implicitfast_integrate(m: Any, d: Any, scratch: OptimizedFwdPositionScratch, stream=None) -> None:
@@ -611,13 +560,11 @@ def implicitfast_integrate(m: Any, d: Any, scratch: OptimizedFwdPositionScratch,
     (M - h qDeriv) x = efc.Ma through the tree L'DL or blocked dense kernel, then the
     advance with x.  The free-body correction of mujoco-warp 3.16
     (``_implicit_free_body_correction``, :3768-3780) is upstream-only and not applied."""
-    from . import binding as B
-
-    if int(m.opt.integrator) != int(B.types.IntegratorType.IMPLICITFAST):
+    if int(m.opt.integrator) != int(binding.types.IntegratorType.IMPLICITFAST):
         raise NotImplementedError("only the implicit-fast integrator has a path here")
     if scratch.implicit_qderiv is None or scratch.implicit_qacc is None:
         raise RuntimeError("implicit-fast scratch is not attached (attach_implicit_scratch)")
-    if int(getattr(m, "nu", 0) or 0) and not (int(m.opt.disableflags) & B.upstream_constants()["disable_actuation"]):
+    if int(getattr(m, "nu", 0) or 0) and not (int(m.opt.disableflags) & binding.upstream_constants()["disable_actuation"]):
         coefficients = _fused_gain_coefficients(m, d, scratch)
         if coefficients is None:
             actuator_velocity_gain(m, d, scratch.implicit_actuator_vel, scratch)
@@ -626,6 +573,6 @@ def implicitfast_integrate(m: Any, d: Any, scratch: OptimizedFwdPositionScratch,
     _implicit_matrix(m, d, scratch.implicit_qderiv, scratch, coefficients, stream)
     _factor_solve_i_dense(
         m, d, scratch.implicit_qderiv, scratch.implicit_qacc, d.efc.Ma, scratch.dense_factor_solve,
-        tree_factor_solve=scratch.tree_factor_solve, stream=stream, slot="implicit",
+        tree_factor_solve=scratch.tree_factor_solve, stream=stream,
     )
     _advance_with_scratch(m, d, scratch.implicit_qacc, scratch, stream=stream)

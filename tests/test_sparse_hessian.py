@@ -494,7 +494,6 @@ def test_library_uploaded_plan_gives_the_same_bits(cuda_device):
     native = sparse_hessian.NativePlan(plan)
     assert native.struct.nfac == plan.nfac and native.struct.nfsweep == plan.struct.nfsweep
     plan.struct = native.struct
-    del scratch._imn_solve_call  # structs are cached per scratch
     dd.qacc.zero_()
     runtime.solve_with_scratch(md, dd, scratch, use_optimized_kernel=True)
     torch.cuda.synchronize()
