@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes
 import operator
+import weakref
 from typing import Any
 
 import numpy as np
@@ -178,17 +179,21 @@ _TABLES: dict = {}
 
 
 def table_to_host(a: Any) -> np.ndarray:
-    """Host copy of a constant model table, read from the device once per buffer: a copy
+    """Host copy of a constant model table, read from the device once per array: a copy
     in every call would synchronise the stream and cannot be captured in a CUDA graph.
     Only for arrays whose contents never change after model set-up."""
     if isinstance(a, np.ndarray):
         return a
     key = (addr(a), tuple(shape(a)))
-    hit = _TABLES.get(key)
-    if hit is None:
+    seen, hit = _TABLES.get(key, (None, None))
+    if seen is None or seen() is not a:  # unknown, or the address of an array that is gone
         if len(_TABLES) > 256:
             _TABLES.clear()
-        hit = _TABLES[key] = np.array(to_host(a), copy=True)
+        hit = np.array(to_host(a), copy=True)
+        try:
+            _TABLES[key] = weakref.ref(a), hit
+        except TypeError:  # an array type that cannot be watched is read every time
+            pass
     return hit
 
 

@@ -267,3 +267,14 @@ def test_host_near_device_binds_to_the_gpus_node_and_restores(tmp_path):
         assert near.node is None and os.sched_getaffinity(0) == before
     with host_batch.host_near_device(pci_bus_id="0000:ff:00.0", sysfs=str(tmp_path)) as near:
         assert near.node is None and os.sched_getaffinity(0) == before
+
+
+def test_a_table_at_the_address_of_an_earlier_one_is_read_anew():
+    import torch
+
+    from instantmimic_b200 import arrays
+
+    storage = torch.zeros(4, dtype=torch.int32)
+    assert arrays.table_to_host(storage[:]).tolist() == [0, 0, 0, 0]
+    storage.fill_(3)  # another model's table, where the first one's memory was
+    assert arrays.table_to_host(storage[:]).tolist() == [3, 3, 3, 3]
