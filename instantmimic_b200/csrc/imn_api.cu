@@ -204,10 +204,7 @@ static int launch_mul_m(const ImnModel* m, const float* M, int64_t M_ld, const f
     if (nworld >= 4096 && g < 8 && tile_bytes <= 56 * 1024) {
       const int bulk = M_ld == m->nM && v_ld == m->nv && (reinterpret_cast<uintptr_t>(M) & 15) == 0 &&
                        (reinterpret_cast<uintptr_t>(v) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-      cudaError_t e = cudaFuncSetAttribute(mul_m_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(mul_m_tile_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared);
+      cudaError_t e = allow_shared(mul_m_tile_kernel, tile_bytes, true);
       if (e != cudaSuccess) return set_error("mul_m: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
       e = launch_chained(mul_m_tile_kernel, (nworld + 31) / 32, 32 * kTileWarps, tile_bytes, stream, m->nv, m->nM,
                          m->M_mulm_rowadr, m->M_mulm_col, m->M_mulm_madr, M, M_ld, v, v_ld, out, out_ld, copy_to, niter, zero,

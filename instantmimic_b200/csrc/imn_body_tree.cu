@@ -421,8 +421,8 @@ static int launch_tree(const char* who, void (*kernel)(Args...), int gw, size_t 
   const size_t bytes = floats_per_world * 4 * per_cta;
   if (bytes > 227 * 1024)
     return set_error("%s: %zu bytes of shared memory per block exceed the 227 KB of an SM", who, bytes), IMN_ERR_LIMIT;
-  if (bytes > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  {
+    const cudaError_t e = allow_shared(kernel, bytes);
     if (e != cudaSuccess) return set_error("%s: cudaFuncSetAttribute: %s", who, cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
   const cudaError_t e =
@@ -440,9 +440,7 @@ static bool use_tiles(int nworld, size_t bytes) { return nworld >= 4096 && bytes
 template <typename... Args>
 static int launch_tile(const char* who, void (*kernel)(Args...), size_t bytes, int nworld, void* stream, Args... args) {
   if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    const cudaError_t e = allow_shared(kernel, bytes, true);
     if (e != cudaSuccess) return set_error("%s: cudaFuncSetAttribute: %s", who, cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
   const cudaError_t e = launch_chained(kernel, (nworld + 31) / 32, 32 * kTileWarps, bytes, (cudaStream_t)stream, args...);

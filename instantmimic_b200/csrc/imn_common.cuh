@@ -45,6 +45,21 @@ __device__ __forceinline__ void chain_begin() {
   chain_release();
 }
 
+// Largest dynamic shared memory one CTA may opt into on sm_100 (227 KB).
+static const int kMaxSmem = 227 * 1024;
+
+// Before a launch with `bytes` of dynamic shared memory.  More than 48 KB a block have to be allowed first, a
+// limit of the function that all threads of the process share: it is always raised to the maximum,
+// so that no call lowers it between another one's and that one's launch.
+// whole_sm: several blocks are to fill an SM; the driver otherwise sizes the carve-out for one.
+template <typename... P>
+static inline cudaError_t allow_shared(void (*kernel)(P...), size_t bytes, bool whole_sm = false) {
+  cudaError_t e = cudaSuccess;
+  if (whole_sm) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  if (e == cudaSuccess && bytes > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  return e;
+}
+
 template <typename... P, typename... A>
 static inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, size_t bytes, cudaStream_t stream,
                                          A&&... args) {

@@ -323,8 +323,8 @@ extern "C" int imn_implicit_matrix(const ImnImplicit* p, const float* M, int64_t
   while (warps > 1 && per_warp * warps > 227 * 1024) warps /= 2;
   const size_t bytes = per_warp * warps;
   if (bytes > 227 * 1024) return imn::set_error("imn_implicit_matrix: nM %d too large", p->nM), IMN_ERR_LIMIT;
-  if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  {
+    const cudaError_t e = imn::allow_shared(kernel, bytes);
     if (e != cudaSuccess)
       return imn::set_error("imn_implicit_matrix: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
@@ -344,8 +344,8 @@ extern "C" int imn_advance(const ImnAdvance* p, const float* qacc, int64_t qacc_
   if (nworld == 0) return IMN_OK;
   const size_t bytes = sizeof(float) * 32 * ((size_t)imn::advance_stride(p->nq) + 2 * (size_t)imn::advance_stride(p->nv));
   if (bytes > 227 * 1024) return imn::set_error("imn_advance: nq %d too large", p->nq), IMN_ERR_LIMIT;
-  if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(imn::advance_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  {
+    const cudaError_t e = imn::allow_shared(imn::advance_kernel, bytes);
     if (e != cudaSuccess)
       return imn::set_error("imn_advance: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }

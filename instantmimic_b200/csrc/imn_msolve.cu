@@ -400,8 +400,8 @@ extern "C" int imn_tree_ldl_solve(const ImnTreePlan* plan, const float* M, int64
     return imn::set_error("imn_tree_ldl_solve: plan needs %zu bytes of shared memory per block (max %d)", bytes,
                           227 * 1024),
            IMN_ERR_LIMIT;
-  if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(imn::tree_ldl_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  {
+    const cudaError_t e = imn::allow_shared(imn::tree_ldl_kernel, bytes);
     if (e != cudaSuccess)
       return imn::set_error("imn_tree_ldl_solve: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
@@ -445,10 +445,7 @@ extern "C" int imn_blocked_dense_factor_solve(const ImnBlockedPlan* plan, const 
                           227 * 1024),
            IMN_ERR_LIMIT;
   {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                         cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess && bytes > 48 * 1024)
-      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    const cudaError_t e = imn::allow_shared(kernel, bytes, true);
     if (e != cudaSuccess)
       return imn::set_error("imn_blocked_dense_factor_solve: cudaFuncSetAttribute: %s", cudaGetErrorString(e)),
              IMN_ERR_LAUNCH;

@@ -75,8 +75,6 @@ static int g_wait_polls = 1 << 22;
 static int g_withhold_copies = 0;
 
 
-// Largest dynamic shared memory one CTA may opt into on sm_100 (227 KB).
-static const int kMaxSmem = 227 * 1024;
 // Most warps (worlds in hand) of a CTA: bounds the registers at 128 with a resident J, 168 with a
 // streamed one, whose worlds take more shared memory and are fewer.
 static const int kResidentWarps = 16, kStreamedWarps = 12;
@@ -864,8 +862,7 @@ extern "C" int imn_solve(const ImnModel* m, const ImnData* d, const ImnCtx* cx, 
                            : sp.pairs ? (stats ? imn::newton_kernel<2, true>(res, g) : imn::newton_kernel<2, false>(res, g))
                                       : (stats ? imn::newton_kernel<1, true>(res, g) : imn::newton_kernel<1, false>(res, g));
   {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess && bytes > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const cudaError_t e = imn::allow_shared(kern, bytes, true);
     if (e != cudaSuccess)
       return imn::set_error("imn_solve: cudaFuncSetAttribute: %s", cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }

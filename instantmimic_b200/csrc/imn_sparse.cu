@@ -78,9 +78,8 @@ extern "C" int imn_sparse_factor_nonfused(const ImnSparsePlan* plan, const uint8
   const size_t bytes = sizeof(float) * (((plan->nslots + 3) & ~3) + 3 * (size_t)n4);
   if (bytes > 227 * 1024)
     return imn::set_error("imn_sparse_factor_nonfused: factor needs %zu bytes of shared memory", bytes), IMN_ERR_LIMIT;
-  if (bytes > 48 * 1024) {
-    cudaError_t e =
-        cudaFuncSetAttribute(imn::sparse_nonfused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  {
+    const cudaError_t e = imn::allow_shared(imn::sparse_nonfused_kernel, bytes);
     if (e != cudaSuccess)
       return imn::set_error("imn_sparse_factor_nonfused: cudaFuncSetAttribute: %s", cudaGetErrorString(e)),
              IMN_ERR_LAUNCH;
