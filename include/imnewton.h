@@ -30,7 +30,7 @@
 extern "C" {
 #endif
 
-#define IMN_ABI_VERSION 5
+#define IMN_ABI_VERSION 6
 
 typedef enum ImnStatus {
   IMN_OK = 0,
@@ -163,25 +163,14 @@ typedef struct ImnSparsePlan {
   const uint16_t* s_b;      /* SH_SB  [nfac]                                   */
   const int32_t* s_m;       /* SH_SM  [nfac]                                   */
   const uint32_t* gat;      /* SH_GAT [nfac] (non-fused path)                  */
-  /* The level tables once more, laid out for the fused kernel: one record per
-   * (sweep, lane), so that a lane fetches all it needs for a sweep with one load
-   * and can fetch the next sweep's record ahead of time.  A sweep is 32 / team
-   * entries of one level.
-   *   fsweep [nfsweep][32][4]: {slot | (col+1) << 16, run_ab, run_kl of the entry's
-   *     first run, flags}; flags bit 0 = the lane has an entry, bit 1 = last sweep
-   *     of its level, bits 2-4 = log2(team), bits 8-15 = further runs of the entry,
-   *     bits 16-31 = index of the first of those in run_ab / run_kl.
-   *   bsweep [nbsweep][32]: slot | src << 16 | dst << 23 | has-work << 30 |
-   *     last-of-level << 31 (backward solve).
-   * NULL / 0 when the plan is only used by the non-fused kernel. */
-  const uint32_t* fsweep;
-  const uint32_t* bsweep;
-  int32_t nfsweep, nbsweep;
-  /* What the fused kernel reads: the sweeps once more with every operand as a byte offset
-   * from N[0] (1/D starts up4(nslots) floats behind N), one record per (step, lane).  The
-   * entries of a level are dealt to its sweeps anew (most terms first); entries that neither
-   * have a term nor are a diagonal are left out.  A sweep is as many steps as its entry
-   * with the most runs has runs.
+  /* What the fused kernel reads of the level tables: one record per (step, lane) with every
+   * operand as a byte offset from N[0] (1/D starts up4(nslots) floats behind N), so that a lane
+   * fetches all it needs for a step with one load and can fetch the next step's record ahead of
+   * time.  A sweep is 32 / team entries of one level (nfsweep, nbsweep: the level tables' own
+   * count of sweeps; 0 when the plan is only used by the non-fused kernel).  The factor's
+   * entries are dealt to its sweeps anew (most terms first); entries that neither have a term
+   * nor are a diagonal are left out.  A sweep is as many steps as its entry with the most runs
+   * has runs.
    *   fstep [nfstep + 1][32][4]: {a | b << 16, d | slot << 16, terms | diagonal's 1/D << 16
    *     (0: not a diagonal), flags}; a, b, d start at the lane's own first term of the run and
    *     advance by the team width; flags bit 0 = the lane stores the entry, bit 1 = last step
@@ -192,7 +181,9 @@ typedef struct ImnSparsePlan {
    *   bstep [nbsweep + 1][32][2]: {slot | source's right-hand side << 16, source's 1/D |
    *     destination's right-hand side << 16}; bit 0 of word 0 = the lane has work, of
    *     word 1 = last of its level.
-   * The spare record at the end of both is only prefetched.  */
+   * The spare record at the end of both is only prefetched.  NULL / 0 when the plan is only used
+   * by the non-fused kernel. */
+  int32_t nfsweep, nbsweep;
   const uint32_t* fstep;
   const uint32_t* bstep;
   int32_t nfstep;

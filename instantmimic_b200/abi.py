@@ -16,7 +16,7 @@ I32 = C.c_int32
 I64 = C.c_int64
 F32 = C.c_float
 
-IMN_ABI_VERSION = 5
+IMN_ABI_VERSION = 6
 
 IMN_OK = 0
 IMN_ERR_NULL = -1
@@ -112,12 +112,10 @@ SPARSE_TABLES = (
     ("s_b", "uint16"),
     ("s_m", "int32"),
     ("gat", "uint32"),
-    ("fsweep", "uint32"),
-    ("bsweep", "uint32"),
 )
 
 
-# the same sweeps with every operand as a byte offset (uint32; sparse_hessian.pack_steps)
+# the sweeps of the level tables with every operand as a byte offset (uint32; sparse_hessian.pack_steps)
 SPARSE_STEPS = ("fstep", "bstep")
 
 

@@ -131,7 +131,6 @@ extern "C" int imn_sparse_plan_create(const ImnSparsePlan* host, ImnSparsePlan**
       TAB(b_dst, host->nback > 0 ? host->nback : 1), TAB(pair, nv * nv), TAB(f_lvl, host->nlevels + 1),
       TAB(f_row, nv), TAB(row_start, nv), TAB(rk_ptr, nv + 1), TAB(rk, nrk), TAB(pmask, nv * words),
       TAB(s_a, host->nfac), TAB(s_b, host->nfac), TAB(s_m, host->nfac), TAB(gat, host->nfac),
-      TAB(fsweep, (size_t)host->nfsweep * 128), TAB(bsweep, (size_t)host->nbsweep * 32),
       TAB(fstep, host->nfstep > 0 ? ((size_t)host->nfstep + 1) * 128 : 0),
       TAB(bstep, host->nfstep > 0 ? ((size_t)host->nbsweep + 1) * 64 : 0),
   };

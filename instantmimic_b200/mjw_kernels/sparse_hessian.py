@@ -355,13 +355,12 @@ def build_plan(m: Any, body_groups: Sequence[Sequence[int]], block: int, path: s
         rk_ptr=rk_ptr.tolist(), rk=rk.tolist() or [0], pmask=pmask.reshape(-1).tolist(), s_a=s_a.tolist(),
         s_b=s_b.tolist(), s_m=s_m.tolist(), gat=gat.tolist(),
     )
-    raw["fsweep"], raw["bsweep"] = _pack_sweeps(raw) if path == "fused" else ([], [])
     tables = {}
     for name, dtype in abi.SPARSE_TABLES:
         vals = raw[name] if len(raw[name]) else [0]
         tables[name] = np.asarray(vals, dtype=np.int64).astype(dtype)
-    if path != "fused":
-        tables["fsweep"], tables["bsweep"] = tables["fsweep"][:0], tables["bsweep"][:0]
+    for name, records in zip(("fsweep", "bsweep"), _pack_sweeps(raw) if path == "fused" else ([], [])):
+        tables[name] = np.asarray(records, dtype=np.int64).astype(np.uint32)  # stay on the host
     return SparseHessianPlan(
         nv=nv, nv_pad=nv_pad, block=block, nslots=nslots, nterms=nterms, levels=len(levels),
         density=nfac / (nv * (nv + 1) / 2), path=path, nfac=nfac, tables=tables, adjacency=adj,
@@ -370,9 +369,15 @@ def build_plan(m: Any, body_groups: Sequence[Sequence[int]], block: int, path: s
 
 
 def _pack_sweeps(raw: dict) -> tuple[list[int], list[int]]:
-    """The level tables as one record per (sweep, lane) for the fused kernel (layout in
-    include/imnewton.h).  A sweep is the 32 / team entries of a level that the warp
-    works on at once; lanes of a team carry the same record."""
+    """The level tables as one record per (sweep, lane), from which ``pack_steps`` makes the records the
+    fused kernel reads.  A sweep is the 32 / team entries of a level that the warp works on at
+    once; lanes of a team carry the same record.
+
+    ``fsweep`` [sweeps][32][4]: {slot | (col + 1) << 16, run_ab, run_kl of the entry's first run, flags}; flags
+    bit 0 = the lane has an entry, bit 1 = last sweep of its level, bits 2-4 = log2(team), bits 8-15 =
+    further runs of the entry, bits 16-31 = index of the first of those in run_ab / run_kl.
+    ``bsweep`` [sweeps][32]: slot | src << 16 | dst << 23 | has-work << 30 | last-of-level << 31
+    (backward solve)."""
     lvl_ptr, lvl_team = raw["lvl_ptr"], raw["lvl_team"]
     run_ptr, run_ab, run_kl = raw["run_ptr"], raw["run_ab"], raw["run_kl"]
     fs: list[int] = []
@@ -516,8 +521,6 @@ def plan_struct(plan: SparseHessianPlan, arrays: dict) -> abi.ImnSparsePlan:
         setattr(st, name, addr(arrays[name]))
     st.nfsweep = int(plan.tables["fsweep"].shape[0]) // 128
     st.nbsweep = int(plan.tables["bsweep"].shape[0]) // 32
-    if not st.nfsweep:
-        st.fsweep = st.bsweep = None
     for name in abi.SPARSE_STEPS:
         setattr(st, name, addr(arrays.get(name)))
     st.nfstep, st.pairs = int(plan.steps.get("nfstep", 0)), int(plan.steps.get("pairs", 0))
