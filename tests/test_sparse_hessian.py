@@ -436,8 +436,8 @@ def test_nonfused_sparse_factor_matches_oracle_and_dense_search(oracle, cuda_dev
 
 
 def test_sweep_records_restate_the_level_tables():
-    """The per-(sweep, lane) records the fused kernel reads (include/imnewton.h) carry the
-    same entries, runs and level boundaries as the level tables they are packed from."""
+    """The per-(sweep, lane) records from which the fused kernel's step records are packed carry the
+    same entries, runs and level boundaries as the level tables."""
     for name in ("humanoid", "snu"):
         m, _, _ = synthetic.make_workload(name, 1, seed=0)
         plan = sparse_hessian.build_plan(m, _single_body_groups(m), 32 if m.nv_pad < 64 else 64, "fused")
@@ -479,6 +479,182 @@ def test_sweep_records_restate_the_level_tables():
     big, _, _ = synthetic.make_workload("humanoid", 1, seed=0)
     nf = sparse_hessian.build_plan(big, _single_body_groups(big), 64, "nonfused")
     assert nf.tables["fsweep"].size == 0 and sparse_hessian.host_struct(nf).nfsweep == 0
+
+
+def _plan_models():
+    """(model, groups) of plans of several shapes: the three named trees, a tree whose sweeps go in pairs, trees
+    with groups that couple limbs (several runs per entry, tables beyond the shared-memory limit)."""
+    for name in ("humanoid", "snu", "g1"):
+        m, _, _ = synthetic.make_workload(name, 1, seed=0)
+        yield name, m, _single_body_groups(m)
+    for nv, coupled in ((64, 0), (79, 8), (79, 10)):
+        yield f"limb{nv}+{coupled}", *_coupled_limbs(nv, coupled)
+
+
+def _coupled_limbs(nv, coupled):
+    parent, body = synthetic.limb_tree(nv)
+    m = put_model(parent, body_of_dof=body)
+    rng = np.random.default_rng(0)
+    pairs = [sorted(rng.choice(np.arange(1, len(m.body_dofadr)), 2, replace=False).tolist()) for _ in range(coupled)]
+    return m, _single_body_groups(m) + pairs
+
+
+def _lane_terms(team, runs):
+    """Per lane of a team its (a, b, k) terms in the order it adds them."""
+    return tuple(tuple((a + t, b + t, k + t) for a, b, k, n in runs for t in range(lane, n, team)) for lane in range(team))
+
+
+def test_step_records_give_every_entry_its_terms_in_order():
+    """Interprets ``fstep`` as the fused kernel does, pairs of sweeps included: level by level the same
+    entries as the level tables, each with the same terms in the same order on the same lane of a
+    team of the same width, and nothing that a level stores is read in it."""
+    paired = 0
+    for name, m, groups in _plan_models():
+        plan = sparse_hessian.build_plan(m, groups, 32 if m.nv_pad < 64 else 64, "fused")
+        t, inv0 = plan.tables, (plan.nfac + plan.nv + 3) // 4 * 4
+        want = []
+        for lvl, team in enumerate(t["lvl_team"].astype(int)):
+            entries = {}
+            for e in range(int(t["lvl_ptr"][lvl]), int(t["lvl_ptr"][lvl + 1])):
+                r = range(int(t["run_ptr"][e]), int(t["run_ptr"][e + 1]))
+                runs = [(int(t["run_ab"][q]) & 0xFFFF, int(t["run_ab"][q]) >> 16, int(t["run_kl"][q]) & 0xFFFF,
+                         int(t["run_kl"][q]) >> 16) for q in r]
+                if runs or t["ent_col"][e] >= 0:  # the others change nothing
+                    entries[int(t["ent_slot"][e])] = (int(t["ent_col"][e]), _lane_terms(team, runs))
+            if entries:
+                want.append(entries)
+        f = plan.steps["fstep"].reshape(-1, 32, 4).astype(np.int64)
+        assert f.shape[0] == plan.steps["nfstep"] + 1 and not f[-1].any()
+        got, level, pending = [], {}, [[] for _ in range(32)]
+
+        def run_of(rec, lane, most):
+            n, step = int(rec[2]) & 0xFFFF, 1 << ((int(rec[3]) >> 2) & 7)
+            assert n <= most
+            a, b, d = int(rec[0]) & 0xFFFF, int(rec[0]) >> 16, int(rec[1]) & 0xFFFF
+            assert not (a % 4 or b % 4 or d % 4)
+            return [(a // 4 + step * q, b // 4 + step * q, d // 4 - inv0 + step * q) for q in range(n)]
+
+        def close(rec):
+            team = 1 << ((int(rec[0, 3]) >> 2) & 7)
+            any_diagonal = False
+            for first in range(0, 32, team):
+                lanes = range(first, first + team)
+                assert all(not rec[q, 3] & 1 for q in lanes if q != first)
+                terms = tuple(tuple(pending[q]) for q in lanes)
+                if not rec[first, 3] & 1:
+                    assert not any(terms)
+                    continue
+                slot, diagonal = int(rec[first, 1]) >> 18, int(rec[first, 2]) >> 16
+                any_diagonal |= diagonal != 0
+                assert slot not in level
+                level[slot] = (diagonal // 4 - inv0 if diagonal else -1, terms)
+            assert bool(rec[0, 3] & 64) >= any_diagonal
+            for q in range(32):
+                pending[q] = []
+
+        k = 0
+        while k < plan.steps["nfstep"]:
+            rec = f[k]
+            flags = rec[:, 3] & ~1
+            assert (flags == flags[0]).all()  # the warp branches on them
+            width = 2 if flags[0] & 128 else 1
+            paired += width - 1
+            most = int(flags[0] >> 8) & 0xFF
+            for part in f[k:k + width]:
+                for lane in range(32):
+                    pending[lane] += run_of(part[lane], lane, most)
+                if part[0, 3] & 32:
+                    close(part)
+            assert width == 1 or (f[k:k + 2, 0, 3] & 32).all() and (f[k, 0, 3] ^ f[k + 1, 0, 3]) & 0x1C == 0
+            k += width
+            if f[k - 1, 0, 3] & 2:
+                got.append(level)
+                level = {}
+        assert got == want and not level, name
+        for entries in got:
+            read = {slot for _, terms in entries.values() for lane in terms for a, b, _ in lane for slot in (a, b)}
+            inverse = {d for _, terms in entries.values() for lane in terms for _, _, d in lane}
+            assert not read & set(entries) and not inverse & {c for c, _ in entries.values()}
+    assert paired
+
+
+def test_backward_step_records_give_every_push_once_and_level_by_level():
+    for name, m, groups in _plan_models():
+        plan = sparse_hessian.build_plan(m, groups, 32 if m.nv_pad < 64 else 64, "fused")
+        t, inv0 = plan.tables, (plan.nfac + plan.nv + 3) // 4 * 4
+        want = [sorted(zip(*(t[k][int(a):int(b)].tolist() for k in ("b_slot", "b_src", "b_dst"))))
+                for a, b in zip(t["b_lvl"][:-1], t["b_lvl"][1:]) if a < b]
+        got, level = [], []
+        records = plan.steps["bstep"].reshape(-1, 32, 2).astype(np.int64)
+        assert not records[-1].any()
+        for rec in records[:-1]:
+            for w0, w1 in rec.tolist():
+                if not w0 & 1:
+                    continue
+                src = (w0 >> 18) - plan.nfac
+                assert ((w1 & 0xFFFC) >> 2) - inv0 == src
+                level.append(((w0 & 0xFFFC) >> 2, src, (w1 >> 18) - plan.nfac))
+            assert (rec[:, 1] & 1 == rec[0, 1] & 1).all()
+            if rec[0, 1] & 1:
+                got.append(sorted(level))
+                assert not {s for _, s, _ in level} & {q for _, _, q in level}
+                level = []
+        assert got == want and not level, name
+
+
+def test_lane_program_of_m_v_takes_every_row_once_in_table_order():
+    """Interprets ``M_mulm_lanes`` as ``products`` does: every row's terms in the order of the row table
+    followed by terms with the zero behind the vector, its sum stored once it is whole."""
+    models = [m for _, m, _ in _plan_models()]
+    for nv in (1, 31, 32, 33, 79):
+        parent, body = synthetic.chain_tree(nv)
+        models.append(put_model(parent, body_of_dof=body))
+    for m in models:
+        nv, lanes = m.nv, np.asarray(m.M_mulm_lanes).view(np.uint32).reshape(-1, 32, 4).astype(np.int64)
+        rowadr, col, madr = (np.asarray(a).astype(int) for a in (m.M_mulm_rowadr, m.M_mulm_col, m.M_mulm_madr))
+        stored = {}
+        for lane in range(32):
+            terms = []
+            for words in lanes[:-1, lane].tolist():
+                terms += [((w & 0x1FC) >> 2, w >> 18) for w in words]
+                row = (words[1] >> 9) & 0x7F
+                assert stored.get(row, (lane,))[0] == lane or row == nv
+                stored[row] = (lane, terms)
+                if words[0] & 0x200:
+                    terms = []
+        stored.pop(nv, None)  # lanes that are done
+        assert sorted(stored) == list(range(nv))
+        for row, (_, terms) in stored.items():
+            k = range(rowadr[row], rowadr[row + 1])
+            assert terms[:len(k)] == [(int(col[q]), int(madr[q])) for q in k]
+            assert all(v == nv and e < m.nM for v, e in terms[len(k):]) and len(terms) - len(k) < 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("coupled", [8, 10])
+@pytest.mark.parametrize("worlds", [24, 700])
+def test_plan_whose_tables_stay_in_global_memory(oracle, cuda_device, worlds, coupled):
+    """Tables of more than a third of an SM's shared memory (79 dofs, groups that couple limbs) are read from
+    global memory; with sweeps in pairs and without, a team per world and a warp."""
+    from instantmimic_b200 import mjw_model
+    from instantmimic_b200.mjw_kernels import newton_fusion
+
+    m, groups = _coupled_limbs(79, coupled)
+    d, _ = synthetic.make_problem(m, worlds, 48, seed=coupled, nefc_range=(8, 48), rowless_fraction=0.1)
+    got, scratch, (md, dd) = _cuda_sparse(m, d, cuda_device, groups)
+    plan = scratch.solver_context.sparse_hessian_plan
+    words = plan.steps["fstep"].size + plan.steps["bstep"].size + m.M_mulm_lanes.size + plan.nfac + m.nv
+    assert 4 * words > 227 * 1024 // 3 and plan.steps["pairs"] == (coupled == 8)
+    info = newton_fusion.solve_call(md, dd, scratch.solver_context, scratch.solver_nsolving).launch_info()
+    # the CTA's shared memory does not hold them
+    assert info.smem_bytes < 4 * words or info.smem_bytes + 4 * words > 227 * 1024
+    want, wctx = _oracle_sparse(oracle, m, d, plan)
+    live = np.arange(d.njmax)[None, :] < np.minimum(d.nefc, d.njmax)[:, None]
+    np.testing.assert_array_equal(got.solver_niter, want.solver_niter)
+    np.testing.assert_array_equal(got.efc.state[live], want.efc.state[live])
+    np.testing.assert_array_equal(got.qacc, want.qacc)
+    np.testing.assert_array_equal(got.efc.force[live], want.efc.force[live])
+    assert mjw_model.to_host(dd).overflow.max() == want.overflow.max()
 
 
 @pytest.mark.gpu
