@@ -119,8 +119,9 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   g.tB = t, t += sp ? (sp->nbsweep + 1) * 64 : 0;
   g.tS = t, t += sp ? up4(sp->nfac) : 0;
   g.tO = t, t += sp ? up4(m.nv) : 0;
-  // tables stay in global memory when they would take more than a third of an SM's shared memory
-  g.tsm = 4 * t <= kMaxSmem / 3;
+  // a plan's tables stay in global memory when they would take more than a third of an SM's shared memory;
+  // without a plan there is the M v program only, at most 31 KB for 79 dofs
+  g.tsm = !sp || 4 * t <= kMaxSmem / 3;
   g.tab = g.tsm ? t : 0;
   g.wait_polls = g_wait_polls;
   g.withhold_copies = g_withhold_copies;
@@ -674,7 +675,9 @@ static Kernel newton_kernel(bool resident, const Geom& g) {
 }
 template <int SPARSE, bool STATS>
 static Kernel newton_kernel(bool resident, const Geom& g) {
-  return g.tsm ? newton_kernel<SPARSE, STATS, true>(resident, g) : newton_kernel<SPARSE, STATS, false>(resident, g);
+  if constexpr (SPARSE != 0)
+    if (!g.tsm) return newton_kernel<SPARSE, STATS, false>(resident, g);
+  return newton_kernel<SPARSE, STATS, true>(resident, g);
 }
 
 __global__ void start_counters(int* nsolving, int* work_counter, int nworld) {
