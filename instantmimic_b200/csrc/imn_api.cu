@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(256) mul_m_kernel(const int nv, const int* __r
                                                     float* __restrict__ out, const int64_t out_ld,
                                                     float* __restrict__ copy_to, int* __restrict__ niter,
                                                     float* __restrict__ zero, const int nworld) {
-  chain_begin();
+  chain_wait();
   extern __shared__ uint32_t tab[];  // packed (col | madr << 16) entries, then nv + 1 row starts
   const int nnz = rowadr[nv];
   int* radr = reinterpret_cast<int*>(tab + nnz);
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
                       float* __restrict__ copy_to, int* __restrict__ niter, float* __restrict__ zero, const int nworld,
                       const int bulk) {
   extern __shared__ __align__(16) float tile[];
-  chain_begin();
+  chain_wait();
   const int nnz = rowadr[nv];
   float* Mt = tile + 4;  // the first 16 bytes hold the mbarrier
   float* vt = Mt + ((32 * nM + 3) & ~3);

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
     tree_accumulate_kernel(const ImnBodyTree T, float* __restrict__ values, const int64_t world_ld, const int C,
                            const int skip_root_parent, const int nworld) {
   extern __shared__ __align__(16) float tree_smem[];
-  chain_begin();
+  chain_wait();
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int n = T.nbody * C;
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
     crb_kernel(const ImnBodyTree T, const float* __restrict__ cinert, const float* __restrict__ cdof,
                float* __restrict__ crb, float* __restrict__ M, const int64_t M_ld, const int nworld) {
   extern __shared__ __align__(16) float tree_smem[];
-  chain_begin();
+  chain_wait();
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int sl = t.sl, w = t.w;
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
                const int64_t qvel_ld, float* __restrict__ cacc_out, float* __restrict__ cfrc_out,
                float* __restrict__ qfrc_bias, const int64_t bias_ld, const int nworld) {
   extern __shared__ __align__(16) float tree_smem[];
-  chain_begin();
+  chain_wait();
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int sl = t.sl, w = t.w;
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
                    const float* __restrict__ cdof, float* __restrict__ cvel_out, float* __restrict__ cdof_dot_out,
                    const int nworld) {
   extern __shared__ __align__(16) float tree_smem[];
-  chain_begin();
+  chain_wait();
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int sl = t.sl, w = t.w;

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(32 * kTileWarps)
                         const float* __restrict__ cdof, float* __restrict__ cvel_out, float* __restrict__ cdof_dot_out,
                         const int nworld) {
   extern __shared__ __align__(16) float tile_smem[];
-  chain_begin();
+  chain_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = blockIdx.x * 32;
   const int nb6 = T.nbody * 6, nv6 = T.nv * 6, sb = odd(nb6), sv = odd(nv6), sq = odd(T.nv);
   float* cvel_t = tile_smem;

@@ -28,22 +28,17 @@ int sm_count();  // of the current device; 148 where there is none
 // released it or left, and waits in chain_wait until the predecessor's results are visible.
 // Every kernel launched by launch_chained waits before it touches global memory; as it releases its
 // successor only after its own wait, a waiting kernel has one unfinished kernel before it, and everything
-// earlier is complete.
-// A grid of few blocks releases at once, so that the launch of the next overlaps it.  A larger one
-// does so by leaving: blocks of the next kernel that become resident while it drains pile up on the SMs that
-// drain first, where an ordinary launch spreads them evenly (blocked dense factor + solve of 4096
-// worlds: 76 -> 95 us when every kernel released at once).
-// 16 humanoid worlds, a substep of 12 launches: 161 -> 146 us; 8192 worlds, the smooth stages 65 -> 55,
-// the implicit-fast tail 34 -> 29.
+// earlier is complete.  (Ordinary launches: a substep of 12 launches with 16 humanoid worlds 161 us
+// against 146, the smooth stages of 8192 worlds 65 against 55, the implicit-fast tail 34 against 29.)
+// A stage releases its successor by leaving (no call).  Released at once, the successor's blocks become
+// resident while the grid drains and pile up on the SMs that drain first, where a later launch spreads them
+// evenly, and a grid of few blocks gains nothing either.  us when every stage releases at once / grids of
+// up to 64 blocks / none: factor with three right-hand sides and second solve, 4096 worlds 86 / 67 / 67, 256
+// worlds 41.4 / 41.4 / 38.3; smooth stages, 8192 worlds 59 / 52 / 52, 2048 worlds 46 / 39 / 39; tail, 512 worlds
+// 15.8 / 15.8 / 14.8.  The counter kernels of a solve, a block each, do release at once: the solve
+// stages its tables meanwhile (substep of 512 worlds 145.1 -> 144.3 us, 4096 56-dof worlds 1096.6 -> 1094.1).
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-static const int kFewBlocks = 64;  // under half of the SMs
-__device__ __forceinline__ void chain_release() {
-  if (gridDim.x <= kFewBlocks) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void chain_begin() {
-  chain_wait();
-  chain_release();
-}
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Largest dynamic shared memory one CTA may opt into on sm_100 (227 KB).
 static const int kMaxSmem = 227 * 1024;

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(32 * kMatrixWarps)
     implicit_matrix_kernel(const ImnImplicit P, const float* __restrict__ M, const int64_t M_ld,
                            float* __restrict__ out, const int64_t out_ld, const int nworld) {
   extern __shared__ float qd_all[];
-  chain_begin();
+  chain_wait();
   const int lane = threadIdx.x & 31, w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= nworld) return;
   const int row = (P.nM + 3) & ~3;
@@ -241,7 +241,7 @@ __host__ __device__ inline int advance_stride(int n) { return (n & 3) == 0 ? (n 
 __global__ void __launch_bounds__(32 * kAdvanceWarps)
     advance_kernel(const ImnAdvance P, const float* __restrict__ qacc, const int64_t qacc_ld, const int nworld) {
   extern __shared__ __align__(16) float rows[];
-  chain_begin();
+  chain_wait();
   // row strides: the lanes of a warp read the same element of 32 rows; a row length that
   // shares a factor of 4 or more with the 32 banks is padded to an odd stride
   const int tq = advance_stride(P.nq), tv = advance_stride(P.nv);

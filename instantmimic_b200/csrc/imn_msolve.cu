@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, KM == 2 ? 7 : 4)
                          const int* __restrict__ active, const int rhs, const int mode, const int carry,
                          const int ldu, const int per_world, const int vec, const int nworld) {
   extern __shared__ __align__(16) float sm[];
-  chain_begin();
+  chain_wait();
   const int l = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int w = blockIdx.x * kDenseWarps + warp;
   if (w >= nworld || (active && active[w] == 0)) return;

@@ -234,8 +234,7 @@ std::string generate(const std::string& name, const int32_t* prog, const int32_t
          ") " + name + "(const float* __restrict__ M, long long M_ld, const float* __restrict__ y,\n"
          "    long long y_ld, float* __restrict__ x, long long x_ld, int nworld, int bulk) {\n"
          "  extern __shared__ __align__(16) float slots[];\n"
-         "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");  // chain_begin of imn_common.cuh\n"
-         "  if (gridDim.x <= 64) asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n"
+         "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");  // chain_wait of imn_common.cuh\n"
          "  const int lw = threadIdx.x & 31, part = threadIdx.x >> 5;\n"
          "  const int world = blockIdx.x * 32 + lw;\n"
          "  const bool live = world < nworld;\n"
