@@ -45,3 +45,22 @@ def test_host_batch_pipeline_matches_oracle(oracle, cuda_device, mode, grouped):
         np.testing.assert_array_equal(out["state"].numpy()[live], want.efc.state[live])
         np.testing.assert_array_equal(out["force"].numpy()[live].view(np.uint32), want.efc.force[live].view(np.uint32))
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("worlds", [1129, 1130, 2300])
+def test_results_that_go_back_in_pieces(oracle, cuda_device, worlds):
+    """Either side of one piece, and several pieces with a remainder."""
+    m, d, _ = synthetic.make_workload("humanoid", worlds, seed=6, iterations=4)
+    want, _, _ = run_oracle(oracle, m, d, matrices=False)
+    pipe = host_batch.HostBatchPipeline(mjw_model.to_device(m, cuda_device), d, cuda_device, slots=2, mode="sparse8")
+    sizes = [p.numel() for p, _ in pipe.slots[0]["sparse"]["pieces"]]
+    total = host_batch.result_layout(worlds, d.njmax, m.nv)[1]
+    assert sum(sizes) == total and max(sizes) <= 1 << 20 and len(sizes) == -(-total // (1 << 20))
+    pipe.submit(0, host_batch.pin_batch(d))
+    out = pipe.result(0)
+    live = np.arange(d.njmax)[None, :] < d.nefc[:, None]
+    for name, ref in (("qacc", want.qacc), ("qfrc_constraint", want.qfrc_constraint), ("Ma", want.efc.Ma),
+                      ("solver_niter", want.solver_niter), ("overflow", want.overflow)):
+        np.testing.assert_array_equal(out[name].numpy().view(np.uint32), ref.view(np.uint32), err_msg=name)
+    for name in ("force", "state"):
+        np.testing.assert_array_equal(out[name].numpy()[live], getattr(want.efc, name)[live], err_msg=name)
