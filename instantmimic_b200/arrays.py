@@ -161,7 +161,7 @@ def is_device(a: Any) -> bool:
 
 
 def length(a: Any) -> int:
-    return int(a.shape[0])
+    return a.shape[0]
 
 
 def to_host(a: Any) -> np.ndarray:

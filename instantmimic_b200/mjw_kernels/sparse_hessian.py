@@ -489,8 +489,9 @@ def pack_steps(t: dict, nv: int, nfac: int) -> dict:
         out[s, n - 1, :, 3] |= 32 | ends_level[s] | (64 if diag[s].any() else 0)
         steps += list(out[s, :n])
         single += [False] * (n - 1) + [n == 1 and not ends_level[s]]
-    # Pairs: where they cover most steps (large trees, whose levels are several sweeps wide).  Elsewhere the kernel
-    # without them is the faster one: 35 dofs with 10 of 21 steps in pairs, 2330 -> 2409 us per solve.
+    # Pairs: where they cover two thirds of the steps (large trees, whose levels are several sweeps wide): 56
+    # dofs, 40 of 47 steps, 1187 -> 1090 us per solve.  Elsewhere the kernel without them is the faster
+    # one: 35 dofs with 10 of 21 steps in pairs, 2330 -> 2409.
     first = []
     for k in range(len(steps) - 1):
         if single[k] and int(steps[k + 1][0, 3]) & 32 and not (first and first[-1] == k - 1):

@@ -162,20 +162,15 @@ def _per_body(a: Any, nworld: int, nbody: int, width: int, name: str) -> int:
     return addr(a)
 
 
-def _all_per_body(arrays: tuple, nworld: int, extents: tuple, names: tuple) -> tuple:
-    """The same for several arrays; extents: (rows, width) of each."""
-    if dense(arrays, [(nworld, n, width) for n, width in extents]):
+def _all_per_body(arrays: tuple, shapes: list, names: tuple) -> tuple:
+    """The same for several arrays of the given shapes."""
+    if dense(arrays, shapes):
         return addrs(arrays)
-    return tuple([_per_body(a, nworld, n, width, "d." + name) for a, (n, width), name in zip(arrays, extents, names)])
+    return tuple([_per_body(a, *dims, "d." + name) for a, dims, name in zip(arrays, shapes, names)])
 
 
 def _row_ld(a: Any) -> int:
     return elem_strides(a)[0]
-
-
-_CRB = calls.getter("cinert", "cdof", "crb")
-_RNE_NAMES = ("cinert", "cvel", "cdof", "cdof_dot", "cacc", "cfrc_int")
-_RNE = calls.getter(*_RNE_NAMES)
 
 
 def accumulate(m: Any, d: Any, values: Any, components: int, skip_root_parent: bool, scratch: TreeReductionScratch,
@@ -197,9 +192,9 @@ def crb(m: Any, d: Any, scratch: TreeReductionScratch | None = None, stream=None
     """d.crb and d.M from d.cinert and d.cdof (tree_fusion.py:186-206)."""
     _need(scratch, "crb")
 
-    nb, nv, W = length(m.body_parentid), m.nv, int(d.nworld)
-    cinert, cdof, crb = _all_per_body(_CRB(d), W, ((nb, 10), (nv, 6), (nb, 10)), ("cinert", "cdof", "crb"))
-    M = d.M
+    nb, nv, W, M = length(m.body_parentid), m.nv, int(d.nworld), d.M
+    cinert, cdof, crb = _all_per_body((d.cinert, d.cdof, d.crb), [(W, nb, 10), (W, nv, 6), (W, nb, 10)],
+                                      ("cinert", "cdof", "crb"))
     calls.call("imn_crb", (pack_tree_inertia(m, scratch), cinert, cdof, crb, addr(M), _row_ld(M), W), stream)
 
 
@@ -208,8 +203,11 @@ def rne(m: Any, d: Any, scratch: TreeReductionScratch | None = None, stream=None
     _need(scratch, "rne")
 
     nb, nv, W = length(m.body_parentid), m.nv, int(d.nworld)
+    per_body, per_dof = (W, nb, 6), (W, nv, 6)
     cinert, cvel, cdof, cdof_dot, cacc, cfrc_int = _all_per_body(
-        _RNE(d), W, ((nb, 10), (nb, 6), (nv, 6), (nv, 6), (nb, 6), (nb, 6)), _RNE_NAMES)
+        (d.cinert, d.cvel, d.cdof, d.cdof_dot, d.cacc, d.cfrc_int),
+        [(W, nb, 10), per_body, per_dof, per_dof, per_body, per_body],
+        ("cinert", "cvel", "cdof", "cdof_dot", "cacc", "cfrc_int"))
     qvel, qfrc_bias = d.qvel, d.qfrc_bias
-    calls.call("imn_rne", (pack_tree_gravity(m, scratch), cinert, cvel, cdof, cdof_dot, addr(qvel), _row_ld(qvel),
-                           cacc, cfrc_int, addr(qfrc_bias), _row_ld(qfrc_bias), W), stream)
+    calls.call("imn_rne", (pack_tree_gravity(m, scratch), cinert, cvel, cdof, cdof_dot, addr(qvel), _row_ld(qvel), cacc, cfrc_int,
+                           addr(qfrc_bias), _row_ld(qfrc_bias), W), stream)

@@ -15,13 +15,12 @@ from ..arrays import addr, length
 from . import tree_fusion
 
 
-_DATA = calls.getter("cdof", "cvel", "cdof_dot")
-
-
 def com_vel(m: Any, d: Any, tree: Any, stream=None) -> None:
     """d.cvel and d.cdof_dot from d.qvel and d.cdof."""
     tree_fusion._need(tree, "com_vel")
     nb, nv, W, qvel = length(m.body_parentid), m.nv, int(d.nworld), d.qvel
-    cdof, cvel, cdof_dot = tree_fusion._all_per_body(_DATA(d), W, ((nv, 6), (nb, 6), (nv, 6)), ("cdof", "cvel", "cdof_dot"))
-    calls.call("imn_com_vel", (tree_fusion.pack_tree_joints(m, tree), addr(qvel), tree_fusion._row_ld(qvel), cdof, cvel,
-                               cdof_dot, W), stream)
+    per_dof = (W, nv, 6)
+    cdof, cvel, cdof_dot = tree_fusion._all_per_body((d.cdof, d.cvel, d.cdof_dot), [per_dof, (W, nb, 6), per_dof],
+                                                     ("cdof", "cvel", "cdof_dot"))
+    calls.call("imn_com_vel", (tree_fusion.pack_tree_joints(m, tree), addr(qvel), tree_fusion._row_ld(qvel), cdof, cvel, cdof_dot,
+                               W), stream)
