@@ -119,8 +119,13 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   g.tB = t, t += sp ? (sp->nbsweep + 1) * 64 : 0;
   g.tS = t, t += sp ? up4(sp->nfac) : 0;
   g.tO = t, t += sp ? up4(m.nv) : 0;
-  // a plan's tables stay in global memory when they would take more than a third of an SM's shared memory;
-  // without a plan there is the M v program only, at most 31 KB for 79 dofs
+  // A plan's tables stay in global memory when they would take more than a third of an SM's shared memory;
+  // without a plan there is the M v program only, at most 31 KB for 79 dofs.  us per solve, tables in shared /
+  // global memory: 34 dofs (19 KB) 592 worlds 155 / 171, 8192 worlds 562 / 547 (14 worlds per SM against 16);
+  // 56 dofs (43 KB) 4096 worlds 1114 / 1193 (9 against 11); 79 dofs (57 KB) 1401 / 1940.  Beyond the
+  // third: 64 dofs with coupled limbs (81 KB) 592 worlds 472 / 688, 4096 worlds 1803 / 1955; 79 dofs
+  // (106 KB) 661 / 869, 3186 / 3312; (137 KB) 1437 / 1112, 7720 / 4234.  The third keeps the tables of every
+  // tree alone on chip and errs on the side of more worlds; the crossing lies near half an SM.
   g.tsm = !sp || 4 * t <= kMaxSmem / 3;
   g.tab = g.tsm ? t : 0;
   g.wait_polls = g_wait_polls;
@@ -148,8 +153,8 @@ __device__ __noinline__ void warn_limit(int which, unsigned limit) {
 // others read from ends in team_sync.
 // The solve is written as one loop whose trip is "take a world if none is in hand, else run one
 // pass of it" rather than as a load followed by a pass loop: the same statements, but the compiler
-// lays the single loop out better (measured: 0.836 -> 0.796 ms per 8192 humanoid worlds at the same
-// occupancy).
+// lays the single loop out better (when a CTA held one world: 0.836 -> 0.796 ms per 8192 humanoid worlds at
+// the same occupancy).
 template <bool JRES, bool J16, int SPARSE, bool STATS, bool TSM, bool TEAM>
 __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& d, const ImnCtx& cx, const Geom& g,
                                               const ImnSparsePlan& sp) {
@@ -775,10 +780,13 @@ static int worlds_per_sm(const Geom& g, int most) {
 
 // J resident in shared memory or streamed through the 32-row tile.  Resident J is
 // read once from HBM; a streamed J is re-read from L2 in every stage but leaves room
-// for more worlds per SM.  Measured on B200 (dense factor): humanoid (njmax 64) 12
-// resident vs 16 streamed worlds per SM: resident 7 % faster; SNU-like (njmax 128) 4 vs
-// 7: streamed 1.22x faster; G1-like (njmax 250) 4 vs 11: streamed 1.6x faster.  Hence:
-// stream when it holds at least 1.6x the worlds.
+// for more worlds per SM.  Stream when it holds at least 1.6x the worlds.  us per solve of a batch that
+// fills the GPU, resident / streamed (worlds per SM): 34 dofs x 64 rows 563 / 709 (14 / 12), dense factor 940 /
+// 1007 (13 / 12); 27 x 128 dense 476 / 536 (8 / 12); 35 x 128 dense 750 / 829 (8 / 12: 1.5x); 64 x 64
+// dense 1831 / 1779 (5 / 5); 48 x 96 dense 1381 / 1201 (5 / 10); 56 x 128 rows 1423 / 1115 (4 / 9); 64 x 128
+// dense 3650 / 2487 (3 / 5: 1.7x); 35 x 250 4600 / 2334 (4 / 12).  The ratio is that of full SMs; batches of up to 4
+// worlds per SM fit either way and differ by a few per cent: 56 x 128, 16 worlds 250 / 263, 592 worlds
+// 317 / 340; 35 x 250 240 / 232, 249 / 254.
 //
 // Warps per world: a world's rows, dofs and Hessian entries can be dealt to several warps; the line
 // search, the row lists and the factor cannot, and each stage costs a barrier.  A team of p warps is taken

@@ -22,8 +22,8 @@ struct World {
   float *Jsm, *A, *qacc, *Ma, *search, *mv, *grad, *qfs, *xsm, *dinv;
   // the world's M stays in global memory: its nM values are read once per iteration by
   // `products` (independent loads, issued together) and once by the Hessian assembly, and
-  // the shared memory they would take holds more worlds per SM instead (measured: humanoid
-  // 0.792 -> 0.785 ms per 8192 worlds, SNU-like 1.820 -> 1.736 ms per 4096)
+  // the shared memory they would take holds more worlds per SM instead (when a CTA held one world:
+  // humanoid 0.792 -> 0.785 ms per 8192 worlds, SNU-like 1.820 -> 1.736 ms per 4096)
   const float* M;
   float *Jaref, *jv, *Dsm, *force;
   const float* floss;  // global memory: only friction-loss rows read it
