@@ -175,9 +175,8 @@ typedef struct ImnSparsePlan {
    *     (0: not a diagonal), flags}; a, b, d start at the lane's own first term of the run and
    *     advance by the team width; flags bit 0 = the lane stores the entry, bit 1 = last step
    *     of its level, bits 2-4 = log2(team), bit 5 = last step of its sweep, bit 6 = a
-   *     lane of the sweep holds a diagonal entry, bit 7 = this step and the next, two sweeps
-   *     of a level, are done together (bits 8-15 then count for both), bits 8-15 = most
-   *     terms of a lane.
+   *     lane of the sweep holds a diagonal entry, bit 7 = this step and the next are two sweeps
+   *     of a level (bits 8-15 then count for both), bits 8-15 = most terms of a lane.
    *   bstep [nbsweep + 1][32][2]: {slot | source's right-hand side << 16, source's 1/D |
    *     destination's right-hand side << 16}; bit 0 of word 0 = the lane has work, of
    *     word 1 = last of its level.
@@ -187,7 +186,7 @@ typedef struct ImnSparsePlan {
   const uint32_t* fstep;
   const uint32_t* bstep;
   int32_t nfstep;
-  int32_t pairs; /* whether fstep has steps marked with bit 7 */
+  int32_t pairs; /* whether two thirds of the steps are marked with bit 7: a team of warps shares the levels */
 } ImnSparsePlan;
 
 /* Solver context: the arrays mujoco_warp's `_create_solver_context` allocates

@@ -507,17 +507,20 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
             hessian_dense<JRES, J16, TEAM>(s, quad_count, first);
         }
         PROF(9);
-        // the factorisation is a chain of levels or rows: part 0's
-        if (TEAM && part != 0) {
-        } else if (SPARSE) {
+        // the sweeps of a sparse factor's levels can be shared by the team; the solves and the dense factor are chains: part 0's
+        if (SPARSE && (first || quad_count > 0)) {
           // refactor the packed H, or solve with the resident factor
           // (sparse_hessian.py:490-547)
-          if (first || quad_count > 0) {
-            sp_load_rhs<TSM>(sp, s.tab, s.N, s.grad, lane);
-            IMN_MARK(s, 1);
-            sp_factor_steps<TSM, SPARSE == 2>(sp, s.tab, s.N, lane);
-            IMN_MARK(s, 2);
-          } else {
+          sp_load_rhs<TSM>(sp, s.tab, s.N, s.grad, tid, threads);
+          team_sync<TEAM>(s);
+          IMN_MARK(s, 1);
+          if (SPARSE == 2 || part == 0)
+            sp_factor_steps<TSM, SPARSE == 2>(sp, s.tab, s.N, lane, part, g.parts, [&] { team_sync<SPARSE == 2>(s); });
+          IMN_MARK(s, 2);
+        }
+        if (TEAM && part != 0) {
+        } else if (SPARSE) {
+          if (!(first || quad_count > 0)) {
             sp_forward(sp, s.N, s.iD, s.grad, lane);
             IMN_MARK(s, 3);
           }
@@ -653,8 +656,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
 
 // Two entry points over the same body, with the register bounds that follow from the most worlds
 // in hand (kResidentWarps, kStreamedWarps).
-// SPARSE: 0 the dense factor, 1 a sparse plan, 2 a sparse plan whose sweeps go in pairs (ImnSparsePlan::pairs):
-// beside the code for pairs the kernels of plans without them run 1 to 3 % slower.
+// SPARSE: 0 the dense factor, 1 a sparse plan, 2 a sparse plan whose sweeps a team shares (sp_factor_steps).
 // STATS compiles the work counters of ImnCtx.stats in: four more live values in a kernel that is
 // short of registers cost 9 % of its speed (measured), so the counting variants run only for
 // callers that pass the stats array.
@@ -676,16 +678,20 @@ static Kernel newton_kernel(bool resident, bool j16) {
                   : (Kernel)newton_kernel_streamed<false, SPARSE, STATS, TSM, TEAM>;
 }
 template <int SPARSE, bool STATS, bool TSM>
-static Kernel newton_kernel(bool resident, const Geom& g) {
+static Kernel newton_kernel(bool resident, const Geom& g, bool share) {
   if constexpr (!STATS)
-    if (g.parts > 1) return newton_kernel<SPARSE, STATS, TSM, true>(resident, g.j16);
+    if (g.parts > 1) {
+      if constexpr (SPARSE != 0)
+        if (share) return newton_kernel<2, STATS, TSM, true>(resident, g.j16);
+      return newton_kernel<SPARSE, STATS, TSM, true>(resident, g.j16);
+    }
   return newton_kernel<SPARSE, STATS, TSM, false>(resident, g.j16);
 }
 template <int SPARSE, bool STATS>
-static Kernel newton_kernel(bool resident, const Geom& g) {
+static Kernel newton_kernel(bool resident, const Geom& g, bool share) {
   if constexpr (SPARSE != 0)
-    if (!g.tsm) return newton_kernel<SPARSE, STATS, false>(resident, g);
-  return newton_kernel<SPARSE, STATS, true>(resident, g);
+    if (!g.tsm) return newton_kernel<SPARSE, STATS, false>(resident, g, share);
+  return newton_kernel<SPARSE, STATS, true>(resident, g, share);
 }
 
 __global__ void start_counters(int* nsolving, int* work_counter, int nworld) {
@@ -872,11 +878,10 @@ extern "C" int imn_solve(const ImnModel* m, const ImnData* d, const ImnCtx* cx, 
   rc = imn::plan_launch(m, d, cx->sparse_plan, cx->stats != nullptr, &g, &res, &grid);
   if (rc) return rc;
   const int bytes = 4 * (g.tab + g.warps * g.total);
-  const bool sparse = cx->sparse_plan != nullptr, stats = cx->stats != nullptr;
+  const bool sparse = cx->sparse_plan != nullptr, stats = cx->stats != nullptr, share = sparse && cx->sparse_plan->pairs;
   const ImnSparsePlan sp = sparse ? *cx->sparse_plan : ImnSparsePlan{};
-  const imn::Kernel kern = !sparse    ? (stats ? imn::newton_kernel<0, true>(res, g) : imn::newton_kernel<0, false>(res, g))
-                           : sp.pairs ? (stats ? imn::newton_kernel<2, true>(res, g) : imn::newton_kernel<2, false>(res, g))
-                                      : (stats ? imn::newton_kernel<1, true>(res, g) : imn::newton_kernel<1, false>(res, g));
+  const imn::Kernel kern = sparse ? (stats ? imn::newton_kernel<1, true>(res, g, share) : imn::newton_kernel<1, false>(res, g, share))
+                                  : (stats ? imn::newton_kernel<0, true>(res, g, share) : imn::newton_kernel<0, false>(res, g, share));
   {
     const cudaError_t e = imn::allow_shared(kern, bytes, true);
     if (e != cudaSuccess)

@@ -32,12 +32,11 @@ __device__ __forceinline__ int tab_orig(const Tables& tab, const ImnSparsePlan& 
   return TSM ? (int)tab.orig[j] : (int)__ldg(P.orig + j);
 }
 
-// N[rhs + j] = grad[dof of elimination index j]
+// N[rhs + j] = grad[dof of elimination index j], thread `t` of `threads`; the caller's barrier follows
 template <bool TSM>
-__device__ __forceinline__ void sp_load_rhs(const ImnSparsePlan& P, const Tables& tab, float* N, const float* grad, int lane) {
+__device__ __forceinline__ void sp_load_rhs(const ImnSparsePlan& P, const Tables& tab, float* N, const float* grad, int t, int threads) {
 #pragma unroll 1
-  for (int j = lane; j < P.nv; j += 32) N[P.nfac + j] = grad[tab_orig<TSM>(tab, P, j)];
-  __syncwarp();
+  for (int j = t; j < P.nv; j += threads) N[P.nfac + j] = grad[tab_orig<TSM>(tab, P, j)];
 }
 // N[rhs + j] = grad[dof of elimination index j]
 __device__ __forceinline__ void sp_load_rhs(const ImnSparsePlan& P, float* N, const float* grad, int lane) {
@@ -86,112 +85,109 @@ __device__ __forceinline__ void sp_factor_levels(const ImnSparsePlan& P, float* 
   }
 }
 
-// The same factorisation driven by the step records (ImnSparsePlan::fstep): one 128-bit load,
-// issued a step ahead, gives a lane its run of terms and its entry as byte offsets from N[0], so
-// that a term costs its three reads, two multiplications and a predicate.  Teams of one lane, where
-// most terms are, take four terms per trip with constant offsets between them; reads past a lane's
-// last term stay inside the world's shared memory and are not added.  (A lane that took the terms
-// of its run one by one from scaled indices spent 180 cycles per term step: 34-dof humanoid, 8192
-// worlds, 15 k cycles per factorisation.)
 __device__ __forceinline__ float sp_at(const float* N, uint32_t offset) {
   return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(N) + offset);
 }
-// Two sweeps of a level, whose chains of reads and sums run side by side (56 dofs, levels of up to
-// three sweeps, 4096 worlds: 1187 -> 1090 us per solve; four terms per trip instead of two: 1125).
-__device__ __forceinline__ void sp_two_sweeps(float* N, const uint4 e, const uint4 g) {
-  uint32_t a = e.x & 0xFFFFu, b = e.x >> 16, d = e.y & 0xFFFFu, A = g.x & 0xFFFFu, B = g.x >> 16, D = g.y & 0xFFFFu;
-  int n = (int)(e.z & 0xFFFFu), m = (int)(g.z & 0xFFFFu);
-  const uint32_t slot = e.y >> 16, Slot = g.y >> 16, stride = 4u << ((e.w >> 2) & 7u);
-  const float start = sp_at(N, slot), Start = sp_at(N, Slot);
-  float v = 0.0f, V = 0.0f;
+// The same factorisation driven by the step records (ImnSparsePlan::fstep): one 128-bit load,
+// issued a step ahead, gives a lane its run of terms and its entry as byte offsets from N[0], so
+// that a term costs its three reads, two multiplications and a predicate.
+//
+// A factorisation is a chain of steps, most of them with few terms, so what counts is a step's own
+// latency.  The records of a tree's plan begin with the sweeps of a lane per entry and one run of
+// terms; these have a loop of their own that asks a record for nothing but its terms and its diagonals.
+// With one loop for every kind of step, a step without any terms took 300 cycles, 100 of them in the
+// test for a reduction tree that it does not have, 130 in 1 / w (which only steps with a diagonal
+// need); the loop for them takes 50.  us per solve, one loop -> two: 34 dofs (16 steps) 16 worlds 125.6 -> 112.5,
+// 8192 worlds 561 -> 539; 35 dofs (21 steps) 16 worlds 229 -> 207, 16384 worlds 2330 -> 2277; 56 dofs (47 steps), 4096
+// worlds 1097 -> 1088.  In full batches the size of the code counts as much: with the next four terms'
+// reads in flight 112.5 / 550 / 207 / 2345 / 1123, with two sweeps of a level at once on top 56 dofs at 1200.
+//
+// SHARE: the warps of a team take the sweeps of a level in turn, for plans whose sweeps mostly have company in
+// their level (ImnSparsePlan::pairs).  56 dofs (47 steps in 22 levels): 16 worlds 272 -> 245 us, 592 worlds 356 -> 330.
+// Elsewhere the barriers cost more than the few extra sweeps: 34 dofs (16 in 13) 112.4 -> 114.1, 592 worlds
+// 139.9 -> 145.5; 35 dofs (21 in 16) 207.0 -> 208.0.
+// Reads past a lane's last term are not added.  They stay inside the world's shared memory: a lane
+// reads fewer than (terms of the step + 4) x team elements past its first one, at most 5 nv, and six
+// vectors of up4(nv + 1) elements follow 1 / D.
+// v plus the lane's terms of a record
+__device__ __forceinline__ float sp_terms(const float* N, const uint4 rec, uint32_t stride, float v) {
+  uint32_t a = rec.x & 0xFFFFu, b = rec.x >> 16, d = rec.y & 0xFFFFu;
+  int count = (int)(rec.z & 0xFFFFu);
 #pragma unroll 1
-  for (int left = (int)((e.w >> 8) & 0xFFu); left > 0; left -= 2, n -= 2, m -= 2) {
-    const float p0 = sp_at(N, a) * sp_at(N, b), q0 = sp_at(N, d), P0 = sp_at(N, A) * sp_at(N, B), Q0 = sp_at(N, D);
-    a += stride, b += stride, d += stride, A += stride, B += stride, D += stride;
-    const float p1 = sp_at(N, a) * sp_at(N, b), q1 = sp_at(N, d), P1 = sp_at(N, A) * sp_at(N, B), Q1 = sp_at(N, D);
-    a += stride, b += stride, d += stride, A += stride, B += stride, D += stride;
-    if (n > 0) v = fmaf(p0, q0, v);
-    if (m > 0) V = fmaf(P0, Q0, V);
-    if (n > 1) v = fmaf(p1, q1, v);
-    if (m > 1) V = fmaf(P1, Q1, V);
+  for (int left = (int)((rec.w >> 8) & 0xFFu); left > 0; left -= 4, count -= 4) {
+    float ab[4], q[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) ab[k] = sp_at(N, a + stride * k) * sp_at(N, b + stride * k), q[k] = sp_at(N, d + stride * k);
+    a += 4 * stride, b += 4 * stride, d += 4 * stride;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (count > k) v = fmaf(ab[k], q[k], v);
   }
-  const int T = 1 << ((e.w >> 2) & 7u);
-#pragma unroll 1
-  for (int off = T >> 1; off > 0; off >>= 1) {
-    const float x = __shfl_down_sync(IMN_FULL_MASK, v, off, T), X = __shfl_down_sync(IMN_FULL_MASK, V, off, T);
-    v = v + x, V = V + X;
-  }
-  const float w = start - v, W = Start - V;
+  return v;
+}
+__device__ __forceinline__ void sp_store(float* N, const uint4 rec, float w) {
   char* at = reinterpret_cast<char*>(N);
-  if (e.w & 1u) *reinterpret_cast<float*>(at + slot) = w;
-  if (g.w & 1u) *reinterpret_cast<float*>(at + Slot) = W;
-  if ((e.w | g.w) & 64u) {
-    const uint32_t di = e.z >> 16, Di = g.z >> 16;
-    const float inv = 1.0f / (di ? w : 1.0f), Inv = 1.0f / (Di ? W : 1.0f);
-    if (di) *reinterpret_cast<float*>(at + di) = inv;
-    if (Di) *reinterpret_cast<float*>(at + Di) = Inv;
+  if (rec.w & 1u) *reinterpret_cast<float*>(at + (rec.y >> 16)) = w;
+  if (rec.w & 64u) {
+    const uint32_t diag = rec.z >> 16;
+    const float inv = 1.0f / (diag ? w : 1.0f);
+    if (diag) *reinterpret_cast<float*>(at + diag) = inv;
   }
 }
 
-template <bool TSM, bool PAIR>
-__device__ __forceinline__ void sp_factor_steps(const ImnSparsePlan& P, const Tables& tables, float* N, int lane) {
+// `part` of `parts` warps; sync() orders the team's warps.
+template <bool TSM, bool SHARE, class Sync>
+__device__ __forceinline__ void sp_factor_steps(const ImnSparsePlan& P, const Tables& tables, float* N, int lane, int part, int parts,
+                                                Sync sync) {
   const uint4* tab = tables.fstep + lane;
   uint4 cur = tab_at<TSM>(tab);
-  float v = 0.0f;
+  int s = P.nfstep;
+  int turn = 0;  // the warp whose sweep it is
+  // a lane per entry, one run each
 #pragma unroll 1
-  for (int s = P.nfstep; s > 0; --s) {
+  for (; s > 0 && (cur.w & 0x3Cu) == 32u; --s) {
     tab += 32;
     const uint4 nxt = tab_at<TSM>(tab);
-    const uint32_t fl = cur.w, slot = cur.y >> 16;
-    if (PAIR && (fl & 128u)) {  // two sweeps of the level at once
-      tab += 32;
-      const uint4 then = tab_at<TSM>(tab);
-      sp_two_sweeps(N, cur, nxt);
-      if (nxt.w & 2u) __syncwarp();
-      cur = then;
-      --s;
-      continue;
+    if (!SHARE || turn == part) {
+      const float start = sp_at(N, cur.y >> 16);
+      const float v = sp_terms(N, cur, 4u, 0.0f);
+      sp_store(N, cur, start - v);
     }
-    uint32_t a = cur.x & 0xFFFFu, b = cur.x >> 16, d = cur.y & 0xFFFFu;
-    int cnt = (int)(cur.z & 0xFFFFu);
-    const float start = sp_at(N, slot);
-    int left = (int)((fl >> 8) & 0xFFu);
-    if ((fl & 0x1Cu) == 0u) {
-#pragma unroll 1
-      for (; left > 0; left -= 4, cnt -= 4, a += 16, b += 16, d += 16) {
-        float p[4], q[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) p[k] = sp_at(N, a + 4 * k) * sp_at(N, b + 4 * k), q[k] = sp_at(N, d + 4 * k);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (cnt > k) v = fmaf(p[k], q[k], v);
-      }
+    if (SHARE) {
+      turn = turn + 1 < parts ? turn + 1 : 0;
+      if (cur.w & 2u) sync(), turn = 0;
     } else {
-      const uint32_t stride = 4u << ((fl >> 2) & 7u);
+      __syncwarp();
+    }
+    cur = nxt;
+  }
+  float v = 0.0f;
 #pragma unroll 1
-      for (; left > 0; left -= 2, cnt -= 2) {
-        const float p0 = sp_at(N, a) * sp_at(N, b), q0 = sp_at(N, d);
-        a += stride, b += stride, d += stride;
-        const float p1 = sp_at(N, a) * sp_at(N, b), q1 = sp_at(N, d);
-        a += stride, b += stride, d += stride;
-        if (cnt > 0) v = fmaf(p0, q0, v);
-        if (cnt > 1) v = fmaf(p1, q1, v);
+  for (; s > 0; --s) {
+    tab += 32;
+    const uint4 nxt = tab_at<TSM>(tab);
+    if (!SHARE || turn == part) {
+      const float start = sp_at(N, cur.y >> 16);
+      const uint32_t log_team = __reduce_or_sync(IMN_FULL_MASK, (cur.w >> 2) & 7u);  // the same in every lane, and known to be
+      v = sp_terms(N, cur, 4u << log_team, v);
+      if (cur.w & 32u) {
+        if (log_team > 3) {
+          if (log_team > 4) v = v + __shfl_down_sync(IMN_FULL_MASK, v, 16, 32);
+          v = v + __shfl_down_sync(IMN_FULL_MASK, v, 8, 16);
+        }
+        if (log_team > 2) v = v + __shfl_down_sync(IMN_FULL_MASK, v, 4, 8);
+        if (log_team > 1) v = v + __shfl_down_sync(IMN_FULL_MASK, v, 2, 4);
+        if (log_team > 0) v = v + __shfl_down_sync(IMN_FULL_MASK, v, 1, 2);
+        sp_store(N, cur, start - v);
+        v = 0.0f;
       }
     }
-    if (fl & 32u) {
-      const int T = 1 << ((fl >> 2) & 7u);
-#pragma unroll 1
-      for (int off = T >> 1; off > 0; off >>= 1) v = v + __shfl_down_sync(IMN_FULL_MASK, v, off, T);
-      const float w = start - v;
-      if (fl & 1u) *reinterpret_cast<float*>(reinterpret_cast<char*>(N) + slot) = w;
-      if (fl & 64u) {
-        const uint32_t diag = cur.z >> 16;
-        const float inv = 1.0f / (diag ? w : 1.0f);
-        if (diag) *reinterpret_cast<float*>(reinterpret_cast<char*>(N) + diag) = inv;
-      }
-      v = 0.0f;
+    if (SHARE) {
+      if (cur.w & 32u) turn = turn + 1 < parts ? turn + 1 : 0;
+      if (cur.w & 2u) sync(), turn = 0;
+    } else {
+      __syncwarp();
     }
-    if (fl & 2u) __syncwarp();
     cur = nxt;
   }
 }

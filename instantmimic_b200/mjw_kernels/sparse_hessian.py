@@ -452,7 +452,7 @@ def _deal_entries(t: dict) -> np.ndarray:
 def pack_steps(t: dict, nv: int, nfac: int) -> dict:
     """The sweep records with every operand as a byte offset from N[0] and one record per run
     of terms (layout in include/imnewton.h): the kernel neither scales indices nor looks further
-    runs up.  Two sweeps of one run each in the same level are marked to be done together."""
+    runs up.  Two sweeps of one run each in the same level are marked as a pair."""
     if t["fsweep"].size == 0:
         rec = t["fsweep"].astype(np.int64).reshape(-1, 32, 4)
     else:
@@ -489,9 +489,9 @@ def pack_steps(t: dict, nv: int, nfac: int) -> dict:
         out[s, n - 1, :, 3] |= 32 | ends_level[s] | (64 if diag[s].any() else 0)
         steps += list(out[s, :n])
         single += [False] * (n - 1) + [n == 1 and not ends_level[s]]
-    # Pairs: where they cover two thirds of the steps (large trees, whose levels are several sweeps wide): 56
-    # dofs, 40 of 47 steps, 1187 -> 1090 us per solve.  Elsewhere the kernel without them is the faster
-    # one: 35 dofs with 10 of 21 steps in pairs, 2330 -> 2409.
+    # Pairs: where they cover two thirds of the steps (large trees, whose levels are several sweeps wide) the warps of
+    # a team share the levels: 56 dofs, 40 of 47 steps, 16 worlds 272 -> 245 us per solve.  Elsewhere the barriers cost
+    # more: 35 dofs with 10 of 21 steps in pairs, 207 -> 208, 34 dofs with 6 of 16 112 -> 114.
     first = []
     for k in range(len(steps) - 1):
         if single[k] and int(steps[k + 1][0, 3]) & 32 and not (first and first[-1] == k - 1):
