@@ -60,7 +60,7 @@ struct Geom {
   // tables in shared memory (Tables), in words from its start; the worlds' slices (`total` words
   // each, offsets above) follow at `tab` words.  warps: worlds in hand per CTA
   bool tsm;
-  int tM, tF, tB, tS, tO, tab, warps;
+  int tM, tF, tB, tS, tO, tP, tab, warps;
   // warps per world (make_geom); the tiles of a streamed J are `tile` words apart
   int parts, tile, oBox;
   bool early;  // the launch before this one is its own counter kernel, which writes no table
@@ -119,6 +119,7 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   g.tB = t, t += sp ? (sp->nbsweep + 1) * 64 : 0;
   g.tS = t, t += sp ? up4(sp->nfac) : 0;
   g.tO = t, t += sp ? up4(m.nv) : 0;
+  g.tP = t, t += sp ? up4(m.nv * g.mwords) : 0;
   // A plan's tables stay in global memory when they would take more than a third of an SM's shared memory;
   // without a plan there is the M v program only, at most 31 KB for 79 dofs.  us per solve, tables in shared /
   // global memory: 34 dofs (19 KB) 592 worlds 155 / 171, 8192 worlds 562 / 547 (14 worlds per SM against 16);
@@ -199,10 +200,12 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
     s.tab.bstep = reinterpret_cast<const uint2*>(smem_all + g.tB);
     s.tab.slots = reinterpret_cast<const uint32_t*>(smem_all + g.tS);
     s.tab.orig = reinterpret_cast<const uint32_t*>(smem_all + g.tO);
+    s.tab.pmask = reinterpret_cast<const uint32_t*>(smem_all + g.tP);
   } else {
     s.tab.mulm = reinterpret_cast<const uint4*>(m.M_mulm_lanes);
     s.tab.fstep = reinterpret_cast<const uint4*>(sp.fstep);
     s.tab.bstep = reinterpret_cast<const uint2*>(sp.bstep);
+    s.tab.pmask = sp.pmask;
   }
   s.M_rowadr = m.M_rowadr, s.M_rownnz = m.M_rownnz, s.M_colind = m.M_colind;
   int* const load_phase_at = static_cast<int*>(bar) + 2;  // the barrier itself takes two words
@@ -239,6 +242,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         reinterpret_cast<uint32_t*>(smem_all + g.tS)[i] =
             4u * __ldg(sp.s_a + i) | (4u * __ldg(sp.s_b + i)) << 9 | (uint32_t)(__ldg(sp.s_m + i) + 1) << 18;
       for (int i = threadIdx.x; i < nv; i += blockDim.x) reinterpret_cast<uint32_t*>(smem_all + g.tO)[i] = __ldg(sp.orig + i);
+      for (int i = threadIdx.x; i < nv * g.mwords; i += blockDim.x) reinterpret_cast<uint32_t*>(smem_all + g.tP)[i] = __ldg(sp.pmask + i);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
@@ -498,7 +502,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
           if (SPARSE && first) {
             bool bad = false;
 #pragma unroll 1
-            for (int r = lane; r < nefc; r += 32) bad = bad || row_outside(s.masks, r4, g.mwords, r, sp.pmask);
+            for (int r = lane; r < nefc; r += 32) bad = bad || row_outside<TSM>(s.masks, r4, g.mwords, r, s.tab.pmask);
             outside = __any_sync(IMN_FULL_MASK, bad);
           }
           if (SPARSE)

@@ -21,7 +21,7 @@ namespace imn {
 struct Tables {
   const uint4 *mulm, *fstep;
   const uint2* bstep;
-  const uint32_t *slots, *orig;
+  const uint32_t *slots, *orig, *pmask;
 };
 template <bool TSM, class T>
 __device__ __forceinline__ T tab_at(const T* p) {
