@@ -294,6 +294,7 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         nefc = min(R, nefc_in);
         ne = d.ne[w], nef = ne + d.nf[w];
         s.nefc = nefc, s.ne = ne, s.nef = nef;
+        if (TEAM) s.mulm_part = ((nefc + 31) >> 5) % g.parts;  // the one behind those that take a tile of rows
         rowless = nefc_in == 0;
         dofo = (size_t)w * d.dof_ld, efco = (size_t)w * d.efc_ld;
         s.Jg = d.efc_J + (d.J_world_offset ? (size_t)d.J_world_offset[w] : (size_t)w * d.J_ld_world);
@@ -435,9 +436,12 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         if (r < nefc) {
           const float nj = first ? s.Jaref[r] : rounded_step(s.Jaref[r], alpha, s.jv[r]);
           s.Jaref[r] = nj;
-          const bool is_eq = r < ne, is_fr = !is_eq && r < nef;
-          int ns;
-          eval_constraint(is_eq, is_fr, nj, s.Dsm[r], is_fr ? s.floss[r] : 0.0f, f, ns);
+          // an equality or an inequality row without a branch; friction-loss rows are few and come first
+          const float D = s.Dsm[r];
+          const bool quad = r < ne || !(nj >= 0.0f);
+          f = quad ? -D * nj : 0.0f;
+          int ns = quad ? IMN_STATE_QUADRATIC : IMN_STATE_SATISFIED;
+          if (r >= ne && r < nef) eval_friction(nj, D, s.floss[r], f, ns);
           const int old = first ? -1 : s.state[r];
           s.force[r] = f;
           s.state[r] = ns;
@@ -489,14 +493,13 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
         decrement *= rsq;
         grad_scale = ns;
       } else {
-        grad_dot = full_gradient<JRES, TEAM>(s, nfr);
+        full_gradient<JRES, TEAM>(s, nfr);
         if (STATS) {
           ++st_grad;
           if (!first) st_flips += quad_count;
           if (first || quad_count > 0) ++st_factor;
         }
         PROF(8);
-        decrement = 0.0f;
         grad_scale = 1.0f;
         if (first || quad_count > 0) {
           if (SPARSE && first) {
@@ -522,22 +525,24 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
             sp_factor_steps<TSM, SPARSE == 2>(sp, s.tab, s.N, lane, part, g.parts, [&] { team_sync<SPARSE == 2>(s); });
           IMN_MARK(s, 2);
         }
+        SearchSums sum = {0.0f, 0.0f, 0.0f};
         if (TEAM && part != 0) {
         } else if (SPARSE) {
           if (!(first || quad_count > 0)) {
             sp_forward(sp, s.N, s.iD, s.grad, lane);
             IMN_MARK(s, 3);
           }
-          sp_backward_steps<TSM>(sp, s.tab, s.N, s.iD, s.grad, s.search, s.bd, lane, search_dot, decrement);
+          sum = sp_backward_steps<TSM>(sp, s.tab, s.N, s.iD, s.grad, s.search, s.bd, lane);
           IMN_MARK(s, 4);
         } else {
-          factor_solve(s, first || quad_count > 0, search_dot, decrement);
+          sum = factor_solve(s, first || quad_count > 0);
         }
         if (TEAM) {
-          if (tid == 0) s.box[5] = __float_as_int(search_dot), s.box[6] = __float_as_int(decrement);
+          if (tid == 0) s.box[5] = __float_as_int(sum.xx), s.box[6] = __float_as_int(sum.gx), s.box[11] = __float_as_int(sum.gg);
           team_sync<TEAM>(s);
-          search_dot = __int_as_float(s.box[5]), decrement = __int_as_float(s.box[6]);
+          sum = {__int_as_float(s.box[5]), __int_as_float(s.box[6]), __int_as_float(s.box[11])};
         }
+        search_dot = sum.xx, decrement = sum.gx, grad_dot = sum.gg;
         PROF(10);
       }
       bool lost = !JRES && *s.jfail;
@@ -569,9 +574,11 @@ __device__ __forceinline__ void newton_worlds(const ImnModel& m, const ImnData& 
       }
       // ---- convergence (newton_fusion.py:267-295) -------------------------------
       ++niter;
-      const bool converged = alpha == 0.0f || (improvement > 0.0f && improvement / scale < tolerance) ||
-                             sqrtf(grad_dot) / scale < tolerance ||
-                             0.5f * decrement / scale < tolerance;
+      // the three measures over the lanes, one division for all of them, and no branch between them
+      float measure = lane == 0 ? improvement : lane == 1 ? sqrtf(grad_dot) : 0.5f * decrement;
+      measure = measure / scale;
+      const bool converged =
+          __any_sync(IMN_FULL_MASK, alpha == 0.0f || (measure < tolerance && (lane != 0 || improvement > 0.0f)));
       if (converged || niter == m.iterations) {
         if (!converged) {
           if ((m.warn_overflow & m.overflow_iterations) && tid == 0) warn_limit(1, (unsigned)m.iterations);

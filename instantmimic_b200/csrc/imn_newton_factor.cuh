@@ -133,7 +133,7 @@ __device__ __forceinline__ void factor_follow(const World& s, int b0, int c0) {
   __syncwarp();
 }
 
-__device__ __forceinline__ void factor_solve(const World& s, bool factor, float& sum0, float& sum1) {
+__device__ __forceinline__ SearchSums factor_solve(const World& s, bool factor) {
   const int lane = s.lane, nv = s.nv, ldu = s.ldu;
   float* A = s.A;
   if (factor) {
@@ -186,12 +186,14 @@ __device__ __forceinline__ void factor_solve(const World& s, bool factor, float&
     __syncwarp();
   }
   IMN_MARK(s, 14);
-  sum0 = logical_block_sum(nv, s.bd, lane, [&](int i, float a) { return fmaf(s.xsm[i], s.xsm[i], a); });
-  sum1 = logical_block_sum(nv, s.bd, lane, [&](int i, float a) { return fmaf(s.grad[i], s.xsm[i], a); });
-#pragma unroll 1
-  for (int i = lane; i < nv; i += 32) s.search[i] = -s.xsm[i];
+  const SearchSums sum = search_sums(nv, s.bd, lane, [&](int i, float& x, float& gx, float& g) {
+    x = s.xsm[i];
+    gx = g = s.grad[i];
+    s.search[i] = -x;
+  });
   __syncwarp();
   IMN_MARK(s, 15);
+  return sum;
 }
 
 }  // namespace imn

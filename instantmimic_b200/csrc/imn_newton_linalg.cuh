@@ -16,7 +16,7 @@ struct World {
   int nv, ldj, ldp, ldu, bd, nefc, ne, nef, lane, nM;
   // a team of `parts` warps may share the world (the TEAM kernels), each with a row tile, a copy barrier
   // and its words of its own; `box` carries single values from part 0 to the others
-  int part, parts, team_bar, tile_words;
+  int part, parts, team_bar, tile_words, mulm_part;  // mulm_part: the warp that forms M v
   int* box;
   float* tile;
   float *Jsm, *A, *qacc, *Ma, *search, *mv, *grad, *qfs, *xsm, *dinv;
@@ -265,7 +265,7 @@ __device__ __forceinline__ void products(const World& s, const float* v, float* 
   // itself, the table reads touched up to 18 cache lines per instruction, stood in front of the
   // reads of M, and dofs past 32 took a second round (34-dof model, 8192 worlds: 7000 -> 5900 cycles
   // of the world's warp per product; 56-dof model, 4096 worlds: 1745 -> 1669 us per solve).
-  if (!TEAM || ((s.nefc + 31) >> 5) % s.parts == part) {
+  if (!TEAM || s.mulm_part == part) {
     const uint4* prog = s.tab.mulm + lane;
     uint4 p = tab_at<TSM>(prog);
     float acc = 0.0f;
@@ -319,18 +319,17 @@ __device__ __forceinline__ void products(const World& s, const float* v, float* 
 }
 
 // grad = Ma - qfrc_smooth - J^T force over the rows with a nonzero force (a zero
-// force leaves the running sums unchanged), then grad_dot
-// (newton_stages.py:785-795).  Lane = dof.  Every element of J is used once, so a streamed J is read
+// force leaves the running sums unchanged; newton_stages.py:785-795).  Lane = dof.  Every element of J is used once, so a streamed J is read
 // straight from global memory (coalesced), without the detour through the tile; the listed rows go
 // several at a time so that their reads overlap.
 template <bool JRES, bool TEAM>
-__device__ __forceinline__ float full_gradient(const World& s, int nfr) {
+__device__ __forceinline__ void full_gradient(const World& s, int nfr) {
   const int lane = s.lane, nv = s.nv;
   float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
   const int i0 = lane, i1 = lane + 32, i2 = lane + 64;
   const int part = team_part<TEAM>(s), parts = team_parts<TEAM>(s);  // 32 dofs per warp of a team, in turn
-  const bool h0 = i0 < nv && (!TEAM || part == 0), h1 = i1 < nv && (!TEAM || 1 % parts == part),
-             h2 = i2 < nv && (!TEAM || 2 % parts == part);
+  const bool h0 = i0 < nv && (!TEAM || part == 0), h1 = i1 < nv && (!TEAM || part == 1),
+             h2 = i2 < nv && (!TEAM || part == (parts > 2 ? 2 : 0));
   if (TEAM && 32 * part >= nv) nfr = 0;
   constexpr int B = JRES ? 4 : 8;
   const float* J = (JRES ? s.Jsm : s.Jg) + lane;
@@ -351,7 +350,6 @@ __device__ __forceinline__ float full_gradient(const World& s, int nfr) {
   if (h1) s.grad[i1] = (s.Ma[i1] - s.qfs[i1]) - s1;
   if (h2) s.grad[i2] = (s.Ma[i2] - s.qfs[i2]) - s2;
   team_sync<TEAM>(s);
-  return logical_block_sum(nv, s.bd, lane, [&](int i, float acc) { return fmaf(s.grad[i], s.grad[i], acc); });
 }
 
 // The Hessian from the listed rows, dense form.  First call: H = M + sum D J^T J over the

@@ -74,8 +74,6 @@ __device__ __forceinline__ LineSearchResult line_search(const World& s, float se
                                                         float ls_tolerance, float scale, float eps,
                                                         int ls_iterations) {
   const int lane = s.lane, nv = s.nv, ne = s.ne, nef = s.nef, nefc = s.nefc, bd = s.bd;
-  const float snorm = sqrtf(search_dot);
-  const float gtol = fmaxf(tolerance * ls_tolerance * snorm * scale, 1e-06f);
   float q[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 1
   for (int i = lane; i < nv; i += 32) {
@@ -117,16 +115,22 @@ __device__ __forceinline__ LineSearchResult line_search(const World& s, float se
   ls_sum(q, bd, lane);
   const float q1 = q[0], q2 = q[1];
   const Vec3 p0 = v3(0.0f, q1, 2.0f * q2) + v3(q[2], q[3], q[4]);
-  const float q1_abs = sqrtf(2.0f * fmaxf(q[2], 0.0f) * fmaxf(q[4], 0.0f)) + fabsf(q1);
+  // Roots and quotients take 110 cycles each and come in pairs: one for the lower half of the warp, one for the upper.
+  const bool up = lane >= 16;
+  const float root = sqrtf(up ? 2.0f * fmaxf(q[2], 0.0f) * fmaxf(q[4], 0.0f) : search_dot);
+  const float snorm = __shfl_sync(IMN_FULL_MASK, root, 0);
+  const float gtol = fmaxf(tolerance * ls_tolerance * snorm * scale, 1e-06f);
+  const float q1_abs = __shfl_sync(IMN_FULL_MASK, root, 16) + fabsf(q1);
   const float gtol_accept = fmaxf(gtol, eps * q1_abs);
-  out.noise_floor = eps * fmaxf(1.0f, safe_div(q1_abs, p0.c2));
+  const float quotient = safe_div(up ? q1_abs : p0.c1, p0.c2);
+  const float a_in = -__shfl_sync(IMN_FULL_MASK, quotient, 0);
+  out.noise_floor = eps * fmaxf(1.0f, __shfl_sync(IMN_FULL_MASK, quotient, 16));
   if (fabsf(p0.c1) < eps * q1_abs) {
     out.converged = true;
     return out;
   }
 
   // pass 1: the first Newton step
-  const float a_in = -safe_div(p0.c1, p0.c2);
   Vec3 lo, hi;
   float lo_alpha, hi_alpha;
   {
@@ -154,7 +158,9 @@ __device__ __forceinline__ LineSearchResult line_search(const World& s, float se
   // bracket passes
 #pragma unroll 1
   for (int pass = 0; pass < ls_iterations; ++pass) {
-    const float al[3] = {lo_alpha - safe_div(lo.c1, lo.c2), hi_alpha - safe_div(hi.c1, hi.c2), 0.5f * (lo_alpha + hi_alpha)};
+    const float step = safe_div(up ? hi.c1 : lo.c1, up ? hi.c2 : lo.c2);
+    const float al[3] = {lo_alpha - __shfl_sync(IMN_FULL_MASK, step, 0), hi_alpha - __shfl_sync(IMN_FULL_MASK, step, 16),
+                         0.5f * (lo_alpha + hi_alpha)};
     Vec3 acc[3];
     ls_rows<3>(s, rowa, rowb, fric, more, al, acc);
     float r9[9] = {acc[0].c0, acc[0].c1, acc[0].c2, acc[1].c0, acc[1].c1, acc[1].c2, acc[2].c0, acc[2].c1, acc[2].c2};

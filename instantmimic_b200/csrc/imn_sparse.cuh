@@ -11,7 +11,7 @@
 // a fixed order, so results do not depend on scheduling.
 #pragma once
 
-#include "imn_common.cuh"
+#include "imn_newton_dev.cuh"
 
 namespace imn {
 
@@ -252,12 +252,10 @@ __device__ __forceinline__ void sp_backward(const ImnSparsePlan& P, float* N, co
   __syncwarp();
 }
 
-// sp_backward driven by the step records (ImnSparsePlan::bstep).
+// sp_backward driven by the step records (ImnSparsePlan::bstep); returns the sums, grad . grad among them.
 template <bool TSM>
-__device__ __forceinline__ void sp_backward_steps(const ImnSparsePlan& P, const Tables& tables, float* N, const float* iD,
-                                                  const float* grad, float* search, int bd, int lane,
-                                                  float& sum0, float& sum1) {
-  const int rhs = P.nfac, n = P.nv;
+__device__ __forceinline__ SearchSums sp_backward_steps(const ImnSparsePlan& P, const Tables& tables, float* N, const float* iD,
+                                                        const float* grad, float* search, int bd, int lane) {
   const uint2* tab = tables.bstep + lane;
   uint2 cur = tab_at<TSM>(tab);
 #pragma unroll 1
@@ -271,23 +269,14 @@ __device__ __forceinline__ void sp_backward_steps(const ImnSparsePlan& P, const 
     if (cur.y & 1u) __syncwarp();
     cur = nxt;
   }
-  float ra = 0.0f, rb = 0.0f;
-#pragma unroll 1
-  for (int w = 0; w < bd / 32; ++w) {
-    float s0 = 0.0f, s1 = 0.0f;
-#pragma unroll 1
-    for (int j = lane + 32 * w; j < n; j += bd) {
-      const int d = tab_orig<TSM>(tables, P, j);
-      const float v = N[rhs + j] * iD[j];
-      search[d] = -v;
-      s0 = fmaf(v, v, s0);
-      s1 = fmaf(grad[d], v, s1);
-    }
-    ra = ra + warp_tree_sum(s0);
-    rb = rb + warp_tree_sum(s1);
-  }
-  sum0 = ra, sum1 = rb;
+  const SearchSums sum = search_sums(P.nv, bd, lane, [&](int j, float& x, float& gx, float& g) {
+    const int d = tab_orig<TSM>(tables, P, j);
+    x = N[P.nfac + j] * iD[j];
+    gx = grad[d], g = grad[j];
+    search[d] = -x;
+  });
   __syncwarp();
+  return sum;
 }
 
 // Count one pattern violation in the world's counter (last element of its hfactor);
