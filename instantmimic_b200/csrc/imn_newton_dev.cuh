@@ -47,6 +47,38 @@ __device__ __forceinline__ bool mbar_try_wait(void* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// ---- pairs of floats: one instruction for two fused multiply-adds, each rounded as fmaf rounds it ----------
+typedef unsigned long long Pair;
+__device__ __forceinline__ Pair make_pair(float x, float y) {
+  Pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float pair_x(Pair a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+  return x;
+}
+__device__ __forceinline__ float pair_y(Pair a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+  return y;
+}
+__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
+  Pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
+  Pair r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+struct alignas(16) Pair2 {
+  Pair a, b;
+};
+__device__ __forceinline__ Pair2 ld_pair2(const float* p) { return *reinterpret_cast<const Pair2*>(p); }
+
 // ---- row cost pieces (the statement is in oracle/newton_oracle.c) -------------
 __device__ __forceinline__ int row_zone(float x, bool fr, float rf) {
   if (fr) return x <= -rf ? IMN_STATE_LINEARNEG : (x >= rf ? IMN_STATE_LINEARPOS : IMN_STATE_QUADRATIC);

@@ -12,9 +12,11 @@
 // multiply-adds; the pivot is sqrtf; the row is scaled by the reciprocal pivot.
 //
 // Mapping: 16 rows at a time.  A lane owns K columns c = b0 + lane + 32k (K = 1 or 2 by the
-// columns that are left; columns past the 64th follow when the block's rows are done) and keeps the block's 16 running sums of each in registers.  Phase 1 adds
-// the terms of all earlier rows (one shared-memory read of U[t][c] per column and four 128-bit
-// broadcast reads of U[t][b0..b0+15] feed 16 K fused multiply-adds).  Phase 2 eliminates the block's
+// columns that are left; columns past the 64th follow when the block's rows are done) and keeps the block's 16 running
+// sums of each in registers, two rows to a pair, so that one instruction does two of the fused multiply-adds (a
+// register and an instruction per row instead: 48 dofs x 96 rows, 4096 worlds 1140 us against 1067, 32 x 128, 8192 worlds 1784
+// against 1775, others equal).  Phase 1 adds the terms of all earlier rows (one shared-memory read of U[t][c] per
+// column and four 128-bit broadcast reads of U[t][b0..b0+15] feed 8 K pairs).  Phase 2 eliminates the block's
 // rows.  Its chain per row is scale -> own square -> shuffle -> root -> reciprocal: the pivot of row
 // r + 1 is its lane's own sum after row r, which that lane has at once, so it travels while the
 // other sums wait for row r to come back from shared memory as four broadcast reads (the block's
@@ -32,7 +34,7 @@ template <int K>
 __device__ __forceinline__ void factor_block(const World& s, int b0) {
   const int lane = s.lane, nv = s.nv, ldu = s.ldu, nr = min(16, nv - b0);
   float* A = s.A;
-  float acc[K][16];
+  Pair acc[K][8];  // rows 2h and 2h + 1
   int cc[K];
   bool valid[K];
 #pragma unroll
@@ -44,31 +46,31 @@ __device__ __forceinline__ void factor_block(const World& s, int b0) {
     // last hold values that are never stored or read by another lane
     const float* src = (cc[k] < nv ? A + (cc[k] + 1) * ldu : s.grad) + b0;
 #pragma unroll
-    for (int g = 0; g < 16; g += 4) {
-      const float4 h = g < nr ? ld4(src + g) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      acc[k][g] = h.x, acc[k][g + 1] = h.y, acc[k][g + 2] = h.z, acc[k][g + 3] = h.w;
+    for (int g = 0; g < 4; ++g) {
+      Pair2 h = {0ull, 0ull};
+      if (4 * g < nr) h = ld_pair2(src + 4 * g);
+      acc[k][2 * g] = h.a, acc[k][2 * g + 1] = h.b;
     }
   }
   // phase 1: terms of rows t < b0
 #pragma unroll 2
   for (int t = 0; t < b0; ++t) {
     const float* Ut = A + t * ldu;
-    float uc[K];
+    Pair uc[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) uc[k] = Ut[cc[k]];
+    for (int k = 0; k < K; ++k) uc[k] = make_pair(-Ut[cc[k]], -Ut[cc[k]]);
 #pragma unroll
-    for (int g = 0; g < 16; g += 4) {
-      const float4 u = ld4(Ut + b0 + g);  // past the last row: values of the next rows, never stored
+    for (int g = 0; g < 4; ++g) {
+      const Pair2 u = ld_pair2(Ut + b0 + 4 * g);  // past the last row: values of the next rows, never stored
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        acc[k][g] = fmaf(-u.x, uc[k], acc[k][g]), acc[k][g + 1] = fmaf(-u.y, uc[k], acc[k][g + 1]);
-        acc[k][g + 2] = fmaf(-u.z, uc[k], acc[k][g + 2]), acc[k][g + 3] = fmaf(-u.w, uc[k], acc[k][g + 3]);
-      }
+      for (int k = 0; k < K; ++k)
+        acc[k][2 * g] = pair_fma(u.a, uc[k], acc[k][2 * g]), acc[k][2 * g + 1] = pair_fma(u.b, uc[k], acc[k][2 * g + 1]);
     }
   }
   IMN_MARK(s, 12);
-  // phase 2: acc[k][q] belongs to row g + q
-  float pv = __shfl_sync(IMN_FULL_MASK, acc[0][0], 0);
+  // phase 2: acc[k][q / 2] belongs to row g + q
+  const auto row = [&](int k, int q) { return q & 1 ? pair_y(acc[k][q >> 1]) : pair_x(acc[k][q >> 1]); };
+  float pv = __shfl_sync(IMN_FULL_MASK, row(0, 0), 0);
 #pragma unroll 1
   for (int g = 0; g < nr; g += 4) {
 #pragma unroll
@@ -79,29 +81,28 @@ __device__ __forceinline__ void factor_block(const World& s, int b0) {
       float* Ur = A + (b0 + r) * ldu;
       float u[K];
 #pragma unroll
-      for (int k = 0; k < K; ++k) u[k] = acc[k][q] * rinv;
-      pv = __shfl_sync(IMN_FULL_MASK, fmaf(-u[0], u[0], acc[0][q + 1]), r + 1);
+      for (int k = 0; k < K; ++k) u[k] = row(k, q) * rinv;
+      pv = __shfl_sync(IMN_FULL_MASK, fmaf(-u[0], u[0], row(0, q + 1)), r + 1);
 #pragma unroll
       for (int k = 0; k < K; ++k)
         if (valid[k] && cc[k] >= b0 + r) Ur[cc[k]] = k == 0 && lane == r ? dg : u[k];
       if (lane == 0) s.dinv[b0 + r] = rinv;
       __syncwarp();
 #pragma unroll
-      for (int h = 0; h < 16; h += 4) {
-        const float4 m = ld4(Ur + b0 + g + h);
+      for (int h = 0; h < 4; ++h) {
+        const Pair2 m = ld_pair2(Ur + b0 + g + 4 * h);
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-          if (h > q) acc[k][h] = fmaf(-m.x, u[k], acc[k][h]);
-          if (h + 1 > q) acc[k][h + 1] = fmaf(-m.y, u[k], acc[k][h + 1]);
-          if (h + 2 > q) acc[k][h + 2] = fmaf(-m.z, u[k], acc[k][h + 2]);
-          if (h + 3 > q) acc[k][h + 3] = fmaf(-m.w, u[k], acc[k][h + 3]);
+        for (int k = 0; k < K; ++k) {  // sums of finished rows go on as pairs of others
+          const Pair nu = make_pair(-u[k], -u[k]);
+          if (4 * h + 1 > q) acc[k][2 * h] = pair_fma(m.a, nu, acc[k][2 * h]);
+          if (4 * h + 3 > q) acc[k][2 * h + 1] = pair_fma(m.b, nu, acc[k][2 * h + 1]);
         }
       }
     }
 #pragma unroll
     for (int k = 0; k < K; ++k)
 #pragma unroll
-      for (int h = 0; h < 16; ++h) acc[k][h] = h < 12 ? acc[k][h + 4] : 0.0f;
+      for (int h = 0; h < 8; ++h) acc[k][h] = h < 6 ? acc[k][h + 2] : 0ull;
   }
   __syncwarp();
   IMN_MARK(s, 13);
