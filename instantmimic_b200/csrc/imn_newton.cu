@@ -806,12 +806,16 @@ static int worlds_per_sm(const Geom& g, int most) {
 // 317 / 340; 35 x 250 240 / 232, 249 / 254.
 //
 // Warps per world: a world's rows, dofs and Hessian entries can be dealt to several warps; the line
-// search, the row lists and the factor cannot, and each stage costs a barrier.  A team of p warps is taken
-// for sqrt(p) times one: the choice is the largest (worlds in hand) x sqrt(team).  That is one warp where
-// the worlds in hand fill the SM's registers, more for batches of few worlds per SM (1024 34-dof
-// worlds, two warps: 182 -> 174 us; 1000 35-dof worlds, dense: 436 -> 411; 16 worlds, four warps, solve and
-// the rest of a step: 174 -> 161) and for worlds so large that few fit (64 dofs x 512 rows: 5 worlds of a warp
-// 4621 us, 3 of four warps 4153).
+// search, the row lists and most factors cannot, and each stage costs a barrier.  A solve by a team takes kTeamTime of
+// one warp's time (one world per SM, one to four warps: 34 dofs 134 / 126 / 119 / 119 us, 56 dofs 372 / 300 / 263 / 259,
+// 64 dofs x 512 rows 812 / 570 / 476 / 457), but an SM holds fewer teams.  A launch lasts as many solves as its SMs take
+// worlds one after the other: `rounds` if a started round took as long as a full one, share / n if worlds filled
+// in for one another; measured batches lie half-way.  The choice is the least product of the two.  us by the largest
+// (worlds in hand) x sqrt(team), which knows no rounds -> now (best of all four): 34 dofs, 6 worlds per SM 158 -> 142
+// (142), 10 per SM 178 -> 162 (162); 40 x 100 dense, 6: 328 -> 244 (244); 60 dofs, 7: 921 -> 764 (764); 64 x 512, 4: 842 -> 650
+// (650), 12: 1810 -> 1755 (1755); 50 x 100, 8: 444 -> 370 (370); 56 dofs, 7: 393 -> 454 (393).  Over 131 batches of nine models and 1
+// to 28 worlds per SM the mean distance from the best falls from 2.4 % to 0.5 %.
+static const float kTeamTime[5] = {0.0f, 1.0f, 0.82f, 0.70f, 0.60f};
 static const int kMaxParts = 4;
 
 static int plan_launch(const ImnModel* m, const ImnData* d, const ImnSparsePlan* sp, bool stats, Geom* g, bool* resident,
@@ -829,12 +833,13 @@ static int plan_launch(const ImnModel* m, const ImnData* d, const ImnSparsePlan*
   // one CTA per SM; a batch that does not fill the GPU is spread over all SMs
   const int sms = sm_count(), share = max((d->nworld + sms - 1) / sms, 1);
   g->warps = min(share, *resident ? nr : ns);
+  const auto time = [&](const Geom& q) {
+    return ((float)((share + q.warps - 1) / q.warps) + (float)share / (float)q.warps) * kTeamTime[q.parts];
+  };
   for (int parts = 2; parts <= kMaxParts && !stats; ++parts) {  // the counting kernels know no teams
     Geom team = make_geom(*m, *d, *resident, sp, parts);
-    const int n = min(share, worlds_per_sm(team, (*resident ? kResidentWarps : kStreamedWarps) / parts));
-    if ((float)n * sqrtf((float)parts) <= (float)g->warps * sqrtf((float)g->parts)) continue;
-    team.warps = n;
-    *g = team;
+    team.warps = min(share, worlds_per_sm(team, (*resident ? kResidentWarps : kStreamedWarps) / parts));
+    if (team.warps > 0 && time(team) < time(*g)) *g = team;
   }
   const int need = (d->nworld + g->warps - 1) / g->warps;
   *grid = need < sms ? need : sms;
