@@ -184,7 +184,7 @@ class ImnBlockedPlan(C.Structure):
         ("pad", I32),
         ("indices", P),
         ("identity", P),
-        ("nM", I32),
+        ("nM", I32), ("places", P),
     ]
 
 

@@ -93,17 +93,17 @@ __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast
 // an SM holds to cover it: registers for 28 warps per SM (models up to 64 columns), so that 4096 worlds are
 // in flight at once.  4096 humanoid worlds, three right-hand sides, then one with the stored factor:
 // 104 us with two worlds per warp, three column groups throughout and 15 shuffles per row; 95 at 24
-// warps per SM; 69 as it is (65536 worlds: 1432 -> 958).  Two worlds per warp halve the warps and take
+// warps per SM; 67 at 28 (47 with what the comments below say).  Two worlds per warp halve the warps and take
 // three column groups for one or two: slower at every batch size.
 //
 // Rows b0 .. b0 + 15 at the K column groups that are left.  As in the Newton factor
 // (imn_newton_factor.cuh): the pivot of row r + 1 is its own lane's sum after row r and travels at
 // once, the row's block entries come back from shared memory as broadcast reads, four rows per trip.
-template <int K>
+template <int K, int R>
 __device__ __forceinline__ void dense_block(float* A, float* dinv, const int b0, const int n, const int nc, const int ldu,
                                             const int l) {
   const int nr = min(16, n - b0);
-  float acc[K][16];
+  float acc[K][R];
   int cc[K];
   bool valid[K];
 #pragma unroll
@@ -113,7 +113,7 @@ __device__ __forceinline__ void dense_block(float* A, float* dinv, const int b0,
     cc[k] = valid[k] ? c : nc - 1;
     const float* src = A + (cc[k] + 1) * ldu + b0;
 #pragma unroll
-    for (int g = 0; g < 16; g += 4) {
+    for (int g = 0; g < R; g += 4) {
       const float4 h = g < nr ? ld4(src + g) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       acc[k][g] = h.x, acc[k][g + 1] = h.y, acc[k][g + 2] = h.z, acc[k][g + 3] = h.w;
     }
@@ -126,7 +126,7 @@ __device__ __forceinline__ void dense_block(float* A, float* dinv, const int b0,
 #pragma unroll
     for (int k = 0; k < K; ++k) uc[k] = Ut[cc[k]];
 #pragma unroll
-    for (int g = 0; g < 16; g += 4) {
+    for (int g = 0; g < R; g += 4) {
       const float4 u = ld4(Ut + b0 + g);  // past the last row: values that end in sums nobody stores
 #pragma unroll
       for (int k = 0; k < K; ++k) {
@@ -148,14 +148,14 @@ __device__ __forceinline__ void dense_block(float* A, float* dinv, const int b0,
       float u[K];
 #pragma unroll
       for (int k = 0; k < K; ++k) u[k] = acc[k][q] * rinv;
-      pv = __shfl_sync(IMN_FULL_MASK, fmaf(-u[0], u[0], acc[0][q + 1]), r + 1);
+      pv = __shfl_sync(IMN_FULL_MASK, fmaf(-u[0], u[0], q + 1 < R ? acc[0][q + 1] : 0.0f), r + 1);
 #pragma unroll
       for (int k = 0; k < K; ++k)
         if (valid[k] && cc[k] >= b0 + r) Ur[cc[k]] = k == 0 && l == r ? dg : u[k];
       if (l == 0) dinv[b0 + r] = rinv;
       __syncwarp();
 #pragma unroll
-      for (int h = 0; h < 16; h += 4) {
+      for (int h = 0; h < R; h += 4) {
         const float4 m = ld4(Ur + b0 + g + h);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
@@ -169,7 +169,7 @@ __device__ __forceinline__ void dense_block(float* A, float* dinv, const int b0,
 #pragma unroll
     for (int k = 0; k < K; ++k)
 #pragma unroll
-      for (int h = 0; h < 16; ++h) acc[k][h] = h < 12 ? acc[k][h + 4] : 0.0f;
+      for (int h = 0; h < R; ++h) acc[k][h] = h + 4 < R ? acc[k][h + 4] : 0.0f;
   }
   __syncwarp();
 }
@@ -178,12 +178,16 @@ template <int KM>
 __device__ __forceinline__ void dense_factor_carry(float* A, float* dinv, const int n, const int nc, const int ldu, const int l) {
 #pragma unroll 1
   for (int b0 = 0; b0 < n; b0 += 16) {
-    if (nc - b0 <= 32)
-      dense_block<1>(A, dinv, b0, n, nc, ldu, l);
+    // a last block of up to four rows (33 to 36 dofs) keeps no sums of the twelve it does not have
+    // (4096 34-dof worlds 49.8 -> 47.4 us)
+    if (n - b0 <= 4 && nc - b0 <= 32)
+      dense_block<1, 4>(A, dinv, b0, n, nc, ldu, l);
+    else if (nc - b0 <= 32)
+      dense_block<1, 16>(A, dinv, b0, n, nc, ldu, l);
     else if (KM == 2 || nc - b0 <= 64)
-      dense_block<2>(A, dinv, b0, n, nc, ldu, l);
+      dense_block<2, 16>(A, dinv, b0, n, nc, ldu, l);
     else
-      dense_block<KM>(A, dinv, b0, n, nc, ldu, l);
+      dense_block<KM, 16>(A, dinv, b0, n, nc, ldu, l);
   }
 }
 
@@ -289,6 +293,7 @@ __device__ __forceinline__ void dense_substitute(const float* A, const float* di
 template <int KM>
 __global__ void __launch_bounds__(32 * kDenseWarps, KM == 2 ? 7 : 4)
     blocked_dense_kernel(const int nv, const int pad, const int nM, const int* __restrict__ indices,
+                         const uint16_t* __restrict__ places,
                          const float* __restrict__ identity, const float* __restrict__ M, const int64_t M_ld,
                          const float* __restrict__ y, float* __restrict__ Ug, float* __restrict__ x,
                          const int* __restrict__ active, const int rhs, const int mode, const int carry,
@@ -310,25 +315,49 @@ __global__ void __launch_bounds__(32 * kDenseWarps, KM == 2 ? 7 : 4)
   const float* yw = y + (size_t)w * n * rhs;
   for (int q = l; q < n * rhs; q += 32) X[q] = yw[q];
   if (mode == 0) {
-    // gather the blocks on and above the diagonal: table entry
-    // ((kb*nblk + ib)*16 + r)*16 + c addresses M's value of (16 kb + r, 16 ib + c);
-    // index nM is the extra zero slot
+    // the padded diagonal's roots, a lane each
+    const float root = n + l < pad ? sqrtf(__ldg(identity + (((n + l) & 15) << 4 | ((n + l) & 15)))) : 0.0f;
     const float* Mw = M + (size_t)w * M_ld;
-    for (int kb = 0; kb < nblk; ++kb)
-      for (int ib = kb; ib < nblk; ++ib) {
-        const int* tab = indices + ((kb * nblk + ib) << 8);
-#pragma unroll 4
-        for (int q = l; q < 256; q += 32) {
-          const int row = 16 * kb + (q >> 4), colm = 16 * ib + (q & 15);
-          const int idx = __ldg(tab + q);
-          if (row <= colm && colm < n) A[(colm + 1) * ldu + row] = idx < nM ? __ldg(Mw + idx) : 0.0f;
+    if (places) {
+      // M's entries in storage order, coalesced, each to its place; the positions between them are zero.  Looked up
+      // position by position (a read of the table, a branch, a read of M for every position of a block) this was 25 k
+      // of the 78 k cycles of a 34-dof world.  us, 4096 34-dof worlds, three right-hand sides and a second solve 61 -> 50,
+      // 256 worlds 29 -> 24; 8192 56-dof worlds 271 -> 220.
+      constexpr int B = 8;
+      for (int q = l; 4 * q < (n + 1) * ldu; q += 32) *reinterpret_cast<float4*>(A + 4 * q) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      __syncwarp();
+#pragma unroll 1
+      for (int e0 = l; e0 < nM; e0 += 32 * B) {
+        float v[B];
+        int at[B];
+#pragma unroll
+        for (int j = 0; j < B; ++j) {
+          const int e = min(e0 + 32 * j, nM - 1);
+          v[j] = __ldg(Mw + e), at[j] = __ldg(places + e);
         }
+#pragma unroll
+        for (int j = 0; j < B; ++j)
+          if (e0 + 32 * j < nM) A[((at[j] >> 8) + 1) * ldu + (at[j] & 255)] = v[j];
       }
-    __syncwarp();
-    for (int e = l; e < n * carry; e += 32) {
-      const int r = e / carry, q = e - r * carry;
-      A[(n + q + 1) * ldu + r] = X[r * rhs + q];
+    } else {
+      // gather the blocks on and above the diagonal: table entry
+      // ((kb*nblk + ib)*16 + r)*16 + c addresses M's value of (16 kb + r, 16 ib + c);
+      // index nM is the extra zero slot
+      for (int kb = 0; kb < nblk; ++kb)
+        for (int ib = kb; ib < nblk; ++ib) {
+          const int* tab = indices + ((kb * nblk + ib) << 8);
+#pragma unroll 4
+          for (int q = l; q < 256; q += 32) {
+            const int row = 16 * kb + (q >> 4), colm = 16 * ib + (q & 15);
+            const int idx = __ldg(tab + q);
+            if (row <= colm && colm < n) A[(colm + 1) * ldu + row] = idx < nM ? __ldg(Mw + idx) : 0.0f;
+          }
+        }
     }
+    __syncwarp();
+#pragma unroll 1
+    for (int q = 0; q < carry; ++q)
+      for (int r = l; r < n; r += 32) A[(n + q + 1) * ldu + r] = X[r * rhs + q];
     __syncwarp();
     dense_factor_carry<KM>(A, dinv, n, nc, ldu, l);
     // the factor, padded: zeros below the diagonal, the padded diagonal's own root; four columns
@@ -350,19 +379,33 @@ __global__ void __launch_bounds__(32 * kDenseWarps, KM == 2 ? 7 : 4)
         for (int c = l; c < pad; c += 32) Ur[c] = (c >= r && c < n) ? Ar[c] : 0.0f;
       }
     }
+#pragma unroll 1
     for (int r = n; r < pad; ++r) {
-      const float dg = sqrtf(identity[((r & 15) << 4) | (r & 15)]);
-      for (int c = l; c < pad; c += 32) Uw[r * pad + c] = c == r ? dg : 0.0f;
+      const float dg = __shfl_sync(IMN_FULL_MASK, root, r - n);
+#pragma unroll 3
+      for (int cl = l; cl < pad; cl += 32) Uw[r * pad + cl] = cl == r ? dg : 0.0f;
     }
-    for (int e = l; e < n * carry; e += 32) {
-      const int r = e / carry, q = e - r * carry;
-      X[r * rhs + q] = A[r * ldu + n + q];
-    }
+#pragma unroll 1
+    for (int q = 0; q < carry; ++q)
+      for (int r = l; r < n; r += 32) X[r * rhs + q] = A[r * ldu + n + q];
   } else {
     if (vec) {
-#pragma unroll 8
-      for (int r = vr; r < n; r += vrows)
-        if (c + 3 >= r && c < n) *reinterpret_cast<float4*>(A + r * ldu + c) = *reinterpret_cast<const float4*>(Uw + r * pad + c);
+      // six reads in flight, then their stores (one after the other: 10 k of the 20 k cycles of a second solve of 34-dof worlds)
+      constexpr int B = 6;
+#pragma unroll 1
+      for (int r0 = vr; r0 < n; r0 += B * vrows) {
+        float4 v[B];
+#pragma unroll
+        for (int j = 0; j < B; ++j) {
+          const int r = min(r0 + j * vrows, n - 1);
+          v[j] = *reinterpret_cast<const float4*>(Uw + r * pad + c);
+        }
+#pragma unroll
+        for (int j = 0; j < B; ++j) {
+          const int r = r0 + j * vrows;
+          if (r < n && c + 3 >= r && c < n) *reinterpret_cast<float4*>(A + r * ldu + c) = v[j];
+        }
+      }
     } else {
       for (int r = 0; r < n; ++r)
         for (int c = r + l; c < n; c += 32) A[r * ldu + c] = Uw[r * pad + c];
@@ -452,7 +495,7 @@ extern "C" int imn_blocked_dense_factor_solve(const ImnBlockedPlan* plan, const 
   }
   const int vec = (reinterpret_cast<uintptr_t>(U) & 15) == 0;  // pad is a multiple of 16 floats
   const cudaError_t e = imn::launch_chained(kernel, (nworld + per_cta - 1) / per_cta, 32 * imn::kDenseWarps, bytes,
-                                            (cudaStream_t)stream, plan->nv, plan->pad, plan->nM, plan->indices, plan->identity,
+                                            (cudaStream_t)stream, plan->nv, plan->pad, plan->nM, plan->indices, plan->places, plan->identity,
                                             M, M_ld, y, U, x, active, rhs_count, mode, carry, ldu, per_world, vec, nworld);
   if (e != cudaSuccess)
     return imn::set_error("imn_blocked_dense_factor_solve: launch failed: %s", cudaGetErrorString(e)),

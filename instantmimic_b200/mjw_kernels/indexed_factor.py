@@ -36,6 +36,7 @@ class BlockedDenseFactorSolveScratch:
     U: Any  # (nworld, pad, pad) factor workspace
     indices: Any  # (pad * pad,) block-major gather table; nM addresses the zero slot
     identity: Any  # (256,) ones on the padded diagonal of the last block
+    places: Any  # (nM,) row | column << 8 of every entry of M, as raw bytes
     struct: abi.ImnBlockedPlan
 
 
@@ -56,6 +57,14 @@ def dense_index_table(m: Any) -> np.ndarray:
             c = int(colind[e])
             table[k, c] = table[c, k] = e
     return table
+
+
+def entry_places(table: np.ndarray, nM: int) -> np.ndarray:
+    """(nM,) position row | column << 8, row <= column, of every CSR entry of M: ``table`` the other way round."""
+    places = np.zeros(nM, np.uint16)
+    rows, cols = np.nonzero(np.triu(table < nM))
+    places[table[rows, cols]] = rows | cols << 8
+    return places
 
 
 def block_major_layout(table: np.ndarray, pad: int, zero_index: int) -> np.ndarray:
@@ -92,16 +101,18 @@ def create_blocked_dense_factor_solve_scratch(
         return None
     pad = _round_up(nv, BLOCK_SIZE)
     nM = int(d.M.shape[1])
-    layout = block_major_layout(dense_index_table(m), pad, nM)
-    indices = torch.from_numpy(layout).to(device)
+    table = dense_index_table(m)
+    indices = torch.from_numpy(block_major_layout(table, pad, nM)).to(device)
+    # torch's uint16 has no arithmetic; the raw bytes do
+    places = torch.from_numpy(entry_places(table, nM).view(np.uint8)).to(device)
     identity = torch.from_numpy(pad_identity(nv, pad)).to(device)
     U = torch.zeros((nworld, pad, pad), dtype=torch.float32, device=device)
     st = abi.ImnBlockedPlan()
     st.nv, st.pad, st.nM = nv, pad, nM
-    st.indices, st.identity = addr(indices), addr(identity)
+    st.indices, st.identity, st.places = addr(indices), addr(identity), addr(places)
     return BlockedDenseFactorSolveScratch(
         nv=nv, pad=pad, block_size=BLOCK_SIZE, block_dim=BLOCK_DIM, U=U, indices=indices,
-        identity=identity, struct=st,
+        identity=identity, places=places, struct=st,
     )
 
 

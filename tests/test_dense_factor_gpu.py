@@ -32,3 +32,38 @@ def test_dense_factor_edges(oracle, cuda_device, nv, rhs, offset):
     np.testing.assert_array_equal(x.cpu().numpy(), want_x)
     np.testing.assert_array_equal(x2.cpu().numpy(), want_x)
     np.testing.assert_array_equal(U.cpu().numpy(), want_U)
+
+
+@pytest.mark.parametrize("places", [True, False])
+@pytest.mark.parametrize("nv,rhs", [(33, 1), (36, 28), (36, 29), (37, 3), (52, 2), (80, 1)])
+def test_last_block_and_entry_places(oracle, cuda_device, nv, rhs, places):
+    """Last blocks of one, four and five rows, with as many columns as the narrow form takes and one more; M's entries
+    laid out by their places and looked up position by position."""
+    import torch
+
+    worlds = 7
+    m, Mv, _, pad, layout, ident, y = _blocked_case(nv, worlds, rhs)
+    md = mjw_model.to_device(m, cuda_device)
+    dd = mjw_model.to_device(mjw_model.make_data(m, worlds, 4), cuda_device)
+    scratch = indexed_factor.create_blocked_dense_factor_solve_scratch(md, dd, cuda_device)
+    if not places:
+        scratch.struct.places = None
+    Mt, yt = torch.from_numpy(Mv).to(cuda_device), torch.from_numpy(y).to(cuda_device)
+    active = torch.ones(worlds, dtype=torch.int32, device=cuda_device)
+    active[3] = 0
+    x, x2, U = torch.zeros_like(yt), torch.zeros_like(yt), torch.full((worlds, pad, pad), 7.0, device=cuda_device)
+    indexed_factor.factor_multi_solve(scratch, Mt, yt, active, U, x, rhs)
+    indexed_factor.multi_solve(scratch, U, yt, active, x2, rhs)
+    want_x, want_U = oracle.blocked_dense_factor_solve(nv, pad, layout, ident, Mv, y)
+    want_x[3], want_U[3] = 0.0, 7.0
+    np.testing.assert_array_equal(x.cpu().numpy(), want_x)
+    np.testing.assert_array_equal(x2.cpu().numpy(), want_x)
+    np.testing.assert_array_equal(U.cpu().numpy(), want_U)
+
+
+def test_entry_places_are_the_index_table_the_other_way_round():
+    m = _blocked_case(35, 1, 1)[0]
+    table = indexed_factor.dense_index_table(m)
+    places = indexed_factor.entry_places(table, int(m.nM))
+    rows, cols = places & 0xFF, places >> 8
+    assert (rows <= cols).all() and np.array_equal(table[rows, cols], np.arange(m.nM))
