@@ -136,43 +136,88 @@ __device__ __forceinline__ Team<GW> make_team(int nworld) {
   return t;
 }
 
+// ---- everything on its way at once ----------------------------------------------------
+//
+// A stage is a few levels of short arithmetic; what took the time was reads that waited for one another: the
+// level's tables (position -> body -> parent, dofs, joints), one dependent read from global memory after the other in
+// every level, qvel inside them, and inputs fetched where they are needed.  A warp now sends for all of
+// its worlds' inputs and for the tables of the tree (six words per body and two per dof, in its own shared
+// memory: no block barrier) with asynchronous copies, waits once, and walks the levels in
+// shared memory.  @TREEFIG@
+__device__ __forceinline__ void async_word(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+}
+// a world's run of n floats by the lanes of its team
+template <int GW>
+__device__ __forceinline__ void async_run(float* dst, const float* src, int n, int sl) {
+#pragma unroll 4
+  for (int i = sl; i < n; i += GW) async_word(dst + i, src + i);
+}
+// The warp's copies of the tables; those that a stage does not send for stay unused.
+struct WarpTables {
+  int *bodies, *child_ptr, *child_ids, *parent, *dofadr, *dofnum, *offsets, *dof_body;
+};
+__host__ __device__ inline int table_words(int nbody, int nlevels, int nv) { return 6 * nbody + 1 + nlevels + 1 + nv; }
+// behind the worlds of the CTA (32 / GW per warp, `per_world` floats each), a warp's tables after the other's
+template <int GW>
+__device__ __forceinline__ int* table_space(const ImnBodyTree& T, float* smem, int per_world) {
+  return reinterpret_cast<int*>(smem + (size_t)kTreeWarps * (32 / GW) * per_world) +
+         (threadIdx.x >> 5) * table_words(T.nbody, T.nlevels, T.nv);
+}
+__device__ __forceinline__ WarpTables warp_tables(const ImnBodyTree& T, int* at) {
+  WarpTables t;
+  t.bodies = at, t.child_ids = t.bodies + T.nbody, t.parent = t.child_ids + T.nbody, t.dofadr = t.parent + T.nbody;
+  t.dofnum = t.dofadr + T.nbody, t.child_ptr = t.dofnum + T.nbody, t.offsets = t.child_ptr + T.nbody + 1;
+  t.dof_body = t.offsets + T.nlevels + 1;
+  return t;
+}
+__device__ __forceinline__ void send_words(int* dst, const int* src, int n) {
+#pragma unroll 1
+  for (int i = threadIdx.x & 31; i < n; i += 32) async_word(dst + i, src + i);
+}
+// what a sweep up reads (child_ptr has an entry per position and one behind; the leaves' children take one pointer each)
+__device__ __forceinline__ void send_sweep(const ImnBodyTree& T, const WarpTables& t) {
+  send_words(t.offsets, T.level_offsets, T.nlevels + 1);
+  send_words(t.bodies, T.level_bodies, T.nbody);
+  send_words(t.child_ptr, T.child_ptr, T.nbody + 1);
+  send_words(t.child_ids, T.child_ids, T.nbody - 1);
+}
+__device__ __forceinline__ void send_levels(const ImnBodyTree& T, const WarpTables& t) {
+  send_words(t.parent, T.body_parentid, T.nbody);
+  send_words(t.dofadr, T.body_dofadr, T.nbody);
+  send_words(t.dofnum, T.body_dofnum, T.nbody);
+}
+
 // Bottom-up sweep over the team's values (nbody x C floats in shared memory): the
 // parents of a level take their children of the next level, in level-list order
 // (tree_fusion.py:94-112).  child_ptr is indexed by the parent's position in the level
-// list.
-template <int GW>
-__device__ __forceinline__ void sweep_up(const ImnBodyTree& T, float* v, int C, bool skip_root_parent, int sl) {
+// list.  FIXED: the number of components where it is known (a division by it otherwise).
+template <int GW, int FIXED>
+__device__ __forceinline__ void sweep_up(const WarpTables& t, int nlevels, float* v, int components, bool skip_root_parent, int sl) {
+  const int C = FIXED ? FIXED : components;
 #pragma unroll 1
-  for (int level = T.nlevels - 1; level > 0; --level) {
-    const int pstart = T.level_offsets[level - 1];
-    const int pcount = T.level_offsets[level] - pstart;
+  for (int level = nlevels - 1; level > 0; --level) {
+    const int pstart = t.offsets[level - 1];
+    const int pcount = t.offsets[level] - pstart;
 #pragma unroll 1
     for (int entry = sl; entry < pcount * C; entry += GW) {
       const int pos = pstart + entry / C, comp = entry - (entry / C) * C;
-      const int parent = T.level_bodies[pos];
+      const int parent = t.bodies[pos];
       if (skip_root_parent && parent == 0) continue;
       float value = v[parent * C + comp];
-      const int cend = T.child_ptr[pos + 1];
+      const int cend = t.child_ptr[pos + 1];
 #pragma unroll 1
-      for (int k = T.child_ptr[pos]; k < cend; ++k) value = value + v[T.child_ids[k] * C + comp];
+      for (int k = t.child_ptr[pos]; k < cend; ++k) value = value + v[t.child_ids[k] * C + comp];
       v[parent * C + comp] = value;
     }
     __syncwarp();
   }
 }
 
-// Per-world runs are a few hundred floats: four loads in flight per lane.
-template <int GW>
-__device__ __forceinline__ void copy_in(float* dst, const float* __restrict__ src, int n, int sl) {
-  int i = sl;
-#pragma unroll 1
-  for (; i + 3 * GW < n; i += 4 * GW) {
-    const float a = src[i], b = src[i + GW], c = src[i + 2 * GW], d = src[i + 3 * GW];
-    dst[i] = a, dst[i + GW] = b, dst[i + 2 * GW] = c, dst[i + 3 * GW] = d;
-  }
-#pragma unroll 1
-  for (; i < n; i += GW) dst[i] = src[i];
-}
 template <int GW>
 __device__ __forceinline__ void copy_out(float* __restrict__ dst, const float* src, int n, int sl, bool live) {
   if (!live) return;
@@ -188,12 +233,17 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   chain_wait();
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
-  const int n = T.nbody * C;
-  float* v = tree_smem + (size_t)t.slot * ((n + 3) & ~3);
+  const int n = T.nbody * C, per_world = (n + 3) & ~3;
+  float* v = tree_smem + (size_t)t.slot * per_world;
+  const WarpTables tab = warp_tables(T, table_space<GW>(T, tree_smem, per_world));
   float* g = values + (size_t)t.w * world_ld;
-  copy_in<GW>(v, g, n, t.sl);
-  __syncwarp();
-  sweep_up<GW>(T, v, C, skip_root_parent != 0, t.sl);
+  async_run<GW>(v, g, n, t.sl);
+  send_sweep(T, tab);
+  async_wait();
+  if (C == 3)
+    sweep_up<GW, 3>(tab, T.nlevels, v, C, skip_root_parent != 0, t.sl);
+  else
+    sweep_up<GW, 0>(tab, T.nlevels, v, C, skip_root_parent != 0, t.sl);
   copy_out<GW>(g, v, n, t.sl, t.live);
 }
 
@@ -210,14 +260,17 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int sl = t.sl, w = t.w;
-  const int nb10 = T.nbody * 10, nv6 = T.nv * 6;
-  float* c = tree_smem + (size_t)t.slot * (((nb10 + 3) & ~3) + 2 * ((nv6 + 3) & ~3));
+  const int nb10 = T.nbody * 10, nv6 = T.nv * 6, per_world = ((nb10 + 3) & ~3) + 2 * ((nv6 + 3) & ~3);
+  float* c = tree_smem + (size_t)t.slot * per_world;
   float* dof = c + ((nb10 + 3) & ~3);
   float* bufs = dof + ((nv6 + 3) & ~3);
-  copy_in<GW>(c, cinert + (size_t)w * nb10, nb10, sl);
-  copy_in<GW>(dof, cdof + (size_t)w * nv6, nv6, sl);
-  __syncwarp();
-  sweep_up<GW>(T, c, 10, true, sl);
+  const WarpTables tab = warp_tables(T, table_space<GW>(T, tree_smem, per_world));
+  async_run<GW>(c, cinert + (size_t)w * nb10, nb10, sl);
+  async_run<GW>(dof, cdof + (size_t)w * nv6, nv6, sl);
+  send_sweep(T, tab);
+  send_words(tab.dof_body, T.dof_bodyid, T.nv);
+  async_wait();
+  sweep_up<GW, 10>(tab, T.nlevels, c, 10, true, sl);
   copy_out<GW>(crb + (size_t)w * nb10, c, nb10, sl, t.live);
   const float* arm = T.dof_armature + (size_t)(w % T.n_armature) * T.nv;
   float* Mw = M + (size_t)w * M_ld;
@@ -225,17 +278,31 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   // cdof_j . buf_i -- the ancestor walk of the reference flattened over M's CSR, so that
   // every lane is busy and consecutive lanes store consecutive entries
 #pragma unroll 1
-  for (int i = sl; i < T.nv; i += GW) st6(bufs + 6 * i, inert_vec(c + 10 * T.dof_bodyid[i], ld6(dof + 6 * i)));
+  for (int i = sl; i < T.nv; i += GW) st6(bufs + 6 * i, inert_vec(c + 10 * tab.dof_body[i], ld6(dof + 6 * i)));
   __syncwarp();
-#pragma unroll 2
-  for (int e = sl; e < T.nM; e += GW) {
-    const int i = T.M_rowidx[e], j = T.M_colind[e];
-    float v = dot6(ld6(dof + 6 * j), ld6(bufs + 6 * i));
-    if (i == j) v = arm[i] + v;
-    if (t.live) Mw[e] = v;
+  constexpr int B = 4;  // entries whose indices are read together
+#pragma unroll 1
+  for (int e0 = sl; e0 < T.nM; e0 += B * GW) {
+    int i[B], j[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      const int e = min(e0 + k * GW, T.nM - 1);
+      i[k] = __ldg(T.M_rowidx + e), j[k] = __ldg(T.M_colind + e);
+    }
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      const int e = e0 + k * GW;
+      if (e >= T.nM) break;
+      float v = dot6(ld6(dof + 6 * j[k]), ld6(bufs + 6 * i[k]));
+      if (i[k] == j[k]) v = arm[i[k]] + v;
+      if (t.live) Mw[e] = v;
+    }
   }
 }
 
+__host__ __device__ inline int rne_floats(int nbody, int nv) {
+  return 2 * ((nbody * 6 + 3) & ~3) + 2 * ((nv * 6 + 3) & ~3) + ((nbody * 10 + 3) & ~3) + ((nv + 3) & ~3);
+}
 // rne without accelerations (tree_fusion.py:209-222): cacc down the tree from
 // -gravity, per-body forces cinert cacc + cvel x* (cinert cvel), summed up the tree,
 // projected on the dofs.
@@ -250,26 +317,36 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int sl = t.sl, w = t.w;
-  const int nb6 = T.nbody * 6, nv6 = T.nv * 6, nb6p = (nb6 + 3) & ~3, nv6p = (nv6 + 3) & ~3;
-  float* cacc = tree_smem + (size_t)t.slot * (2 * nb6p + nv6p);
-  float* cfrc = cacc + nb6p;
-  float* dd = cfrc + nb6p;  // cdof_dot, then cdof
-  copy_in<GW>(dd, cdof_dot + (size_t)w * nv6, nv6, sl);
+  const int nb6 = T.nbody * 6, nv6 = T.nv * 6, nb6p = (nb6 + 3) & ~3, nv6p = (nv6 + 3) & ~3, nvp = (T.nv + 3) & ~3;
+  const int nb10 = T.nbody * 10, nb10p = (nb10 + 3) & ~3, per_world = rne_floats(T.nbody, T.nv);
+  float* cacc = tree_smem + (size_t)t.slot * per_world;
+  float* cfrc = cacc + nb6p;  // cvel until the body's force replaces it
+  float* dd = cfrc + nb6p;    // cdof_dot
+  float* dof = dd + nv6p;
+  float* inert = dof + nv6p;
+  float* qv = inert + nb10p;
+  const WarpTables tab = warp_tables(T, table_space<GW>(T, tree_smem, per_world));
+  async_run<GW>(dd, cdof_dot + (size_t)w * nv6, nv6, sl);
+  async_run<GW>(qv, qvel + (size_t)w * qvel_ld, T.nv, sl);
+  async_run<GW>(inert, cinert + (size_t)w * nb10, nb10, sl);
+  async_run<GW>(cfrc, cvel + (size_t)w * nb6, nb6, sl);
+  async_run<GW>(dof, cdof + (size_t)w * nv6, nv6, sl);
+  send_sweep(T, tab);
+  send_levels(T, tab);
+  send_words(tab.dof_body, T.dof_bodyid, T.nv);
   if (sl < 6) {
     const float* g = T.gravity + 3 * (size_t)(w % T.n_gravity);
     cacc[sl] = (sl < 3 || !T.gravity_enabled) ? 0.0f : -g[sl - 3];
-    cfrc[sl] = 0.0f;
   }
-  __syncwarp();
-  const float* qv = qvel + (size_t)w * qvel_ld;
+  async_wait();
 #pragma unroll 1
   for (int level = 1; level < T.nlevels; ++level) {
-    const int end = T.level_offsets[level + 1];
+    const int end = tab.offsets[level + 1];
 #pragma unroll 1
-    for (int pos = T.level_offsets[level] + sl; pos < end; pos += GW) {
-      const int b = T.level_bodies[pos];
-      Sp6 a = ld6(cacc + 6 * T.body_parentid[b]);
-      const int d0 = T.body_dofadr[b], d1 = d0 + T.body_dofnum[b];
+    for (int pos = tab.offsets[level] + sl; pos < end; pos += GW) {
+      const int b = tab.bodies[pos];
+      Sp6 a = ld6(cacc + 6 * tab.parent[b]);
+      const int d0 = tab.dofadr[b], d1 = d0 + tab.dofnum[b];
 #pragma unroll 1
       for (int dofid = d0; dofid < d1; ++dofid) a = axpy6(a, ld6(dd + 6 * dofid), qv[dofid]);
       st6(cacc + 6 * b, a);
@@ -278,28 +355,31 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   }
   copy_out<GW>(cacc_out + (size_t)w * nb6, cacc, nb6, sl, t.live);
 #pragma unroll 1
-  for (int b = 1 + sl; b < T.nbody; b += GW) {
-    const float* I = cinert + ((size_t)w * T.nbody + b) * 10;
-    float in[10];
-#pragma unroll
-    for (int k = 0; k < 10; ++k) in[k] = I[k];
-    const Sp6 v = ld6(cvel + ((size_t)w * T.nbody + b) * 6);
-    const Sp6 f = inert_vec(in, ld6(cacc + 6 * b));
-    const Sp6 x = motion_cross_force(v, inert_vec(in, v));
+  for (int b = sl; b < T.nbody; b += GW) {
     Sp6 r;
+    if (b == 0) {
 #pragma unroll
-    for (int k = 0; k < 6; ++k) r.v[k] = f.v[k] + x.v[k];
+      for (int k = 0; k < 6; ++k) r.v[k] = 0.0f;
+    } else {
+      float in[10];
+#pragma unroll
+      for (int k = 0; k < 10; ++k) in[k] = inert[10 * b + k];
+      const Sp6 v = ld6(cfrc + 6 * b);
+      const Sp6 f = inert_vec(in, ld6(cacc + 6 * b));
+      const Sp6 x = motion_cross_force(v, inert_vec(in, v));
+#pragma unroll
+      for (int k = 0; k < 6; ++k) r.v[k] = f.v[k] + x.v[k];
+    }
     st6(cfrc + 6 * b, r);
   }
   __syncwarp();
-  copy_in<GW>(dd, cdof + (size_t)w * nv6, nv6, sl);  // cdof_dot is no longer needed
-  sweep_up<GW>(T, cfrc, 6, false, sl);
+  sweep_up<GW, 6>(tab, T.nlevels, cfrc, 6, false, sl);
   __syncwarp();
   copy_out<GW>(cfrc_out + (size_t)w * nb6, cfrc, nb6, sl, t.live);
   float* bias = qfrc_bias + (size_t)w * bias_ld;
 #pragma unroll 1
   for (int i = sl; i < T.nv; i += GW) {
-    const float e = dot6(ld6(dd + 6 * i), ld6(cfrc + 6 * T.dof_bodyid[i]));
+    const float e = dot6(ld6(dof + 6 * i), ld6(cfrc + 6 * tab.dof_body[i]));
     if (t.live) bias[i] = e;
   }
 }
@@ -318,30 +398,47 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int sl = t.sl, w = t.w;
-  const int nb6 = T.nbody * 6, nv6 = T.nv * 6, nb6p = (nb6 + 3) & ~3, nv6p = (nv6 + 3) & ~3;
-  float* cvel = tree_smem + (size_t)t.slot * (nb6p + 2 * nv6p);
+  const int nb6 = T.nbody * 6, nv6 = T.nv * 6, nb6p = (nb6 + 3) & ~3, nv6p = (nv6 + 3) & ~3, nvp = (T.nv + 3) & ~3;
+  const int per_world = nb6p + 2 * nv6p + nvp;
+  float* cvel = tree_smem + (size_t)t.slot * per_world;
   float* dof = cvel + nb6p;
   float* dot = dof + nv6p;
-  copy_in<GW>(dof, cdof + (size_t)w * nv6, nv6, sl);
-  __syncwarp();
-  const float* qv = qvel + (size_t)w * qvel_ld;
+  float* qv = dot + nv6p;
+  const WarpTables tab = warp_tables(T, table_space<GW>(T, tree_smem, per_world));
+  int* const jntadr = tab.child_ids;  // a walk down reads no children
+  int* const jntnum = tab.child_ptr;
+  int* const kind = tab.dofnum;  // of the body's first joint
+  async_run<GW>(dof, cdof + (size_t)w * nv6, nv6, sl);
+  async_run<GW>(qv, qvel + (size_t)w * qvel_ld, T.nv, sl);
+  send_words(tab.offsets, T.level_offsets, T.nlevels + 1);
+  send_words(tab.bodies, T.level_bodies, T.nbody);
+  send_words(tab.parent, T.body_parentid, T.nbody);
+  send_words(tab.dofadr, T.body_dofadr, T.nbody);
+  send_words(jntnum, T.body_jntnum, T.nbody);
+#pragma unroll 1
+  for (int b = threadIdx.x & 31; b < T.nbody; b += 32) {
+    const int adr = T.body_jntadr[b];
+    jntadr[b] = adr;
+    kind[b] = T.body_jntnum[b] > 0 ? T.jnt_type[adr] : 0;
+  }
+  async_wait();
 #pragma unroll 1
   for (int level = 0; level < T.nlevels; ++level) {
-    const int end = T.level_offsets[level + 1];
+    const int end = tab.offsets[level + 1];
 #pragma unroll 1
-    for (int pos = T.level_offsets[level] + sl; pos < end; pos += GW) {
-      const int b = T.level_bodies[pos];
+    for (int pos = tab.offsets[level] + sl; pos < end; pos += GW) {
+      const int b = tab.bodies[pos];
       Sp6 v;
       if (b == 0) {
 #pragma unroll
         for (int k = 0; k < 6; ++k) v.v[k] = 0.0f;
       } else {
-        v = ld6(cvel + 6 * T.body_parentid[b]);
-        int dofid = T.body_dofadr[b];
-        const int j1 = T.body_jntadr[b] + T.body_jntnum[b];
+        v = ld6(cvel + 6 * tab.parent[b]);
+        int dofid = tab.dofadr[b], type = kind[b];
+        const int j0 = jntadr[b], j1 = j0 + jntnum[b];
 #pragma unroll 1
-        for (int j = T.body_jntadr[b]; j < j1; ++j) {
-          const int type = T.jnt_type[j];
+        for (int j = j0; j < j1; ++j) {
+          if (j > j0) type = T.jnt_type[j];
           if (type == IMN_JNT_FREE) {
             Sp6 zero;
 #pragma unroll
@@ -413,12 +510,12 @@ static int team_lanes(const ImnBodyTree* T, int at_least = 8) {
 }
 
 template <typename... Args>
-static int launch_tree(const char* who, void (*kernel)(Args...), int gw, size_t floats_per_world, int nworld,
+static int launch_tree(const char* who, const ImnBodyTree* T, void (*kernel)(Args...), int gw, size_t floats_per_world, int nworld,
                        void* stream, Args... args) {
   if (nworld < 0) return set_error("%s: negative world count", who), IMN_ERR_SHAPE;
   if (nworld == 0) return IMN_OK;
   const int per_cta = kTreeWarps * (32 / gw);
-  const size_t bytes = floats_per_world * 4 * per_cta;
+  const size_t bytes = floats_per_world * 4 * per_cta + 4 * (size_t)kTreeWarps * table_words(T->nbody, T->nlevels, T->nv);
   if (bytes > 227 * 1024)
     return set_error("%s: %zu bytes of shared memory per block exceed the 227 KB of an SM", who, bytes), IMN_ERR_LIMIT;
   {
@@ -451,9 +548,9 @@ static size_t oddz(size_t n) { return n | 1; }
 
 // KERNEL<8 | 16 | 32> by the tree's team width
 #define IMN_TEAM_LAUNCH(LANES, KERNEL, FLOATS, NWORLD, STREAM, ...)                                \
-  ((LANES) == 8    ? imn::launch_tree(who, KERNEL<8>, 8, FLOATS, NWORLD, STREAM, __VA_ARGS__)   \
-   : (LANES) == 16 ? imn::launch_tree(who, KERNEL<16>, 16, FLOATS, NWORLD, STREAM, __VA_ARGS__) \
-                   : imn::launch_tree(who, KERNEL<32>, 32, FLOATS, NWORLD, STREAM, __VA_ARGS__))
+  ((LANES) == 8    ? imn::launch_tree(who, T, KERNEL<8>, 8, FLOATS, NWORLD, STREAM, __VA_ARGS__)   \
+   : (LANES) == 16 ? imn::launch_tree(who, T, KERNEL<16>, 16, FLOATS, NWORLD, STREAM, __VA_ARGS__) \
+                   : imn::launch_tree(who, T, KERNEL<32>, 32, FLOATS, NWORLD, STREAM, __VA_ARGS__))
 
 }  // namespace imn
 
@@ -494,7 +591,7 @@ extern "C" int imn_rne(const ImnBodyTree* T, const float* cinert, const float* c
     return imn::set_error("%s: NULL array", who), IMN_ERR_NULL;
   if (T->n_gravity <= 0 || qvel_ld < T->nv || bias_ld < T->nv)
     return imn::set_error("%s: bad gravity count or stride", who), IMN_ERR_SHAPE;
-  return IMN_TEAM_LAUNCH(imn::team_lanes(T, 16), imn::rne_kernel, 2 * imn::up4z((size_t)T->nbody * 6) + imn::up4z((size_t)T->nv * 6), nworld,
+  return IMN_TEAM_LAUNCH(imn::team_lanes(T, 16), imn::rne_kernel, (size_t)imn::rne_floats(T->nbody, T->nv), nworld,
                          stream, *T, cinert, cvel, cdof, cdof_dot, qvel, qvel_ld, cacc, cfrc_int, qfrc_bias, bias_ld,
                          (int)nworld);
 }
@@ -514,6 +611,6 @@ extern "C" int imn_com_vel(const ImnBodyTree* T, const float* qvel, int64_t qvel
       return imn::launch_tile(who, imn::com_vel_tile_kernel, bytes, nworld, stream, *T, qvel, qvel_ld, cdof, cvel,
                               cdof_dot, (int)nworld);
   }
-  return IMN_TEAM_LAUNCH(imn::team_lanes(T), imn::com_vel_kernel, imn::up4z((size_t)T->nbody * 6) + 2 * imn::up4z((size_t)T->nv * 6),
+  return IMN_TEAM_LAUNCH(imn::team_lanes(T), imn::com_vel_kernel, imn::up4z((size_t)T->nbody * 6) + 2 * imn::up4z((size_t)T->nv * 6) + imn::up4z(T->nv),
                          nworld, stream, *T, qvel, qvel_ld, cdof, cvel, cdof_dot, (int)nworld);
 }
