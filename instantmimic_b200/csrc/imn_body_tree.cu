@@ -151,11 +151,19 @@ __device__ __forceinline__ void async_wait() {
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncwarp();
 }
-// a world's run of n floats by the lanes of its team
+// A world's run of n floats by the lanes of its team: 16 bytes a piece where the runs are whole pieces on 16-byte
+// boundaries (`dst` always is), four bytes elsewhere.
 template <int GW>
 __device__ __forceinline__ void async_run(float* dst, const float* src, int n, int sl) {
+  if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll 2
+    for (int i = 4 * sl; i < n; i += 4 * GW)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + i)), "l"(src + i)
+                   : "memory");
+  } else {
 #pragma unroll 4
-  for (int i = sl; i < n; i += GW) async_word(dst + i, src + i);
+    for (int i = sl; i < n; i += GW) async_word(dst + i, src + i);
+  }
 }
 // The warp's copies of the tables; those that a stage does not send for stay unused.
 struct WarpTables {
@@ -221,6 +229,11 @@ __device__ __forceinline__ void sweep_up(const WarpTables& t, int nlevels, float
 template <int GW>
 __device__ __forceinline__ void copy_out(float* __restrict__ dst, const float* src, int n, int sl, bool live) {
   if (!live) return;
+  if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll 2
+    for (int i = 4 * sl; i < n; i += 4 * GW) *reinterpret_cast<float4*>(dst + i) = *reinterpret_cast<const float4*>(src + i);
+    return;
+  }
 #pragma unroll 4
   for (int i = sl; i < n; i += GW) dst[i] = src[i];
 }
@@ -280,7 +293,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
 #pragma unroll 1
   for (int i = sl; i < T.nv; i += GW) st6(bufs + 6 * i, inert_vec(c + 10 * tab.dof_body[i], ld6(dof + 6 * i)));
   __syncwarp();
-  constexpr int B = 4;  // entries whose indices are read together
+  constexpr int B = 2;  // entries whose indices are read together (four: 8192 34-dof worlds 13.5 -> 15.8 us, others equal)
 #pragma unroll 1
   for (int e0 = sl; e0 < T.nM; e0 += B * GW) {
     int i[B], j[B];
@@ -474,11 +487,6 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   copy_out<GW>(cdof_dot_out + (size_t)w * nv6, dot, nv6, sl, t.live);
 }
 
-}  // namespace imn
-
-#include "imn_body_tree_tile.cuh"
-
-namespace imn {
 
 static int check_tree(const ImnBodyTree* T, const char* who, bool need_dofs) {
   if (!T) return set_error("%s: NULL tree", who), IMN_ERR_NULL;
@@ -529,22 +537,6 @@ static int launch_tree(const char* who, const ImnBodyTree* T, void (*kernel)(Arg
 }
 
 static size_t up4z(size_t n) { return (n + 3) & ~(size_t)3; }
-
-// The lane-per-world kernels take over from 4096 worlds on (128 blocks of 32 worlds: below
-// that the teams fill the GPU better) when two blocks' rows fit an SM's shared memory.
-static bool use_tiles(int nworld, size_t bytes) { return nworld >= 4096 && bytes <= 113 * 1024; }
-
-template <typename... Args>
-static int launch_tile(const char* who, void (*kernel)(Args...), size_t bytes, int nworld, void* stream, Args... args) {
-  if (bytes > 48 * 1024) {
-    const cudaError_t e = allow_shared(kernel, bytes, true);
-    if (e != cudaSuccess) return set_error("%s: cudaFuncSetAttribute: %s", who, cudaGetErrorString(e)), IMN_ERR_LAUNCH;
-  }
-  const cudaError_t e = launch_chained(kernel, (nworld + 31) / 32, 32 * kTileWarps, bytes, (cudaStream_t)stream, args...);
-  if (e != cudaSuccess) return set_error("%s: launch failed: %s", who, cudaGetErrorString(e)), IMN_ERR_LAUNCH;
-  return IMN_OK;
-}
-static size_t oddz(size_t n) { return n | 1; }
 
 // KERNEL<8 | 16 | 32> by the tree's team width
 #define IMN_TEAM_LAUNCH(LANES, KERNEL, FLOATS, NWORLD, STREAM, ...)                                \
@@ -604,13 +596,6 @@ extern "C" int imn_com_vel(const ImnBodyTree* T, const float* qvel, int64_t qvel
   if (!qvel || !cdof || !cvel || !cdof_dot || !T->body_jntadr || !T->body_jntnum || !T->jnt_type)
     return imn::set_error("%s: NULL array", who), IMN_ERR_NULL;
   if (qvel_ld < T->nv) return imn::set_error("%s: qvel stride < nv", who), IMN_ERR_SHAPE;
-  {
-    const size_t bytes =
-        128 * (imn::oddz((size_t)T->nbody * 6) + 2 * imn::oddz((size_t)T->nv * 6) + imn::oddz(T->nv));
-    if (imn::use_tiles(nworld, bytes))
-      return imn::launch_tile(who, imn::com_vel_tile_kernel, bytes, nworld, stream, *T, qvel, qvel_ld, cdof, cvel,
-                              cdof_dot, (int)nworld);
-  }
   return IMN_TEAM_LAUNCH(imn::team_lanes(T), imn::com_vel_kernel, imn::up4z((size_t)T->nbody * 6) + 2 * imn::up4z((size_t)T->nv * 6) + imn::up4z(T->nv),
                          nworld, stream, *T, qvel, qvel_ld, cdof, cvel, cdof_dot, (int)nworld);
 }
