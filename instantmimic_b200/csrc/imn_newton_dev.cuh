@@ -240,6 +240,7 @@ __device__ __forceinline__ void ls_sum(float (&v)[N], int bd, int lane) {
       }
     }
   };
+  const float zero = bd == 64 ? 0.0f : -0.0f;  // x + -0 is x
   fold(a, v, N, 16);
   fold(b, a, N1, 8);
   fold(c, b, N2, 4);
@@ -250,7 +251,7 @@ __device__ __forceinline__ void ls_sum(float (&v)[N], int bd, int lane) {
     // value k went up at step s when its index at that step was odd
     const int src = ((k & 1) ? 16 : 0) | ((k & 2) ? 8 : 0) | ((k & 4) ? 4 : 0) | ((k & 8) ? 2 : 0);
     v[k] = __shfl_sync(IMN_FULL_MASK, e, src);
-    if (bd == 64) v[k] = v[k] + 0.0f;
+    v[k] = v[k] + zero;
   }
 }
 

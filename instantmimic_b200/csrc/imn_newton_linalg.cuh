@@ -331,7 +331,10 @@ __device__ __forceinline__ void full_gradient(const World& s, int nfr) {
   const bool h0 = i0 < nv && (!TEAM || part == 0), h1 = i1 < nv && (!TEAM || part == 1),
              h2 = i2 < nv && (!TEAM || part == (parts > 2 ? 2 : 0));
   if (TEAM && 32 * part >= nv) nfr = 0;
-  constexpr int B = JRES ? 4 : 8;
+  // rows in flight: reads of a streamed J come from L2, which a team alone on its warps has to cover itself; where the
+  // other worlds do, the shorter code counts (eight -> four: 56 dofs, 4096 worlds 1057 -> 1048 us, 35 dofs x 250 rows,
+  // 16384 worlds 2152 -> 2112; in teams 64 dofs x 512 rows 3711 -> 3933, 16 worlds of 56 dofs 226 -> 236)
+  constexpr int B = !JRES && TEAM ? 8 : 4;
   const float* J = (JRES ? s.Jsm : s.Jg) + lane;
 #pragma unroll 1
   for (int a = 0; a < nfr; a += B) {
@@ -471,8 +474,10 @@ __device__ __noinline__ void count_violations(bool first, const float* Jw, int l
 template <bool JRES, bool J16, bool TSM, bool TEAM>
 __device__ __forceinline__ void hessian_sparse(const World& s, int count, bool first, bool outside, const ImnSparsePlan& SP) {
   const int lane = s.lane, nv = s.nv, nfac = SP.nfac;
-  // slots a lane sums at a time: few in a team, whose warps take turns at the slots
-  constexpr int Q = TEAM ? 5 : JRES ? 10 : 12;
+  // slots a lane sums at a time: few in a team, whose warps take turns at the slots, and beside a streamed J, where the
+  // shorter code counts for more than the second look at a row (twelve -> six: 56 dofs, 4096 worlds 1067 -> 1057 us, 35
+  // dofs x 250 rows, 16384 worlds 2183 -> 2152; ten -> five with J resident: 34 dofs, 8192 worlds 511 -> 517)
+  constexpr int Q = TEAM ? 5 : JRES ? 10 : 6;
   const int part = team_part<TEAM>(s), parts = team_parts<TEAM>(s);
   const int step = JRES ? max(count, 1) : 32 * parts;
   // a list without rows still has to place M (first call)
