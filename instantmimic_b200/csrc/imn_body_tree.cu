@@ -126,7 +126,7 @@ struct Team {
 template <int GW>
 __device__ __forceinline__ Team<GW> make_team(int nworld) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per = 32 / GW;
-  const int first = (blockIdx.x * kTreeWarps + warp) * per, sub = lane / GW;
+  const int first = (blockIdx.x * (blockDim.x >> 5) + warp) * per, sub = lane / GW;
   Team<GW> t;
   t.sl = lane - sub * GW;
   t.live = first + sub < nworld;
@@ -173,7 +173,7 @@ __host__ __device__ inline int table_words(int nbody, int nlevels, int nv) { ret
 // behind the worlds of the CTA (32 / GW per warp, `per_world` floats each), a warp's tables after the other's
 template <int GW>
 __device__ __forceinline__ int* table_space(const ImnBodyTree& T, float* smem, int per_world) {
-  return reinterpret_cast<int*>(smem + (size_t)kTreeWarps * (32 / GW) * per_world) +
+  return reinterpret_cast<int*>(smem + (size_t)(blockDim.x >> 5) * (32 / GW) * per_world) +
          (threadIdx.x >> 5) * table_words(T.nbody, T.nlevels, T.nv);
 }
 __device__ __forceinline__ WarpTables warp_tables(const ImnBodyTree& T, int* at) {
@@ -504,7 +504,8 @@ static int check_tree(const ImnBodyTree* T, const char* who, bool need_dofs) {
 // Lanes per world: the tree's team_lanes when it is 8, 16 or 32 (the host mirror sets the
 // smallest that covers the widest level), else a whole warp.
 // Per kernel the width is raised to what was measured fastest on a B200 (65536 worlds,
-// 14-body / 34-dof and 24-body / 56-dof humanoids, widths 8 / 16 / 32 in us):
+// 14-body / 34-dof and 24-body / 56-dof humanoids, widths 8 / 16 / 32 in us, when every level still read its tables
+// from global memory):
 //   tree sum, 3 components   19 / 25 / 41     29 / 39 / 64    -> the tree's width
 //   com_vel                  64 / 70 / 111   132 / 121 / 163  -> the tree's width
 //   rne                      99 / 74 / 113   189 / 139 / 159  -> at least 16
@@ -522,8 +523,12 @@ static int launch_tree(const char* who, const ImnBodyTree* T, void (*kernel)(Arg
                        void* stream, Args... args) {
   if (nworld < 0) return set_error("%s: negative world count", who), IMN_ERR_SHAPE;
   if (nworld == 0) return IMN_OK;
-  const int per_cta = kTreeWarps * (32 / gw);
-  const size_t bytes = floats_per_world * 4 * per_cta + 4 * (size_t)kTreeWarps * table_words(T->nbody, T->nlevels, T->nv);
+  // four warps a block, fewer for trees of hundreds of bodies, whose worlds would not fit
+  int warps = kTreeWarps;
+  const size_t warp_bytes = 4 * (floats_per_world * (32 / gw) + table_words(T->nbody, T->nlevels, T->nv));
+  while (warps > 1 && warps * warp_bytes > 227 * 1024) warps /= 2;
+  const int per_cta = warps * (32 / gw);
+  const size_t bytes = warps * warp_bytes;
   if (bytes > 227 * 1024)
     return set_error("%s: %zu bytes of shared memory per block exceed the 227 KB of an SM", who, bytes), IMN_ERR_LIMIT;
   {
@@ -531,7 +536,7 @@ static int launch_tree(const char* who, const ImnBodyTree* T, void (*kernel)(Arg
     if (e != cudaSuccess) return set_error("%s: cudaFuncSetAttribute: %s", who, cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   }
   const cudaError_t e =
-      launch_chained(kernel, (nworld + per_cta - 1) / per_cta, 32 * kTreeWarps, bytes, (cudaStream_t)stream, args...);
+      launch_chained(kernel, (nworld + per_cta - 1) / per_cta, 32 * warps, bytes, (cudaStream_t)stream, args...);
   if (e != cudaSuccess) return set_error("%s: launch failed: %s", who, cudaGetErrorString(e)), IMN_ERR_LAUNCH;
   return IMN_OK;
 }

@@ -331,6 +331,32 @@ def test_cuda_smooth_stages_bit_exact(name, nworld, team):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nv,team", [(400, 16), (700, 16), (700, 32)])
+def test_cuda_smooth_stages_of_trees_of_hundreds_of_bodies(nv, team):
+    """Four warps' worlds do not fit a block's shared memory: blocks of two and of one warp."""
+    from dataclasses import replace
+
+    from instantmimic_b200.mjw_model import make_data, put_model
+
+    parent, body = synthetic.chain_tree(nv)
+    m = put_model(parent, body_of_dof=body)
+    d = make_data(m, 7, 1)
+    synthetic.add_smooth_state(m, d, seed=3)
+    scratch = tree_fusion.create_tree_reduction_scratch(m, deterministic=True)
+    md, dd = mjw_model.to_device(m, _device()), mjw_model.to_device(d, _device())
+    sd = replace(tree_fusion.create_tree_reduction_scratch(md, deterministic=True), team_lanes=team)
+    for stage in (velocity_fusion.com_vel, tree_fusion.crb, tree_fusion.rne, tree_fusion.subtree_com_accumulate):
+        stage(md, dd, sd)
+    oracle.com_vel(m, d, scratch)
+    oracle.crb(m, d, scratch)
+    oracle.rne(m, d, scratch)
+    oracle.body_tree_accumulate(m, scratch, d.subtree_com, 3, False)
+    got = mjw_model.to_host(dd)
+    for field in ("cvel", "cdof_dot", "crb", "cacc", "cfrc_int", "qfrc_bias", "subtree_com"):
+        np.testing.assert_array_equal(getattr(got, field), getattr(d, field), err_msg=field)
+
+
+@pytest.mark.gpu
 def test_cuda_tree_entry_points_check_their_arguments():
     import torch
 
