@@ -37,10 +37,10 @@ namespace imn {
 
 // Phase timers, compiled only into the profiling build (-DIMN_PROFILE).
 #ifdef IMN_PROFILE
-__device__ unsigned long long g_prof[16];
-#define PROF_DECL long long prof_t = clock64(); long long prof_acc[16] = {0}; s.prof_acc = prof_acc; s.prof_t = &prof_t
+__device__ unsigned long long g_prof[24];
+#define PROF_DECL long long prof_t = clock64(); long long prof_acc[24] = {0}; s.prof_acc = prof_acc; s.prof_t = &prof_t
 #define PROF(k) do { const long long t_ = clock64(); prof_acc[k] += t_ - prof_t; prof_t = t_; } while (0)
-#define PROF_FLUSH do { if (tid == 0) for (int k_ = 0; k_ < 16; ++k_) atomicAdd(&g_prof[k_], (unsigned long long)prof_acc[k_]); } while (0)
+#define PROF_FLUSH do { if (tid == 0) for (int k_ = 0; k_ < 24; ++k_) atomicAdd(&g_prof[k_], (unsigned long long)prof_acc[k_]); } while (0)
 #else
 #define PROF_DECL
 #define PROF(k)
@@ -850,9 +850,9 @@ static int plan_launch(const ImnModel* m, const ImnData* d, const ImnSparsePlan*
 
 #ifdef IMN_PROFILE
 extern "C" int imn_debug_profile(unsigned long long* out, int reset) {
-  cudaMemcpyFromSymbol(out, imn::g_prof, sizeof(unsigned long long) * 16);
+  cudaMemcpyFromSymbol(out, imn::g_prof, sizeof(unsigned long long) * 24);
   if (reset) {
-    unsigned long long z[16] = {0};
+    unsigned long long z[24] = {0};
     cudaMemcpyToSymbol(imn::g_prof, z, sizeof z);
   }
   return 0;
