@@ -141,7 +141,7 @@ __device__ __forceinline__ Team<GW> make_team(int nworld) {
 // A stage is a few levels of short arithmetic; what took the time was reads that waited for one another: the
 // level's tables (position -> body -> parent, dofs, joints), one dependent read from global memory after the other in
 // every level, qvel inside them, and inputs fetched where they are needed.  A warp now sends for all of
-// its worlds' inputs and for the tables of the tree (six words per body and two per dof, in its own shared
+// its worlds' inputs and for the tables of the tree (six words per body and one per dof, in its own shared
 // memory: no block barrier) with asynchronous copies, waits once, and walks the levels in
 // shared memory.  Five smooth stages in a graph, us: 34 dofs 64 worlds 36.2 -> 27.7, 1000 worlds 40.8 -> 31.0, 8192 worlds
 // 52.3 -> 50.1; 56 dofs 500 worlds 84.3 -> 67.5, 4096 worlds 87.9 -> 73.0; 35 dofs 16384 worlds 148.8 -> 137.9.  (com_vel with a
