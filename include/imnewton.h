@@ -263,7 +263,8 @@ typedef struct ImnBlockedPlan {
   const int32_t* indices; /* device (pad*pad) block-major gather; nM = zero    */
   const float* identity;  /* device (256): ones on the padded diagonal         */
   int32_t nM;
-  const uint16_t* places; /* device (nM): row | column << 8, row <= column, of M's entries; NULL: through indices */
+  const uint16_t* places; /* device (nM): row | column << 8, row <= column, of M's entries; 0xFFFF: an entry that
+                           * `indices` does not name; NULL: through indices */
 } ImnBlockedPlan;
 
 /* mujoco mjtJoint values (Model.jnt_type). */

@@ -290,6 +290,9 @@ __device__ __forceinline__ void dense_substitute(const float* A, const float* di
   for (int q = 0; q < rhs; q += 2 * RQ) dense_back<RQ>(A, dinv, X, n, ldu, rhs, q, l);
 }
 
+// an entry of M whose position belongs to a later one (ImnBlockedPlan::places)
+constexpr int kNoPlace = 0xFFFF;
+
 template <int KM>
 __global__ void __launch_bounds__(32 * kDenseWarps, KM == 2 ? 7 : 4)
     blocked_dense_kernel(const int nv, const int pad, const int nM, const int* __restrict__ indices,
@@ -337,7 +340,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, KM == 2 ? 7 : 4)
         }
 #pragma unroll
         for (int j = 0; j < B; ++j)
-          if (e0 + 32 * j < nM) A[((at[j] >> 8) + 1) * ldu + (at[j] & 255)] = v[j];
+          if (e0 + 32 * j < nM && at[j] != kNoPlace) A[((at[j] >> 8) + 1) * ldu + (at[j] & 255)] = v[j];
       }
     } else {
       // gather the blocks on and above the diagonal: table entry

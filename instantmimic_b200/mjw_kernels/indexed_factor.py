@@ -25,6 +25,7 @@ from ..arrays import addr, elem_strides, is_contiguous, to_host
 BLOCK_SIZE = 16
 BLOCK_DIM = 64
 MIN_NV = 32
+NO_PLACE = 0xFFFF
 
 
 @dataclass
@@ -36,7 +37,7 @@ class BlockedDenseFactorSolveScratch:
     U: Any  # (nworld, pad, pad) factor workspace
     indices: Any  # (pad * pad,) block-major gather table; nM addresses the zero slot
     identity: Any  # (256,) ones on the padded diagonal of the last block
-    places: Any  # (nM,) row | column << 8 of every entry of M, as raw bytes
+    places: Any  # (nM,) row | column << 8 of every entry of M or NO_PLACE, as raw bytes
     struct: abi.ImnBlockedPlan
 
 
@@ -60,8 +61,9 @@ def dense_index_table(m: Any) -> np.ndarray:
 
 
 def entry_places(table: np.ndarray, nM: int) -> np.ndarray:
-    """(nM,) position row | column << 8, row <= column, of every CSR entry of M: ``table`` the other way round."""
-    places = np.zeros(nM, np.uint16)
+    """(nM,) position row | column << 8, row <= column, of every CSR entry of M: ``table`` the other way round.
+    An entry that the table does not name (a later one has its position) has none: NO_PLACE."""
+    places = np.full(nM, NO_PLACE, np.uint16)
     rows, cols = np.nonzero(np.triu(table < nM))
     places[table[rows, cols]] = rows | cols << 8
     return places
@@ -100,7 +102,7 @@ def create_blocked_dense_factor_solve_scratch(
     if not isinstance(nworld, int) or nworld <= 0 or getattr(d, "M", None) is None:
         return None
     pad = _round_up(nv, BLOCK_SIZE)
-    nM = int(d.M.shape[1])
+    nM = min(int(d.M.shape[1]), int(m.M_colind.shape[0]))  # M's rows may be wider than their entries
     table = dense_index_table(m)
     indices = torch.from_numpy(block_major_layout(table, pad, nM)).to(device)
     # torch's uint16 has no arithmetic; the raw bytes do

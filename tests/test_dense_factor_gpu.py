@@ -61,6 +61,30 @@ def test_last_block_and_entry_places(oracle, cuda_device, nv, rhs, places):
     np.testing.assert_array_equal(U.cpu().numpy(), want_U)
 
 
+@pytest.mark.parametrize("filler", [0.0, 9.0])
+@pytest.mark.parametrize("places", [True, False])
+def test_rows_of_m_wider_than_their_entries(oracle, cuda_device, places, filler):
+    import torch
+
+    nv, rhs, worlds = 34, 2, 5
+    m, Mv, _, pad, layout, ident, y = _blocked_case(nv, worlds, rhs)
+    md = mjw_model.to_device(m, cuda_device)
+    d = mjw_model.make_data(m, worlds, 4)
+    d.M = np.concatenate([Mv, np.full((worlds, 2), filler, np.float32)], 1)
+    dd = mjw_model.to_device(d, cuda_device)
+    scratch = indexed_factor.create_blocked_dense_factor_solve_scratch(md, dd, cuda_device)
+    if not places:
+        scratch.struct.places = None
+    yt = torch.from_numpy(y).to(cuda_device)
+    x, x2 = torch.zeros_like(yt), torch.zeros_like(yt)
+    indexed_factor.factor_multi_solve(scratch, dd.M, yt, None, scratch.U, x, rhs)
+    indexed_factor.multi_solve(scratch, scratch.U, yt, None, x2, rhs)
+    want_x, want_U = oracle.blocked_dense_factor_solve(nv, pad, layout, ident, Mv, y)
+    np.testing.assert_array_equal(x.cpu().numpy(), want_x)
+    np.testing.assert_array_equal(x2.cpu().numpy(), want_x)
+    np.testing.assert_array_equal(scratch.U.cpu().numpy(), want_U)
+
+
 def test_entry_places_are_the_index_table_the_other_way_round():
     m = _blocked_case(35, 1, 1)[0]
     table = indexed_factor.dense_index_table(m)

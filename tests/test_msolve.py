@@ -9,7 +9,7 @@ import pytest
 
 from instantmimic_b200 import synthetic
 from instantmimic_b200.mjw_kernels import indexed_factor, tree_ldl
-from instantmimic_b200.mjw_model import put_model
+from instantmimic_b200.mjw_model import make_data, put_model
 
 
 def _branched_tree():
@@ -168,6 +168,55 @@ def test_blocked_oracle_matches_numpy_and_reuses_its_factor(oracle, nv):
     # a second solve from the stored factor is bit-identical to the fresh one
     x2, _ = oracle.blocked_dense_factor_solve(nv, pad, layout, ident, None, y, U=U, mode=1)
     np.testing.assert_array_equal(x, x2)
+
+
+def _wide_matrix_model(nv):
+    """A model and its Data with M two columns wider than the entries it stores."""
+    parent, body = synthetic.limb_tree(nv)
+    m = put_model(parent, body_of_dof=body)
+    d = make_data(m, 3, 4)
+    d.M = np.zeros((3, m.nM + 2), np.float32)
+    return m, d
+
+
+def _laid_out(scratch, m, row):
+    """M's upper triangle of one world by the plan's entry places, as the kernel lays it out."""
+    places = scratch.places.numpy().view(np.uint16)[:scratch.struct.nM]
+    dense = np.zeros((m.nv, m.nv), np.float32)
+    for e, at in enumerate(places.tolist()):
+        if at != 0xFFFF:
+            assert (at & 255) <= at >> 8 < m.nv
+            dense[at & 255, at >> 8] = row[e]
+    return dense
+
+
+@pytest.mark.parametrize("filler", [0.0, 9.0])
+def test_rows_of_m_wider_than_its_entries_are_not_taken_for_entries(filler):
+    m, d = _wide_matrix_model(35)
+    Mv, Md = synthetic.random_mass_matrices(m, 3, np.random.default_rng(0))
+    d.M[:] = filler
+    d.M[:, :m.nM] = Mv
+    scratch = indexed_factor.create_blocked_dense_factor_solve_scratch(m, d, "cpu")
+    np.testing.assert_array_equal(_laid_out(scratch, m, d.M[1]), np.triu(Md[1]).astype(np.float32))
+    # the index table's zero entries are no column of M either
+    zero = scratch.indices.numpy() >= scratch.struct.nM
+    assert zero.any() and scratch.indices.numpy()[~zero].max() == m.nM - 1
+
+
+def test_entries_of_m_that_share_a_place():
+    """Both triangles stored: the later of the two entries is the one that counts, as in the index table."""
+    m, d = _wide_matrix_model(35)
+    table = indexed_factor.dense_index_table(m)
+    rows, cols = np.nonzero(table < m.nM)  # row by row, both triangles
+    m.M_rownnz = np.bincount(rows, minlength=m.nv).astype(np.int32)
+    m.M_rowadr = (np.cumsum(m.M_rownnz) - m.M_rownnz).astype(np.int32)
+    m.M_colind = cols.astype(np.int32)
+    d.M = np.arange(1.0, 1.0 + 3 * cols.size, dtype=np.float32).reshape(3, -1)
+    scratch = indexed_factor.create_blocked_dense_factor_solve_scratch(m, d, "cpu")
+    want = np.zeros((m.nv, m.nv), np.float32)
+    for e, (r, c) in enumerate(zip(rows.tolist(), cols.tolist())):
+        want[min(r, c), max(r, c)] = d.M[2, e]
+    np.testing.assert_array_equal(_laid_out(scratch, m, d.M[2]), want)
 
 
 def test_plan_compiles_to_a_straight_line_kernel_without_a_gpu():
