@@ -806,16 +806,21 @@ static int worlds_per_sm(const Geom& g, int most) {
 // 317 / 340; 35 x 250 240 / 232, 249 / 254.
 //
 // Warps per world: a world's rows, dofs and Hessian entries can be dealt to several warps; the line
-// search, the row lists and most factors cannot, and each stage costs a barrier.  A solve by a team takes kTeamTime of
-// one warp's time (one world per SM, one to four warps: 34 dofs 134 / 126 / 119 / 119 us, 56 dofs 372 / 300 / 263 / 259,
-// 64 dofs x 512 rows 812 / 570 / 476 / 457), but an SM holds fewer teams.  A launch lasts as many solves as its SMs take
-// worlds one after the other: `rounds` if a started round took as long as a full one, share / n if worlds filled
-// in for one another; measured batches lie half-way.  The choice is the least product of the two.  us by the largest
-// (worlds in hand) x sqrt(team), which knows no rounds -> now (best of all four): 34 dofs, 6 worlds per SM 158 -> 142
-// (142), 10 per SM 178 -> 162 (162); 40 x 100 dense, 6: 328 -> 244 (244); 60 dofs, 7: 921 -> 764 (764); 64 x 512, 4: 842 -> 650
-// (650), 12: 1810 -> 1755 (1755); 50 x 100, 8: 444 -> 370 (370); 56 dofs, 7: 393 -> 454 (393).  Over 131 batches of nine models and 1
-// to 28 worlds per SM the mean distance from the best falls from 2.4 % to 0.5 %.
-static const float kTeamTime[5] = {0.0f, 1.0f, 0.82f, 0.70f, 0.60f};
+// search, the row lists and most factors cannot, and each stage costs a barrier.  How much of a solve can be dealt
+// follows J: streamed, its rows come from L2, and more warps hide that (one world per SM, one to four warps, us: 56 dofs
+// 414 / 314 / 289 / 276, 35 x 250 264 / 223 / 193 / 187, 64 x 512 879 / 594 / 519 / 494); resident, the chains are most of
+// it (34 dofs 135 / 126 / 120 / 120, 40 x 100 dense 248 / 211 / 203 / 204, 60 x 64 dense 444 / 384 / 371 / 355).
+// With n worlds in hand a solve takes kTeamTime + n kCrowded of one warp's time alone.  A launch lasts as many solves as
+// its SMs take worlds one after the other: share / n if worlds filled in for one another, `rounds` if a started round
+// took as long as a full one.  Worlds go by falling row counts, so a last round is short: a tenth of `rounds`, nothing
+// where J is resident.  The choice is the least product.  Over 289 batches (17 models, 1 to 28 worlds per SM) the mean distance from the best
+// of the four is 0.4 %, 2.1 % by the largest (worlds in hand) x sqrt(team), and none is more than 3.3 % behind
+// that; 1.2 % with one column of times for every J and half of `rounds` (56 dofs, 7 worlds per SM, 473 us where two warps
+// take 429; 35 x 512, 28 per SM 1758 / 1566).  What is left are batches of one world more than teams of two
+// hold: where worlds differ in rows two warps are ahead (35 x 96 dense, 9 per SM 308 against 345 us), where all have
+// the same count one is (27 x 32 dense 131 against 150), and the rule takes two.
+static const float kTeamTime[2][5] = {{0.0f, 1.0f, 0.72f, 0.58f, 0.55f}, {0.0f, 1.0f, 0.84f, 0.81f, 0.74f}};  // [J resident]
+static const float kCrowded[2] = {0.03f, 0.01f}, kRounds[2] = {0.1f, 0.0f};
 static const int kMaxParts = 4;
 
 static int plan_launch(const ImnModel* m, const ImnData* d, const ImnSparsePlan* sp, bool stats, Geom* g, bool* resident,
@@ -834,7 +839,9 @@ static int plan_launch(const ImnModel* m, const ImnData* d, const ImnSparsePlan*
   const int sms = sm_count(), share = max((d->nworld + sms - 1) / sms, 1);
   g->warps = min(share, *resident ? nr : ns);
   const auto time = [&](const Geom& q) {
-    return ((float)((share + q.warps - 1) / q.warps) + (float)share / (float)q.warps) * kTeamTime[q.parts];
+    const float n = (float)q.warps, rounds = (float)((share + q.warps - 1) / q.warps);
+    const float turns = (float)share / n;
+    return (turns + kRounds[*resident] * (rounds - turns)) * (kTeamTime[*resident][q.parts] + n * kCrowded[*resident]);
   };
   for (int parts = 2; parts <= kMaxParts && !stats; ++parts) {  // the counting kernels know no teams
     Geom team = make_geom(*m, *d, *resident, sp, parts);

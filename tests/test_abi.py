@@ -101,6 +101,44 @@ def test_launch_info_reports_geometry_without_a_gpu():
     assert info.j_resident == 0  # 512 rows x 64 dofs stream through the staging tile
 
 
+@pytest.mark.parametrize("name,per_sm,worlds", [
+    # one world more than teams of two hold: they are ahead where worlds differ in rows (473 us against 429, 336 / 306)
+    ("snu", 7, 6), ("g1", 7, 6),
+    # the same with the dense factor (345 / 308), and its full batches (323 / 278 us, 3502 / 2773, 1758 / 1566)
+    ("chain35x96", 9, 8), ("humanoid dense", 14, 13), ("limb64x512", 20, 4), ("limb35x512", 28, 6), ("chain60x64", 7, 6),
+    # few worlds: all in hand, with as many warps as there is room for; full batches: a warp each
+    ("snu", 1, 1), ("limb64x512", 3, 3), ("humanoid", 6, 6), ("humanoid", 28, 14), ("snu", 28, 9), ("g1", 28, 12)])
+def test_worlds_in_hand_follow_the_measured_best(name, per_sm, worlds):
+    """Host-only: worlds an SM takes at once, by worlds per SM."""
+    import numpy as np
+
+    from instantmimic_b200 import binding, synthetic
+    from instantmimic_b200.mjw_kernels import sparse_hessian
+    from instantmimic_b200.mjw_model import make_data, put_model
+    from helpers import host_ctx
+
+    kind, _, rows = name.partition("x")
+    if kind[:5] in ("chain", "limb6", "limb3"):
+        parent, body = (synthetic.chain_tree if kind[:5] == "chain" else synthetic.limb_tree)(int(kind.lstrip("chainlimb")))
+        m = put_model(parent, body_of_dof=body)
+        d, plan = make_data(m, 4, int(rows)), None
+    else:
+        kind, _, dense = name.partition(" ")
+        m, d, _ = synthetic.make_workload(kind, 4, seed=0)
+        groups = [[b] for b in range(1, len(m.body_dofadr))]
+        plan = None if dense else sparse_hessian.build_plan(m, groups, 32 if m.nv_pad < 64 else 64, "fused")
+    ms, ds = binding.model_struct(m), binding.data_struct(m, d)
+    cs = binding.ctx_struct(ds, host_ctx(m, d), np.zeros(1, np.int32))
+    cs.stats = None
+    ds.nworld = 148 * per_sm
+    if plan is not None:
+        host = sparse_hessian.host_struct(plan)
+        cs.sparse_plan = C.pointer(host)
+    info = abi.ImnLaunchInfo()
+    assert _lib.lib().imn_launch_info(C.byref(ms), C.byref(ds), C.byref(cs), C.byref(info)) == 0, _lib.lib().imn_last_error()
+    assert info.worlds_per_cta == worlds
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "_LIB", None)
     monkeypatch.setattr(_lib, "_PATH", tmp_path / "absent.so")
