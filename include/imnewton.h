@@ -30,7 +30,7 @@
 extern "C" {
 #endif
 
-#define IMN_ABI_VERSION 6
+#define IMN_ABI_VERSION 7
 
 typedef enum ImnStatus {
   IMN_OK = 0,

@@ -16,7 +16,7 @@ I32 = C.c_int32
 I64 = C.c_int64
 F32 = C.c_float
 
-IMN_ABI_VERSION = 6
+IMN_ABI_VERSION = 7
 
 IMN_OK = 0
 IMN_ERR_NULL = -1

@@ -45,6 +45,22 @@ def test_ctypes_structs_match_the_compiler(tmp_path):
         assert C.sizeof(getattr(abi, s)) == int(sizes[s]), s
 
 
+# sizeof every struct of a layout version: a struct that changes takes the next number
+_LAYOUTS = {
+    6: dict(ImnAdvance=96, ImnBallLimits=304, ImnBlockedPlan=32, ImnBodyTree=168, ImnCtx=208, ImnData=208, ImnImplicit=152,
+            ImnLaunchInfo=20, ImnModel=144, ImnSparsePlan=256, ImnTreePlan=48),
+    7: dict(ImnAdvance=96, ImnBallLimits=304, ImnBlockedPlan=40, ImnBodyTree=168, ImnCtx=208, ImnData=208, ImnImplicit=152,
+            ImnLaunchInfo=20, ImnModel=144, ImnSparsePlan=256, ImnTreePlan=48),
+}
+
+
+def test_struct_sizes_are_those_of_the_layout_version():
+    """A host built against another version's header is refused by the number, so a layout has one number."""
+    sizes = {name: C.sizeof(getattr(abi, name)) for name in dir(abi) if name.startswith("Imn")}
+    assert sizes == _LAYOUTS[_lib.lib().imn_abi_version()]
+    assert int(re.search(r"#define IMN_ABI_VERSION (\d+)", HEADER.read_text())[1]) == abi.IMN_ABI_VERSION
+
+
 def test_validation_rejects_bad_calls_before_any_launch():
     lib = _lib.lib()
     m, d, c = abi.ImnModel(), abi.ImnData(), abi.ImnCtx()
