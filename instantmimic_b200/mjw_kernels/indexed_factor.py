@@ -37,8 +37,8 @@ class BlockedDenseFactorSolveScratch:
     U: Any  # (nworld, pad, pad) factor workspace
     indices: Any  # (pad * pad,) block-major gather table; nM addresses the zero slot
     identity: Any  # (256,) ones on the padded diagonal of the last block
-    places: Any  # (nM,) row | column << 8 of every entry of M or NO_PLACE, as raw bytes
     struct: abi.ImnBlockedPlan
+    places: Any = None  # (nM,) row | column << 8 of every entry of M or NO_PLACE, as raw bytes
 
 
 def _round_up(value: int, multiple: int) -> int:
@@ -114,7 +114,7 @@ def create_blocked_dense_factor_solve_scratch(
     st.indices, st.identity, st.places = addr(indices), addr(identity), addr(places)
     return BlockedDenseFactorSolveScratch(
         nv=nv, pad=pad, block_size=BLOCK_SIZE, block_dim=BLOCK_DIM, U=U, indices=indices,
-        identity=identity, places=places, struct=st,
+        identity=identity, struct=st, places=places,
     )
 
 

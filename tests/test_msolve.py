@@ -203,6 +203,18 @@ def test_rows_of_m_wider_than_its_entries_are_not_taken_for_entries(filler):
     assert zero.any() and scratch.indices.numpy()[~zero].max() == m.nM - 1
 
 
+def test_a_plan_of_the_index_table_alone_is_still_one():
+    """A caller that builds the plan itself need not name the entries' places (imn_blocked_dense_factor_solve then looks
+    every position up)."""
+    m, d = _wide_matrix_model(35)
+    made = indexed_factor.create_blocked_dense_factor_solve_scratch(m, d, "cpu")
+    struct = type(made.struct).from_buffer_copy(made.struct)
+    struct.places = None
+    own = indexed_factor.BlockedDenseFactorSolveScratch(
+        made.nv, made.pad, made.block_size, made.block_dim, made.U, made.indices, made.identity, struct)
+    assert own.struct is struct and own.places is None
+
+
 def test_entries_of_m_that_share_a_place():
     """Both triangles stored: the later of the two entries is the one that counts, as in the index table."""
     m, d = _wide_matrix_model(35)
