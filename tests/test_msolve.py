@@ -203,6 +203,37 @@ def test_rows_of_m_wider_than_its_entries_are_not_taken_for_entries(filler):
     assert zero.any() and scratch.indices.numpy()[~zero].max() == m.nM - 1
 
 
+def _table_entry_by_entry(m):
+    """dense_index_table as it is defined: every stored entry in turn, both triangles."""
+    table = np.full((m.nv, m.nv), len(m.M_colind), np.int32)
+    for k in range(m.nv):
+        for e in range(m.M_rowadr[k], m.M_rowadr[k] + m.M_rownnz[k]):
+            table[k, m.M_colind[e]] = table[m.M_colind[e], k] = e
+    return table
+
+
+def test_plan_tables_are_made_at_once_and_sent_at_once(monkeypatch):
+    """The plan is set up as often as M changes its shape: no loop over M's entries, one copy to the device."""
+    import torch
+
+    m, d = _wide_matrix_model(56)
+    np.testing.assert_array_equal(indexed_factor.dense_index_table(m), _table_entry_by_entry(m))
+    rng = np.random.default_rng(3)  # rows apart in storage, entries stored twice
+    m.M_rownnz = rng.integers(0, 5, m.nv).astype(np.int32)
+    m.M_rowadr = (7 * rng.permutation(m.nv)).astype(np.int32)
+    m.M_colind = rng.integers(0, m.nv, 7 * m.nv).astype(np.int32)
+    np.testing.assert_array_equal(indexed_factor.dense_index_table(m), _table_entry_by_entry(m))
+    sent, to = [], torch.Tensor.to
+    monkeypatch.setattr(torch.Tensor, "to", lambda t, *a, **k: sent.append(t.numel()) or to(t, *a, **k))
+    scratch = indexed_factor.create_blocked_dense_factor_solve_scratch(m, d, "cpu")
+    assert len(sent) == 1
+    base = scratch.indices.untyped_storage().data_ptr()
+    for t, name in ((scratch.indices, "indices"), (scratch.identity, "identity"), (scratch.places, "places")):
+        assert t.untyped_storage().data_ptr() == base and getattr(scratch.struct, name) == t.data_ptr()
+    assert scratch.indices.dtype == torch.int32 and scratch.identity.dtype == torch.float32
+    np.testing.assert_array_equal(scratch.identity.numpy(), indexed_factor.pad_identity(56, 64))
+
+
 def test_a_plan_of_the_index_table_alone_is_still_one():
     """A caller that builds the plan itself need not name the entries' places (imn_blocked_dense_factor_solve then looks
     every position up)."""
