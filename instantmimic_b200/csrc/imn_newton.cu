@@ -119,7 +119,8 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   g.tB = t, t += sp ? (sp->nbsweep + 1) * 64 : 0;
   g.tS = t, t += sp ? up4(sp->nfac) : 0;
   g.tO = t, t += sp ? up4(m.nv) : 0;
-  g.tP = t, t += sp ? up4(m.nv * g.mwords) : 0;
+  g.tP = t;
+  const int masks = sp ? up4(m.nv * g.mwords) : 0;
   // A plan's tables stay in global memory when they would take more than a third of an SM's shared memory;
   // without a plan there is the M v program only, at most 31 KB for 79 dofs.  us per solve, tables in shared /
   // global memory: 34 dofs (19 KB) 592 worlds 155 / 171, 8192 worlds 562 / 547 (14 worlds per SM against 16);
@@ -128,7 +129,10 @@ static Geom make_geom(const ImnModel& m, const ImnData& d, bool resident, const 
   // (106 KB) 661 / 869, 3186 / 3312; (137 KB) 1437 / 1112, 7720 / 4234.  The third keeps the tables of every
   // tree alone on chip and errs on the side of more worlds; the crossing lies near half an SM.
   g.tsm = !sp || 4 * t <= kMaxSmem / 3;
-  g.tab = g.tsm ? t : 0;
+  // The pattern's masks (up to 960 bytes) came to the staged tables last: a world of thousands of rows that leaves no
+  // room for them reads all tables from global memory rather than being refused (79 dofs: row limits 4457 to 4484).
+  if (parts == 1 && 4 * (t + g.total) <= kMaxSmem && 4 * (t + masks + g.total) > kMaxSmem) g.tsm = false;
+  g.tab = g.tsm ? t + masks : 0;
   g.wait_polls = g_wait_polls;
   g.withhold_copies = g_withhold_copies;
   return g;

@@ -155,6 +155,30 @@ def test_worlds_in_hand_follow_the_measured_best(name, per_sm, worlds):
     assert info.worlds_per_cta == worlds
 
 
+@pytest.mark.parametrize("nv,most", [(35, 6752), (64, 5688), (79, 4484)])
+def test_the_largest_worlds_of_a_plan_stay_accepted(nv, most):
+    """Host-only: what is staged beside the tables does not lower the row limit of a world."""
+    import numpy as np
+
+    from instantmimic_b200 import binding, synthetic
+    from instantmimic_b200.mjw_kernels import sparse_hessian
+    from instantmimic_b200.mjw_model import make_data, put_model
+    from helpers import host_ctx
+
+    parent, body = synthetic.limb_tree(nv)
+    m = put_model(parent, body_of_dof=body)
+    groups = [[b] for b in range(1, len(m.body_dofadr))]
+    host = sparse_hessian.host_struct(sparse_hessian.build_plan(m, groups, 32 if m.nv_pad < 64 else 64, "fused"))
+    for njmax, status in ((most, 0), (most + 1, abi.IMN_ERR_LIMIT)):
+        d = make_data(m, 2, njmax)
+        ms, ds = binding.model_struct(m), binding.data_struct(m, d)
+        cs = binding.ctx_struct(ds, host_ctx(m, d), np.zeros(1, np.int32))
+        cs.stats, cs.sparse_plan = None, C.pointer(host)
+        info = abi.ImnLaunchInfo()
+        assert _lib.lib().imn_launch_info(C.byref(ms), C.byref(ds), C.byref(cs), C.byref(info)) == status
+        assert status or info.smem_bytes <= 227 * 1024
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "_LIB", None)
     monkeypatch.setattr(_lib, "_PATH", tmp_path / "absent.so")
