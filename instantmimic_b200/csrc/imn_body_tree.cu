@@ -173,17 +173,34 @@ struct WarpTables {
   int *bodies, *child_ptr, *child_ids, *parent, *dofadr, *dofnum, *offsets, *dof_body;
 };
 __host__ __device__ inline int table_words(int nbody, int nlevels, int nv) { return 6 * nbody + 1 + nlevels + 1 + nv; }
+__host__ __device__ inline int sweep_words(int nbody, int nlevels) { return 3 * nbody + 1 + nlevels + 1; }
 // behind the worlds of the CTA (32 / GW per warp, `per_world` floats each), a warp's tables after the other's
 template <int GW>
+__device__ __forceinline__ int* table_space(float* smem, int per_world, int words) {
+  return reinterpret_cast<int*>(smem + (size_t)(blockDim.x >> 5) * (32 / GW) * per_world) + (threadIdx.x >> 5) * words;
+}
+template <int GW>
 __device__ __forceinline__ int* table_space(const ImnBodyTree& T, float* smem, int per_world) {
-  return reinterpret_cast<int*>(smem + (size_t)(blockDim.x >> 5) * (32 / GW) * per_world) +
-         (threadIdx.x >> 5) * table_words(T.nbody, T.nlevels, T.nv);
+  return table_space<GW>(smem, per_world, table_words(T.nbody, T.nlevels, T.nv));
 }
 __device__ __forceinline__ WarpTables warp_tables(const ImnBodyTree& T, int* at) {
   WarpTables t;
   t.bodies = at, t.child_ids = t.bodies + T.nbody, t.parent = t.child_ids + T.nbody, t.dofadr = t.parent + T.nbody;
   t.dofnum = t.dofadr + T.nbody, t.child_ptr = t.dofnum + T.nbody, t.offsets = t.child_ptr + T.nbody + 1;
   t.dof_body = t.offsets + T.nlevels + 1;
+  return t;
+}
+// of the tree alone, without a look at its dofs: what a sweep up reads
+__device__ __forceinline__ WarpTables sweep_tables(const ImnBodyTree& T, int* at) {
+  WarpTables t = {};
+  t.bodies = at, t.child_ids = t.bodies + T.nbody, t.child_ptr = t.child_ids + T.nbody, t.offsets = t.child_ptr + T.nbody + 1;
+  return t;
+}
+// the same where it is in global memory
+__device__ __forceinline__ WarpTables sweep_tables(const ImnBodyTree& T) {
+  WarpTables t = {};
+  t.bodies = const_cast<int*>(T.level_bodies), t.child_ids = const_cast<int*>(T.child_ids);
+  t.child_ptr = const_cast<int*>(T.child_ptr), t.offsets = const_cast<int*>(T.level_offsets);
   return t;
 }
 __device__ __forceinline__ void send_words(int* dst, const int* src, int n) {
@@ -244,19 +261,21 @@ __device__ __forceinline__ void copy_out(float* __restrict__ dst, const float* s
 template <int GW>
 __global__ void __launch_bounds__(32 * kTreeWarps)
     tree_accumulate_kernel(const ImnBodyTree T, float* __restrict__ values, const int64_t world_ld, const int C,
-                           const int skip_root_parent, const int nworld) {
+                           const int skip_root_parent, const int staged, const int nworld) {
   extern __shared__ __align__(16) float tree_smem[];
   chain_wait();
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int n = T.nbody * C, per_world = (n + 3) & ~3;
   float* v = tree_smem + (size_t)t.slot * per_world;
-  const WarpTables tab = warp_tables(T, table_space<GW>(T, tree_smem, per_world));
+  const WarpTables tab = sweep_tables(T, table_space<GW>(tree_smem, per_world, sweep_words(T.nbody, T.nlevels)));
   float* g = values + (size_t)t.w * world_ld;
   async_run<GW>(v, g, n, t.sl);
-  send_sweep(T, tab);
+  if (staged) send_sweep(T, tab);
   async_wait();
-  if (C == 3)
+  if (!staged)
+    sweep_up<GW, 0>(sweep_tables(T), T.nlevels, v, C, skip_root_parent != 0, t.sl);
+  else if (C == 3)
     sweep_up<GW, 3>(tab, T.nlevels, v, C, skip_root_parent != 0, t.sl);
   else
     sweep_up<GW, 0>(tab, T.nlevels, v, C, skip_root_parent != 0, t.sl);
@@ -333,7 +352,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   const Team<GW> t = make_team<GW>(nworld);
   if (t.none) return;
   const int sl = t.sl, w = t.w;
-  const int nb6 = T.nbody * 6, nv6 = T.nv * 6, nb6p = (nb6 + 3) & ~3, nv6p = (nv6 + 3) & ~3, nvp = (T.nv + 3) & ~3;
+  const int nb6 = T.nbody * 6, nv6 = T.nv * 6, nb6p = (nb6 + 3) & ~3, nv6p = (nv6 + 3) & ~3;
   const int nb10 = T.nbody * 10, nb10p = (nb10 + 3) & ~3, per_world = rne_floats(T.nbody, T.nv);
   float* cacc = tree_smem + (size_t)t.slot * per_world;
   float* cfrc = cacc + nb6p;  // cvel until the body's force replaces it
@@ -522,13 +541,13 @@ static int team_lanes(const ImnBodyTree* T, int at_least = 8) {
 }
 
 template <typename... Args>
-static int launch_tree(const char* who, const ImnBodyTree* T, void (*kernel)(Args...), int gw, size_t floats_per_world, int nworld,
-                       void* stream, Args... args) {
+static int launch_tree(const char* who, void (*kernel)(Args...), int gw, size_t floats_per_world,
+                       int table_words, int nworld, void* stream, Args... args) {
   if (nworld < 0) return set_error("%s: negative world count", who), IMN_ERR_SHAPE;
   if (nworld == 0) return IMN_OK;
   // four warps a block, fewer for trees of hundreds of bodies, whose worlds would not fit
   int warps = kTreeWarps;
-  const size_t warp_bytes = 4 * (floats_per_world * (32 / gw) + table_words(T->nbody, T->nlevels, T->nv));
+  const size_t warp_bytes = 4 * (floats_per_world * (32 / gw) + table_words);
   while (warps > 1 && warps * warp_bytes > 227 * 1024) warps /= 2;
   const int per_cta = warps * (32 / gw);
   const size_t bytes = warps * warp_bytes;
@@ -547,10 +566,10 @@ static int launch_tree(const char* who, const ImnBodyTree* T, void (*kernel)(Arg
 static size_t up4z(size_t n) { return (n + 3) & ~(size_t)3; }
 
 // KERNEL<8 | 16 | 32> by the tree's team width
-#define IMN_TEAM_LAUNCH(LANES, KERNEL, FLOATS, NWORLD, STREAM, ...)                                \
-  ((LANES) == 8    ? imn::launch_tree(who, T, KERNEL<8>, 8, FLOATS, NWORLD, STREAM, __VA_ARGS__)   \
-   : (LANES) == 16 ? imn::launch_tree(who, T, KERNEL<16>, 16, FLOATS, NWORLD, STREAM, __VA_ARGS__) \
-                   : imn::launch_tree(who, T, KERNEL<32>, 32, FLOATS, NWORLD, STREAM, __VA_ARGS__))
+#define IMN_TEAM_LAUNCH(LANES, KERNEL, FLOATS, TABLES, NWORLD, STREAM, ...)                               \
+  ((LANES) == 8    ? imn::launch_tree(who, KERNEL<8>, 8, FLOATS, TABLES, NWORLD, STREAM, __VA_ARGS__)   \
+   : (LANES) == 16 ? imn::launch_tree(who, KERNEL<16>, 16, FLOATS, TABLES, NWORLD, STREAM, __VA_ARGS__) \
+                   : imn::launch_tree(who, KERNEL<32>, 32, FLOATS, TABLES, NWORLD, STREAM, __VA_ARGS__))
 
 }  // namespace imn
 
@@ -564,8 +583,13 @@ extern "C" int imn_body_tree_accumulate(const ImnBodyTree* T, float* values, int
     return imn::set_error("%s: components %d / world stride %lld do not hold %d bodies", who, components,
                           (long long)world_ld, T->nbody),
            IMN_ERR_SHAPE;
-  return IMN_TEAM_LAUNCH(imn::team_lanes(T), imn::tree_accumulate_kernel, imn::up4z((size_t)T->nbody * components), nworld, stream, *T,
-                         values, world_ld, (int)components, (int)skip_root_parent, (int)nworld);
+  // A tree whose tables do not fit behind a warp's worlds (one component, a warp per world, from 12 to 15 thousand
+  // bodies on) is walked in global memory.
+  const int lanes = imn::team_lanes(T), words = imn::sweep_words(T->nbody, T->nlevels);
+  const size_t floats = imn::up4z((size_t)T->nbody * components);
+  const int staged = 4 * (floats * (32 / lanes) + words) <= 227 * 1024;
+  return IMN_TEAM_LAUNCH(lanes, imn::tree_accumulate_kernel, floats, staged ? words : 0, nworld, stream, *T, values, world_ld,
+                         (int)components, (int)skip_root_parent, staged, (int)nworld);
 }
 
 extern "C" int imn_crb(const ImnBodyTree* T, const float* cinert, const float* cdof, float* crb, float* M,
@@ -577,8 +601,8 @@ extern "C" int imn_crb(const ImnBodyTree* T, const float* cinert, const float* c
     return imn::set_error("%s: NULL array", who), IMN_ERR_NULL;
   if (T->n_armature <= 0 || M_ld < T->nM) return imn::set_error("%s: bad armature count or M stride", who), IMN_ERR_SHAPE;
   return IMN_TEAM_LAUNCH(imn::team_lanes(T, 32), imn::crb_kernel,
-                         imn::up4z((size_t)T->nbody * 10) + 2 * imn::up4z((size_t)T->nv * 6), nworld,
-                         stream, *T, cinert, cdof, crb, M, M_ld, (int)nworld);
+                         imn::up4z((size_t)T->nbody * 10) + 2 * imn::up4z((size_t)T->nv * 6),
+                         imn::table_words(T->nbody, T->nlevels, T->nv), nworld, stream, *T, cinert, cdof, crb, M, M_ld, (int)nworld);
 }
 
 extern "C" int imn_rne(const ImnBodyTree* T, const float* cinert, const float* cvel, const float* cdof,
@@ -591,8 +615,8 @@ extern "C" int imn_rne(const ImnBodyTree* T, const float* cinert, const float* c
     return imn::set_error("%s: NULL array", who), IMN_ERR_NULL;
   if (T->n_gravity <= 0 || qvel_ld < T->nv || bias_ld < T->nv)
     return imn::set_error("%s: bad gravity count or stride", who), IMN_ERR_SHAPE;
-  return IMN_TEAM_LAUNCH(imn::team_lanes(T, 16), imn::rne_kernel, (size_t)imn::rne_floats(T->nbody, T->nv), nworld,
-                         stream, *T, cinert, cvel, cdof, cdof_dot, qvel, qvel_ld, cacc, cfrc_int, qfrc_bias, bias_ld,
+  return IMN_TEAM_LAUNCH(imn::team_lanes(T, 16), imn::rne_kernel, (size_t)imn::rne_floats(T->nbody, T->nv),
+                         imn::table_words(T->nbody, T->nlevels, T->nv), nworld, stream, *T, cinert, cvel, cdof, cdof_dot, qvel, qvel_ld, cacc, cfrc_int, qfrc_bias, bias_ld,
                          (int)nworld);
 }
 
@@ -605,5 +629,5 @@ extern "C" int imn_com_vel(const ImnBodyTree* T, const float* qvel, int64_t qvel
     return imn::set_error("%s: NULL array", who), IMN_ERR_NULL;
   if (qvel_ld < T->nv) return imn::set_error("%s: qvel stride < nv", who), IMN_ERR_SHAPE;
   return IMN_TEAM_LAUNCH(imn::team_lanes(T), imn::com_vel_kernel, imn::up4z((size_t)T->nbody * 6) + 2 * imn::up4z((size_t)T->nv * 6) + imn::up4z(T->nv),
-                         nworld, stream, *T, qvel, qvel_ld, cdof, cvel, cdof_dot, (int)nworld);
+                         imn::table_words(T->nbody, T->nlevels, T->nv), nworld, stream, *T, qvel, qvel_ld, cdof, cvel, cdof_dot, (int)nworld);
 }

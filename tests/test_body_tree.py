@@ -357,6 +357,37 @@ def test_cuda_smooth_stages_of_trees_of_hundreds_of_bodies(nv, team):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("bodies,depth", [(14000, 2), (14000, 5000)])
+def test_cuda_accumulate_of_trees_of_thousands_of_bodies(bodies, depth):
+    """A warp's world fits a block's shared memory, and so do the tables of the flat tree; those of the deep one stay in
+    global memory.  The sum reads nothing of the dofs, so their count does not matter either."""
+    import ctypes as C
+
+    import torch
+
+    from instantmimic_b200 import _lib
+
+    parents = np.zeros(bodies, np.int32)  # a chain, the other bodies on the world body
+    parents[1:depth] = np.arange(depth - 1)
+    depths = np.where(np.arange(bodies) < depth, np.arange(bodies), 1)
+    levels = [np.flatnonzero(depths == k).astype(np.int32) for k in range(depth)]
+    dev = SimpleNamespace(body_parentid=torch.from_numpy(parents).to(_device()),
+                          body_tree=[torch.from_numpy(x).to(_device()) for x in levels])
+    scratch = tree_fusion.create_tree_reduction_scratch(dev)
+    assert scratch.team_lanes == 32
+    initial = np.random.default_rng(7).uniform(0.1, 1.0, (3, bodies, 1)).astype(np.float32)
+    expected = depth_ordered_sum(initial, parents, levels, False)
+    for nv in (0, 10**8):
+        values = torch.from_numpy(initial).to(_device())
+        tree = tree_fusion.tree_struct(dev, scratch)
+        tree.nv = nv
+        stream = torch.cuda.current_stream().cuda_stream
+        rc = _lib.lib().imn_body_tree_accumulate(C.byref(tree), values.data_ptr(), bodies, 1, 0, 3, stream)
+        assert rc == 0, _lib.lib().imn_last_error()
+        np.testing.assert_array_equal(values.cpu().numpy(), expected)
+
+
+@pytest.mark.gpu
 def test_cuda_tree_entry_points_check_their_arguments():
     import torch
 
