@@ -176,7 +176,8 @@ typedef struct ImnSparsePlan {
    *     advance by the team width; flags bit 0 = the lane stores the entry, bit 1 = last step
    *     of its level, bits 2-4 = log2(team), bit 5 = last step of its sweep, bit 6 = a
    *     lane of the sweep holds a diagonal entry, bit 7 = this step and the next are two sweeps
-   *     of a level (bits 8-15 then count for both), bits 8-15 = most terms of a lane.
+   *     of a level (counted for `pairs`; no kernel reads it), bits 8-15 = most terms of a lane
+   *     of the step.
    *   bstep [nbsweep + 1][32][2]: {slot | source's right-hand side << 16, source's 1/D |
    *     destination's right-hand side << 16}; bit 0 of word 0 = the lane has work, of
    *     word 1 = last of its level.

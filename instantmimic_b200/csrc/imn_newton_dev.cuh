@@ -69,11 +69,6 @@ __device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
-  Pair r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 struct alignas(16) Pair2 {
   Pair a, b;
 };

@@ -498,8 +498,7 @@ def pack_steps(t: dict, nv: int, nfac: int) -> dict:
             first.append(k)
     pairs = 3 * 2 * len(first) >= 2 * len(steps)
     for k in first if pairs else []:
-        most = max(int(steps[k][0, 3] >> 8), int(steps[k + 1][0, 3] >> 8))
-        steps[k][:, 3] = (steps[k][:, 3] & 0xFF) | 128 | most << 8
+        steps[k][:, 3] |= 128  # the kernel looks at `pairs` alone
     b = t["bsweep"].astype(np.int64).reshape(-1, 32)
     src, dst, work = (b >> 16) & 0x7F, (b >> 23) & 0x7F, ((b >> 30) & 1) == 1
     back = np.zeros((b.shape[0] + 1, 32, 2), np.int64)

@@ -578,6 +578,48 @@ def test_step_records_give_every_entry_its_terms_in_order():
     assert paired
 
 
+@pytest.mark.parametrize("warps", [1, 2, 4])
+def test_step_records_read_by_one_or_several_warps(warps):
+    """Walks ``fstep`` a record at a time, as the factor does: a sweep per warp in turn, a barrier at a level's end and
+    nowhere else.  A lane's reads, those past its last term among them (four terms a trip), stay between N and the
+    six dof vectors behind 1 / D, and no warp reads between two barriers what another one stores."""
+    for name, m, groups in _plan_models():
+        plan = sparse_hessian.build_plan(m, groups, 32 if m.nv_pad < 64 else 64, "fused")
+        up4 = lambda n: (n + 3) // 4 * 4  # noqa: E731
+        inv0 = up4(plan.nfac + plan.nv)
+        room = 4 * (inv0 + up4(plan.nv) + 6 * up4(plan.nv + 1))
+        f = plan.steps["fstep"].reshape(-1, 32, 4).astype(np.int64)[:plan.steps["nfstep"]]
+        turn, carried, one_lane = 0, None, True
+        reads, stores = {}, {}  # byte offset: warp
+        for rec in f:
+            flags = int(rec[0, 3]) & ~1
+            assert ((rec[:, 3] & ~1) == flags).all()
+            # the records of a lane per entry and one run come first, and the loop for them asks for no more
+            one_lane = one_lane and flags & 0x3C == 32
+            stride = 4 << ((flags >> 2) & 7)
+            trips = -(-((flags >> 8) & 0xFF) // 4)
+            assert carried in (None, turn)  # the runs of a sweep stay with its warp
+            for x, y, z, _ in rec.tolist():
+                for at in (x & 0xFFFF, x >> 16, y & 0xFFFF):
+                    assert at + stride * max(4 * trips - 1, 0) + 4 <= room, name
+                    for q in range(z & 0xFFFF):
+                        reads.setdefault(at + stride * q, set()).add(turn)
+            if flags & 32:
+                for x, y, z, w in rec.tolist():
+                    for at in ([y >> 16] if w & 1 else []) + ([z >> 16] if z >> 16 else []):
+                        assert at not in stores
+                        stores[at] = turn
+            else:
+                assert not one_lane and not flags & 2
+            carried = None if flags & 32 else turn
+            if flags & 32:
+                turn = (turn + 1) % warps
+            if flags & 2:
+                assert not set(stores) & set(reads), name
+                turn, reads, stores = 0, {}, {}
+        assert carried is None and not reads and not stores  # the last sweep ends its level
+
+
 def test_backward_step_records_give_every_push_once_and_level_by_level():
     for name, m, groups in _plan_models():
         plan = sparse_hessian.build_plan(m, groups, 32 if m.nv_pad < 64 else 64, "fused")
