@@ -329,8 +329,8 @@ typedef struct ImnBodyTree {
   const int32_t* level_bodies;  /* (nbody) m.body_tree concatenated, level 0 first  */
   const int32_t* level_offsets; /* (nlevels + 1)                                    */
   const int32_t* child_ptr;     /* (nbody + 1) by position in level_bodies: the     */
-  const int32_t* child_ids;     /* children of that body in level-list order (the
-                                 * world body is nobody's child); no counterpart in
+  const int32_t* child_ids;     /* (nbody - 1) children of that body in level-list order
+                                 * (the world body is nobody's child); no counterpart in
                                  * the reference, which scans the whole next level  */
   const int32_t* body_jntnum;   /* (nbody) */
   const int32_t* body_jntadr;   /* (nbody) */

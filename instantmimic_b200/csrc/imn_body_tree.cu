@@ -32,7 +32,7 @@
 
 namespace imn {
 
-static const int kTreeWarps = 4;
+static const int kTreeWarps = 4, kVelWarps = 2;
 
 struct Sp6 {
   float v[6];
@@ -141,7 +141,7 @@ __device__ __forceinline__ Team<GW> make_team(int nworld) {
 // A stage is a few levels of short arithmetic; what took the time was reads that waited for one another: the
 // level's tables (position -> body -> parent, dofs, joints), one dependent read from global memory after the other in
 // every level, qvel inside them, and inputs fetched where they are needed.  A warp now sends for all of
-// its worlds' inputs and for the tables of the tree (six words per body and one per dof, in its own shared
+// its worlds' inputs and for the tables of the tree that the stage reads (four to six words per body, in its own shared
 // memory: no block barrier) with asynchronous copies, waits once, and walks the levels in
 // shared memory.  Five smooth stages in a graph, us: 34 dofs 64 worlds 36.2 -> 27.7, 1000 worlds 40.8 -> 31.0, 8192 worlds
 // 52.3 -> 50.1; 56 dofs 500 worlds 84.3 -> 67.5, 4096 worlds 87.9 -> 73.0; 35 dofs 16384 worlds 148.8 -> 137.9.  (com_vel with a
@@ -168,28 +168,16 @@ __device__ __forceinline__ void async_run(float* dst, const float* src, int n, i
     for (int i = sl; i < n; i += GW) async_word(dst + i, src + i);
   }
 }
-// The warp's copies of the tables; those that a stage does not send for stay unused.
+// The warp's copies of the tables; a stage lays out those that it reads.
 struct WarpTables {
   int *bodies, *child_ptr, *child_ids, *parent, *dofadr, *dofnum, *offsets, *dof_body;
 };
-__host__ __device__ inline int table_words(int nbody, int nlevels, int nv) { return 6 * nbody + 1 + nlevels + 1 + nv; }
-__host__ __device__ inline int sweep_words(int nbody, int nlevels) { return 3 * nbody + 1 + nlevels + 1; }
-// behind the worlds of the CTA (32 / GW per warp, `per_world` floats each), a warp's tables after the other's
+// behind the worlds of the CTA (32 / GW per warp, `per_world` floats each), a warp's `words` of tables after the other's
 template <int GW>
 __device__ __forceinline__ int* table_space(float* smem, int per_world, int words) {
   return reinterpret_cast<int*>(smem + (size_t)(blockDim.x >> 5) * (32 / GW) * per_world) + (threadIdx.x >> 5) * words;
 }
-template <int GW>
-__device__ __forceinline__ int* table_space(const ImnBodyTree& T, float* smem, int per_world) {
-  return table_space<GW>(smem, per_world, table_words(T.nbody, T.nlevels, T.nv));
-}
-__device__ __forceinline__ WarpTables warp_tables(const ImnBodyTree& T, int* at) {
-  WarpTables t;
-  t.bodies = at, t.child_ids = t.bodies + T.nbody, t.parent = t.child_ids + T.nbody, t.dofadr = t.parent + T.nbody;
-  t.dofnum = t.dofadr + T.nbody, t.child_ptr = t.dofnum + T.nbody, t.offsets = t.child_ptr + T.nbody + 1;
-  t.dof_body = t.offsets + T.nlevels + 1;
-  return t;
-}
+__host__ __device__ inline int sweep_words(int nbody, int nlevels) { return 3 * nbody + 1 + nlevels + 1; }
 // of the tree alone, without a look at its dofs: what a sweep up reads
 __device__ __forceinline__ WarpTables sweep_tables(const ImnBodyTree& T, int* at) {
   WarpTables t = {};
@@ -286,6 +274,11 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
 // out of it: tree_fusion.py:190-191), then M (tree_fusion.py:192-206): row i of M holds
 // i's ancestors in ascending order with the diagonal last; entry (i, j) is
 // cdof_j . (crb[body_i] cdof_i), the diagonal on top of the armature.
+// One world per warp (GW = 32).
+__host__ __device__ inline bool sweep_in_bufs(int nbody, int nlevels, int nv) { return sweep_words(nbody, nlevels) <= 6 * nv; }
+__host__ __device__ inline int crb_words(int nbody, int nlevels, int nv) {
+  return nv + (sweep_in_bufs(nbody, nlevels, nv) ? 0 : sweep_words(nbody, nlevels));
+}
 template <int GW>
 __global__ void __launch_bounds__(32 * kTreeWarps)
     crb_kernel(const ImnBodyTree T, const float* __restrict__ cinert, const float* __restrict__ cdof,
@@ -299,7 +292,10 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   float* c = tree_smem + (size_t)t.slot * per_world;
   float* dof = c + ((nb10 + 3) & ~3);
   float* bufs = dof + ((nv6 + 3) & ~3);
-  const WarpTables tab = warp_tables(T, table_space<GW>(T, tree_smem, per_world));
+  // the sweep's tables lie where `bufs` of the warp's world will, or behind the worlds where they take more
+  int* const behind = table_space<GW>(tree_smem, per_world, crb_words(T.nbody, T.nlevels, T.nv));
+  WarpTables tab = sweep_tables(T, sweep_in_bufs(T.nbody, T.nlevels, T.nv) ? reinterpret_cast<int*>(bufs) : behind + T.nv);
+  tab.dof_body = behind;
   async_run<GW>(c, cinert + (size_t)w * nb10, nb10, sl);
   async_run<GW>(dof, cdof + (size_t)w * nv6, nv6, sl);
   send_sweep(T, tab);
@@ -336,8 +332,9 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
 }
 
 __host__ __device__ inline int rne_floats(int nbody, int nv) {
-  return 2 * ((nbody * 6 + 3) & ~3) + 2 * ((nv * 6 + 3) & ~3) + ((nbody * 10 + 3) & ~3) + ((nv + 3) & ~3);
+  return 2 * ((nbody * 6 + 3) & ~3) + ((nv * 6 + 3) & ~3) + ((nbody * 10 + 3) & ~3) + ((nv + 3) & ~3);
 }
+__host__ __device__ inline int rne_words(int nbody, int nlevels) { return 4 * nbody + nlevels + 1; }
 // rne without accelerations (tree_fusion.py:209-222): cacc down the tree from
 // -gravity, per-body forces cinert cacc + cvel x* (cinert cvel), summed up the tree,
 // projected on the dofs.
@@ -356,19 +353,22 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   const int nb10 = T.nbody * 10, nb10p = (nb10 + 3) & ~3, per_world = rne_floats(T.nbody, T.nv);
   float* cacc = tree_smem + (size_t)t.slot * per_world;
   float* cfrc = cacc + nb6p;  // cvel until the body's force replaces it
-  float* dd = cfrc + nb6p;    // cdof_dot
-  float* dof = dd + nv6p;
-  float* inert = dof + nv6p;
+  float* dd = cfrc + nb6p;    // cdof_dot, then cdof
+  float* inert = dd + nv6p;
   float* qv = inert + nb10p;
-  const WarpTables tab = warp_tables(T, table_space<GW>(T, tree_smem, per_world));
+  // the walk down's tables; those of the sweep up take their place, the dofs' bodies that of the warp's first qvel
+  WarpTables tab = {};
+  tab.bodies = table_space<GW>(tree_smem, per_world, rne_words(T.nbody, T.nlevels)), tab.offsets = tab.bodies + T.nbody;
+  tab.parent = tab.offsets + T.nlevels + 1, tab.dofadr = tab.parent + T.nbody, tab.dofnum = tab.dofadr + T.nbody;
+  tab.child_ptr = tab.parent, tab.child_ids = tab.child_ptr + T.nbody + 1;
+  tab.dof_body = reinterpret_cast<int*>(qv - (size_t)(t.slot % (32 / GW)) * per_world);
   async_run<GW>(dd, cdof_dot + (size_t)w * nv6, nv6, sl);
   async_run<GW>(qv, qvel + (size_t)w * qvel_ld, T.nv, sl);
   async_run<GW>(inert, cinert + (size_t)w * nb10, nb10, sl);
   async_run<GW>(cfrc, cvel + (size_t)w * nb6, nb6, sl);
-  async_run<GW>(dof, cdof + (size_t)w * nv6, nv6, sl);
-  send_sweep(T, tab);
+  send_words(tab.offsets, T.level_offsets, T.nlevels + 1);
+  send_words(tab.bodies, T.level_bodies, T.nbody);
   send_levels(T, tab);
-  send_words(tab.dof_body, T.dof_bodyid, T.nv);
   if (sl < 6) {
     const float* g = T.gravity + 3 * (size_t)(w % T.n_gravity);
     cacc[sl] = (sl < 3 || !T.gravity_enabled) ? 0.0f : -g[sl - 3];
@@ -388,6 +388,11 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
     }
     __syncwarp();
   }
+  // what comes next arrives during the forces
+  send_words(tab.child_ptr, T.child_ptr, T.nbody + 1);
+  send_words(tab.child_ids, T.child_ids, T.nbody - 1);
+  send_words(tab.dof_body, T.dof_bodyid, T.nv);
+  async_run<GW>(dd, cdof + (size_t)w * nv6, nv6, sl);
   copy_out<GW>(cacc_out + (size_t)w * nb6, cacc, nb6, sl, t.live);
 #pragma unroll 1
   for (int b = sl; b < T.nbody; b += GW) {
@@ -407,18 +412,19 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
     }
     st6(cfrc + 6 * b, r);
   }
-  __syncwarp();
+  async_wait();
   sweep_up<GW, 6>(tab, T.nlevels, cfrc, 6, false, sl);
   __syncwarp();
   copy_out<GW>(cfrc_out + (size_t)w * nb6, cfrc, nb6, sl, t.live);
   float* bias = qfrc_bias + (size_t)w * bias_ld;
 #pragma unroll 1
   for (int i = sl; i < T.nv; i += GW) {
-    const float e = dot6(ld6(dof + 6 * i), ld6(cfrc + 6 * tab.dof_body[i]));
+    const float e = dot6(ld6(dd + 6 * i), ld6(cfrc + 6 * tab.dof_body[i]));
     if (t.live) bias[i] = e;
   }
 }
 
+__host__ __device__ inline int vel_words(int nbody, int nlevels) { return 6 * nbody + nlevels + 1; }
 // Body velocities by depth (velocity_fusion.py:15-103): cvel of a body is its parent's
 // plus cdof qvel of its own dofs; cdof_dot of a dof is cvel x cdof taken before that
 // dof's own contribution (for a free joint: the three translations first, zero
@@ -439,10 +445,12 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
   float* dof = cvel + nb6p;
   float* dot = dof + nv6p;
   float* qv = dot + nv6p;
-  const WarpTables tab = warp_tables(T, table_space<GW>(T, tree_smem, per_world));
-  int* const jntadr = tab.child_ids;  // a walk down reads no children
-  int* const jntnum = tab.child_ptr;
-  int* const kind = tab.dofnum;  // of the body's first joint
+  WarpTables tab = {};
+  tab.bodies = table_space<GW>(tree_smem, per_world, vel_words(T.nbody, T.nlevels)), tab.offsets = tab.bodies + T.nbody;
+  tab.parent = tab.offsets + T.nlevels + 1, tab.dofadr = tab.parent + T.nbody;
+  int* const jntadr = tab.dofadr + T.nbody;
+  int* const jntnum = jntadr + T.nbody;
+  int* const kind = jntnum + T.nbody;  // of the body's first joint
   async_run<GW>(dof, cdof + (size_t)w * nv6, nv6, sl);
   async_run<GW>(qv, qvel + (size_t)w * qvel_ld, T.nv, sl);
   send_words(tab.offsets, T.level_offsets, T.nlevels + 1);
@@ -525,28 +533,33 @@ static int check_tree(const ImnBodyTree* T, const char* who, bool need_dofs) {
 
 // Lanes per world: the tree's team_lanes when it is 8, 16 or 32 (the host mirror sets the
 // smallest that covers the widest level), else a whole warp.
-// Per kernel the width is raised to what was measured fastest on a B200 (65536 worlds,
-// 14-body / 34-dof and 24-body / 56-dof humanoids, widths 8 / 16 / 32 in us, when every level still read its tables
-// from global memory):
-//   tree sum, 3 components   19 / 25 / 41     29 / 39 / 64    -> the tree's width
-//   com_vel                  64 / 70 / 111   132 / 121 / 163  -> the tree's width
-//   rne                      99 / 74 / 113   189 / 139 / 159  -> at least 16
-//   crb                     141 / 101 / 88   473 / 255 / 187  -> 32
+// Per kernel the width is raised to what was measured fastest for full batches on a B200 (65536 worlds, 34-dof
+// humanoid, 56-dof SNU-like, 35-dof G1-like tree, widths 8 / 16 / 32 in us):
+//   tree sum, 3 components   12 / 18 / 32     17 / 25 / 40     33 / 32 / 57    -> the tree's width
+//   com_vel                  45 / 58 / 108    75 / 96 / 152    76 / 86 / 154   -> the tree's width
+//   rne                      53 / 62 / 96    104 / 96 / 128   161 / 135 / 155  -> at least 16
+//   crb                     115 / 85 / 84    365 / 232 / 171  245 / 153 / 133  -> 32
 // A narrow team fills the lanes during the per-body arithmetic but multiplies the shared
 // memory of a CTA (16 worlds instead of 4), which costs resident warps: crb keeps three
 // per-world arrays on chip and its entry loop fills a whole warp anyway.
+//
+// What a warp's worlds and tables take decides how many warps an SM holds.  With tables for every stage in
+// every stage's space, cdof beside cdof_dot and blocks of four warps throughout, us for 8192, 16384 and 65536 worlds:
+// com_vel SNU 16.5, 28.5, 83; crb SNU 30.9, -, 171, G1 20.1, -, 133; rne SNU 18.9, -, 111, G1 22.4, -, 149.
+// Each stage its own tables, those of one phase in the place of another's: crb SNU 25.3, 47, 168, G1 20.1, 38, 132; rne SNU
+// 14.9, 28, 96, G1 18.7, 39, 135; com_vel in blocks of two warps SNU 10.8, 22.8, 75 (of four 16.9, 28.8, 84, of one 10.8,
+// 22.7, 73; G1 11.9 / 12.7 / 12.0 at 8192).  The other stages lose in blocks of two (crb SNU 31.6, 50, 169).
 static int team_lanes(const ImnBodyTree* T, int at_least = 8) {
   const int lanes = (T->team_lanes == 8 || T->team_lanes == 16) ? T->team_lanes : 32;
   return lanes > at_least ? lanes : at_least;
 }
 
 template <typename... Args>
-static int launch_tree(const char* who, void (*kernel)(Args...), int gw, size_t floats_per_world,
+static int launch_tree(const char* who, void (*kernel)(Args...), int warps, int gw, size_t floats_per_world,
                        int table_words, int nworld, void* stream, Args... args) {
   if (nworld < 0) return set_error("%s: negative world count", who), IMN_ERR_SHAPE;
   if (nworld == 0) return IMN_OK;
-  // four warps a block, fewer for trees of hundreds of bodies, whose worlds would not fit
-  int warps = kTreeWarps;
+  // fewer warps a block for trees of hundreds of bodies, whose worlds would not fit
   const size_t warp_bytes = 4 * (floats_per_world * (32 / gw) + table_words);
   while (warps > 1 && warps * warp_bytes > 227 * 1024) warps /= 2;
   const int per_cta = warps * (32 / gw);
@@ -566,10 +579,10 @@ static int launch_tree(const char* who, void (*kernel)(Args...), int gw, size_t 
 static size_t up4z(size_t n) { return (n + 3) & ~(size_t)3; }
 
 // KERNEL<8 | 16 | 32> by the tree's team width
-#define IMN_TEAM_LAUNCH(LANES, KERNEL, FLOATS, TABLES, NWORLD, STREAM, ...)                               \
-  ((LANES) == 8    ? imn::launch_tree(who, KERNEL<8>, 8, FLOATS, TABLES, NWORLD, STREAM, __VA_ARGS__)   \
-   : (LANES) == 16 ? imn::launch_tree(who, KERNEL<16>, 16, FLOATS, TABLES, NWORLD, STREAM, __VA_ARGS__) \
-                   : imn::launch_tree(who, KERNEL<32>, 32, FLOATS, TABLES, NWORLD, STREAM, __VA_ARGS__))
+#define IMN_TEAM_LAUNCH(LANES, KERNEL, WARPS, FLOATS, TABLES, NWORLD, STREAM, ...)                        \
+  ((LANES) == 8    ? imn::launch_tree(who, KERNEL<8>, WARPS, 8, FLOATS, TABLES, NWORLD, STREAM, __VA_ARGS__)   \
+   : (LANES) == 16 ? imn::launch_tree(who, KERNEL<16>, WARPS, 16, FLOATS, TABLES, NWORLD, STREAM, __VA_ARGS__) \
+                   : imn::launch_tree(who, KERNEL<32>, WARPS, 32, FLOATS, TABLES, NWORLD, STREAM, __VA_ARGS__))
 
 }  // namespace imn
 
@@ -588,7 +601,7 @@ extern "C" int imn_body_tree_accumulate(const ImnBodyTree* T, float* values, int
   const int lanes = imn::team_lanes(T), words = imn::sweep_words(T->nbody, T->nlevels);
   const size_t floats = imn::up4z((size_t)T->nbody * components);
   const int staged = 4 * (floats * (32 / lanes) + words) <= 227 * 1024;
-  return IMN_TEAM_LAUNCH(lanes, imn::tree_accumulate_kernel, floats, staged ? words : 0, nworld, stream, *T, values, world_ld,
+  return IMN_TEAM_LAUNCH(lanes, imn::tree_accumulate_kernel, imn::kTreeWarps, floats, staged ? words : 0, nworld, stream, *T, values, world_ld,
                          (int)components, (int)skip_root_parent, staged, (int)nworld);
 }
 
@@ -600,9 +613,9 @@ extern "C" int imn_crb(const ImnBodyTree* T, const float* cinert, const float* c
   if (!cinert || !cdof || !crb || !M || !T->dof_armature || !T->M_rowidx || !T->M_colind)
     return imn::set_error("%s: NULL array", who), IMN_ERR_NULL;
   if (T->n_armature <= 0 || M_ld < T->nM) return imn::set_error("%s: bad armature count or M stride", who), IMN_ERR_SHAPE;
-  return IMN_TEAM_LAUNCH(imn::team_lanes(T, 32), imn::crb_kernel,
+  return imn::launch_tree(who, imn::crb_kernel<32>, imn::kTreeWarps, 32,
                          imn::up4z((size_t)T->nbody * 10) + 2 * imn::up4z((size_t)T->nv * 6),
-                         imn::table_words(T->nbody, T->nlevels, T->nv), nworld, stream, *T, cinert, cdof, crb, M, M_ld, (int)nworld);
+                         imn::crb_words(T->nbody, T->nlevels, T->nv), nworld, stream, *T, cinert, cdof, crb, M, M_ld, (int)nworld);
 }
 
 extern "C" int imn_rne(const ImnBodyTree* T, const float* cinert, const float* cvel, const float* cdof,
@@ -615,8 +628,8 @@ extern "C" int imn_rne(const ImnBodyTree* T, const float* cinert, const float* c
     return imn::set_error("%s: NULL array", who), IMN_ERR_NULL;
   if (T->n_gravity <= 0 || qvel_ld < T->nv || bias_ld < T->nv)
     return imn::set_error("%s: bad gravity count or stride", who), IMN_ERR_SHAPE;
-  return IMN_TEAM_LAUNCH(imn::team_lanes(T, 16), imn::rne_kernel, (size_t)imn::rne_floats(T->nbody, T->nv),
-                         imn::table_words(T->nbody, T->nlevels, T->nv), nworld, stream, *T, cinert, cvel, cdof, cdof_dot, qvel, qvel_ld, cacc, cfrc_int, qfrc_bias, bias_ld,
+  return IMN_TEAM_LAUNCH(imn::team_lanes(T, 16), imn::rne_kernel, imn::kTreeWarps, (size_t)imn::rne_floats(T->nbody, T->nv),
+                         imn::rne_words(T->nbody, T->nlevels), nworld, stream, *T, cinert, cvel, cdof, cdof_dot, qvel, qvel_ld, cacc, cfrc_int, qfrc_bias, bias_ld,
                          (int)nworld);
 }
 
@@ -628,6 +641,6 @@ extern "C" int imn_com_vel(const ImnBodyTree* T, const float* qvel, int64_t qvel
   if (!qvel || !cdof || !cvel || !cdof_dot || !T->body_jntadr || !T->body_jntnum || !T->jnt_type)
     return imn::set_error("%s: NULL array", who), IMN_ERR_NULL;
   if (qvel_ld < T->nv) return imn::set_error("%s: qvel stride < nv", who), IMN_ERR_SHAPE;
-  return IMN_TEAM_LAUNCH(imn::team_lanes(T), imn::com_vel_kernel, imn::up4z((size_t)T->nbody * 6) + 2 * imn::up4z((size_t)T->nv * 6) + imn::up4z(T->nv),
-                         imn::table_words(T->nbody, T->nlevels, T->nv), nworld, stream, *T, qvel, qvel_ld, cdof, cvel, cdof_dot, (int)nworld);
+  return IMN_TEAM_LAUNCH(imn::team_lanes(T), imn::com_vel_kernel, imn::kVelWarps, imn::up4z((size_t)T->nbody * 6) + 2 * imn::up4z((size_t)T->nv * 6) + imn::up4z(T->nv),
+                         imn::vel_words(T->nbody, T->nlevels), nworld, stream, *T, qvel, qvel_ld, cdof, cvel, cdof_dot, (int)nworld);
 }

@@ -357,6 +357,35 @@ def test_cuda_smooth_stages_of_trees_of_hundreds_of_bodies(nv, team):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("fixed", [0, 60])
+def test_cuda_smooth_stages_of_trees_with_few_dofs(fixed):
+    """Three dofs and a chain of bodies without any: the sweep's tables take more than the dofs' products leave."""
+    from instantmimic_b200.mjw_model import make_data, put_model
+
+    parent, body = synthetic.chain_tree(3)
+    m = put_model(parent, body_of_dof=body)
+    nbody = len(m.body_parentid)
+    m.body_parentid = np.concatenate([m.body_parentid, np.arange(nbody - 1, nbody - 1 + fixed)]).astype(np.int32)
+    for name, value in (("body_dofadr", -1), ("body_jntadr", -1), ("body_dofnum", 0), ("body_jntnum", 0)):
+        setattr(m, name, np.concatenate([getattr(m, name), np.full(fixed, value)]).astype(np.int32))
+    m.body_tree = list(m.body_tree) + [np.array([b], np.int32) for b in range(nbody, nbody + fixed)]
+    d = make_data(m, 7, 1)
+    synthetic.add_smooth_state(m, d, seed=3)
+    scratch = tree_fusion.create_tree_reduction_scratch(m, deterministic=True)
+    md, dd = mjw_model.to_device(m, _device()), mjw_model.to_device(d, _device())
+    sd = tree_fusion.create_tree_reduction_scratch(md, deterministic=True)
+    for stage in (velocity_fusion.com_vel, tree_fusion.crb, tree_fusion.rne, tree_fusion.subtree_com_accumulate):
+        stage(md, dd, sd)
+    oracle.com_vel(m, d, scratch)
+    oracle.crb(m, d, scratch)
+    oracle.rne(m, d, scratch)
+    oracle.body_tree_accumulate(m, scratch, d.subtree_com, 3, False)
+    got = mjw_model.to_host(dd)
+    for field in ("cvel", "cdof_dot", "crb", "M", "cacc", "cfrc_int", "qfrc_bias", "subtree_com"):
+        np.testing.assert_array_equal(getattr(got, field), getattr(d, field), err_msg=field)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("bodies,depth", [(14000, 2), (14000, 5000)])
 def test_cuda_accumulate_of_trees_of_thousands_of_bodies(bodies, depth):
     """A warp's world fits a block's shared memory, and so do the tables of the flat tree; those of the deep one stay in
