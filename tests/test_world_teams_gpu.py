@@ -44,3 +44,25 @@ def test_worlds_per_sm(oracle, cuda_device, name, sparse, per_sm):
     for a, b in ((got.qacc, want.qacc), (got.efc.Ma, want.efc.Ma), (got.qfrc_constraint, want.qfrc_constraint),
                  (got.efc.force[live], want.efc.force[live])):
         np.testing.assert_array_equal(np.ascontiguousarray(a).view(np.uint32), np.ascontiguousarray(b).view(np.uint32))
+
+
+def test_worlds_that_leave_the_staged_masks_no_room(oracle, cuda_device):
+    """The largest row limit of the humanoid's plan: a world that fits beside the plan's tables and not beside the masks
+    as well, whose tables stay in global memory."""
+    m, d, _ = synthetic.make_workload("humanoid", 3, seed=3, iterations=6, ls_iterations=6)
+    rows, most = d.njmax, 6840
+    for name, a in vars(d.efc).items():
+        if isinstance(a, np.ndarray) and a.ndim >= 2 and a.shape[1] == rows:
+            setattr(d.efc, name, np.concatenate([a, np.zeros((3, most - rows, *a.shape[2:]), a.dtype)], 1))
+    d.njmax = most
+    md, dd = mjw_model.to_device(m, cuda_device), mjw_model.to_device(copy.deepcopy(d), cuda_device)
+    scratch = runtime.make_optimized_fwd_position_scratch(md, dd, cuda_device)
+    groups = [[b] for b in range(1, len(m.body_dofadr))]
+    assert runtime.refresh_sparse_hessian(md, dd, scratch, groups, cuda_device) == "enabled"
+    plan = sparse_hessian.host_struct(scratch.solver_context.sparse_hessian_plan)
+    runtime.solve_with_scratch(md, dd, scratch, use_optimized_kernel=True)
+    got, want = mjw_model.to_host(dd), copy.deepcopy(d)
+    oracle.solve(m, want, host_ctx(m, want), np.zeros(1, np.int32), sparse_plan_struct=plan)
+    np.testing.assert_array_equal(got.solver_niter, want.solver_niter)
+    for a, b in ((got.qacc, want.qacc), (got.efc.Ma, want.efc.Ma), (got.qfrc_constraint, want.qfrc_constraint)):
+        np.testing.assert_array_equal(np.ascontiguousarray(a).view(np.uint32), np.ascontiguousarray(b).view(np.uint32))
