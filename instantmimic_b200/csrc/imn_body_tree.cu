@@ -143,10 +143,10 @@ __device__ __forceinline__ Team<GW> make_team(int nworld) {
 // every level, qvel inside them, and inputs fetched where they are needed.  A warp now sends for all of
 // its worlds' inputs and for the tables of the tree that the stage reads (four to six words per body, in its own shared
 // memory: no block barrier) with asynchronous copies, waits once, and walks the levels in
-// shared memory.  Five smooth stages in a graph, us: 34 dofs 64 worlds 36.2 -> 27.7, 1000 worlds 40.8 -> 31.0, 8192 worlds
-// 52.3 -> 50.1; 56 dofs 500 worlds 84.3 -> 67.5, 4096 worlds 87.9 -> 73.0; 35 dofs 16384 worlds 148.8 -> 137.9.  (com_vel with a
+// shared memory.  Five smooth stages in a graph, us: 34 dofs 64 worlds 37.0 -> 28.6, 1000 worlds 40.6 -> 31.3, 8192 worlds
+// 52.0 -> 46.5; 56 dofs 500 worlds 83.9 -> 66.9, 4096 worlds 86.9 -> 72.0; 35 dofs 16384 worlds 148.1 -> 133.0.  (com_vel with a
 // lane per world, 32 worlds per block, was ahead of the teams from 4096 worlds on and is not any more: 65536 worlds of 34
-// dofs 53.6 us against 44.9, 56 dofs 97.0 against 83.6, 35 dofs 93.4 against 75.0.)
+// dofs 53.4 us against 45.1, 56 dofs 97.0 against 75.0, 35 dofs 93.2 against 76.4.)
 __device__ __forceinline__ void async_word(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(32 * kTreeWarps)
     }
     __syncwarp();
   }
-  // what comes next arrives during the forces
+  // what comes next arrives during the forces (64 to 512 worlds, where space does not count: 5.5 -> 5.8 us)
   send_words(tab.child_ptr, T.child_ptr, T.nbody + 1);
   send_words(tab.child_ids, T.child_ids, T.nbody - 1);
   send_words(tab.dof_body, T.dof_bodyid, T.nv);

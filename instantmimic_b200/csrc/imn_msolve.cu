@@ -179,7 +179,8 @@ __device__ __forceinline__ void dense_factor_carry(float* A, float* dinv, const 
 #pragma unroll 1
   for (int b0 = 0; b0 < n; b0 += 16) {
     // a last block of up to four rows (33 to 36 dofs) keeps no sums of the twelve it does not have
-    // (4096 34-dof worlds 49.8 -> 47.4 us)
+    // (4096 34-dof worlds 49.8 -> 47.4 us).  The same for up to eight rows is not worth its code: 8192 56-dof worlds 228.0 ->
+    // 226.7, 512 32.8 -> 33.1, and 4096 34-dof worlds 45.8 -> 47.0.
     if (n - b0 <= 4 && nc - b0 <= 32)
       dense_block<1, 4>(A, dinv, b0, n, nc, ldu, l);
     else if (nc - b0 <= 32)
